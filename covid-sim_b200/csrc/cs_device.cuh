@@ -358,7 +358,7 @@ __device__ __forceinline__ double bound_of(const DevPop& d, int b, int B)
 {
     if (d.bounds_static) {
         const int bx = b / d.nby, by = b % d.nby, Bx = B / d.nby, By = B % d.nby;
-        return (double)__ldg(d.bound_c + ((size_t)by * d.nby + By) * d.nbx + (bx > Bx ? bx - Bx : Bx - bx));
+        return (double)__ldg(d.bound_c + ((size_t)by * d.nbx + (bx > Bx ? bx - Bx : Bx - bx)) * d.nby + By);
     }
     return d.block_bound_tab[(size_t)b * d.NB + B];
 }

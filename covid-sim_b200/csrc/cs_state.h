@@ -166,7 +166,7 @@ struct DevPop {
     BlockInfo* block_info;       // [NB], S0 rebuilt with S0
     double* block_row_cum;     // [NB][NB]
     // bound(b, B), which depends on the row of b, the row of B and the distance of
-    // their columns only: [nby][nby][nbx], FP32 rounded up, filled once per geometry
+    // their columns only: [nby (row of b)][nbx (distance)][nby (row of B)], FP32 rounded up, filled once per geometry
     const float* bound_c;
     double* block_bound_tab;   // [NB][NB] bound(b, B) evaluated per UpdateProbs call, when bound_c
                                // could not be filled (a distance beyond the kernel table)

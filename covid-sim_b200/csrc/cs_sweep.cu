@@ -726,25 +726,42 @@ __global__ void k_tot_prob_finish(DevPop d, const float* Ag, const float* Bg)
     }
 }
 
+// The proposal blocks' cell lists: running S0 and guide table, one warp per block.
+// Bound: the gather of the cells' S0 (dependent loads); a warp reads 32 cells at once
+// and scans them, where one thread per block walked its cells one by one (100 of them
+// at 600 x 600 cells: 182 us, now 10).
 __global__ void k_block_S0(DevPop d)
 {
     if (d.gate && !*d.gate) return;
-    for (int B = blockIdx.x * blockDim.x + threadIdx.x; B < d.NB; B += gridDim.x * blockDim.x) {
+    const int lane = threadIdx.x & 31;
+    const int nwarps = (gridDim.x * blockDim.x) >> 5;
+    for (int B = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; B < d.NB; B += nwarps) {
+        const int k0 = d.block_cell_ofs[B], k1 = d.block_cell_ofs[B + 1];
         long long s = 0;
-        int k0 = d.block_cell_ofs[B], k1 = d.block_cell_ofs[B + 1];
-        for (int k = k0; k < k1; k++) {
-            int m = d.block_cells[k], s0 = d.S0[m];
-            s += s0;
-            d.block_cell_info[k] = BlockCell{(int32_t)s, m, d.cell_start[m], s0};
+        for (int kb = k0; kb < k1; kb += 32) {
+            const int k = kb + lane;
+            const int m = k < k1 ? d.block_cells[k] : 0, s0 = k < k1 ? d.S0[m] : 0;
+            long long x = s0;
+            for (int o = 1; o < 32; o <<= 1) {
+                const long long y = __shfl_up_sync(0xffffffffu, x, o);
+                if (lane >= o) x += y;
+            }
+            if (k < k1) d.block_cell_info[k] = BlockCell{(int32_t)(s + x), m, d.cell_start[m], s0};
+            s += __shfl_sync(0xffffffffu, x, 31);
         }
-        d.block_info[B] = BlockInfo{s, k0, k1};
+        if (lane == 0) d.block_info[B] = BlockInfo{s, k0, k1};
+        __syncwarp();
         // cut points of the block's cells: entry k0+q = first cell whose running S0
-        // exceeds q/nc of the block total
-        int nc = k1 - k0, j = k0;
-        for (int q = 0; q < nc; q++) {
-            double thr = (double)q * (double)s / (double)nc;
-            while (j < k1 - 1 && (double)d.block_cell_info[j].cum <= thr) j++;
-            d.cell_guide[k0 + q] = (int16_t)(j - k0);
+        // exceeds q/nc of the block total (the last cell if none)
+        const int nc = k1 - k0;
+        for (int q = lane; q < nc; q += 32) {
+            const double thr = (double)q * (double)s / (double)nc;
+            int lo = k0, hi = k1 - 1;
+            while (lo < hi) {
+                const int mid = (lo + hi) >> 1;
+                if ((double)d.block_cell_info[mid].cum <= thr) lo = mid + 1; else hi = mid;
+            }
+            d.cell_guide[k0 + q] = (int16_t)(lo - k0);
         }
     }
 }
@@ -758,56 +775,159 @@ __global__ void k_block_bounds_all(DevPop d, float* bound_c, unsigned long long*
     const cs_params& P = *d.P;
     const size_t n = (size_t)d.nby * d.nby * d.nbx;
     for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < n; e += (size_t)gridDim.x * blockDim.x) {
-        const int dx = (int)(e % d.nbx), By = (int)((e / d.nbx) % d.nby), by = (int)(e / ((size_t)d.nbx * d.nby));
+        const int By = (int)(e % d.nby), dx = (int)((e / d.nby) % d.nbx), by = (int)(e / ((size_t)d.nbx * d.nby));
         bound_c[e] = __double2float_ru(block_bound_rel(d, P, by, By, dx, oor));
     }
 }
 
 // Row b of the proposal table: running sum over B of S0_B * bound(b, B), added in
 // B order so the doubles round exactly as a sequential loop.
-__global__ void k_block_rows(DevPop d)
+//
+// Bound: the chain of NB dependent additions of a row, which the rounding order fixes.
+// A block owns 32 rows, one per lane of its first warp, which does nothing but add; the
+// other seven warps form the next 32 x 32 weights and store the sums of the last ones,
+// through three buffers.  Loads run one tile ahead of their use.  (One warp
+// per row passed every addition through a shuffle and searched the guide table's entries
+// in the row, 12 dependent loads each: 490 us at NB = 3600, now 98 us and 80 us for
+// k_block_guides.)
+constexpr int kRowsPerBlock = 32;
+__global__ void __launch_bounds__(256) k_block_rows(DevPop d)
 {
     if (d.gate && !*d.gate) return;
     const cs_params& P = *d.P;
-    int lane = threadIdx.x & 31;
-    int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    int nwarps = (gridDim.x * blockDim.x) >> 5;
-    for (int b = warp; b < d.NB; b += nwarps) {
-        double* row = d.block_row_cum + (size_t)b * d.NB;
-        double* btab = d.bounds_static ? nullptr : d.block_bound_tab + (size_t)b * d.NB;
-        double s = 0.0;
-        for (int B0 = 0; B0 < d.NB; B0 += 32) {
-            int B = B0 + lane;
-            double w = 0.0;
-            if (B < d.NB && d.block_info[B].S0 > 0) {
-                double bound;
-                if (d.bounds_static) bound = bound_of(d, b, B);
-                else btab[B] = bound = block_bound(d, P, b, B, CSB_CTR(err_kernel_range));
-                w = (double)d.block_info[B].S0 * bound;
+    constexpr int kMine = (kRowsPerBlock + 6) / 7;   // rows of a weight-forming warp
+    __shared__ double tile[3][32][kRowsPerBlock + 1];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, NB = d.NB, nby = d.nby;
+    const int ntiles = (NB + 31) / 32;
+    for (int b0 = blockIdx.x * kRowsPerBlock; b0 < NB; b0 += gridDim.x * kRowsPerBlock) {
+        // warps 1..7: rows warp-1, warp+6, ... ; their block columns and bound rows
+        int bx[kMine];
+        const float* brow[kMine];
+#pragma unroll
+        for (int q = 0; q < kMine; q++) {
+            const int b = min(b0 + warp - 1 + 7 * q, NB - 1);
+            bx[q] = max(b, 0) / nby;
+            brow[q] = d.bound_c + (size_t)(max(b, 0) % nby) * d.nbx * nby;
+        }
+        int Bx = lane / nby, By = lane % nby;   // this lane's target block of the next tile to read
+        long long S0 = 0;
+        float f[kMine];
+        auto read = [&](int i) {   // issue tile i's loads
+            const int B = i * 32 + lane;
+            S0 = B < NB ? d.block_info[B].S0 : 0;
+            if (d.bounds_static && B < NB) {
+#pragma unroll
+                for (int q = 0; q < kMine; q++) f[q] = __ldg(brow[q] + (size_t)abs(Bx - bx[q]) * nby + By);
             }
-            for (int k = 0; k < 32; k++) {
-                double wk = __shfl_sync(0xffffffffu, w, k);
-                if (B0 + k < d.NB) {
-                    s = s + wk;
-                    if (lane == k) row[B] = s;
+            for (By += 32; By >= nby; By -= nby) Bx++;
+        };
+        auto form = [&](int i) {   // tile i's weights from what read(i) loaded
+            const int B = i * 32 + lane;
+#pragma unroll
+            for (int q = 0; q < kMine; q++) {
+                const int r = warp - 1 + 7 * q, b = b0 + r;
+                if (r >= kRowsPerBlock) break;
+                double w = 0.0;
+                if (S0 > 0 && b < NB) {
+                    double bound = (double)f[q];
+                    if (!d.bounds_static)
+                        d.block_bound_tab[(size_t)b * NB + B] = bound = block_bound(d, P, b, B, CSB_CTR(err_kernel_range));
+                    w = (double)S0 * bound;
+                }
+                tile[i % 3][lane][r] = w;
+            }
+        };
+        auto store = [&](int i) {
+            const int B = i * 32 + lane;
+            if (B >= NB) return;
+#pragma unroll
+            for (int q = 0; q < kMine; q++) {
+                const int r = warp - 1 + 7 * q;
+                if (r < kRowsPerBlock && b0 + r < NB) d.block_row_cum[(size_t)(b0 + r) * NB + B] = tile[i % 3][lane][r];
+            }
+        };
+        if (warp > 0) {
+            read(0);
+            form(0);
+            if (ntiles > 1) read(1);
+        }
+        __syncthreads();
+        double s = 0.0;
+        for (int i = 0; i < ntiles; i++) {
+            if (warp == 0) {
+                double v[32];
+#pragma unroll
+                for (int k = 0; k < 32; k++) v[k] = tile[i % 3][k][lane];
+#pragma unroll
+                for (int k = 0; k < 32; k++) {
+                    s = s + v[k];
+                    tile[i % 3][k][lane] = s;
+                }
+            } else {
+                if (i + 1 < ntiles) form(i + 1);
+                if (i + 2 < ntiles) read(i + 2);
+                if (i > 0) store(i - 1);
+            }
+            __syncthreads();
+        }
+        if (warp > 0) store(ntiles - 1);
+        __syncthreads();   // the buffers are refilled for the next rows
+    }
+}
+
+// guide[k] of row b = first B whose running weight exceeds k/NB of the row total (the
+// last block if none).  B is the answer for the k from n(B-1) to n(B), n(B) the number of
+// thresholds below row[B]; so every B with one marks its first k, and a running maximum
+// over k fills the rest.  n(B) comes from one product, and from the thresholds themselves
+// where that lies too near an integer to tell.  One warp per row; dynamic shared memory
+// holds its NB marks.  Bound: reading the rows once (8 B per entry).
+__global__ void k_block_guides(DevPop d)
+{
+    if (d.gate && !*d.gate) return;
+    extern __shared__ int16_t s_guide[];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, wpb = blockDim.x >> 5, NB = d.NB;
+    int16_t* mark = s_guide + (size_t)warp * NB;
+    for (int b = blockIdx.x * wpb + warp; b < NB; b += gridDim.x * wpb) {
+        const double* row = d.block_row_cum + (size_t)b * NB;
+        const double total = row[NB - 1], per = (double)NB / total;
+        for (int k = lane; k < NB; k += 32) mark[k] = 0;
+        __syncwarp();
+        int before = 0;   // n of the block before this warp's 32
+        double vn = lane < NB ? row[lane] : 0.0, vn2 = lane + 32 < NB ? row[lane + 32] : 0.0;   // read two steps ahead
+        for (int B0 = 0; B0 < NB; B0 += 32) {
+            const int B = B0 + lane;
+            int n = NB;
+            const double v = vn;
+            vn = vn2;
+            if (B + 64 < NB) vn2 = row[B + 64];
+            if (B < NB) {
+                const double x = v * per, f = floor(x);
+                if (x > 1e-6 && x < (double)NB && x - f > 1e-6 && x - f < 1.0 - 1e-6) {
+                    n = (int)f + 1;
+                } else {
+                    n = (x > 0.0) ? (int)fmin(x, (double)NB) : 0;
+                    while (n < NB && (double)n * total / (double)NB < v) n++;
+                    while (n > 0 && !((double)(n - 1) * total / (double)NB < v)) n--;
                 }
             }
+            int p = __shfl_up_sync(0xffffffffu, n, 1);
+            if (lane == 0) p = before;
+            if (B < NB && n > p && p < NB) mark[p] = (int16_t)B;
+            before = __shfl_sync(0xffffffffu, n, 31);
+            if (B0 + 32 >= NB) before = __shfl_sync(0xffffffffu, n, (NB - 1) & 31);
         }
-        // guide[k] = first B whose running weight exceeds k/NB of the row total (the
-        // last block if none): thresholds and the row both ascend, so each lane
-        // finds its entries by binary search
         __syncwarp();
-        int16_t* guide = d.block_guide + (size_t)b * d.NB;
-        const double total = s;
-        for (int k = lane; k < d.NB; k += 32) {
-            double thr = (double)k * total / (double)d.NB;
-            int lo = 0, hi = d.NB - 1;
-            while (lo < hi) {
-                int mid = (lo + hi) >> 1;
-                if (row[mid] <= thr) lo = mid + 1; else hi = mid;
-            }
-            guide[k] = (int16_t)lo;
+        int run = 0;
+        int16_t* guide = d.block_guide + (size_t)b * NB;
+        for (int k0 = 0; k0 < NB; k0 += 32) {
+            const int k = k0 + lane;
+            int g = k < NB ? (k >= before ? NB - 1 : (int)mark[k]) : 0;
+            for (int o = 1; o < 32; o <<= 1) g = max(g, __shfl_up_sync(0xffffffffu, g, o));
+            g = max(g, run);
+            run = __shfl_sync(0xffffffffu, g, 31);
+            if (k < NB) guide[k] = (int16_t)g;
         }
+        __syncwarp();
     }
 }
 
@@ -2746,6 +2866,8 @@ int cs_gpu_set_params(cs_gpu_ctx* c, const cs_params* params)
 static int build_block_bounds(cs_gpu_ctx* c)
 {
     DevPop& d = c->d;
+    if (2 * (size_t)d.NB > (48u << 10))   // k_block_guides' marks
+        CK(cudaFuncSetAttribute(k_block_guides, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 * 32767));
     if (!d.bounds_static) return CS_OK;
     unsigned long long* oor = nullptr;
     CK(cudaMalloc(&oor, sizeof(unsigned long long)));
@@ -2794,11 +2916,13 @@ static int build_kernel_rows(cs_gpu_ctx* c)
     return CS_OK;
 }
 
-// bytes of p to zero (a kernel rather than a memset so that a day graph can gate it)
-__global__ void k_zero_gated(unsigned char* p, size_t bytes, const int32_t* gate)
+// n words of p and m bytes of q to zero (a kernel rather than memsets so that a day
+// graph can gate it)
+__global__ void k_zero_gated(float* p, size_t n, unsigned char* q, size_t m, const int32_t* gate)
 {
     if (gate && !*gate) return;
-    for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < bytes; e += (size_t)gridDim.x * blockDim.x) p[e] = 0;
+    for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < n; e += (size_t)gridDim.x * blockDim.x) p[e] = 0.f;
+    for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < m; e += (size_t)gridDim.x * blockDim.x) q[e] = 0;
 }
 
 // The dynamic shared memory the row kernel needs, raised above the default before
@@ -2828,8 +2952,8 @@ static int tot_prob_pass(cs_gpu_ctx* c, bool denominators)
     const cs_params& P = c->hp;
     size_t G = (size_t)P.ncw * P.nch;
     if (d.gate) {
-        LAUNCH(k_zero_gated, c->grid, kThreads, (unsigned char*)c->S0g, sizeof(float) * G, d.gate);
-        LAUNCH(k_zero_gated, 4, kThreads, c->rowS, (size_t)P.nch, d.gate);
+        LAUNCH(k_zero_gated, (int)std::min<size_t>(c->grid, (G + kThreads - 1) / kThreads), kThreads, c->S0g, G, c->rowS,
+               (size_t)P.nch, d.gate);
     } else {
         CK(cudaMemsetAsync(c->S0g, 0, sizeof(float) * G, c->stream));
         CK(cudaMemsetAsync(c->rowS, 0, P.nch, c->stream));
@@ -2861,11 +2985,22 @@ static int tot_prob_pass(cs_gpu_ctx* c, bool denominators)
     return CS_OK;
 }
 
+// The proposal blocks from the current S0: cell lists, rows, the rows' guide tables
+// (as many warps a block as the marks leave room for in the default shared memory, one
+// at the largest block counts, whose 64 KB are enabled at creation).
+static int guide_warps(int NB) { return std::max(1, std::min(8, (int)((48u << 10) / (2u * (unsigned)NB)))); }
+
 static int rebuild_blocks(cs_gpu_ctx* c)
 {
     DevPop& d = c->d;
-    LAUNCH(k_block_S0, (d.NB + kThreads - 1) / kThreads, kThreads, d);
-    LAUNCH(k_block_rows, (d.NB * 32 + kThreads - 1) / kThreads, kThreads, d);
+    LAUNCH(k_block_S0, (d.NB * 32 + kThreads - 1) / kThreads, kThreads, d);
+    LAUNCH(k_block_rows, (d.NB + kRowsPerBlock - 1) / kRowsPerBlock, kThreads, d);
+    const int wpb = guide_warps(d.NB);
+    if (c->prof) prof_begin(c, "k_block_guides");
+    k_block_guides<<<(d.NB + wpb - 1) / wpb, 32 * wpb, 2 * (size_t)wpb * d.NB, c->stream>>>(d);
+    if (c->prof) prof_end(c);
+    c->launches++;
+    CK(cudaGetLastError());
     return CS_OK;
 }
 
@@ -4267,7 +4402,5 @@ extern "C" int cs_gpu_update_probs_static(cs_gpu_ctx* c, int do_place)
     c->launches++;
     CK(cudaGetLastError());
     LAUNCH(k_tot_prob_finish, cgrid, kThreads, d, Ag, c->Bg);
-    LAUNCH(k_block_S0, (d.NB + kThreads - 1) / kThreads, kThreads, d);
-    LAUNCH(k_block_rows, (d.NB * 32 + kThreads - 1) / kThreads, kThreads, d);
-    return CS_OK;
+    return rebuild_blocks(c);
 }
