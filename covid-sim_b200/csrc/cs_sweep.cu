@@ -224,6 +224,7 @@ struct cs_gpu_ctx {
     int series_cap = 0;
     int day_every_step = -1;    // the probs_every_step the day graph was captured with
     long long geometry_gen = 0; // bumped when set_params replaces the kernel-row table
+    size_t tp_pair_smem = 0;    // dynamic shared memory enabled for k_tot_prob_pairs
     size_t tp_smem[2] = {0, 0}; // dynamic shared memory enabled for k_tot_prob_rows<false>, <true>
     // staging of cs_gpu_place_events / cs_gpu_set_mcell_status
     cs_place_event* d_ev = nullptr;
@@ -514,18 +515,21 @@ __global__ void k_kernel_rows(DevPop d, float* Gtab, unsigned long long* oor)
     }
 }
 
+// Cell values on the grid, row by row (index y * ncw + x), so that the row kernels
+// read a target row contiguously.
 __global__ void k_grid_values(DevPop d, float* S0g, float* Ng, uint8_t* rowS, uint8_t* rowN)
 {
     if (d.gate && !*d.gate) return;
-    int nch = d.P->nch;
+    const int nch = d.P->nch, ncw = d.P->ncw;
     for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < d.NC; c += gridDim.x * blockDim.x) {
-        int g = d.cell_grid[c];
+        const int x = d.cell_grid[c] / nch, y = d.cell_grid[c] % nch;
+        const size_t g = (size_t)y * ncw + x;
         S0g[g] = (float)d.S0[c];
-        if (d.S0[c] > 0) rowS[g % nch] = 1;
+        if (d.S0[c] > 0) rowS[y] = 1;
         if (Ng) {
             int n = d.cell_start[c + 1] - d.cell_start[c];
             Ng[g] = (float)n;
-            if (n > 0) rowN[g % nch] = 1;
+            if (n > 0) rowN[y] = 1;
         }
     }
 }
@@ -633,8 +637,8 @@ __global__ void __launch_bounds__(256) k_tot_prob_rows(DevPop d, const float* S0
                     G[tp_phys(gm.off - k)] = v;
                 }
                 if (r == 0) {
-                    Srow[k] = S0g[(size_t)k * nch + ym];
-                    if (kDenominators) Nrow[k] = Ng[(size_t)k * nch + ym];
+                    Srow[k] = S0g[(size_t)ym * ncw + k];
+                    if (kDenominators) Nrow[k] = Ng[(size_t)ym * ncw + k];
                 }
             }
             __syncthreads();
@@ -688,6 +692,185 @@ __global__ void __launch_bounds__(256) k_tot_prob_rows(DevPop d, const float* S0
         if (xl < ncw) {
             Aout[zofs + (size_t)xl * nch + yl] = A[j];
             if (kDenominators) Bout[zofs + (size_t)xl * nch + yl] = B[j];
+        }
+    }
+}
+
+// The numerators A on the packed FP32 pipe: a thread owns the same eight source
+// columns of TWO neighbouring source rows, and every quantity is a pair over those
+// rows (kernel rows interleaved in shared memory, S0 duplicated), so one fma.rn.f32x2
+// does both rows' term.  Each half rounds as a scalar fused multiply-add and the order
+// of the terms is k_tot_prob_rows' own, so the sums are the same bits.
+//
+// Bound: the FP32 pipe (ncw^2 * nch^2 FMAs).  The scalar kernel spends an issue slot per
+// term plus 31 shared-memory loads per 128 terms and waits twice per target row for its
+// loads; here 128 instructions do 256 terms, a window takes 24 loads (its last seven
+// pairs are the next window's first), and the next target row is copied in (cp.async)
+// while this one is summed.  At 600 x 600 cells 7.2 -> 5.4 ms, 68 % of the pipe's cycles
+// (53 % before); at 240 x 240 cells 350 -> 220 us.  What is left is the pipe's own
+// throttle: three warps a scheduler, in bursts of 128 packed instructions.
+constexpr int kTotPairThreads = 384;
+constexpr size_t kMaxBlockSmem = 227 * 1024;
+struct TotPairGeom {
+    int ncwR, off, gphys;  // as TotProbGeom, in pairs
+    int nchunks, chunks_per_block;
+    int need;              // threads per pair of source rows: ceil(ncw / 8)
+    int npair;             // pairs of source rows per block
+    int threads, xblocks;
+    __host__ __device__ int buf() const { return npair * gphys + ncwR; }   // pairs per buffer
+    size_t smem() const { return 2 * sizeof(float2) * (size_t)buf(); }
+};
+
+static TotPairGeom tot_pair_geom(int ncw, int nch, bool partial)
+{
+    TotPairGeom g;
+    g.ncwR = (ncw + kTotProbSpan - 1) / kTotProbSpan * kTotProbSpan;
+    g.off = g.ncwR + 7;
+    g.gphys = tp_phys(g.off + g.ncwR + kTotProbSpan) + 2;
+    g.gphys += g.gphys & 1;   // keeps S0 after the kernel rows 16-byte aligned (float4 reads)
+    g.nchunks = (nch + kTotProbRowChunk - 1) / kTotProbRowChunk;
+    g.chunks_per_block = partial ? 1 : g.nchunks;
+    g.need = (ncw + kTotProbCols - 1) / kTotProbCols;
+    // Row pairs per block: the count that leaves the fewest lanes idle in a multiple of
+    // 128 threads.  Four warps are the unit because a block's warps go round the SM's four
+    // schedulers: at 600 columns two pairs (150 threads, five warps) gave one scheduler
+    // two warps of every block and the others one, and ran at 53 % of the FP32 pipe.
+    g.npair = 1;
+    g.threads = 256;
+    double best = 0.0;
+    for (int k = 1; k * g.need <= kTotPairThreads && 2 * (k - 1) < nch; k++) {
+        const int t = (k * g.need + 127) / 128 * 128;
+        const double used = (double)(k * g.need) / (double)t;
+        TotPairGeom h = g;
+        h.npair = k;
+        if (used > best + 0.02 && (k == 1 || h.smem() <= kMaxBlockSmem)) {
+            best = used;
+            g.npair = k;
+            g.threads = t;
+        }
+    }
+    g.xblocks = g.npair * g.need <= g.threads ? 1 : (g.need + g.threads - 1) / g.threads;
+    return g;
+}
+
+__global__ void __launch_bounds__(kTotPairThreads, 1) k_tot_prob_pairs(DevPop d, const float* __restrict__ S0g,
+                                                           const uint8_t* __restrict__ rowS, float* __restrict__ Aout,
+                                                           TotPairGeom gm, const float* __restrict__ Gtab)
+{
+    if (d.gate && !*d.gate) return;
+    const cs_params& P = *d.P;
+    const int ncw = P.ncw, nch = P.nch;
+    extern __shared__ __align__(16) float2 sh2[];
+    const int sub = gm.xblocks == 1 ? (int)threadIdx.x / gm.need : 0;
+    const int jcol = gm.xblocks == 1 ? (int)threadIdx.x % gm.need : (int)(blockIdx.x * blockDim.x + threadIdx.x);
+    const int yb = 2 * (int)blockIdx.y * gm.npair;   // the block's first source row
+    const int yl = yb + 2 * sub;
+    const int xl0 = (sub < gm.npair && yl < nch) ? jcol * kTotProbCols : ncw;   // ncw: no outputs
+    const int q0 = blockIdx.z * gm.chunks_per_block;
+    const int q1 = min(q0 + gm.chunks_per_block, gm.nchunks);
+    for (int k = threadIdx.x; k < 2 * gm.buf(); k += blockDim.x) sh2[k] = make_float2(0.f, 0.f);
+    __syncthreads();
+    auto copy4 = [](float* dst, const float* src) {
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" :: "r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
+    };
+    // target row ym into buffer w: the source rows' kernel values, mirrored and
+    // interleaved, and S0 twice; left in flight
+    auto fill = [&](int w, int ym) {
+        float2* base = sh2 + (size_t)w * gm.buf();
+        for (int r = 0; r < gm.npair; r++) {
+            const int y0 = yb + 2 * r, y1 = min(y0 + 1, nch - 1);   // an odd last row pairs with itself
+            if (y0 >= nch) break;
+            float2* G = base + (size_t)r * gm.gphys;
+            if (Gtab) {
+                const float *g0 = Gtab + ((size_t)y0 * nch + ym) * ncw, *g1 = Gtab + ((size_t)y1 * nch + ym) * ncw;
+                for (int k = threadIdx.x; k < ncw; k += blockDim.x) {
+                    float2 *p = G + tp_phys(gm.off + k), *m = G + tp_phys(gm.off - k);
+                    copy4(&p->x, g0 + k);
+                    copy4(&p->y, g1 + k);
+                    copy4(&m->x, g0 + k);
+                    copy4(&m->y, g1 + k);
+                }
+            } else {
+                for (int k = threadIdx.x; k < ncw; k += blockDim.x) {
+                    float2 v;
+                    v.x = (float)row_kernel(d, P, k, y0, ym, CSB_CTR(err_kernel_range));
+                    v.y = y1 > y0 ? (float)row_kernel(d, P, k, y1, ym, CSB_CTR(err_kernel_range)) : v.x;
+                    G[tp_phys(gm.off + k)] = v;
+                    G[tp_phys(gm.off - k)] = v;
+                }
+            }
+        }
+        float2* S = base + (size_t)gm.npair * gm.gphys;
+        for (int k = threadIdx.x; k < ncw; k += blockDim.x) {
+            copy4(&S[k].x, S0g + (size_t)ym * ncw + k);
+            copy4(&S[k].y, S0g + (size_t)ym * ncw + k);
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    const int yend = min(nch, q1 * kTotProbRowChunk);
+    auto next_row = [&](int ym) {   // the first target row at or after ym with susceptibles
+        while (ym < yend && !rowS[ym]) ym++;
+        return ym;
+    };
+    float2 A[kTotProbCols];
+#pragma unroll
+    for (int j = 0; j < kTotProbCols; j++) A[j] = make_float2(0.f, 0.f);
+    const int t0 = 9 * ((gm.off - 7 - xl0) / 8);   // as k_tot_prob_rows, in pairs
+    int w = 0, ym = next_row(q0 * kTotProbRowChunk);
+    if (ym < yend) fill(0, ym);
+    for (int q = q0; q < q1; q++) {
+        float2 a[kTotProbCols];
+#pragma unroll
+        for (int j = 0; j < kTotProbCols; j++) a[j] = make_float2(0.f, 0.f);
+        const int ym1 = min(nch, (q + 1) * kTotProbRowChunk);
+        while (ym < ym1) {
+            asm volatile("cp.async.wait_group 0;" ::: "memory");
+            __syncthreads();   // row ym is in, and every thread is done with the other buffer
+            const int nx = next_row(ym + 1);
+            if (nx < yend) fill(w ^ 1, nx);
+            if (xl0 < ncw) {
+                const float2* Gp = sh2 + (size_t)w * gm.buf() + (size_t)sub * gm.gphys;
+                const float2* Srow = sh2 + (size_t)w * gm.buf() + (size_t)gm.npair * gm.gphys;
+                float2 sa[kTotProbCols];
+#pragma unroll
+                for (int j = 0; j < kTotProbCols; j++) sa[j] = make_float2(0.f, 0.f);
+                // a window's last seven pairs are the next one's first
+                float2 win[kTotProbSpan + kTotProbCols - 1];
+#pragma unroll
+                for (int r = 0; r < kTotProbCols - 1; r++) win[kTotProbSpan + r] = Gp[t0 + r];
+#pragma unroll 2
+                for (int xm0 = 0, t = t0; xm0 < gm.ncwR; xm0 += kTotProbSpan, t += 18) {
+#pragma unroll
+                    for (int r = 0; r < kTotProbCols - 1; r++) win[r] = win[kTotProbSpan + r];
+#pragma unroll
+                    for (int r = kTotProbCols - 1; r < kTotProbSpan + kTotProbCols - 1; r++) win[r] = Gp[t + r + (r >> 3)];
+                    const float4* s4 = reinterpret_cast<const float4*>(Srow + xm0);
+#pragma unroll
+                    for (int u2 = 0; u2 < kTotProbSpan / 2; u2++) {
+                        const float4 sv = s4[u2];
+                        const float2 s0 = make_float2(sv.x, sv.y), s1 = make_float2(sv.z, sv.w);
+#pragma unroll
+                        for (int j = 0; j < kTotProbCols; j++) sa[j] = __ffma2_rn(s0, win[2 * u2 - j + 7], sa[j]);
+#pragma unroll
+                        for (int j = 0; j < kTotProbCols; j++) sa[j] = __ffma2_rn(s1, win[2 * u2 + 1 - j + 7], sa[j]);
+                    }
+                }
+#pragma unroll
+                for (int j = 0; j < kTotProbCols; j++) a[j] = make_float2(a[j].x + sa[j].x, a[j].y + sa[j].y);
+            }
+            w ^= 1;
+            ym = nx;
+        }
+#pragma unroll
+        for (int j = 0; j < kTotProbCols; j++) A[j] = make_float2(A[j].x + a[j].x, A[j].y + a[j].y);
+    }
+    const size_t zofs = (size_t)blockIdx.z * ncw * nch;
+#pragma unroll
+    for (int j = 0; j < kTotProbCols; j++) {
+        const int xl = xl0 + j;
+        if (xl < ncw) {
+            Aout[zofs + (size_t)xl * nch + yl] = A[j].x;
+            if (yl + 1 < nch) Aout[zofs + (size_t)xl * nch + yl + 1] = A[j].y;
         }
     }
 }
@@ -2937,11 +3120,45 @@ static int tot_prob_smem(cs_gpu_ctx* c, bool denominators, size_t smem)
     return CS_OK;
 }
 
+// Numerators on the packed pipe, unless a grid is so wide that its interleaved kernel
+// rows do not fit shared memory twice (about 4,400 columns); k_tot_prob_rows needs a quarter.
+static bool tot_prob_packed(const cs_params& P) { return tot_pair_geom(P.ncw, P.nch, true).smem() <= kMaxBlockSmem; }
+
 static int tot_prob_prepare(cs_gpu_ctx* c)
 {
     const cs_params& P = c->hp;
-    const TotProbGeom gm = tot_prob_geom(P.ncw, P.nch, true);
-    return tot_prob_smem(c, false, gm.smem(false));
+    if (!tot_prob_packed(P)) return tot_prob_smem(c, false, tot_prob_geom(P.ncw, P.nch, true).smem(false));
+    const size_t smem = tot_pair_geom(P.ncw, P.nch, true).smem();
+    if (smem <= 48 * 1024 || smem <= c->tp_pair_smem) return CS_OK;
+    CK(cudaFuncSetAttribute(k_tot_prob_pairs, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    c->tp_pair_smem = smem;
+    return CS_OK;
+}
+
+// Launch the numerators' row kernel: every chunk's partial sums into out (partial), or
+// the final sums.
+static int tot_prob_numerators(cs_gpu_ctx* c, const float* S0g, const uint8_t* rowS, float* out, bool partial)
+{
+    const cs_params& P = c->hp;
+    int r = tot_prob_prepare(c);
+    if (r) return r;
+    if (c->prof) prof_begin(c, partial ? "k_tot_prob_rows" : "k_tot_prob_rows_static");
+    if (tot_prob_packed(P)) {
+        const TotPairGeom gm = tot_pair_geom(P.ncw, P.nch, partial);
+        const dim3 grid(gm.xblocks, (P.nch + 2 * gm.npair - 1) / (2 * gm.npair), gm.nchunks / gm.chunks_per_block);
+        k_tot_prob_pairs<<<grid, gm.threads, gm.smem(), c->stream>>>(c->d, S0g, rowS, out, gm, c->Gtab);
+    } else {
+        const TotProbGeom gm = tot_prob_geom(P.ncw, P.nch, partial);
+        dim3 grid;
+        int tpb;
+        tot_prob_launch_shape(P.ncw, P.nch, gm, &grid, &tpb);
+        k_tot_prob_rows<false><<<grid, tpb, gm.smem(false), c->stream>>>(c->d, S0g, nullptr, rowS, nullptr, out, nullptr,
+                                                                         gm, c->Gtab);
+    }
+    if (c->prof) prof_end(c);
+    c->launches++;
+    CK(cudaGetLastError());
+    return CS_OK;
 }
 
 // One pass of the tot_prob row kernel: A from the current S0 (and, at creation,
@@ -2964,21 +3181,20 @@ static int tot_prob_pass(cs_gpu_ctx* c, bool denominators)
     }
     LAUNCH(k_grid_values, (d.NC + kThreads - 1) / kThreads, kThreads, d, c->S0g, denominators ? c->Ng : nullptr, c->rowS, c->rowN);
     const TotProbGeom gm = tot_prob_geom(P.ncw, P.nch, true);
-    dim3 grid;
-    int tpb;
-    tot_prob_launch_shape(P.ncw, P.nch, gm, &grid, &tpb);
-    const size_t smem = gm.smem(denominators);
-    int r = tot_prob_smem(c, denominators, smem);
-    if (r) return r;
-    if (c->prof) prof_begin(c, "k_tot_prob_rows");
+    int r;
     if (denominators) {
+        dim3 grid;
+        int tpb;
+        tot_prob_launch_shape(P.ncw, P.nch, gm, &grid, &tpb);
+        const size_t smem = gm.smem(true);
+        if ((r = tot_prob_smem(c, true, smem))) return r;
+        if (c->prof) prof_begin(c, "k_tot_prob_rows");
         k_tot_prob_rows<true><<<grid, tpb, smem, c->stream>>>(d, c->S0g, c->Ng, c->rowS, c->rowN, c->Apart, c->Bpart, gm, c->Gtab);
-    } else {
-        k_tot_prob_rows<false><<<grid, tpb, smem, c->stream>>>(d, c->S0g, nullptr, c->rowS, nullptr, c->Apart, nullptr, gm, c->Gtab);
-    }
-    if (c->prof) prof_end(c);
-    c->launches++;
-    CK(cudaGetLastError());
+        if (c->prof) prof_end(c);
+        c->launches++;
+        CK(cudaGetLastError());
+    } else if ((r = tot_prob_numerators(c, c->S0g, c->rowS, c->Apart, true)))
+        return r;
     const int rgrid = (int)((G + kThreads - 1) / kThreads);
     LAUNCH(k_tot_prob_reduce, rgrid, kThreads, c->Apart, gm.nchunks, G, c->Ag, d.gate);
     if (denominators) LAUNCH(k_tot_prob_reduce, rgrid, kThreads, c->Bpart, gm.nchunks, G, c->Bg, d.gate);
@@ -4389,18 +4605,8 @@ extern "C" int cs_gpu_update_probs_static(cs_gpu_ctx* c, int do_place)
     LAUNCH(k_grid_values, cgrid, kThreads, d, S0g, (float*)nullptr, rowS, (uint8_t*)nullptr);
     // All row chunks of a column block run in one block (grid z = 1): the chunked
     // form's per-chunk partial sums would need nchunks x G more floats of scratch.
-    const TotProbGeom gm = tot_prob_geom(P.ncw, P.nch, false);
-    dim3 grid;
-    int tpb;
-    tot_prob_launch_shape(P.ncw, P.nch, gm, &grid, &tpb);
-    const size_t smem = gm.smem(false);
-    int r = tot_prob_smem(c, false, smem);
+    int r = tot_prob_numerators(c, S0g, rowS, Ag, false);
     if (r) return r;
-    if (c->prof) prof_begin(c, "k_tot_prob_rows_static");
-    k_tot_prob_rows<false><<<grid, tpb, smem, c->stream>>>(d, S0g, nullptr, rowS, nullptr, Ag, nullptr, gm, c->Gtab);
-    if (c->prof) prof_end(c);
-    c->launches++;
-    CK(cudaGetLastError());
     LAUNCH(k_tot_prob_finish, cgrid, kThreads, d, Ag, c->Bg);
     return rebuild_blocks(c);
 }
