@@ -177,16 +177,14 @@ def kernel_bytes(name, w, n_cells_steps):
         return 20 * w["work_place_candidates"] + 16 * w["work_infectors"]
     if name == "k_spatial":
         return 33 * w["work_spatial_draws"]
-    if name in ("k_apply_infections", "k_partition_S"):
+    if name in ("k_apply_infections", "k_partition_S", "k_infections"):
         return 12 * w["work_new_infections"]
-    if name == "k_incub_gather":
-        return 16 * w["work_incub_people"] + 16 * n_cells_steps
-    if name == "k_incub_events":
-        return 32 * w["work_transitions"]
-    if name == "k_incub_finish":
-        return 8 * w["work_transitions"]
-    if name == "k_build_active":   # the infectors, once per timestep
-        return 12 * w["work_infectors"] + 16 * n_cells_steps
+    if name == "k_scan":   # the infector list, the transition scan and the cells' counts, one pass
+        return 12 * w["work_infectors"] + 16 * w["work_incub_people"] + 16 * n_cells_steps
+    if name in ("k_onsets", "k_progress"):   # the transitions, counted once for the two
+        return 16 * w["work_transitions"]
+    if name == "k_moves":
+        return 8 * w["work_transitions"] + 12 * w["work_new_infections"]
     return None
 
 

@@ -96,7 +96,8 @@ struct DevStep {
     unsigned long long seed;
 };
 
-// Transition flags per person for one IncubRecoverySweep.
+// Transition flags per person between the transitions and the list moves of one step: set
+// on people who cross two blocks in it, cleared by the move that reads them.
 enum : uint8_t { kStepLtoI = 1, kStepItoRD = 2 };
 
 // Everything the kernels need, passed by value.
@@ -127,7 +128,7 @@ struct DevPop {
     // Each latent or infectious person's next transition time: the least of the
     // times IncubRecoverySweep tests (latent_time; case onset, recovery and the
     // severity times) that is not yet past, 0xFFFF when none is.  The transition
-    // gather reads it alone; k_incub_events re-tests the person's own times.
+    // scan reads it alone; k_onsets and k_progress re-test the person's own times.
     // ev_init, when nonzero, has the next gather form it from those times (set by
     // a state upload or run reset).
     uint16_t* next_ev;
@@ -154,8 +155,8 @@ struct DevPop {
     DevIv* iv;
     DevStep* step;
     const unsigned long long* seed_src;  // the run's seed, written by begin_run / upload_state
-    const double* t_src;                 // when set (batched graphs), k_set_step takes t from here
-    int32_t* step_clock;                 // when set (day graphs), k_set_step takes t = clock * dt and advances it
+    const double* t_src;                 // when set (batched graphs), the step takes t from here
+    int32_t* step_clock;                 // when set (day graphs), the step takes t = clock * dt and k_moves advances it
     const int32_t* gate;                 // when set (day graphs), UpdateProbs kernels run only if *gate
     int32_t* close_window;     // [2] every place closed at ts has [0] <= ts < [1]
     // spatial proposal blocks
@@ -180,9 +181,10 @@ struct DevPop {
     int32_t* counts;           // [kCntN] device-side sizes (see kCnt*)
     int32_t* touched;          // [NC] cells whose lists change this phase
     uint8_t* cell_flag;        // [NC]
-    int32_t* act;              // [N] active people (infectors / latent+infectious)
-    int32_t* act_cell;         // [N]
-    int32_t* cnt;              // [NC] per-cell moves of the current phase (zero between phases)
+    int2* act;                 // [N] the step's infectors (person, cell)
+    int2* events;              // [N] the step's transitions (person, cell): latent people from the front, infectious from the back
+    int32_t* cnt_s;            // [NC] the step's S -> L moves per cell (zero between steps)
+    int32_t* cnt;              // [NC] L -> I (low 16 bits) and I -> R/D (high) moves per cell
     int32_t* cnt_ofs;          // [N] first contact-map entry of each active infector
     int32_t* cmap;             // [2N] active-list index of the infector owning each spatial contact
     int32_t cmap_cap;
@@ -201,12 +203,12 @@ struct DevPop {
     cs_counters* C;
 };
 
-// kCntHH is last: the infect sweep zeroes the counters before it (kCntN - 1 of
+// kCntHH is last: the infect sweep alone zeroes the counters before it (kCntN - 1 of
 // them) and leaves the household list, which its false cases may have filled, to
 // the incub sweep's household pass.  The step's transition events are two lists in
-// act / act_cell: latent people from the front (kCntEvents), infectious people
-// from the back (kCntEventsInf), so that a warp of the transition kernel mostly
-// takes one branch.
+// `events`: latent people from the front (kCntEvents), infectious people from the
+// back (kCntEventsInf), so that a warp of the transition kernel mostly takes one
+// branch.
 enum { kCntQueue = 0, kCntTouched = 1, kCntAct = 2, kCntContacts = 3, kCntPlaceWork = 4, kCntEvents = 5,
        kCntCarer = 6, kCntFalse = 7, kCntEventsInf = 8, kCntHH = 9, kCntN = 10 };
 

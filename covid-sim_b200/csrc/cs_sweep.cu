@@ -7,21 +7,22 @@
 // built on the device, with no host round trip inside a step (so a step can be
 // replayed as a CUDA graph):
 //
-//   InfectSweep
-//     k_build_active         infectious people of every cell, one list
+//     k_set_step             the step's scalars        beside
+//     k_scan                 the infectious people, and the people with a transition this
+//                            step, of every cell: two lists
 //     k_infector_hh_spatial  household pass and spatial Poisson count per infector;
 //                            reserves each infector's entries of the contact map
-//     k_infector_places      place passes, one thread per (infector, place type)
-//     k_spatial              spatial contacts: block proposal + rejection, eight
+//     k_infector_places      place passes, one thread per (infector, place type), beside
+//     k_spatial              spatial contacts: block proposal + rejection, several
 //                            draws of a contact evaluated together
-//     k_apply_infections     DoInfect for every claimed person (lowest key wins)
-//     k_partition_S          S -> L cell-list moves, one warp per touched cell
-//   IncubRecoverySweep
-//     k_incub_gather         the latent and infectious people with an event this step,
-//                            read from the cells' lists
-//     k_incub_events         DoIncub / DoCase / severity / recovery / death per person
-//     k_incub_finish         L -> I and I -> R/D cell-list moves per touched cell, then
-//                            the deferred adult-carer absence and household quarantine
+//     k_infections           DoInfect for every claimed person (lowest key wins), beside
+//     k_onsets               DoIncub, beside
+//     k_progress             DoCase / severity / recovery / death per person
+//     k_moves                S -> L, L -> I and I -> R/D cell-list moves per touched cell,
+//     k_households           beside the deferred adult-carer absence and household
+//                            quarantine
+// The sweeps called one by one (and a timestep with false positives) apply the infections
+// and their moves first (k_apply_infections, k_partition_S) and scan for transitions after.
 //
 // Determinism: all random numbers come from Philox streams keyed by
 // (seed, step, entity, purpose); conflicting infections resolve by atomicMin on a
@@ -135,13 +136,17 @@ __device__ __forceinline__ int2 block_reserve2(int32_t* count_a, int32_t na, int
     return r;
 }
 
-__device__ __forceinline__ void mark_cell(const DevPop& d, int c)
+// Cell flags of a step: its lists change; someone infected this step also turned
+// infectious; someone who turned infectious this step also left the infectious block.
+enum : unsigned { kCellTouched = 1, kCellRelayS = 2, kCellRelayL = 4 };
+
+__device__ __forceinline__ void mark_cell(const DevPop& d, int c, unsigned bits)
 {
     // cell_flag is a byte array; use the containing 32-bit word for the atomic.
     unsigned int* w = (unsigned int*)(d.cell_flag + (c & ~3));
-    unsigned int bit = 1u << ((c & 3) * 8);
-    unsigned int old = atomicOr(w, bit);
-    if (!(old & bit)) d.touched[append(d.counts + kCntTouched)] = c;
+    const unsigned sh = (c & 3) * 8;
+    unsigned int old = atomicOr(w, (bits | kCellTouched) << sh);
+    if (!(old & ((unsigned)kCellTouched << sh))) d.touched[append(d.counts + kCntTouched)] = c;
 }
 
 __device__ __forceinline__ bool flag_household(const DevPop& d, int h, uint8_t f)
@@ -175,6 +180,46 @@ struct StaticStore {
     }
 };
 
+// Streams beside a main one, for the kernels of a timestep that run side by side (branches
+// of the captured graphs).
+struct Branches {
+    static constexpr int kN = 2;
+    cudaStream_t s[kN] = {};
+    cudaEvent_t fork = nullptr, join[kN] = {};
+    cudaError_t create()
+    {
+        cudaError_t e = cudaEventCreateWithFlags(&fork, cudaEventDisableTiming);
+        for (int i = 0; i < kN && e == cudaSuccess; i++) {
+            e = cudaStreamCreateWithFlags(&s[i], cudaStreamNonBlocking);
+            if (e == cudaSuccess) e = cudaEventCreateWithFlags(&join[i], cudaEventDisableTiming);
+        }
+        return e;
+    }
+    void destroy()
+    {
+        for (int i = 0; i < kN; i++) {
+            if (s[i]) { cudaStreamSynchronize(s[i]); cudaStreamDestroy(s[i]); }
+            if (join[i]) cudaEventDestroy(join[i]);
+        }
+        if (fork) cudaEventDestroy(fork);
+    }
+    cudaError_t begin(cudaStream_t main, int n)   // branches 0..n-1 start after main's work so far
+    {
+        cudaError_t e = cudaEventRecord(fork, main);
+        for (int i = 0; i < n && e == cudaSuccess; i++) e = cudaStreamWaitEvent(s[i], fork, 0);
+        return e;
+    }
+    cudaError_t end(cudaStream_t main, int n)     // main goes on after branches 0..n-1
+    {
+        cudaError_t e = cudaSuccess;
+        for (int i = 0; i < n && e == cudaSuccess; i++) {
+            e = cudaEventRecord(join[i], s[i]);
+            if (e == cudaSuccess) e = cudaStreamWaitEvent(main, join[i], 0);
+        }
+        return e;
+    }
+};
+
 struct DayCtl;
 
 struct cs_gpu_ctx {
@@ -186,8 +231,7 @@ struct cs_gpu_ctx {
     void* packed = nullptr;    // device staging of cs_gpu_get_sample_packed
     cudaStream_t own_stream = nullptr;     // the context's stream while a batch lends it another
     cudaStream_t stream = nullptr;
-    cudaStream_t side = nullptr;           // the place pass's branch beside the spatial pass
-    cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
+    Branches br;                           // kernels of a timestep that run side by side
     char err[512] = {0};
     long long launches = 0;
     DevPop d{};
@@ -208,6 +252,7 @@ struct cs_gpu_ctx {
     float *Apart = nullptr, *Bpart = nullptr;   // per row-chunk partial sums
     uint64_t seed = 0;
     bool run_started = false;
+    bool lists_stale = false;   // the last timestep left its touched-cell and household lists for the next scan to empty
     int grid = 148 * 8;
     int spatial_lanes = 8;   // lanes per spatial contact (2, 4, 8 or 16)
     // one timestep captured as a CUDA graph and replayed
@@ -1114,63 +1159,245 @@ __global__ void k_block_guides(DevPop d)
     }
 }
 
-// ======================================================== active-list build
-// The step's active people, cell by cell: infectious, slots [S+L, S+L+I) (mode 0),
-// or latent and infectious, slots [S, S+L+I) (mode 1).  The cells come in tiles of
-// blockDim.x; Q = gridDim.x / tiles blocks share a tile, block q copying its chunks
-// q, q + Q, ... of blockDim.x entries (entry j by the thread whose turn it is), so a
-// cell with thousands of active people costs no more than its share and the launch
-// has the parallelism of the list.  Each chunk reserves its entries at once, so the
-// list's order varies from launch to launch; nothing that reads it depends on the
-// order (random streams are keyed by person and contact, conflicting claims resolve
-// by key, tallies are integer sums, and cell lists are reordered by position).
-__device__ __forceinline__ void k_build_active_body(const DevPop& d, int mode)
+// ============================================================ step scalars
+typedef DevStep StepScalars;
+
+__device__ __forceinline__ double step_time(const DevPop& d, const cs_params& P, double t)
 {
-    __shared__ int s_first[kThreads], s_ofs[kThreads], s_n[kThreads];
-    const int ntiles = (d.NC + blockDim.x - 1) / blockDim.x;
+    if (d.t_src) t = *d.t_src;
+    if (d.step_clock) t = (double)*d.step_clock * P.ModelTimeStep;
+    return t;
+}
+__device__ __forceinline__ int step_number(const cs_params& P, double t) { return (int)(uint16_t)(P.TimeStepsPerDay * t); }
+
+// The step's scalars from the parameters, on the device (src/Sweep.cpp:292-301);
+// empty_lists: also the lists that the timestep before left for this one to empty.
+__device__ __forceinline__ void k_set_step_body(const DevPop& d, double t, unsigned long long seed, int empty_lists)
+{
+    const cs_params& P = *d.P;
+    t = step_time(d, P, t);
+    if (d.seed_src) seed = *d.seed_src;
+    DevStep st;
+    st.t = t;
+    st.ts = step_number(P, t);
+    st.blanket = P.DoBlanketMoveRestr && (t >= P.MoveRestrTimeStart) && (t < P.MoveRestrTimeStart + P.MoveRestrDuration);
+    st.fp = P.ModelTimeStep / (1 - P.FalsePositiveRate);
+    st.seas = P.Seasonality;
+    st.sp_beta = P.DoSpatial ? st.seas * st.fp * P.LocalBeta : 0.0;
+    st.hh_beta = P.DoHouseholds ? st.seas * st.fp * P.HouseholdTrans : 0.0;
+    st.seed = seed;
+    *d.step = st;
+    if (empty_lists) d.counts[kCntTouched] = d.counts[kCntHH] = 0;
+}
+__global__ void k_set_step(DevPop d, double t, unsigned long long seed, int empty_lists) { k_set_step_body(d, t, seed, empty_lists); }
+__global__ void k_set_step_multi(const DevPop* __restrict__ pops, int empty_lists) { k_set_step_body(pops[blockIdx.x], 0.0, 0ull, empty_lists); }
+
+// The gather's test from the person's own times, forming next_ev on the way (the
+// first gather after an upload or reset); kept out of line, off the common path.
+// (The arrays come as pointers: a DevPop passed by reference to an out-of-line
+// function would be copied to every thread's stack.)
+__device__ __noinline__ bool gather_test_from_times(const cs_params* __restrict__ P, const PersonHot* hot,
+                                                    const uint16_t* const* times, uint16_t* next_ev, int p, int ts)
+{
+    const int delay = (int)(P->LatentToSymptDelay / P->ModelTimeStep);
+    const PersonHot h = hot[p];
+    if (h.inf == CS_INF_LATENT) {
+        next_ev[p] = h.latent_time;
+        return h.latent_time == ts;
+    }
+    // times: recovery, SARI, critical, stepdown
+    const int v[5] = {(uint16_t)(h.latent_time + delay), times[0][p], P->DoSeverity ? times[1][p] : 0xFFFF,
+                      P->DoSeverity ? times[2][p] : 0xFFFF, P->DoSeverity ? times[3][p] : 0xFFFF};
+    int best = 0xFFFF;
+    bool ev = false;
+    for (int k = 0; k < 5; k++) {
+        if (k >= 2 && !P->DoSeverity) break;
+        if (v[k] == ts) ev = true;
+        if (v[k] >= ts && v[k] < best) best = v[k];
+    }
+    next_ev[p] = (uint16_t)best;
+    return ev;
+}
+
+// A warp's staging of the (person, cell) pairs it appends to a list: 32 at a time go out
+// with one reservation, so a list costs one atomic per 32 entries whatever the fraction
+// of the warp's people that join it.
+struct WarpAppend {
+    int2* buf;   // 64 entries of shared memory
+    int n;
+};
+template <bool kBack>
+__device__ __forceinline__ void warp_append(WarpAppend& w, bool pred, int2 v, int32_t* count, int2* list, int back)
+{
+    const int lane = threadIdx.x & 31;
+    const unsigned m = __ballot_sync(0xffffffffu, pred);
+    if (!m) return;
+    if (pred) w.buf[w.n + __popc(m & ((1u << lane) - 1u))] = v;
+    w.n += __popc(m);
+    __syncwarp();
+    if (w.n < 32) return;
+    int base = 0;
+    if (lane == 0) base = atomicAdd(count, 32);
+    base = __shfl_sync(0xffffffffu, base, 0);
+    list[kBack ? back - (base + lane) : base + lane] = w.buf[lane];
+    const int2 rest = w.buf[32 + lane];
+    __syncwarp();
+    w.n -= 32;
+    if (lane < w.n) w.buf[lane] = rest;
+    __syncwarp();
+}
+template <bool kBack>
+__device__ __forceinline__ void warp_append_flush(WarpAppend& w, int32_t* count, int2* list, int back)
+{
+    const int lane = threadIdx.x & 31;
+    int base = 0;
+    if (w.n == 0) return;
+    if (lane == 0) base = atomicAdd(count, w.n);
+    base = __shfl_sync(0xffffffffu, base, 0);
+    if (lane < w.n) list[kBack ? back - (base + lane) : base + lane] = w.buf[lane];
+}
+
+// The step's lists from the cells, in one pass: the infectious people (slots
+// [S+L, S+L+I) of each cell, kActive) and the latent and infectious people one of whose
+// transition times is now (slots [S, S+L+I), kEvents; IncubRecoverySweep's scan,
+// src/Sweep.cpp:920-977).  The infections of the step do not move these slots and do not
+// touch these people's times, so the scan for transitions can run ahead of them; a person
+// infected this step whose latent period ends this step is handled with its infection.
+//
+// The cells come in tiles of kThreads; up to Q = gridDim.x / tiles blocks share a tile,
+// block q taking the q-th part of its entries (as many parts as fill a block each), so a
+// cell with thousands of active people costs no more than its share and the launch has the
+// parallelism of the list.  An infector's
+// place in the list is its rank among the part's infectors (known from the cells' counts:
+// one reservation per part); the transitions are rare and go through warp_append, latent
+// people from the front of the list and infectious people from its back.  The lists'
+// order varies from launch to launch; nothing that reads them depends on it (random
+// streams are keyed by person and contact, claims resolve by key, tallies are integer
+// sums, cell lists are reordered by position).
+//
+// Bound: the cells' counts (16 B each), the slots (4 B) and one 2-byte time per latent or
+// infectious person (a 32-byte sector when alone in it).  Two kernels read the same cells
+// and slots before this one did both, 3.9 + 5.2 us with hardly anyone infected and
+// 23 + 47 us at the peak of 10 M people.
+constexpr int kScanUnroll = 4;   // entries of a thread in flight together
+template <bool kActive, bool kEvents>
+__device__ __forceinline__ void k_scan_body(const DevPop& d, double t)
+{
+    constexpr int kWarps = kThreads / 32;
+    __shared__ int s_first[kThreads], s_ofs[kThreads], s_ofsI[kThreads], s_L[kThreads];
+    __shared__ int2 s_warp[kWarps];
+    __shared__ int s_ts, s_base, s_r0, s_r1;
+    __shared__ int2 s_buf[kWarps][2][64];
+    if (threadIdx.x == 0) s_ts = step_number(*d.P, step_time(d, *d.P, t));   // k_set_step runs beside this kernel
+    const bool init = kEvents && *d.ev_init != 0;   // next_ev is formed from the people's own times
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    WarpAppend lat{s_buf[warp][0], 0}, inf{s_buf[warp][1], 0};
+    long long people = 0;
+    const int ntiles = (d.NC + kThreads - 1) / kThreads;
     const int Q = max(1, (int)gridDim.x / ntiles), part = blockIdx.x % Q;
     for (int tile = blockIdx.x / Q; tile < ntiles; tile += max(1, (int)gridDim.x / Q)) {
-        const int c0 = tile * blockDim.x;
+        const int c0 = tile * kThreads;
         const int c = c0 + threadIdx.x;
-        int first = 0, n = 0;
+        int first = 0, nl = 0, ni = 0;
         if (c < d.NC) {
-            first = d.cell_start[c] + d.S[c] + (mode == 0 ? d.L[c] : 0);
-            n = mode == 0 ? d.I[c] : d.L[c] + d.I[c];
+            first = d.cell_start[c] + d.S[c];
+            nl = d.L[c];
+            ni = d.I[c];
+            if (!kEvents) { first += nl; nl = 0; }
         }
-        const int o = block_reserve2(nullptr, n, nullptr, 0).x;   // the block's own prefix of n
-        s_first[threadIdx.x] = first;
-        s_ofs[threadIdx.x] = o;
-        s_n[threadIdx.x] = n;
+        // the tile's prefixes of entries and of infectors
+        int ox = nl + ni, oy = ni;
+        for (int o = 1; o < 32; o <<= 1) {
+            const int yx = __shfl_up_sync(0xffffffffu, ox, o), yy = __shfl_up_sync(0xffffffffu, oy, o);
+            if (lane >= o) { ox += yx; oy += yy; }
+        }
+        if (lane == 31) s_warp[warp] = make_int2(ox, oy);
         __syncthreads();
-        const int total = s_ofs[blockDim.x - 1] + s_n[blockDim.x - 1];
-        for (int j0 = part * blockDim.x; j0 < total; j0 += Q * blockDim.x) {   // block-uniform: every thread reserves
-            const int j = j0 + (int)threadIdx.x;
-            const bool valid = j < total;
-            int p = 0, cell = 0;
-            if (valid) {
-                int lo = 0, hi = blockDim.x - 1;   // the last cell whose entries start at or before j
-                while (lo < hi) {
-                    const int mid = (lo + hi + 1) >> 1;
-                    if (s_ofs[mid] <= j) lo = mid; else hi = mid - 1;
+        int total = 0;
+        ox -= nl + ni;
+        oy -= ni;
+#pragma unroll
+        for (int w = 0; w < kWarps; w++) {
+            const int2 v = s_warp[w];
+            if (w < warp) { ox += v.x; oy += v.y; }
+            total += v.x;
+        }
+        // the tile's entries in as many parts as fill a block, at most Q; this block's is [j0, j1)
+        const int parts = min(Q, (total + kThreads - 1) / kThreads);
+        const int j0 = part < parts ? (int)((long long)total * part / parts) : 0;
+        const int j1 = part < parts ? (int)((long long)total * (part + 1) / parts) : 0;
+        s_first[threadIdx.x] = first;
+        s_ofs[threadIdx.x] = ox;
+        s_ofsI[threadIdx.x] = oy;
+        s_L[threadIdx.x] = nl;
+        if (kActive && j1 > j0) {   // infectors before entries j0 and j1
+            if (ox <= j0 && j0 < ox + nl + ni) s_r0 = oy + max(0, j0 - ox - nl);
+            if (ox < j1 && j1 <= ox + nl + ni) s_r1 = oy + max(0, j1 - ox - nl);
+        }
+        __syncthreads();
+        if (kActive && threadIdx.x == 0 && j1 > j0) s_base = (s_r1 > s_r0 ? atomicAdd(d.counts + kCntAct, s_r1 - s_r0) : 0) - s_r0;
+        const int ts = s_ts;
+        if (kEvents && threadIdx.x == 0 && part == 0) people += total;
+        for (int jb = j0; jb < j1; jb += kScanUnroll * kThreads) {
+            int2 pc[kScanUnroll];
+            int at[kScanUnroll];   // place among the tile's infectors, -1 for a latent person, -2 past the end
+            bool ev[kScanUnroll];
+#pragma unroll
+            for (int u = 0; u < kScanUnroll; u++) {
+                const int j = jb + u * kThreads + (int)threadIdx.x;
+                at[u] = -2;
+                pc[u] = make_int2(0, 0);
+                if (j < j1) {
+                    int lo = 0, hi = kThreads - 1;   // the last cell whose entries start at or before j
+                    while (lo < hi) {
+                        const int mid = (lo + hi + 1) >> 1;
+                        if (s_ofs[mid] <= j) lo = mid; else hi = mid - 1;
+                    }
+                    const int k = j - s_ofs[lo];   // the cell's slots run latent, then infectious
+                    pc[u] = make_int2(d.slots[s_first[lo] + k], c0 + lo);
+                    at[u] = k < s_L[lo] ? -1 : s_ofsI[lo] + k - s_L[lo];
                 }
-                p = d.slots[s_first[lo] + (j - s_ofs[lo])];
-                cell = c0 + lo;
             }
-            const int e = block_reserve2(d.counts + kCntAct, valid ? 1 : 0, nullptr, 0).x;
-            if (valid) {
-                d.act[e] = p;
-                d.act_cell[e] = cell;
+#pragma unroll
+            for (int u = 0; u < kScanUnroll; u++) {
+                ev[u] = false;
+                if (kEvents && at[u] != -2) {
+                    if (init) {
+                        const uint16_t* times[4] = {d.recovery_time, d.sari_time, d.critical_time, d.stepdown_time};
+                        ev[u] = gather_test_from_times(d.P, d.hot, times, d.next_ev, pc[u].x, ts);
+                    } else {
+                        ev[u] = d.next_ev[pc[u].x] == ts;
+                    }
+                }
+            }
+            if (kActive) {
+                if (jb == j0) __syncthreads();   // s_base
+#pragma unroll
+                for (int u = 0; u < kScanUnroll; u++)
+                    if (at[u] >= 0) d.act[s_base + at[u]] = pc[u];
+            }
+            if (kEvents) {
+#pragma unroll
+                for (int u = 0; u < kScanUnroll; u++) {
+                    warp_append<false>(lat, ev[u] && at[u] == -1, pc[u], d.counts + kCntEvents, d.events, 0);
+                    warp_append<true>(inf, ev[u] && at[u] >= 0, pc[u], d.counts + kCntEventsInf, d.events, d.N - 1);
+                }
             }
         }
         __syncthreads();   // the shared arrays are refilled for the next cells
     }
+    if (kEvents) {
+        warp_append_flush<false>(lat, d.counts + kCntEvents, d.events, 0);
+        warp_append_flush<true>(inf, d.counts + kCntEventsInf, d.events, d.N - 1);
+        if (threadIdx.x == 0 && people) cnt_add(CSB_CTR(work_incub_people), people);
+    }
 }
-__global__ void k_build_active(DevPop d, int mode) { k_build_active_body(d, mode); }
-__global__ void k_build_active_multi(const DevPop* __restrict__ pops, int mode) { k_build_active_body(pops[blockIdx.y], mode); }
+template <bool kActive, bool kEvents>
+__global__ void __launch_bounds__(kThreads) k_scan(DevPop d, double t) { k_scan_body<kActive, kEvents>(d, t); }
+template <bool kActive, bool kEvents>
+__global__ void __launch_bounds__(kThreads) k_scan_multi(const DevPop* __restrict__ pops) { k_scan_body<kActive, kEvents>(pops[blockIdx.y], 0.0); }
 
 // =============================================================== InfectSweep
-typedef DevStep StepScalars;
-
 // AddInfections (src/Sweep.cpp:2031-2065): with probability FalsePositiveRate the
 // entry is a false positive (DoFalseCase for the person) instead of an infection.
 // The draw is keyed by (infector, infectee, infection type), one per entry.
@@ -1190,31 +1417,6 @@ __device__ __forceinline__ void claim_infection(const DevPop& d, const cs_params
     unsigned long long old = atomicMin(d.claim + person, key);
     if (old == ~0ull) d.queue[append(d.counts + kCntQueue)] = person;
 }
-
-// The step's scalars from the parameters, on the device (src/Sweep.cpp:292-301).
-__device__ __forceinline__ void k_set_step_body(const DevPop& d, double t, unsigned long long seed)
-{
-    const cs_params& P = *d.P;
-    if (d.t_src) t = *d.t_src;
-    if (d.step_clock) {
-        int k = *d.step_clock;
-        t = (double)k * P.ModelTimeStep;
-        *d.step_clock = k + 1;
-    }
-    if (d.seed_src) seed = *d.seed_src;
-    DevStep st;
-    st.t = t;
-    st.ts = (int)(uint16_t)(P.TimeStepsPerDay * t);
-    st.blanket = P.DoBlanketMoveRestr && (t >= P.MoveRestrTimeStart) && (t < P.MoveRestrTimeStart + P.MoveRestrDuration);
-    st.fp = P.ModelTimeStep / (1 - P.FalsePositiveRate);
-    st.seas = P.Seasonality;
-    st.sp_beta = P.DoSpatial ? st.seas * st.fp * P.LocalBeta : 0.0;
-    st.hh_beta = P.DoHouseholds ? st.seas * st.fp * P.HouseholdTrans : 0.0;
-    st.seed = seed;
-    *d.step = st;
-}
-__global__ void k_set_step(DevPop d, double t, unsigned long long seed) { k_set_step_body(d, t, seed); }
-__global__ void k_set_step_multi(const DevPop* __restrict__ pops, double t, unsigned long long seed) { k_set_step_body(pops[blockIdx.y], t, seed); }
 
 // Geometric-skip enumeration of the Bernoulli(p) trials over a member list
 // (equivalent to the reference's Binomial count + sample without replacement,
@@ -1281,7 +1483,8 @@ __device__ __forceinline__ void k_infector_hh_spatial_body(const DevPop& d)
         uint8_t closed_i = 0;
         bool absent_i = true;
         if (idx < nact) {
-            int i = d.act[idx], ci = d.act_cell[idx];
+            const int2 ac = d.act[idx];
+            const int i = ac.x, ci = ac.y;
             PersonHot hi = d.hot[i];
             int h = hi.hh;
             int iag = age_group(hi);
@@ -1355,7 +1558,7 @@ __device__ __forceinline__ void k_infector_places_body(const DevPop& d)
     for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
         int2 e = d.place_work[t];
         int idx = e.x >> 3, pt = e.x & 7, link = e.y;
-        int i = d.act[idx];
+        int i = d.act[idx].x;
         PersonHot hi = d.hot[i];
         double PI = st.fp * st.seas * calc_place_inf(hi, P, pt, st.ts);
         if (st.blanket) {
@@ -1437,7 +1640,8 @@ __device__ __forceinline__ void k_spatial_body(const DevPop& d)
     for (int cidx = group; cidx < ncont; cidx += ngroups) {
         int idx = d.cmap[cidx];            // the infector owning contact cidx
         int j = cidx - d.cnt_ofs[idx];
-        int i = d.act[idx], ci = d.act_cell[idx];
+        const int2 ac = d.act[idx];
+        const int i = ac.x, ci = ac.y;
         bool closed_i = d.act_closed[idx] != 0;
         PersonHot hinf = d.hot[i];
         int b = d.cell_block[ci];
@@ -1503,81 +1707,100 @@ __global__ void __launch_bounds__(kThreads, 3) k_spatial(DevPop d) { k_spatial_b
 template <int kSpatialLanes>
 __global__ void __launch_bounds__(kThreads, 3) k_spatial_multi(const DevPop* __restrict__ pops) { k_spatial_body<kSpatialLanes>(pops[blockIdx.y]); }
 
-// DoInfect (src/Update.cpp:100-195) for every person claimed this step.
+// Tallies of DoInfect that every infection adds to, summed per thread and added once per
+// warp: one atomic per thread on a single address would serialise the launch.
+struct InfectTally {
+    long long n = 0, kw = 0, n_tg = 0, tg = 0, si = 0, rad_q = 0, rad_max = 0;
+};
+__device__ __forceinline__ void infect_tally_add(const DevPop& d, const InfectTally& q)
+{
+    cnt_add_warp(CSB_CTR(cumI), q.n);
+    cnt_add_warp(CSB_CTR(cumI_keyworker[1]), q.kw);
+    cnt_add_warp(CSB_CTR(cumI_keyworker[0]), q.n - q.kw);
+    cnt_add_warp(CSB_CTR(cumTG), q.tg);
+    cnt_add_warp(CSB_CTR(cumSI), q.si);
+    cnt_add_warp(CSB_CTR(nTG), q.n_tg);
+    cnt_add_warp(CSB_CTR(sumRad2_q), q.rad_q);
+    long long m = q.rad_max;
+    for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
+    if ((threadIdx.x & 31) == 0 && m > 0) atomicMax((long long*)CSB_CTR(maxRad2_bits), m);
+}
+
+// DoInfect (src/Update.cpp:100-195) for claimed person p, on a register copy of the
+// record that the caller writes back; returns the person's cell.
+__device__ __forceinline__ int do_infect(const DevPop& d, const cs_params& P, int p, PersonHot& h, double t, int ts,
+                                         uint64_t seed, double ox, double oy, InfectTally& q)
+{
+    const unsigned long long key = d.claim[p];
+    d.claim[p] = ~0ull;
+    const int32_t infector = (int32_t)(uint32_t)(key >> 8);
+    const int code = (int)(key & 0xff);
+    const int16_t it = (infector >= 0)
+        ? (int16_t)(code + CS_INFECT_TYPE_MASK * (1 + d.infect_type[infector] / CS_INFECT_TYPE_MASK))
+        : (int16_t)code;
+    h = d.hot[p];
+    h.inf = CS_INF_LATENT;
+    d.infection_time[p] = (uint16_t)ts;
+    d.infector[p] = infector;
+    d.infect_type[p] = it;
+    const int cell = d.mcell_cell[h.mcell];
+    atomicSub(d.S + cell, 1);
+    atomicAdd(d.L + cell, 1);
+    d.mark[d.cell_start[cell] + d.listpos[p]] = 1;
+    atomicAdd(d.cnt_s + cell, 1);   // moves out of this cell's S block
+    q.n++;
+    if (infector != -2) {   // a seed's radius is 0 (the origin moved to it)
+        const HouseholdRec hr = load_household(d, h.hh);
+        const double x = (double)hr.x - ox, y = (double)hr.y - oy;
+        const double r2 = x * x + y * y;
+        q.rad_q += (long long)(r2 * 4294967296.0);
+        q.rad_max = max(q.rad_max, __double_as_longlong(r2));
+    }
+    cnt_add(CSB_STAGED(cumItype[it % CS_INFECT_TYPE_MASK]), 1);
+    cnt_add(CSB_STAGED(cumIa[age_group(h)]), 1);
+    if (h.pflags & CS_PF_KEYWORKER) q.kw++;
+    const int ad = d.mcell_adunit[h.mcell];
+    if (ad >= 0 && ad < CS_MAX_ADUNITS) cnt_add(CSB_STAGED(cumI_adunit[ad]), 1);
+    if (P.DoLatent) {
+        Stream s(seed, CS_RNG_LATENT, (uint32_t)ts, (uint32_t)p, 0);
+        double qq;
+        int i = (int)floor((qq = s.next() * CS_CDF_RES));
+        qq -= (double)i;
+        h.latent_time = (uint16_t)floor(0.5 + (t - P.LatentPeriod * log(qq * P.latent_icdf.v[i + 1] + (1.0 - qq) * P.latent_icdf.v[i])) * P.TimeStepsPerDay);
+    } else
+        h.latent_time = (uint16_t)(t * P.TimeStepsPerDay);
+    if (infector >= 0) {
+        q.tg += ((int)(uint16_t)ts) - ((int)d.infection_time[infector]);
+        q.si += ((int)h.latent_time) - ((int)d.hot[infector].latent_time);
+        q.n_tg++;
+    }
+    return cell;
+}
+
+// DoInfect for every claimed person, alone (seeding, and the sweeps called one by one;
+// a whole timestep's infections go through k_infections).
 __device__ __forceinline__ void k_apply_infections_body(const DevPop& d)
 {
     const cs_params& P = *d.P;
     const double t = d.step->t;
     const int ts = d.step->ts;
     const uint64_t seed = d.step->seed;
-    int nq = d.counts[kCntQueue];
+    const int nq = d.counts[kCntQueue];
     if (blockIdx.x * blockDim.x >= nq) return;   // a block without work stages nothing
     const bool staged = nq >= kStageMinItems;
     stage_begin(d.C, staged);
-    // single-address tallies, summed per thread and added once per warp
-    long long n_inf = 0, n_kw = 0, n_tg = 0, sum_tg = 0, sum_si = 0, rad_q = 0, rad_max = 0;
+    InfectTally tally;
     const double ox = d.rad_origin[0], oy = d.rad_origin[1];
     for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < nq; q += gridDim.x * blockDim.x) {
-        int p = d.queue[q];
-        unsigned long long key = d.claim[p];
-        d.claim[p] = ~0ull;
-        int32_t infector = (int32_t)(uint32_t)(key >> 8);
-        int code = (int)(key & 0xff);
-        int16_t it = (infector >= 0)
-            ? (int16_t)(code + CS_INFECT_TYPE_MASK * (1 + d.infect_type[infector] / CS_INFECT_TYPE_MASK))
-            : (int16_t)code;
-        PersonHot h = d.hot[p];
-        h.inf = CS_INF_LATENT;
-        d.infection_time[p] = (uint16_t)ts;
-        d.infector[p] = infector;
-        d.infect_type[p] = it;
-        int cell = d.mcell_cell[h.mcell];
-        atomicSub(d.S + cell, 1);
-        atomicAdd(d.L + cell, 1);
-        d.mark[d.cell_start[cell] + d.listpos[p]] = 1;
-        atomicAdd(d.cnt + cell, 1);  // transitions out of this cell's S block
-        mark_cell(d, cell);
-        n_inf++;
-        if (infector != -2) {   // a seed's radius is 0 (the origin moved to it)
-            const HouseholdRec hr = load_household(d, h.hh);
-            const double x = (double)hr.x - ox, y = (double)hr.y - oy;
-            const double r2 = x * x + y * y;
-            rad_q += (long long)(r2 * 4294967296.0);
-            rad_max = max(rad_max, __double_as_longlong(r2));
-        }
-        cnt_add(CSB_STAGED(cumItype[it % CS_INFECT_TYPE_MASK]), 1);
-        cnt_add(CSB_STAGED(cumIa[age_group(h)]), 1);
-        if (h.pflags & CS_PF_KEYWORKER) n_kw++;
-        int ad = d.mcell_adunit[h.mcell];
-        if (ad >= 0 && ad < CS_MAX_ADUNITS) cnt_add(CSB_STAGED(cumI_adunit[ad]), 1);
-        if (P.DoLatent) {
-            Stream s(seed, CS_RNG_LATENT, (uint32_t)ts, (uint32_t)p, 0);
-            double qq;
-            int i = (int)floor((qq = s.next() * CS_CDF_RES));
-            qq -= (double)i;
-            h.latent_time = (uint16_t)floor(0.5 + (t - P.LatentPeriod * log(qq * P.latent_icdf.v[i + 1] + (1.0 - qq) * P.latent_icdf.v[i])) * P.TimeStepsPerDay);
-        } else
-            h.latent_time = (uint16_t)(t * P.TimeStepsPerDay);
+        const int p = d.queue[q];
+        PersonHot h;
+        const int cell = do_infect(d, P, p, h, t, ts, seed, ox, oy, tally);
+        mark_cell(d, cell, kCellTouched);
         d.hot[p] = h;
         d.next_ev[p] = h.latent_time;
-        if (infector >= 0) {
-            sum_tg += ((int)(uint16_t)ts) - ((int)d.infection_time[infector]);
-            sum_si += ((int)h.latent_time) - ((int)d.hot[infector].latent_time);
-            n_tg++;
-        }
     }
-    cnt_add_warp(CSB_CTR(cumI), n_inf);
-    cnt_add_warp(CSB_CTR(cumI_keyworker[1]), n_kw);
-    cnt_add_warp(CSB_CTR(cumI_keyworker[0]), n_inf - n_kw);
-    cnt_add_warp(CSB_CTR(cumTG), sum_tg);
-    cnt_add_warp(CSB_CTR(cumSI), sum_si);
-    cnt_add_warp(CSB_CTR(nTG), n_tg);
-    cnt_add_warp(CSB_CTR(sumRad2_q), rad_q);
-    {
-        long long m = rad_max;
-        for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
-        if ((threadIdx.x & 31) == 0 && m > 0) atomicMax((long long*)CSB_CTR(maxRad2_bits), m);
-    }
+    __syncwarp();
+    infect_tally_add(d, tally);
     if (blockIdx.x == 0 && threadIdx.x == 0) cnt_add(CSB_STAGED(work_new_infections), nq);
     stage_flush(d.C, staged);
 }
@@ -1585,66 +1808,136 @@ __global__ void k_apply_infections(DevPop d) { k_apply_infections_body(d); }
 __global__ void k_apply_infections_multi(const DevPop* __restrict__ pops) { k_apply_infections_body(pops[blockIdx.y]); }
 
 // Swap-with-block-end removal of marked slots, high to low (src/Update.cpp:1402-1579
-// UpdateCell sequence).  Moved people get their new listpos.  One warp per block:
-// the warp reads the marks 32 positions at a time from the top and lane 0 applies
-// the swaps in descending position order, as a serial scan would.  A swap writes
-// only at its own position and above, so the marks the warp read for the positions
-// still below are the ones a serial scan would find there.
-__device__ void partition_block_warp(const DevPop& d, int base, int b0, int n, int nmarked, uint8_t want,
-                                     bool relay_exit)
+// UpdateCell sequence).  Moved people get their new listpos.  One warp per block of a
+// cell's list ([b0, b0 + n), cell start `base`).
+//
+// The reference swaps one person at a time: with the marked positions p_0 > p_1 > ... and
+// the block shrinking by one each time, p_j trades places with the block's current last
+// slot.  Each swap waits for two scattered loads when done in memory; here the warp takes
+// up to 32 marks at once, loads the people at the marks and in the tail that the block
+// gives up (two loads in flight for all of them), lets lane 0 play the swaps in shared
+// memory, and writes the outcome back.  A swap touches only its mark and the tail, and no
+// unprocessed mark lies in the tail of a full batch, so batches follow one another as the
+// single swaps would.  `relay`: people whose pstep holds that flag leave the next block
+// too in this step; their new slot gets `relay_mark`.
+struct MoveScratch {
+    int pos[32], head[32], tail[32];
+};
+
+__device__ __forceinline__ void partition_block_warp(const DevPop& d, MoveScratch& w, int base, int b0, int n, int nmarked,
+                                                     uint8_t want, uint8_t relay, uint8_t relay_mark)
 {
+    constexpr int kAhead = 4;   // mark loads in flight per lane
     const int lane = threadIdx.x & 31;
-    int cur = n, removed = 0;
-    for (int top = b0 + n - 1; top >= b0 && removed < nmarked; top -= 32) {
-        const int pos = top - lane;
-        unsigned hits = __ballot_sync(0xffffffffu, pos >= b0 && d.mark[pos] == want);
-        if (lane == 0) {
-            while (hits && removed < nmarked) {
-                const int p = top - (__ffs(hits) - 1);   // lowest lane: highest position
-                hits &= hits - 1;
-                cur--;
-                removed++;
-                const int end = b0 + cur;
-                if (p < end) {
-                    int a = d.slots[p], e = d.slots[end];
-                    d.slots[p] = e;
-                    d.listpos[e] = p - base;
-                    d.slots[end] = a;
-                    d.listpos[a] = end - base;
+    int cur = n, left = nmarked, have = 0;
+    for (int top = b0 + n - 1; top >= b0 && left > 0; top -= 32 * kAhead) {
+        uint8_t mk[kAhead];
+#pragma unroll
+        for (int u = 0; u < kAhead; u++) {
+            const int pos = top - 32 * u - lane;
+            mk[u] = pos >= b0 ? d.mark[pos] : 0;
+        }
+#pragma unroll
+        for (int u = 0; u < kAhead; u++) {
+            unsigned hits = __ballot_sync(0xffffffffu, mk[u] == want);
+            while (hits && left > 0) {   // warp-uniform: the marks come high to low, lowest lane first
+                const int take = min(min(__popc(hits), 32 - have), left);
+                const bool mine = (hits >> lane & 1u) && __popc(hits & ((1u << lane) - 1u)) < take;
+                if (mine) w.pos[have + __popc(hits & ((1u << lane) - 1u))] = top - 32 * u - lane;
+                for (int q = 0; q < take; q++) hits &= hits - 1;
+                have += take;
+                left -= take;
+                if (have < 32 && left > 0) continue;
+                // ---- one batch: `have` marks
+                __syncwarp();
+                const int k = have, T = b0 + cur - k;
+                const int p = lane < k ? w.pos[lane] : 0;
+                if (lane < k) {
+                    w.head[lane] = d.slots[p];
+                    w.tail[lane] = d.slots[T + lane];
                 }
-                d.mark[p] = 0;
-                d.mark[end] = 0;
-                if (relay_exit) {
-                    int a = d.slots[end];
-                    if (d.pstep[a] & kStepItoRD) d.mark[end] = 2;
+                __syncwarp();
+                if (lane == 0)
+                    for (int j = 0; j < k; j++) {
+                        const int e = k - 1 - j, pj = w.pos[j];
+                        if (pj == T + e) continue;
+                        int* at = pj >= T ? &w.tail[pj - T] : &w.head[j];
+                        const int x = *at;
+                        *at = w.tail[e];
+                        w.tail[e] = x;
+                    }
+                __syncwarp();
+                if (lane < k) {
+                    const int a = w.tail[lane];
+                    d.slots[T + lane] = a;
+                    d.listpos[a] = T + lane - base;
+                    if (p < T) {
+                        const int e = w.head[lane];
+                        d.slots[p] = e;
+                        d.listpos[e] = p - base;
+                        d.mark[p] = 0;
+                    }
+                    uint8_t m = 0;
+                    if (relay && (d.pstep[a] & relay)) {
+                        m = relay_mark;
+                        d.pstep[a] = (uint8_t)(d.pstep[a] & ~relay);
+                    }
+                    d.mark[T + lane] = m;
                 }
+                __syncwarp();
+                cur -= k;
+                have = 0;
             }
         }
-        removed = __shfl_sync(0xffffffffu, removed, 0);
-        __syncwarp();
     }
 }
 
-// S -> L list moves for every cell that gained latent people this step, one warp
-// per cell.
+// One touched cell's list moves: S -> L (kS), L -> I and I -> R/D, in that order, each
+// block's new people at the front of the next one.
+template <bool kS, bool kLI>
+__device__ __forceinline__ int partition_cell(const DevPop& d, MoveScratch& w, int c)
+{
+    const int base = d.cell_start[c], S = d.S[c];
+    const int nS = kS ? d.cnt_s[c] : 0;
+    const int v = kLI ? d.cnt[c] : 0;
+    const int L = d.L[c], I = d.I[c];
+    const unsigned f = d.cell_flag[c];
+    const int nLI = v & 0xffff, nIR = (v >> 16) & 0xffff;
+    if (kS && nS)
+        partition_block_warp(d, w, base, base, S + nS, nS, 1, kLI && (f & kCellRelayS) ? kStepLtoI : 0, 1);
+    if (kLI && nLI) partition_block_warp(d, w, base, base + S, L + nLI, nLI, 1, f & kCellRelayL ? kStepItoRD : 0, 2);
+    if (kLI && nIR) partition_block_warp(d, w, base, base + S + L, I + nIR, nIR, 2, 0, 0);
+    __syncwarp();
+    if ((threadIdx.x & 31) == 0) {
+        if (kS && nS) d.cnt_s[c] = 0;
+        if (kLI) d.cnt[c] = 0;
+        d.cell_flag[c] = 0;
+    }
+    return nS > 0 ? 1 : 0;
+}
+
+// The touched cells' moves, one warp per cell, the cells dealt to blocks first so that a
+// short list spreads over the SMs; returns the cells with S -> L moves (lane 0's count).
+template <bool kS, bool kLI>
+__device__ __forceinline__ int partition_touched(const DevPop& d)
+{
+    __shared__ MoveScratch s_move[kThreads / 32];
+    const int nt = d.counts[kCntTouched], warp = threadIdx.x >> 5;
+    int n = 0;
+    for (int k = blockIdx.x + gridDim.x * warp; k < nt; k += gridDim.x * (blockDim.x >> 5))
+        n += partition_cell<kS, kLI>(d, s_move[warp], d.touched[k]);
+    return n;
+}
+
+// S -> L list moves for every cell that gained latent people, alone (with
+// k_apply_infections).
 __device__ __forceinline__ void k_partition_S_body(const DevPop& d)
 {
-    int nt = d.counts[kCntTouched];
-    if (blockIdx.x == 0 && threadIdx.x == 0) cnt_add(CSB_CTR(work_cells_touched), nt);
-    const int warps = (gridDim.x * blockDim.x) >> 5;
-    for (int k = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; k < nt; k += warps) {
-        int c = d.touched[k];
-        int moved = d.cnt[c];
-        int base = d.cell_start[c];
-        partition_block_warp(d, base, base, d.S[c] + moved, moved, 1, false);
-        if ((threadIdx.x & 31) == 0) {
-            d.cnt[c] = 0;
-            d.cell_flag[c] = 0;
-        }
-    }
+    if (blockIdx.x == 0 && threadIdx.x == 0) cnt_add(CSB_CTR(work_cells_touched), d.counts[kCntTouched]);
+    partition_touched<true, false>(d);
 }
-__global__ void k_partition_S(DevPop d) { k_partition_S_body(d); }
-__global__ void k_partition_S_multi(const DevPop* __restrict__ pops) { k_partition_S_body(pops[blockIdx.y]); }
+__global__ void __launch_bounds__(kThreads) k_partition_S(DevPop d) { k_partition_S_body(d); }
+__global__ void __launch_bounds__(kThreads) k_partition_S_multi(const DevPop* __restrict__ pops) { k_partition_S_body(pops[blockIdx.y]); }
 
 // ====================================================== IncubRecoverySweep
 __device__ __forceinline__ void sev_add(const DevPop& d, int ad, int which, int delta, bool cum)
@@ -1922,106 +2215,6 @@ __device__ __forceinline__ uint16_t next_infectious_time(const cs_params& P, uin
     return (uint16_t)best;
 }
 
-// The gather's test from the person's own times, forming next_ev on the way (the
-// first gather after an upload or reset); kept out of line, off the common path.
-// (The arrays come as pointers: a DevPop passed by reference to an out-of-line
-// function would be copied to every thread's stack.)
-__device__ __noinline__ bool gather_test_from_times(const cs_params* __restrict__ P, const PersonHot* hot,
-                                                    const uint16_t* const* times, uint16_t* next_ev, int p, int ts)
-{
-    const int delay = (int)(P->LatentToSymptDelay / P->ModelTimeStep);
-    const PersonHot h = hot[p];
-    if (h.inf == CS_INF_LATENT) {
-        next_ev[p] = h.latent_time;
-        return h.latent_time == ts;
-    }
-    // times: recovery, SARI, critical, stepdown
-    const int v[5] = {(uint16_t)(h.latent_time + delay), times[0][p], P->DoSeverity ? times[1][p] : 0xFFFF,
-                      P->DoSeverity ? times[2][p] : 0xFFFF, P->DoSeverity ? times[3][p] : 0xFFFF};
-    int best = 0xFFFF;
-    bool ev = false;
-    for (int k = 0; k < 5; k++) {
-        if (k >= 2 && !P->DoSeverity) break;
-        if (v[k] == ts) ev = true;
-        if (v[k] >= ts && v[k] < best) best = v[k];
-    }
-    next_ev[p] = (uint16_t)best;
-    return ev;
-}
-
-// Which latent / infectious people have an event this step (latent period ends,
-// case onset, severity change, recovery or death): a light scan that compacts
-// them so the heavy transition kernel runs only on those.
-// IncubRecoverySweep's scan (src/Sweep.cpp:920-977) over the cells' lists: every
-// latent and infectious person (slots [S, S+L+I) of each cell, read block-
-// cooperatively as k_build_active reads a cell's slots, so a dense cell costs no more
-// than its share of the block) joins the step's event list when one of its times is
-// now.  The cells come in tiles of blockDim.x; Q = gridDim.x / tiles blocks share a
-// tile, block q taking its chunks q, q + Q, ... of blockDim.x entries, so the launch
-// has the parallelism of a flat list without building one.  The lists hold (person,
-// cell) in act / act_cell, latent people from the front and infectious people from
-// the back, in no particular order within each: k_incub_events treats each person on
-// its own.
-__device__ __forceinline__ void k_incub_gather_body(const DevPop& d)
-{
-    const int ts = d.step->ts;
-    const bool init = *d.ev_init != 0;   // next_ev is formed from the people's own times
-    __shared__ int s_first[kThreads], s_ofs[kThreads], s_n[kThreads], s_L[kThreads];
-    long long people = 0;
-    const int ntiles = (d.NC + blockDim.x - 1) / blockDim.x;
-    const int Q = max(1, (int)gridDim.x / ntiles), part = blockIdx.x % Q;
-    for (int tile = blockIdx.x / Q; tile < ntiles; tile += max(1, (int)gridDim.x / Q)) {
-        const int c0 = tile * blockDim.x;
-        const int c = c0 + threadIdx.x;
-        int first = 0, n = 0, nl = 0;
-        if (c < d.NC) {
-            first = d.cell_start[c] + d.S[c];
-            nl = d.L[c];
-            n = nl + d.I[c];
-        }
-        const int o = block_reserve2(nullptr, n, nullptr, 0).x;   // the block's own prefix of n
-        s_first[threadIdx.x] = first;
-        s_ofs[threadIdx.x] = o;
-        s_n[threadIdx.x] = n;
-        s_L[threadIdx.x] = nl;
-        __syncthreads();
-        const int total = s_ofs[blockDim.x - 1] + s_n[blockDim.x - 1];
-        if (threadIdx.x == 0 && part == 0) people += total;
-        for (int j0 = part * blockDim.x; j0 < total; j0 += Q * blockDim.x) {   // block-uniform: every thread reserves
-            const int j = j0 + (int)threadIdx.x;
-            bool ev = false, latent = false;
-            int p = 0, cell = 0;
-            if (j < total) {
-                int lo = 0, hi = blockDim.x - 1;   // the last cell whose entries start at or before j
-                while (lo < hi) {
-                    const int mid = (lo + hi + 1) >> 1;
-                    if (s_ofs[mid] <= j) lo = mid; else hi = mid - 1;
-                }
-                latent = j - s_ofs[lo] < s_L[lo];   // the cell's slots run latent, then infectious
-                p = d.slots[s_first[lo] + (j - s_ofs[lo])];
-                cell = c0 + lo;
-                if (init) {
-                    const uint16_t* times[4] = {d.recovery_time, d.sari_time, d.critical_time, d.stepdown_time};
-                    ev = gather_test_from_times(d.P, d.hot, times, d.next_ev, p, ts);
-                } else {
-                    ev = d.next_ev[p] == ts;
-                }
-            }
-            const int2 e = block_reserve2(d.counts + kCntEvents, (ev && latent) ? 1 : 0, d.counts + kCntEventsInf,
-                                          (ev && !latent) ? 1 : 0);
-            if (ev) {
-                const int at = latent ? e.x : d.N - 1 - e.y;
-                d.act[at] = p;
-                d.act_cell[at] = cell;
-            }
-        }
-        __syncthreads();   // the shared arrays are refilled for the next cells
-    }
-    if (threadIdx.x == 0 && people) cnt_add(CSB_CTR(work_incub_people), people);
-}
-__global__ void __launch_bounds__(kThreads) k_incub_gather(DevPop d) { k_incub_gather_body(d); }
-__global__ void __launch_bounds__(kThreads) k_incub_gather_multi(const DevPop* __restrict__ pops) { k_incub_gather_body(pops[blockIdx.y]); }
-
 // DoFalseCase (src/Update.cpp:896-905) for every person with a false-positive
 // entry this step, after the step's infections: detected with probability
 // ControlPropCasesId (counted once the detected cases at the last sample reached
@@ -2063,43 +2256,112 @@ __device__ __forceinline__ void k_apply_false_cases_body(const DevPop& d)
 __global__ void k_apply_false_cases(DevPop d) { k_apply_false_cases_body(d); }
 __global__ void k_apply_false_cases_multi(const DevPop* __restrict__ pops) { k_apply_false_cases_body(pops[blockIdx.y]); }
 
+// How a launch of warps takes a list of n items: `per` items a warp at a time, group g of
+// them by warp g / blocks of block g % blocks.  With few items a launch lasts as long as one
+// item's chain of dependent loads and double-precision draws, and lanes that take different
+// branches of it add theirs up, so while there are fewer items than schedulers (148 SMs
+// of four; shared by a batch's members) each gets a warp of its own, on as many SMs as there
+// are groups.  With many, whole warps in whole blocks: every warp and block adds its
+// tallies to the same few counters at its end.
+struct Groups {
+    int n, per, blocks;
+    __device__ __forceinline__ explicit Groups(int items) : n(items)
+    {
+        const int slots = 592 / (int)gridDim.y, wpb = blockDim.x >> 5;
+        per = max(1, min(32, n / max(1, slots)));
+        const int groups = (n + per - 1) / per;
+        blocks = max(1, min((int)gridDim.x, max(min(groups, 148), (groups + wpb - 1) / wpb)));
+    }
+    __device__ __forceinline__ bool idle_block() const { return (int)blockIdx.x >= blocks || (long long)blockIdx.x * per >= n; }
+    // f(item) for every item of the calling thread; all lanes of a warp make the same calls
+    template <typename F>
+    __device__ __forceinline__ void each(F f) const
+    {
+        const int lane = threadIdx.x & 31;
+        if ((int)blockIdx.x >= blocks) return;
+        for (long long g = blockIdx.x + (long long)blocks * (threadIdx.x >> 5); g * per < n; g += (long long)blocks * (blockDim.x >> 5)) {
+            const long long e = g * per + lane;
+            if (lane < per && e < n) f((int)e);
+        }
+    }
+};
+
+// The step's state changes, one kernel per kind, run side by side: DoInfect for every
+// claimed person (kInfections), DoIncub for the latent people whose time is now (kOnsets),
+// DoCase / severity / recovery / death for the infectious ones (kProgress).  They touch
+// different people (an infection reads its infector's infection time, type and latent
+// time, which no transition changes), share only integer tallies and lists, and meet only
+// in a person infected this step whose latent period ends this step: that thread goes on
+// to the onset itself.
+//
+// (One kernel over all latent and infectious people with a transition, after a second scan
+// and in warps of 32, took 17 us a step with hardly anyone infected, behind 8 us for the
+// infections and 5 for their moves.)
 // cnt[c] low 16 bits: L -> I moves of cell c; high 16 bits: I -> R/D moves.
-__device__ __forceinline__ void k_incub_events_body(const DevPop& d)
+enum ChangeKind { kInfections, kOnsets, kProgress };
+template <ChangeKind kKind>
+__device__ __forceinline__ void k_changes_body(const DevPop& d)
 {
     const cs_params& P = *d.P;
     const double t = d.step->t;
     const int ts = d.step->ts;
     const uint64_t seed = d.step->seed;
     const DevIv iv = *d.iv;
-    const int nlat = d.counts[kCntEvents], nev = nlat + d.counts[kCntEventsInf];
-    if (blockIdx.x == 0 && threadIdx.x == 0) *d.ev_init = 0;   // the gather before this formed next_ev
-    if (blockIdx.x * blockDim.x >= nev) return;   // a block without work stages nothing
-    const bool staged = nev >= kStageMinItems;
+    const int n = d.counts[kKind == kInfections ? kCntQueue : kKind == kOnsets ? kCntEvents : kCntEventsInf];
+    if (kKind == kOnsets && blockIdx.x == 0 && threadIdx.x == 0) *d.ev_init = 0;   // the scan before this formed next_ev
+    const Groups work(n);
+    if (work.idle_block()) return;   // a block without work stages nothing
+    const bool staged = n >= kStageMinItems;
     stage_begin(d.C, staged);
-    for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < nev; e += gridDim.x * blockDim.x) {
-        const int at = e < nlat ? e : d.N - 1 - (e - nlat);   // latent events, then infectious ones
-        const int p = d.act[at], c = d.act_cell[at];
-        PersonHot h = d.hot[p];
-        int pos = d.cell_start[c] + d.listpos[p];
-        if (h.inf == CS_INF_LATENT) {
-            if (h.latent_time != ts) continue;
+    InfectTally tally;
+    const double ox = d.rad_origin[0], oy = d.rad_origin[1];
+    work.each([&](int e) {
+        int p, c, pos = 0;
+        PersonHot h;
+        if (kKind == kInfections) {
+            p = d.queue[e];
+            c = do_infect(d, P, p, h, t, ts, seed, ox, oy, tally);
+            if (h.latent_time != ts) {
+                mark_cell(d, c, kCellTouched);
+                d.hot[p] = h;
+                d.next_ev[p] = h.latent_time;
+                return;
+            }
+        } else {
+            const int2 pc = d.events[kKind == kOnsets ? e : d.N - 1 - e];
+            p = pc.x;
+            c = pc.y;
+            h = d.hot[p];
+            pos = d.cell_start[c] + d.listpos[p];
+        }
+        if (kKind != kProgress) {
+            if (h.latent_time != ts) return;
             PersonTimes tm;
             do_incub(d, P, p, h, ts, seed, tm);
             atomicSub(d.L + c, 1);
             atomicAdd(d.I + c, 1);
             int add = 1;
-            d.mark[pos] = 1;
+            unsigned bits = kCellTouched;
+            uint8_t step = 0;
+            if (kKind == kInfections) {   // still among the S block's marked slots: the move marks the L slot it gives
+                bits |= kCellRelayS;
+                step = kStepLtoI;
+            } else {
+                d.mark[pos] = 1;
+            }
             cnt_add(CSB_STAGED(work_transitions), 1);
             if (infectious_events(d, P, iv, p, h, c, t, ts, seed, tm) & 1) {
-                d.pstep[p] = kStepItoRD;
+                bits |= kCellRelayL;
+                step |= kStepItoRD;
                 add += 1 << 16;
                 d.next_ev[p] = 0xFFFF;
             } else {
                 d.next_ev[p] = next_infectious_time(P, h.latent_time, tm, ts, true);
             }
+            if (step) d.pstep[p] = step;
             d.hot[p] = h;
             atomicAdd(d.cnt + c, add);
-            mark_cell(d, c);
+            mark_cell(d, c, bits);
         } else {
             const PersonTimes tm = load_times(d, P, p);
             int r = infectious_events(d, P, iv, p, h, c, t, ts, seed, tm);
@@ -2107,52 +2369,39 @@ __device__ __forceinline__ void k_incub_events_body(const DevPop& d)
             if (r & 1) {
                 d.mark[pos] = 2;
                 atomicAdd(d.cnt + c, 1 << 16);
-                mark_cell(d, c);
+                mark_cell(d, c, kCellTouched);
                 d.next_ev[p] = 0xFFFF;
             } else {
                 d.next_ev[p] = next_infectious_time(P, h.latent_time, tm, ts, true);
             }
         }
+    });
+    if (kKind == kInfections) {
+        __syncwarp();
+        infect_tally_add(d, tally);
+        if (blockIdx.x == 0 && threadIdx.x == 0) {
+            cnt_add(CSB_STAGED(work_new_infections), n);
+            cnt_add(CSB_STAGED(work_incub_people), n);   // the scan ran ahead of these people's infection
+        }
     }
     stage_flush(d.C, staged);
 }
-__global__ void __launch_bounds__(kThreads, 3) k_incub_events(DevPop d) { k_incub_events_body(d); }
-__global__ void __launch_bounds__(kThreads, 3) k_incub_events_multi(const DevPop* __restrict__ pops) { k_incub_events_body(pops[blockIdx.y]); }
-
-__device__ __forceinline__ void k_partition_LI_body(const DevPop& d)
-{
-    int nt = d.counts[kCntTouched];
-    const int warps = (gridDim.x * blockDim.x) >> 5;
-    for (int k = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; k < nt; k += warps) {
-        int c = d.touched[k];
-        int v = d.cnt[c];
-        int nLI = v & 0xffff, nIR = (v >> 16) & 0xffff;
-        int base = d.cell_start[c];
-        int S = d.S[c], L = d.L[c], I = d.I[c];
-        if (nLI) partition_block_warp(d, base, base + S, L + nLI, nLI, 1, true);
-        if (nIR) partition_block_warp(d, base, base + S + L, I + nIR, nIR, 2, false);
-        if ((threadIdx.x & 31) == 0) {
-            d.cnt[c] = 0;
-            d.cell_flag[c] = 0;
-        }
-    }
-}
-__global__ void k_partition_LI(DevPop d) { k_partition_LI_body(d); }
-__global__ void k_partition_LI_multi(const DevPop* __restrict__ pops) { k_partition_LI_body(pops[blockIdx.y]); }
+__global__ void __launch_bounds__(kThreads, 3) k_infections(DevPop d) { k_changes_body<kInfections>(d); }
+__global__ void __launch_bounds__(kThreads, 3) k_onsets(DevPop d) { k_changes_body<kOnsets>(d); }
+__global__ void __launch_bounds__(kThreads, 3) k_progress(DevPop d) { k_changes_body<kProgress>(d); }
+__global__ void __launch_bounds__(kThreads, 3) k_infections_multi(const DevPop* __restrict__ pops) { k_changes_body<kInfections>(pops[blockIdx.y]); }
+__global__ void __launch_bounds__(kThreads, 3) k_onsets_multi(const DevPop* __restrict__ pops) { k_changes_body<kOnsets>(pops[blockIdx.y]); }
+__global__ void __launch_bounds__(kThreads, 3) k_progress_multi(const DevPop* __restrict__ pops) { k_changes_body<kProgress>(pops[blockIdx.y]); }
 
 // Deferred household actions, once per household, after every per-person
 // transition of the step: the adult-carer absence of DoCase/DoDetectedCase
 // (src/Update.cpp:736-763, 843-868) and household quarantine (src/Update.cpp:676-708).
-__device__ __forceinline__ void k_household_after_body(const DevPop& d)
+__device__ __forceinline__ void household_actions(const DevPop& d)
 {
     const cs_params& P = *d.P;
     const int ts = d.step->ts;
     const uint64_t seed = d.step->seed;
-    // the step's transition flags are only set on event people: clear them
-    const int nlat = d.counts[kCntEvents], nev = nlat + d.counts[kCntEventsInf];
-    for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < nev; e += gridDim.x * blockDim.x)
-        d.pstep[d.act[e < nlat ? e : d.N - 1 - (e - nlat)]] = 0;
-    int nh = d.counts[kCntHH];
+    const int nh = d.counts[kCntHH];
     for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < nh; k += gridDim.x * blockDim.x) {
         int h = d.hh_list[k];
         uint8_t f = d.hh_flag[h];
@@ -2197,22 +2446,28 @@ __device__ __forceinline__ void k_household_after_body(const DevPop& d)
         }
     }
 }
-__global__ void k_household_after(DevPop d) { k_household_after_body(d); }
-__global__ void k_household_after_multi(const DevPop* __restrict__ pops) { k_household_after_body(pops[blockIdx.y]); }
+__global__ void __launch_bounds__(kThreads) k_households(DevPop d) { household_actions(d); }
+__global__ void __launch_bounds__(kThreads) k_households_multi(const DevPop* __restrict__ pops) { household_actions(pops[blockIdx.y]); }
 
-// The cell-list moves and the household actions in one launch: the moves touch the
-// cells' slots and list positions, the household actions people's absences and
-// quarantine, flags and household lists, so neither waits for the other.
-__global__ void k_incub_finish(DevPop d)
+// The end of a timestep: the touched cells' list moves, beside the household actions (the
+// moves touch the cells' slots and list positions, the household actions people's absences
+// and quarantine, flags and household lists).  kS: the step's S -> L moves are among them,
+// and the lists that no later kernel of the step reads go back to empty here (the touched
+// cells' and households' lists, which these two kernels read, when the next step begins).
+template <bool kS>
+__device__ __forceinline__ void k_moves_body(const DevPop& d)
 {
-    k_partition_LI_body(d);
-    k_household_after_body(d);
+    const int n = partition_touched<kS, true>(d);
+    if (kS) {
+        if ((threadIdx.x & 31) == 0 && n) cnt_add(CSB_CTR(work_cells_touched), n);
+        if (blockIdx.x == 0 && threadIdx.x < kCntN && threadIdx.x != kCntTouched && threadIdx.x != kCntHH) d.counts[threadIdx.x] = 0;
+    }
+    if (d.step_clock && blockIdx.x == 0 && threadIdx.x == 0) *d.step_clock += 1;
 }
-__global__ void k_incub_finish_multi(const DevPop* __restrict__ pops)
-{
-    k_partition_LI_body(pops[blockIdx.y]);
-    k_household_after_body(pops[blockIdx.y]);
-}
+template <bool kS>
+__global__ void __launch_bounds__(kThreads) k_moves(DevPop d) { k_moves_body<kS>(d); }
+template <bool kS>
+__global__ void __launch_bounds__(kThreads) k_moves_multi(const DevPop* __restrict__ pops) { k_moves_body<kS>(pops[blockIdx.y]); }
 
 // ============================================================ seeding
 __global__ void k_seed_claims(DevPop d, const int32_t* list, int n)
@@ -2738,7 +2993,7 @@ static int alloc_dynamic(cs_gpu_ctx* c)
         AL(c->rowS, (size_t)params->nch);
     }
     AL(d.claim, N); AL(d.queue, N); AL(d.counts, kCntN); AL(d.touched, NC); AL(d.cell_flag, NC + 4);
-    AL(d.act, N); AL(d.act_cell, N); AL(d.cnt, NC); AL(d.cnt_ofs, N);
+    AL(d.act, N); AL(d.events, N); AL(d.cnt, NC); AL(d.cnt_s, NC); AL(d.cnt_ofs, N);
     AL(d.cmap, 2 * N); d.cmap_cap = (int32_t)(2 * N);
     AL(d.act_closed, N); AL(d.hh_flag, NH + 4); AL(d.hh_list, NH);
     AL(d.carer_win, NH); AL(d.carer_list, NH);
@@ -2751,6 +3006,7 @@ static int alloc_dynamic(cs_gpu_ctx* c)
     CK(cudaMemsetAsync(d.cell_flag, 0, NC + 4, c->stream));
     CK(cudaMemsetAsync(d.hh_flag, 0, NH + 4, c->stream));
     CK(cudaMemsetAsync(d.cnt, 0, sizeof(int32_t) * NC, c->stream));
+    CK(cudaMemsetAsync(d.cnt_s, 0, sizeof(int32_t) * NC, c->stream));
     CK(cudaMemsetAsync(d.pstep, 0, N, c->stream));
     { cs_params* t; UP(t, params, 1); c->dP = t; d.P = t; }
     {
@@ -2786,9 +3042,7 @@ int cs_gpu_create(const cs_population* pop, const cs_params* params, int device,
     c->device = device;
     CK(cudaSetDevice(device));
     CK(cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking));
-    CK(cudaStreamCreateWithFlags(&c->side, cudaStreamNonBlocking));
-    CK(cudaEventCreateWithFlags(&c->ev_fork, cudaEventDisableTiming));
-    CK(cudaEventCreateWithFlags(&c->ev_join, cudaEventDisableTiming));
+    CK(c->br.create());
     int nsm = 148;
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, device);
     c->grid = nsm * 8;
@@ -2947,9 +3201,7 @@ int cs_gpu_create_replica(const cs_gpu_ctx* base, cs_gpu_ctx** out)
     c->device = base->device;
     CK(cudaSetDevice(c->device));
     CK(cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking));
-    CK(cudaStreamCreateWithFlags(&c->side, cudaStreamNonBlocking));
-    CK(cudaEventCreateWithFlags(&c->ev_fork, cudaEventDisableTiming));
-    CK(cudaEventCreateWithFlags(&c->ev_join, cudaEventDisableTiming));
+    CK(c->br.create());
     c->grid = base->grid;
     c->hp = base->hp;
     c->stat = base->stat;
@@ -2977,9 +3229,7 @@ void cs_gpu_destroy(cs_gpu_ctx* c)
     if (c->stream) cudaStreamSynchronize(c->stream);
     for (auto& r : c->ring) { cudaEventDestroy(r.a); cudaEventDestroy(r.b); }
     for (cudaEvent_t e : c->graph_events) cudaEventDestroy(e);
-    if (c->side) { cudaStreamSynchronize(c->side); cudaStreamDestroy(c->side); }
-    if (c->ev_fork) cudaEventDestroy(c->ev_fork);
-    if (c->ev_join) cudaEventDestroy(c->ev_join);
+    c->br.destroy();
     if (c->graph_exec) cudaGraphExecDestroy(c->graph_exec);
     if (c->graph) cudaGraphDestroy(c->graph);
     if (c->day_exec) cudaGraphExecDestroy(c->day_exec);
@@ -3231,15 +3481,25 @@ int cs_gpu_update_probs(cs_gpu_ctx* c, int do_place)
     return rebuild_blocks(c);
 }
 
+// The infections of the claimed people and the false cases, alone.
 static int apply_queue(cs_gpu_ctx* c)
 {
     DevPop& d = c->d;
     LAUNCH(k_apply_infections, c->grid, kThreads, d);
     LAUNCH(k_partition_S, c->grid, kThreads, d);
     if (c->hp.FalsePositiveRate > 0) LAUNCH(k_apply_false_cases, c->grid, kThreads, d);
-    // every sweep leaves its list counters at zero for the next one; the household
-    // list (last) is the incub sweep's
+    // a sweep called alone leaves its list counters at zero for the next one; the
+    // household list (last) is the incub sweep's
     CK(cudaMemsetAsync(d.counts, 0, sizeof(int32_t) * (kCntN - 1), c->stream));
+    return CS_OK;
+}
+
+// List counters at zero before a sweep or seeding called alone, after whole timesteps.
+static int fresh_lists(cs_gpu_ctx* c)
+{
+    if (!c->lists_stale) return CS_OK;
+    CK(cudaMemsetAsync(c->d.counts, 0, sizeof(int32_t) * kCntN, c->stream));
+    c->lists_stale = false;
     return CS_OK;
 }
 
@@ -3255,7 +3515,9 @@ int cs_gpu_seed_infections(cs_gpu_ctx* c, double t, const int32_t* people, int n
         c->seed_cap = n;
     }
     CK(cudaMemcpyAsync(c->d_seed_list, people, sizeof(int32_t) * n, cudaMemcpyHostToDevice, c->stream));
-    LAUNCH(k_set_step, 1, 1, c->d, t, (unsigned long long)c->seed);
+    int r = fresh_lists(c);
+    if (r) return r;
+    LAUNCH(k_set_step, 1, 1, c->d, t, (unsigned long long)c->seed, 0);
     LAUNCH(k_seed_claims, (n + kThreads - 1) / kThreads, kThreads, c->d, c->d_seed_list, n);
     return apply_queue(c);
 }
@@ -3284,6 +3546,8 @@ int cs_gpu_begin_run(cs_gpu_ctx* c, uint64_t seed, const int32_t* seed_people, i
     CK(cudaMemsetAsync(d.C, 0, sizeof(cs_counters), c->stream));
     CK(cudaMemsetAsync(d.counts, 0, sizeof(int32_t) * kCntN, c->stream));
     CK(cudaMemsetAsync(d.cnt, 0, sizeof(int32_t) * d.NC, c->stream));
+    CK(cudaMemsetAsync(d.cnt_s, 0, sizeof(int32_t) * d.NC, c->stream));
+    c->lists_stale = false;
     LAUNCH(k_reset_people, c->grid, kThreads, d, seed);
     LAUNCH(k_reset_slots, c->grid, kThreads, d);
     LAUNCH(k_reset_listpos, (d.NC + kThreads - 1) / kThreads, kThreads, d);
@@ -3295,13 +3559,80 @@ int cs_gpu_begin_run(cs_gpu_ctx* c, uint64_t seed, const int32_t* seed_people, i
     return cs_gpu_seed_infections(c, 0.0, seed_people, n_seed);
 }
 
-static int build_active(cs_gpu_ctx* c, int mode)
+// Every tile of kThreads cells shared by enough blocks to fill the grid.
+static int scan_grid(int NC, int grid)
+{
+    const int ntiles = (NC + kThreads - 1) / kThreads;
+    return ntiles * std::max(1, grid / ntiles);
+}
+
+// LAUNCH on branch i beside the context's stream; while profiling, on the stream itself,
+// so that the kernels run (and are timed) one after the other.
+#define LAUNCH_ON(i, kernel, grid, block, ...)                                                     \
+    do {                                                                                           \
+        if (c->prof) prof_begin(c, #kernel);                                                       \
+        kernel<<<(grid), (block), 0, c->prof ? c->stream : c->br.s[i]>>>(__VA_ARGS__);              \
+        if (c->prof) prof_end(c);                                                                  \
+        c->launches++;                                                                             \
+        CK(cudaGetLastError());                                                                    \
+    } while (0)
+#define FORK(n) do { if (!c->prof) CK(c->br.begin(c->stream, n)); } while (0)
+#define JOIN(n) do { if (!c->prof) CK(c->br.end(c->stream, n)); } while (0)
+
+// The step's scalars, and beside them the scan for the step's lists.
+extern "C++" {
+template <bool kActive, bool kEvents>
+static int begin_step(cs_gpu_ctx* c, double t, bool empty_lists)
 {
     DevPop& d = c->d;
-    // the list counters are zero here: every sweep (and begin_run, upload_state,
-    // seed_infections) ends by zeroing them
-    const int ntiles = (d.NC + kThreads - 1) / kThreads;
-    LAUNCH(k_build_active, ntiles * std::max(1, c->grid / ntiles), kThreads, d, mode);
+    FORK(1);
+    LAUNCH_ON(0, k_set_step, 1, 1, d, t, (unsigned long long)c->seed, empty_lists ? 1 : 0);
+    LAUNCH((k_scan<kActive, kEvents>), scan_grid(d.NC, c->grid), kThreads, d, t);
+    JOIN(1);
+    return CS_OK;
+}
+}
+
+// The infectors' passes over the list the scan built.  The place pass and the spatial pass
+// both read the infector pass's lists and only claim infections (atomicMin on the claim
+// key) and add to counters, so they run side by side.
+static int infector_passes(cs_gpu_ctx* c)
+{
+    DevPop& d = c->d;
+    LAUNCH(k_infector_hh_spatial, c->grid, kThreads, d);
+    FORK(1);
+    LAUNCH_ON(0, k_infector_places, c->grid, kThreads, d);
+    switch (c->spatial_lanes) {
+    case 2: LAUNCH(k_spatial<2>, c->grid, kThreads, d); break;
+    case 4: LAUNCH(k_spatial<4>, c->grid, kThreads, d); break;
+    case 16: LAUNCH(k_spatial<16>, c->grid, kThreads, d); break;
+    default: LAUNCH(k_spatial<8>, c->grid, kThreads, d); break;
+    }
+    JOIN(1);
+    return CS_OK;
+}
+
+static int infect_alone(cs_gpu_ctx* c, double t)
+{
+    int r = begin_step<true, false>(c, t, false);
+    if (!r) r = infector_passes(c);
+    return r ? r : apply_queue(c);
+}
+
+static int incub_alone(cs_gpu_ctx* c, double t)
+{
+    DevPop& d = c->d;
+    int r = begin_step<false, true>(c, t, false);
+    if (r) return r;
+    FORK(1);
+    LAUNCH_ON(0, k_progress, c->grid, kThreads, d);
+    LAUNCH(k_onsets, c->grid, kThreads, d);
+    JOIN(1);
+    FORK(1);
+    LAUNCH_ON(0, k_households, c->grid, kThreads, d);
+    LAUNCH(k_moves<false>, c->grid, kThreads, d);
+    JOIN(1);
+    CK(cudaMemsetAsync(d.counts, 0, sizeof(int32_t) * kCntN, c->stream));   // all list counters
     return CS_OK;
 }
 
@@ -3310,70 +3641,50 @@ int cs_gpu_infect_sweep(cs_gpu_ctx* c, double t, int run)
     (void)run;
     if (!c) return CS_E_ARG;
     if (!c->run_started) return set_err(c, CS_E_STATE, "infect_sweep before begin_run");
-    DevPop& d = c->d;
-    LAUNCH(k_set_step, 1, 1, d, t, (unsigned long long)c->seed);
-    int r = build_active(c, 0);
-    if (r) return r;
-    LAUNCH(k_infector_hh_spatial, c->grid, kThreads, d);
-    // The place pass and the spatial pass both read the infector pass's lists and
-    // only claim infections (atomicMin on the claim key) and add to counters, so the
-    // place pass runs on the side stream beside the spatial pass (a branch of the
-    // captured graphs).  While profiling they run one after the other.
-    const bool fork = c->side && !c->prof;
-    if (fork) {
-        CK(cudaEventRecord(c->ev_fork, c->stream));
-        CK(cudaStreamWaitEvent(c->side, c->ev_fork, 0));
-        k_infector_places<<<c->grid, kThreads, 0, c->side>>>(d);
-        c->launches++;
-        CK(cudaGetLastError());
-        CK(cudaEventRecord(c->ev_join, c->side));
-    } else {
-        LAUNCH(k_infector_places, c->grid, kThreads, d);
-    }
-    switch (c->spatial_lanes) {
-    case 2: LAUNCH(k_spatial<2>, c->grid, kThreads, d); break;
-    case 4: LAUNCH(k_spatial<4>, c->grid, kThreads, d); break;
-    case 16: LAUNCH(k_spatial<16>, c->grid, kThreads, d); break;
-    default: LAUNCH(k_spatial<8>, c->grid, kThreads, d); break;
-    }
-    if (fork) CK(cudaStreamWaitEvent(c->stream, c->ev_join, 0));
-    return apply_queue(c);
-}
-
-// IncubRecoverySweep; set_step false when the infect sweep of the same timestep has
-// just written the step's scalars.
-static int incub_sweep(cs_gpu_ctx* c, double t, bool set_step)
-{
-    DevPop& d = c->d;
-    if (set_step) LAUNCH(k_set_step, 1, 1, d, t, (unsigned long long)c->seed);
-    {   // every tile of kThreads cells shared by enough blocks to fill the grid
-        const int ntiles = (d.NC + kThreads - 1) / kThreads;
-        LAUNCH(k_incub_gather, ntiles * std::max(1, c->grid / ntiles), kThreads, d);
-    }
-    LAUNCH(k_incub_events, c->grid, kThreads, d);
-    LAUNCH(k_incub_finish, c->grid, kThreads, d);
-    CK(cudaMemsetAsync(d.counts, 0, sizeof(int32_t) * kCntN, c->stream));   // all list counters
-    return CS_OK;
+    int r = fresh_lists(c);
+    return r ? r : infect_alone(c, t);
 }
 
 int cs_gpu_incub_recovery_sweep(cs_gpu_ctx* c, double t)
 {
     if (!c) return CS_E_ARG;
     if (!c->run_started) return set_err(c, CS_E_STATE, "incub_recovery_sweep before begin_run");
-    return incub_sweep(c, t, true);
+    int r = fresh_lists(c);
+    return r ? r : incub_alone(c, t);
 }
+
+// One timestep, both sweeps.  With false positives on, a false case is detected between
+// the infections and the transitions, so the sweeps run as they do alone; otherwise one
+// scan serves both, the infections are applied with the transitions, and all list moves
+// come last.
+static bool fused_step(const cs_gpu_ctx* c) { return !(c->hp.FalsePositiveRate > 0); }
 
 static int step_eager(cs_gpu_ctx* c, double t, int run)
 {
-    int r = cs_gpu_infect_sweep(c, t, run);
+    (void)run;
+    if (!fused_step(c)) {
+        int r = infect_alone(c, t);
+        return r ? r : incub_alone(c, t);
+    }
+    DevPop& d = c->d;
+    int r = begin_step<true, true>(c, t, true);
+    if (!r) r = infector_passes(c);
     if (r) return r;
-    return incub_sweep(c, t, false);
+    FORK(2);
+    LAUNCH_ON(0, k_progress, c->grid, kThreads, d);
+    LAUNCH_ON(1, k_infections, c->grid, kThreads, d);
+    LAUNCH(k_onsets, c->grid, kThreads, d);
+    JOIN(2);
+    FORK(1);
+    LAUNCH_ON(0, k_households, c->grid, kThreads, d);
+    LAUNCH(k_moves<true>, c->grid, kThreads, d);
+    JOIN(1);
+    return CS_OK;
 }
 
-// Capture one whole timestep (both sweeps: ten kernels and two memsets, one more
-// kernel with false positives on) as a CUDA graph.  Every kernel reads the step's
-// scalars from device memory written by k_set_step, so a replay only needs the
-// k_set_step node's arguments changed.
+// Capture one whole timestep (both sweeps) as a CUDA graph.  Every kernel reads the step's
+// scalars from device memory written by k_set_step, so a replay only needs the arguments
+// of that node and of the scan (which runs beside it) changed.
 static int capture_step(cs_gpu_ctx* c, double t, int run)
 {
     cudaGraph_t g = nullptr;
@@ -3399,7 +3710,8 @@ static int capture_step(cs_gpu_ctx* c, double t, int run)
         if (ty != cudaGraphNodeTypeKernel) continue;
         cudaKernelNodeParams kp;
         CK(cudaGraphKernelNodeGetParams(nd, &kp));
-        if (kp.func == (void*)k_set_step) {
+        if (kp.func == (void*)k_set_step || kp.func == (void*)k_scan<true, true> || kp.func == (void*)k_scan<true, false> ||
+            kp.func == (void*)k_scan<false, true>) {
             c->set_step_nodes.push_back(nd);
             c->set_step_params.push_back(kp);
         }
@@ -3415,6 +3727,9 @@ int cs_gpu_step(cs_gpu_ctx* c, double t, int run)
 {
     if (!c) return CS_E_ARG;
     if (!c->run_started) return set_err(c, CS_E_STATE, "step before begin_run");
+    if (!fused_step(c))
+        if (int r = fresh_lists(c)) return r;   // its first scan empties no list
+    c->lists_stale = fused_step(c);
     if (!c->use_graph || c->prof) return step_eager(c, t, run);
     if (!c->graph_exec) {
         int r = capture_step(c, t, run);
@@ -3422,8 +3737,9 @@ int cs_gpu_step(cs_gpu_ctx* c, double t, int run)
     }
     DevPop d = c->d;
     unsigned long long seed = c->seed;
+    int empty_lists = fused_step(c) ? 1 : 0;
     for (size_t k = 0; k < c->set_step_nodes.size(); k++) {
-        void* args[] = {&d, &t, &seed};
+        void* args[] = {&d, &t, &seed, &empty_lists};   // k_scan takes the first two
         cudaKernelNodeParams kp = c->set_step_params[k];
         kp.kernelParams = args;
         kp.extra = nullptr;
@@ -3629,6 +3945,8 @@ int cs_gpu_run(cs_gpu_ctx* c, int days, const cs_run_policy* policy, cs_counters
     if (policy) pol = *policy;
     int r = day_ctl_start(c, days, pol);
     if (r) return r;
+    if (!fused_step(c) && (r = fresh_lists(c))) return r;
+    c->lists_stale = fused_step(c);
     c->d.step_clock = c->d_clock;
     c->d.gate = &c->d_ctl->update;
     r = run_days(c, days, spd, pol.probs_every_step != 0);
@@ -3666,6 +3984,8 @@ struct cs_gpu_batch {
     double* d_t = nullptr;   // the timestep's t, read by every member's k_set_step
     DevPop* d_pops = nullptr; // members' DevPop (t taken from d_t)
     int lanes = 8;            // spatial lanes of the batched launches
+    Branches br;              // kernels of a batched timestep that run side by side
+    bool fused = false;       // the form of the timestep the graphs were captured with
     // device run loop (cs_gpu_batch_run): members' DevPop with step clocks and
     // UpdateProbs gates, their control blocks, one graph per day
     DevPop* d_pops_day = nullptr;
@@ -3725,6 +4045,7 @@ int cs_gpu_batch_create(cs_gpu_ctx* const* members, int n, cs_gpu_batch** out)
     }
     BCK(cudaSetDevice(b->device));
     BCK(cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking));
+    BCK(b->br.create());
     BCK(cudaMalloc(&b->d_t, sizeof(double)));
     BCK(cudaMalloc(&b->d_pops, sizeof(DevPop) * n));
     b->members.assign(members, members + n);
@@ -3747,32 +4068,87 @@ const char* cs_gpu_batch_last_error(const cs_gpu_batch* b) { return b ? b->err :
         if (e_ != cudaSuccess) return batch_err(b, CS_E_CUDA, "launch %s: %s", #kernel, cudaGetErrorString(e_)); \
     } while (0)
 
-// The batched timestep, in the order of step_eager (InfectSweep, then
-// IncubRecoverySweep without a second k_set_step).
+#define BLAUNCH_ON(i, kernel, grid, block, ...)                                                    \
+    do {                                                                                           \
+        kernel<<<(grid), (block), 0, b->br.s[i]>>>(__VA_ARGS__);                                   \
+        cudaError_t e_ = cudaGetLastError();                                                       \
+        if (e_ != cudaSuccess) return batch_err(b, CS_E_CUDA, "launch %s: %s", #kernel, cudaGetErrorString(e_)); \
+    } while (0)
+
+// Whether a batched timestep takes step_eager's short form: no member has false positives.
+static bool batch_fused(const cs_gpu_batch* b)
+{
+    for (const cs_gpu_ctx* m : b->members)
+        if (!fused_step(m)) return false;
+    return true;
+}
+
+static long long batch_kernels(const cs_gpu_batch* b) { return batch_fused(b) ? 10 : 12; }
+
+// Members' list counters before a batched timestep or run, as cs_gpu_step and cs_gpu_run
+// treat a lone context's.
+static int batch_lists(cs_gpu_batch* b)
+{
+    const bool fused = batch_fused(b);
+    if (fused != b->fused) {   // a member's false positives were switched on or off
+        BCK(cudaStreamSynchronize(b->stream));
+        batch_drop_graph(b);
+        b->fused = fused;
+    }
+    for (cs_gpu_ctx* m : b->members) {
+        if (!fused)
+            if (int r = fresh_lists(m)) return batch_err(b, r, "%s", m->err);
+        m->lists_stale = fused;
+    }
+    return CS_OK;
+}
+
+// The batched timestep, in the order of step_eager.
 static int batch_enqueue(cs_gpu_batch* b, const DevPop* pops)
 {
     const int R = (int)b->members.size();
     const int grid = b->members[0]->grid;
-    const dim3 g(grid, R), one(1, R);
-    BLAUNCH(k_set_step_multi, one, 1, pops, 0.0, 0ull);
-    BLAUNCH(k_build_active_multi, g, kThreads, pops, 0);
+    const dim3 g(grid, R);
+    int maxc = 0;
+    for (const cs_gpu_ctx* m : b->members) maxc = std::max(maxc, m->d.NC);
+    const dim3 gs(scan_grid(maxc, grid), R);
+    const bool fused = batch_fused(b);
+    BCK(b->br.begin(b->stream, 1));
+    BLAUNCH_ON(0, k_set_step_multi, R, 1, pops, fused ? 1 : 0);
+    if (fused) BLAUNCH((k_scan_multi<true, true>), gs, kThreads, pops);
+    else BLAUNCH((k_scan_multi<true, false>), gs, kThreads, pops);
+    BCK(b->br.end(b->stream, 1));
     BLAUNCH(k_infector_hh_spatial_multi, g, kThreads, pops);
-    BLAUNCH(k_infector_places_multi, g, kThreads, pops);
+    BCK(b->br.begin(b->stream, 1));
+    BLAUNCH_ON(0, k_infector_places_multi, g, kThreads, pops);
     switch (b->lanes) {
     case 2: BLAUNCH(k_spatial_multi<2>, g, kThreads, pops); break;
     case 4: BLAUNCH(k_spatial_multi<4>, g, kThreads, pops); break;
     case 16: BLAUNCH(k_spatial_multi<16>, g, kThreads, pops); break;
     default: BLAUNCH(k_spatial_multi<8>, g, kThreads, pops); break;
     }
+    BCK(b->br.end(b->stream, 1));
+    if (fused) {
+        BCK(b->br.begin(b->stream, 2));
+        BLAUNCH_ON(0, k_progress_multi, g, kThreads, pops);
+        BLAUNCH_ON(1, k_infections_multi, g, kThreads, pops);
+        BLAUNCH(k_onsets_multi, g, kThreads, pops);
+        BCK(b->br.end(b->stream, 2));
+        BCK(b->br.begin(b->stream, 1));
+        BLAUNCH_ON(0, k_households_multi, g, kThreads, pops);
+        BLAUNCH(k_moves_multi<true>, g, kThreads, pops);
+        BCK(b->br.end(b->stream, 1));
+        return CS_OK;
+    }
     BLAUNCH(k_apply_infections_multi, g, kThreads, pops);
     BLAUNCH(k_partition_S_multi, g, kThreads, pops);
-    bool fpr = false;
-    for (const cs_gpu_ctx* m : b->members) fpr |= m->hp.FalsePositiveRate > 0;
-    if (fpr) BLAUNCH(k_apply_false_cases_multi, g, kThreads, pops);
+    BLAUNCH(k_apply_false_cases_multi, g, kThreads, pops);
     BLAUNCH(k_zero_counts_multi, R, 32, pops, (int)(kCntN - 1));   // the household list is the incub sweep's
-    BLAUNCH(k_incub_gather_multi, g, kThreads, pops);
-    BLAUNCH(k_incub_events_multi, g, kThreads, pops);
-    BLAUNCH(k_incub_finish_multi, g, kThreads, pops);
+    BLAUNCH((k_scan_multi<false, true>), gs, kThreads, pops);
+    BLAUNCH(k_onsets_multi, g, kThreads, pops);
+    BLAUNCH(k_progress_multi, g, kThreads, pops);
+    BLAUNCH(k_moves_multi<false>, g, kThreads, pops);
+    BLAUNCH(k_households_multi, g, kThreads, pops);
     BLAUNCH(k_zero_counts_multi, R, 32, pops, (int)kCntN);
     return CS_OK;
 }
@@ -3810,7 +4186,7 @@ static int batch_capture(cs_gpu_batch* b, double t, int run)
     }
     BCK(cudaGraphInstantiate(&b->exec, g, 0));
     b->graph = g;
-    for (int k = 0; k < n; k++) b->member_launches[k] = 11;   // kernels run for each member per step
+    for (int k = 0; k < n; k++) b->member_launches[k] = batch_kernels(b);   // kernels run for each member per step
     return CS_OK;
 }
 
@@ -3819,11 +4195,12 @@ int cs_gpu_batch_step(cs_gpu_batch* b, double t, int run)
     if (!b) return CS_E_ARG;
     for (size_t k = 0; k < b->members.size(); k++)
         if (!b->members[k]->run_started) return batch_err(b, CS_E_STATE, "member %zu: step before begin_run", k);
+    if (int r = batch_lists(b)) return r;
     if (!b->exec) {
         int r = batch_capture(b, t, run);
         if (r) return r;
     }
-    // every member's k_set_step reads t (and its run's seed) from device memory
+    // every member's k_scan reads t (and its run's seed) from device memory
     BCK(cudaMemcpyAsync(b->d_t, &t, sizeof(double), cudaMemcpyHostToDevice, b->stream));
     BCK(cudaGraphLaunch(b->exec, b->stream));
     for (size_t k = 0; k < b->members.size(); k++) b->members[k]->launches += b->member_launches[k];
@@ -3905,7 +4282,7 @@ static int batch_enqueue_day(cs_gpu_batch* b, int spd, bool every_step)
     for (int s = 0; s < spd; s++) {
         int r = batch_enqueue(b, pops);
         if (r) return r;
-        for (int k = 0; k < R; k++) b->member_day_launches[k] += 11;
+        for (int k = 0; k < R; k++) b->member_day_launches[k] += batch_kernels(b);
         if (!every_step && s < spd - 1) continue;
         const int day_end = s == spd - 1 ? 1 : 0;
         BLAUNCH(k_zero_totals_multi, R, 32, pops);
@@ -4010,6 +4387,7 @@ int cs_gpu_batch_run(cs_gpu_batch* b, int days, const cs_run_policy* policies, c
     BCK(cudaMemcpyAsync(b->d_pops_day, hp.data(), sizeof(DevPop) * n, cudaMemcpyHostToDevice, b->stream));
     BCK(cudaMemcpyAsync(b->d_ctls, hc.data(), sizeof(DayCtl*) * n, cudaMemcpyHostToDevice, b->stream));
     BCK(cudaStreamSynchronize(b->stream));
+    if (int r = batch_lists(b)) return r;
     bool stale = !b->day_exec || b->day_every_step != (every ? 1 : 0) || b->day_spd != spd;
     for (int k = 0; k < n && !stale; k++) stale = b->day_geometry[k] != b->members[k]->geometry_gen;
     if (stale) {
@@ -4041,6 +4419,7 @@ void cs_gpu_batch_destroy(cs_gpu_batch* b)
         if (b->ev_join[i]) cudaEventDestroy(b->ev_join[i]);
     }
     if (b->ev_fork) cudaEventDestroy(b->ev_fork);
+    b->br.destroy();
     if (b->d_pops_day) cudaFree(b->d_pops_day);
     if (b->d_ctls) cudaFree(b->d_ctls);
     for (cs_gpu_ctx* m : b->members)
@@ -4529,6 +4908,8 @@ int cs_gpu_upload_state(cs_gpu_ctx* c, uint64_t seed, const cs_state_view* v)
     CK(cudaMemsetAsync(d.mark, 0, N, c->stream));
     CK(cudaMemsetAsync(d.counts, 0, sizeof(int32_t) * kCntN, c->stream));
     CK(cudaMemsetAsync(d.cnt, 0, sizeof(int32_t) * d.NC, c->stream));
+    CK(cudaMemsetAsync(d.cnt_s, 0, sizeof(int32_t) * d.NC, c->stream));
+    c->lists_stale = false;
     CK(cudaMemsetAsync(d.C, 0, sizeof(cs_counters), c->stream));
     CK(cudaMemsetAsync(d.ev_init, 0xff, sizeof(int32_t), c->stream));   // next_ev from the uploaded times
     // the host seeded the run: its LocationInitialInfection is where radii start

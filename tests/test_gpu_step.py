@@ -1,0 +1,75 @@
+"""The whole-timestep path (cs_gpu_step: one scan ahead of the infections, the infections
+beside the transitions, all list moves at the end) against the sweeps called one by one and
+the oracle, state for state (tolerance: none), where the two forms could part: people
+infected and turning infectious in the same timestep (a latent period of a tenth of a step),
+and dying or recovering in it too (an infectious period of no steps), cells with more moves
+in a step than a warp's batch of 32, whole timesteps and single sweeps in turn, and false
+positives switched on and off between steps."""
+import numpy as np
+import pytest
+
+from covidsim_b200 import abi, population, params as prm, sim
+import oracle_py
+from tests.helpers import snapshot, check_lists, STATE_FIELDS
+
+pytestmark = pytest.mark.gpu
+
+
+def _world(n_people, cells, latent, infectious):
+    grid = population.make_grid(nmcl=2)
+    grid.update(ncw=cells, nch=cells, cell_width=1.0 / 120, cell_height=1.0 / 120)
+    pop = population.generate(n_people, grid, sigma=1.0, seed=11)
+    P, lk, hr = prm.build_params(grid, kernel_size=200000)
+    P.LocalBeta = 2.0
+    if latent is not None:
+        P.LatentPeriod = latent
+    if infectious is not None:
+        P.InfectiousPeriod = infectious
+    return pop, P, lk, hr
+
+
+def _same(a, b, where):
+    for k in STATE_FIELDS:
+        assert np.array_equal(a[k], b[k]), "%s: %s differs at %d entries" % (where, k, int(np.sum(a[k] != b[k])))
+
+
+@pytest.mark.parametrize("n_people,cells,latent,infectious,n_seed", [
+    (3000, 1, None, None, 900), (6000, 4, 0.02, None, 300), (6000, 4, 0.02, 0.1, 300), (20000, 30, 0.3, 1.0, 4000)])
+def test_step_matches_single_sweeps_and_oracle(n_people, cells, latent, infectious, n_seed):
+    pop, P, lk, hr = _world(n_people, cells, latent, infectious)
+    whole, single = sim.Simulation(pop, P, lk, hr), sim.Simulation(pop, P, lk, hr)
+    orac = sim.Simulation(pop, P, lk, hr, backend=oracle_py.OracleBackend)
+    seeds = whole.choose_seeds(5, n_seed)
+    for s in (whole, single, orac):
+        s.backend.begin_run(5, seeds)
+    for k in range(48):
+        t = k * P.ModelTimeStep
+        if k in (16, 24):   # the false-positive path, and back
+            for s in (whole, single, orac):
+                q = abi.cs_params.from_buffer_copy(P)
+                q.FalsePositiveRate = 0.2 if k == 16 else 0.0
+                s.backend.set_params(q)
+        if k % 7 == 6:      # whole timesteps and single sweeps of one context in turn
+            whole.backend.infect_sweep(t, 0)
+            whole.backend.incub_recovery_sweep(t)
+        else:
+            whole.backend.step(t, 0)
+        for s in (single, orac):
+            s.backend.infect_sweep(t, 0)
+            s.backend.incub_recovery_sweep(t)
+        if k == 30:
+            for s in (whole, single, orac):
+                s.backend.seed_infections(t, np.arange(0, n_people, 50, dtype=np.int32))
+        if k % 5 == 0 or k in (16, 17, 24, 30, 31, 47):
+            b = snapshot(orac.backend, pop)
+            _same(snapshot(whole.backend, pop), b, "step %d" % k)
+            _same(snapshot(single.backend, pop), b, "sweeps %d" % k)
+    check_lists(b, pop)
+    cs = [abi.counters_to_dict(s.backend.counters()) for s in (whole, single, orac)]
+    assert cs[0] == cs[1]
+    # the mid-run seeding names people already infected; the oracle measures radii from the
+    # last person named, the library from the last one it infects
+    for k in set(cs[0]) - {"sumRad2_q", "maxRad2_bits"}:
+        assert cs[0][k] == cs[2][k], k
+    for s in (whole, single, orac):
+        s.close()
