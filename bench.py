@@ -171,9 +171,9 @@ def kernel_bytes(name, w, n_cells_steps):
     the next-event time -- and 16 B per cell, infector record 40 B, household member 12 B, place candidate 20 B, spatial
     draw 33 B, accepted infection 24 B, infector-list entry 12 B, per-cell counts
     16 B)."""
-    if name == "k_infector_hh_spatial":
+    if name == "k_household":
         return 40 * w["work_infectors"] + 12 * w["work_hh_members"]
-    if name == "k_infector_places":
+    if name == "k_places":
         return 20 * w["work_place_candidates"] + 16 * w["work_infectors"]
     if name == "k_spatial":
         return 33 * w["work_spatial_draws"]

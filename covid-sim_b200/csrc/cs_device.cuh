@@ -7,6 +7,7 @@
 // (population, parameters, seed) alone.
 #pragma once
 
+#include <cstddef>
 #include <cstdint>
 #include <cuda_runtime.h>
 
@@ -41,27 +42,30 @@ __device__ __forceinline__ void philox4x32_10(uint32_t k0, uint32_t k1, uint32_t
 }
 
 // One counter-based stream: {block, entity, ts | purpose << 16, sub} under the run key.
+// A block gives two uniforms; the second waits in a register (not in an array indexed by a
+// counter, which would live in local memory).
 struct Stream {
     uint32_t k0, k1, c1, c2, c3, block;
-    double buf[2];
-    int idx;
+    double hold;
+    bool have;
 
     __device__ __forceinline__ Stream(uint64_t seed, int purpose, uint32_t ts, uint32_t entity, uint32_t sub)
         : k0((uint32_t)seed), k1((uint32_t)(seed >> 32)), c1(entity),
-          c2((ts & 0xffffu) | ((uint32_t)purpose << 16)), c3(sub), block(0), idx(2) {}
+          c2((ts & 0xffffu) | ((uint32_t)purpose << 16)), c3(sub), block(0), hold(0.0), have(false) {}
 
     __device__ __forceinline__ double next()
     {
-        if (idx >= 2) {
-            uint32_t x[4];
-            philox4x32_10(k0, k1, block++, c1, c2, c3, x);
-            uint64_t a = ((uint64_t)x[1] << 32) | x[0];
-            uint64_t b = ((uint64_t)x[3] << 32) | x[2];
-            buf[0] = (double)(a >> 11) * (1.0 / 9007199254740992.0);
-            buf[1] = (double)(b >> 11) * (1.0 / 9007199254740992.0);
-            idx = 0;
+        if (have) {
+            have = false;
+            return hold;
         }
-        return buf[idx++];
+        uint32_t x[4];
+        philox4x32_10(k0, k1, block++, c1, c2, c3, x);
+        uint64_t a = ((uint64_t)x[1] << 32) | x[0];
+        uint64_t b = ((uint64_t)x[3] << 32) | x[2];
+        hold = (double)(b >> 11) * (1.0 / 9007199254740992.0);
+        have = true;
+        return (double)(a >> 11) * (1.0 / 9007199254740992.0);
     }
 };
 
@@ -74,6 +78,9 @@ __device__ inline int32_t sample_poisson(Stream& s, double lambda, unsigned long
     if (!(lambda > 0)) return 0;
     if (lambda < 10.0) {
         double u = s.next();
+        // exp(-lambda) >= 1 - lambda: most draws of a small mean end here without it (the
+        // margin covers the rounding of both sides)
+        if (u < 1.0 - lambda - 1e-12) return 0;
         double p = exp(-lambda), F = p;
         int32_t k = 0;
         while (u > F && k < kMaxLoop) {
@@ -239,16 +246,14 @@ __device__ __forceinline__ double periodic_xy(const cs_params& P, double x, doub
     return x * x + y * y;
 }
 
-// dist2(Person*, Person*) (src/Dist.cpp:49-61) between two households.
-__device__ __forceinline__ double dist2_hh(const DevPop& d, const cs_params& P, int32_t ha, int32_t hb)
+// dist2(Person*, Person*) (src/Dist.cpp:49-61) between two households' locations.
+__device__ __forceinline__ double dist2_xy(const cs_params& P, float2 a, float2 b)
 {
-    float2 a = __ldg(reinterpret_cast<const float2*>(d.hhr + ha));
-    float2 b = __ldg(reinterpret_cast<const float2*>(d.hhr + hb));
-    float ax = a.x, ay = a.y, bx = b.x, by = b.y;
-    if (P.DoUTM_coords) return dist2_utm(P, ax, ay, bx, by);
-    float dx = ax - bx, dy = ay - by;
+    if (P.DoUTM_coords) return dist2_utm(P, a.x, a.y, b.x, b.y);
+    float dx = a.x - b.x, dy = a.y - b.y;
     return periodic_xy(P, fabs(dx), fabs(dy));
 }
+__device__ __forceinline__ float2 person_xy(const DevPop& d, int32_t p) { return __ldg(d.pxy + p); }
 
 // dist2_raw (src/Dist.cpp:163-170), in double from float locations: from a
 // household to a point (a place), and between two households.
@@ -405,6 +410,13 @@ __device__ __forceinline__ PersonLinks load_links(const DevPop& d, int p)
     reinterpret_cast<int4*>(&r)[1] = b;
     return r;
 }
+__device__ __forceinline__ PlaceRec load_place(const DevPop& d, int pt, int l)
+{
+    int4 a = __ldg(reinterpret_cast<const int4*>(d.pl[pt].rec + l));
+    PlaceRec r;
+    reinterpret_cast<int4*>(&r)[0] = a;
+    return r;
+}
 __device__ __forceinline__ HouseholdRec load_household(const DevPop& d, int h)
 {
     int4 a = __ldg(reinterpret_cast<const int4*>(d.hhr + h));
@@ -413,14 +425,32 @@ __device__ __forceinline__ HouseholdRec load_household(const DevPop& d, int h)
     return r;
 }
 
+// ------------------------------------------------- parameters in shared memory
+// A block's copy of the parameters its people's products read: everything before the
+// geometry but the tail of the infectiousness profile (kProfileStaged steps are kept; a
+// later step reads the parameter block itself).  A person's chain touches dozens of these
+// fields one after the other, each a first-touch miss to L2 when read in place; the copy
+// is one round trip for all.  The geometry (distance tables, kernel table scale) stays in
+// global memory.
+constexpr int kProfileStaged = 256;
+constexpr size_t kParamsHead = 2272, kParamsMid = 20608, kParamsEnd = 31280;   // staged: [0, head) and [mid, end)
+static_assert(kParamsHead >= offsetof(cs_params, infectiousness) + kProfileStaged * sizeof(double) && kParamsHead % 16 == 0, "staged range");
+static_assert(kParamsMid <= offsetof(cs_params, PlaceTypeTrans) && kParamsMid % 16 == 0, "staged range");
+static_assert(kParamsEnd >= offsetof(cs_params, sinx) && kParamsEnd % 16 == 0, "staged range");
+
+__device__ __forceinline__ double profile_at(const cs_params& P, const cs_params* Pg, int k)
+{
+    return k < kProfileStaged ? P.infectiousness[k] : Pg->infectiousness[k];
+}
+
 // --------------------------------------- CalcInfSusc (src/CalcInfSusc.cpp)
 // Factors that are exactly 1.0 here (digital contact tracing, treatment,
 // vaccination) are left out; multiplying by 1.0 is exact.
-__device__ __forceinline__ double calc_person_inf(const PersonHot& h, const cs_params& P, int ts)
+__device__ __forceinline__ double calc_person_inf(const DevPop& d, const PersonHot& h, const cs_params& P, int ts)
 {
-    return fabs(h.infness) * P.infectiousness[ts - h.latent_time - 1];
+    return fabs(h.infness) * profile_at(P, d.P, ts - h.latent_time - 1);
 }
-__device__ __forceinline__ double calc_house_inf(const PersonHot& h, uint16_t nhr, const cs_params& P, int ts)
+__device__ __forceinline__ double calc_house_inf(const DevPop& d, const PersonHot& h, uint16_t nhr, const cs_params& P, int ts)
 {
     bool iso = host_isolated(h, P, ts);
     double infn = P.NoInfectiousnessSDinHH ? ((h.infness < 0) ? P.SymptInfectiousness : P.AsymptInfectiousness) : fabs(h.infness);
@@ -429,24 +459,24 @@ __device__ __forceinline__ double calc_house_inf(const PersonHot& h, uint16_t nh
         * P.HouseholdDenomLookup[nhr - 1]
         * (is_ch(h) ? P.CareHomeResidentHouseholdScaling : 1.0)
         * infn
-        * P.infectiousness[ts - h.latent_time - 1];
+        * profile_at(P, d.P, ts - h.latent_time - 1);
 }
-__device__ __forceinline__ double calc_place_inf(const PersonHot& h, const cs_params& P, int pt, int ts)
+__device__ __forceinline__ double calc_place_inf(const DevPop& d, const PersonHot& h, const cs_params& P, int pt, int ts)
 {
     bool iso = host_isolated(h, P, ts), ch = is_ch(h);
     return (iso ? P.Efficacies[CS_NPI_CASE_ISOLATION][pt] : 1.0)
         * ((host_quarantined(h, P, ts) && !ch && !iso) ? P.Efficacies[CS_NPI_HOME_QUARANTINE][pt] : 1.0)
         * ((h.inf == CS_INF_CASE && !ch) ? P.SymptPlaceTypeContactRate[pt] : 1.0)
-        * P.PlaceTypeTrans[pt] / P.PlaceTypeGroupSizeParam1[pt] * calc_person_inf(h, P, ts);
+        * P.PlaceTypeTrans[pt] / P.PlaceTypeGroupSizeParam1[pt] * calc_person_inf(d, h, P, ts);
 }
-__device__ __forceinline__ double calc_spatial_inf(const PersonHot& h, const cs_params& P, int ts)
+__device__ __forceinline__ double calc_spatial_inf(const DevPop& d, const PersonHot& h, const cs_params& P, int ts)
 {
     bool iso = host_isolated(h, P, ts), ch = is_ch(h);
     return (iso ? P.Efficacies[CS_NPI_CASE_ISOLATION][CS_SETTING_SPATIAL] : 1.0)
         * ((host_quarantined(h, P, ts) && !ch && !iso) ? P.Efficacies[CS_NPI_HOME_QUARANTINE][CS_SETTING_SPATIAL] : 1.0)
         * ((h.inf == CS_INF_CASE) ? P.SymptSpatialContactRate : 1.0)
         * P.RelativeSpatialContact[age_group(h)]
-        * calc_person_inf(h, P, ts);
+        * calc_person_inf(d, h, P, ts);
 }
 __device__ __forceinline__ double calc_person_susc(const PersonHot& h, int infector_age_group, const cs_params& P)
 {
@@ -455,7 +485,7 @@ __device__ __forceinline__ double calc_person_susc(const PersonHot& h, int infec
 }
 __device__ __forceinline__ double socdist_factor(const DevPop& d, const PersonHot& h, const cs_params& P, int setting)
 {
-    if (d.socdist[h.mcell] != CS_TREAT_TREATED) return 1.0;
+    if (!d.status_any[kAnySocdist] || d.socdist[h.mcell] != CS_TREAT_TREATED) return 1.0;
     return (h.pflags & CS_PF_ESOCDIST_COMPLY) ? P.Efficacies[CS_NPI_ENHANCED_SOCIAL_DISTANCING][setting]
                                              : P.Efficacies[CS_NPI_SOCIAL_DISTANCING][setting];
 }
@@ -477,6 +507,7 @@ __device__ __forceinline__ double calc_spatial_susc(const DevPop& d, const Perso
 }
 __device__ __forceinline__ bool moverest_differs(const DevPop& d, int ma, int mb)
 {
+    if (!d.status_any[kAnyMoverest]) return false;
     uint8_t a = d.moverest[ma], b = d.moverest[mb];
     return a != b && (a == CS_TREAT_TREATED || b == CS_TREAT_TREATED);
 }

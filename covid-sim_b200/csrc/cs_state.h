@@ -64,8 +64,16 @@ struct __align__(16) BlockInfo {
     int32_t kb, ke;
 };
 
+// A place: where its members start, how many it has, its first group, its microcell; and a
+// group: its first member within the place and its size (one load each).
+struct __align__(16) PlaceRec {
+    int32_t member_ofs, n, group_ofs, mcell;
+};
+
 struct DevPlaces {
     int32_t n;
+    const PlaceRec* rec;       // the next four arrays' entries of a place, together
+    const int2* group;         // (group_start, group_size)
     const int32_t* mcell;
     const int32_t* member_ofs;
     const int32_t* members;
@@ -108,6 +116,7 @@ struct DevPop {
     PersonHot* hot;
     const PersonLinks* links;  // [N]
     const HouseholdRec* hhr;   // [NH]
+    const float2* pxy;         // [N] the person's household's location, for the spatial draws (no detour by the record)
     const int32_t* mcell_cell;
     const int32_t* mcell_adunit;
     const int32_t* cell_grid;
@@ -152,6 +161,7 @@ struct DevPop {
     // microcells
     uint8_t* socdist;
     uint8_t* moverest;
+    int32_t* status_any;       // [2] kAnySocdist, kAnyMoverest: 0 while every microcell's status is 0
     DevIv* iv;
     DevStep* step;
     const unsigned long long* seed_src;  // the run's seed, written by begin_run / upload_state
@@ -185,11 +195,6 @@ struct DevPop {
     int2* events;              // [N] the step's transitions (person, cell): latent people from the front, infectious from the back
     int32_t* cnt_s;            // [NC] the step's S -> L moves per cell (zero between steps)
     int32_t* cnt;              // [NC] L -> I (low 16 bits) and I -> R/D (high) moves per cell
-    int32_t* cnt_ofs;          // [N] first contact-map entry of each active infector
-    int32_t* cmap;             // [2N] active-list index of the infector owning each spatial contact
-    int32_t cmap_cap;
-    uint8_t* act_closed;       // [N] infector's place-closed-and-absent flag
-    int2* place_work;          // [N * NPT] (active index << 3 | place type, place) of each place pass
     uint8_t* hh_flag;          // [NH] deferred household actions
     int32_t* hh_list;          // [NH]
     // households a place closure sends an adult home to (the host closure queue of
@@ -209,7 +214,8 @@ struct DevPop {
 // `events`: latent people from the front (kCntEvents), infectious people from the
 // back (kCntEventsInf), so that a warp of the transition kernel mostly takes one
 // branch.
-enum { kCntQueue = 0, kCntTouched = 1, kCntAct = 2, kCntContacts = 3, kCntPlaceWork = 4, kCntEvents = 5,
-       kCntCarer = 6, kCntFalse = 7, kCntEventsInf = 8, kCntHH = 9, kCntN = 10 };
+enum { kCntQueue = 0, kCntTouched = 1, kCntAct = 2, kCntContacts = 3, kCntEvents = 4,
+       kCntCarer = 5, kCntFalse = 6, kCntEventsInf = 7, kCntHH = 8, kCntN = 9 };
+enum { kAnySocdist = 0, kAnyMoverest = 1 };
 
 }  // namespace csb

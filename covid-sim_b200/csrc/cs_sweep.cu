@@ -10,11 +10,10 @@
 //     k_set_step             the step's scalars        beside
 //     k_scan                 the infectious people, and the people with a transition this
 //                            step, of every cell: two lists
-//     k_infector_hh_spatial  household pass and spatial Poisson count per infector;
-//                            reserves each infector's entries of the contact map
-//     k_infector_places      place passes, one thread per (infector, place type), beside
-//     k_spatial              spatial contacts: block proposal + rejection, several
-//                            draws of a contact evaluated together
+//     k_household            household pass per infector, beside
+//     k_places               place passes per infector, beside
+//     k_spatial              spatial contacts per infector: block proposal + rejection,
+//                            several draws of a contact evaluated together
 //     k_infections           DoInfect for every claimed person (lowest key wins), beside
 //     k_onsets               DoIncub, beside
 //     k_progress             DoCase / severity / recovery / death per person
@@ -254,6 +253,7 @@ struct cs_gpu_ctx {
     bool run_started = false;
     bool lists_stale = false;   // the last timestep left its touched-cell and household lists for the next scan to empty
     int grid = 148 * 8;
+    int nsm = 148;
     int spatial_lanes = 8;   // lanes per spatial contact (2, 4, 8 or 16)
     // one timestep captured as a CUDA graph and replayed
     bool use_graph = true;
@@ -1397,6 +1397,73 @@ __global__ void __launch_bounds__(kThreads) k_scan(DevPop d, double t) { k_scan_
 template <bool kActive, bool kEvents>
 __global__ void __launch_bounds__(kThreads) k_scan_multi(const DevPop* __restrict__ pops) { k_scan_body<kActive, kEvents>(pops[blockIdx.y], 0.0); }
 
+// The block's staged parameters (see kParamsHead): copied by every thread, ready after the
+// call.
+struct __align__(16) StagedParams {
+    unsigned char b[kParamsEnd];
+    // the bytes between the two staged ranges, free for the kernel's own use
+    template <typename T>
+    __device__ __forceinline__ T* spare()
+    {
+        static_assert(sizeof(T) <= kParamsMid - kParamsHead, "fits the gap");
+        return reinterpret_cast<T*>(b + kParamsHead);
+    }
+};
+__device__ __forceinline__ const cs_params& stage_params(StagedParams& sp, const cs_params* Pg)
+{
+    const unsigned char* src = reinterpret_cast<const unsigned char*>(Pg);
+    auto copy = [&](size_t o) {
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" :: "r"((uint32_t)__cvta_generic_to_shared(sp.b + o)), "l"(src + o) : "memory");
+    };
+    for (size_t o = 16 * threadIdx.x; o < kParamsHead; o += 16 * blockDim.x) copy(o);
+    for (size_t o = kParamsMid + 16 * threadIdx.x; o < kParamsEnd; o += 16 * blockDim.x) copy(o);
+    asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
+    __syncthreads();
+    return *reinterpret_cast<const cs_params*>(sp.b);
+}
+
+// How a launch of warps takes a list of n items: `per` items a warp at a time, group g of
+// them by warp g / blocks of block g % blocks.  With few items a launch lasts as long as one
+// item's chain of dependent loads and double-precision draws, and lanes that take different
+// branches of it add theirs up, so while there are fewer items than schedulers (148 SMs
+// of four; shared by a batch's members) each gets a warp of its own, on as many SMs as there
+// are groups.  With many, whole warps in whole blocks: every warp and block adds its
+// tallies to the same few counters at its end.
+struct Groups {
+    int n, per, blocks;
+    __device__ __forceinline__ explicit Groups(int items) : n(items)
+    {
+        const int slots = 592 / (int)gridDim.y, wpb = blockDim.x >> 5;
+        per = max(1, min(32, n / max(1, slots)));
+        const int groups = (n + per - 1) / per;
+        blocks = max(1, min((int)gridDim.x, max(min(groups, 148), (groups + wpb - 1) / wpb)));
+    }
+    __device__ __forceinline__ bool idle_block() const { return (int)blockIdx.x >= blocks || (long long)blockIdx.x * per >= n; }
+    // f(item) for every item of the calling thread; all lanes of a warp make the same calls
+    template <typename F>
+    __device__ __forceinline__ void each(F f) const
+    {
+        const int lane = threadIdx.x & 31;
+        if ((int)blockIdx.x >= blocks) return;
+        for (long long g = blockIdx.x + (long long)blocks * (threadIdx.x >> 5); g * per < n; g += (long long)blocks * (blockDim.x >> 5)) {
+            const long long e = g * per + lane;
+            if (lane < per && e < n) f((int)e);
+        }
+    }
+    // the calling thread's warp's groups, one after the other, and its lane's item of one (-1 for none)
+    __device__ __forceinline__ long long first() const
+    {
+        return (int)blockIdx.x < blocks ? blockIdx.x + (long long)blocks * (threadIdx.x >> 5) : (long long)n;
+    }
+    __device__ __forceinline__ bool more(long long g) const { return g * per < n; }
+    __device__ __forceinline__ long long next(long long g) const { return g + (long long)blocks * (blockDim.x >> 5); }
+    __device__ __forceinline__ int item(long long g) const
+    {
+        const long long e = g * per + (threadIdx.x & 31);
+        return (int)(threadIdx.x & 31) < per && e < n ? (int)e : -1;
+    }
+};
+
 // =============================================================== InfectSweep
 // AddInfections (src/Sweep.cpp:2031-2065): with probability FalsePositiveRate the
 // entry is a false positive (DoFalseCase for the person) instead of an infection.
@@ -1418,28 +1485,115 @@ __device__ __forceinline__ void claim_infection(const DevPop& d, const cs_params
     if (old == ~0ull) d.queue[append(d.counts + kCntQueue)] = person;
 }
 
-// Geometric-skip enumeration of the Bernoulli(p) trials over a member list
-// (equivalent to the reference's Binomial count + sample without replacement,
-// src/Sweep.cpp:463-470 and 563-566).
-__device__ void place_candidates(const DevPop& d, const cs_params& P, const StepScalars& st, int i, const PersonHot& hi,
-                                 int pt, int link, double p, bool between, uint64_t seed)
+// The infectors' three passes run side by side, each from the infector list alone: an
+// infector's household contacts, its contacts at the places it attends and its spatial
+// contacts depend on its record and its own random streams, and meet only in the claims
+// (atomicMin on the claim key) and the tallies.  (A household pass that also listed the
+// infectors' places and spatial contacts for two later kernels cost a launch and three
+// lists more: 11.8 us, then 10.9 beside 9.3, with hardly anyone infected; 13, 10 and 8 side
+// by side now.)
+
+// Household pass (src/Sweep.cpp:331-377), one thread per infector.  Bound: the members'
+// records (32 B each, contiguous), behind three dependent loads.  All members' states are
+// read before the first is acted on.
+__device__ __forceinline__ void k_household_body(const DevPop& d)
 {
+    __shared__ StagedParams sp;
+    const int nact = d.counts[kCntAct];
+    const StepScalars st = *d.step;
+    const Groups work(nact);
+    if (work.idle_block() || !(st.hh_beta > 0)) return;
+    const cs_params& P = stage_params(sp, d.P);
+    const bool anyc = closures_possible(d, st.ts);
+    long long hh_members = 0;
+    work.each([&](int idx) {
+        const int i = d.act[idx].x;
+        const PersonHot hi = d.hot[i];
+        const HouseholdRec hr = load_household(d, hi.hh);
+        const int nh = hr.nh;
+        if (nh <= 1) return;
+        const int f0 = hr.first, f1 = f0 + nh;
+        hh_members += nh;
+        unsigned susc = 0;   // members who are susceptible (a household has at most CS_MAX_HOUSEHOLD_SIZE; more are read below)
+        const int nfast = min(nh, 32);
+        for (int m = 0; m < nfast; m += 4) {
+            int8_t v[4];
+#pragma unroll
+            for (int u = 0; u < 4; u++) v[u] = m + u < nfast ? d.hot[f0 + m + u].inf : (int8_t)CS_INF_IMMUNE_AT_START;
+#pragma unroll
+            for (int u = 0; u < 4; u++) susc |= (v[u] == CS_INF_SUSCEPTIBLE ? 1u : 0u) << ((m + u) & 31);
+        }
+        if (!susc && nh <= 32) return;   // the pass draws for susceptible members only
+        double HI = st.hh_beta * calc_house_inf(d, hi, hr.nhr, P, st.ts);
+        bool absent = false;
+        for (int m = f0; anyc && (m < f1) && (!absent); m++) {
+            // a member counts only when absent: its places are read only then
+            if (!host_absent(d.hot[m], st.ts)) continue;
+            for (int pt = 0; (pt < d.NPT) && (!absent); pt++) {
+                int lk = link_of(d, pt, m);
+                if (lk >= 0) absent = place_closed(d, pt, lk, st.ts);
+            }
+        }
+        if (absent) HI *= P.Efficacies[CS_NPI_PLACE_CLOSURE][CS_SETTING_HOUSE];
+        const int iag = age_group(hi);
+        Stream s(st.seed, CS_RNG_HOUSEHOLD, (uint32_t)st.ts, (uint32_t)i, 0);
+        for (int m = f0; m < f1; m++) {
+            if (m - f0 < 32 && !(susc >> (m - f0) & 1u)) continue;
+            const PersonHot hm = d.hot[m];
+            if (hm.inf == CS_INF_SUSCEPTIBLE) {
+                double foi = HI * calc_house_susc(d, hm, iag, P);
+                if (s.next() < foi) claim_infection(d, P, st, m, i, 1);
+            }
+        }
+    });
+    __syncwarp();
+    cnt_add_warp(CSB_CTR(work_hh_members), hh_members);
+}
+__global__ void __launch_bounds__(kThreads) k_household(DevPop d) { k_household_body(d); }
+__global__ void __launch_bounds__(kThreads) k_household_multi(const DevPop* __restrict__ pops) { k_household_body(pops[blockIdx.y]); }
+
+// Place passes (src/Sweep.cpp:379-647): the Bernoulli(p) trials over the members of an
+// infector's group and of its whole place, enumerated by geometric skips (equivalent to
+// the reference's Binomial count + sample without replacement, :463-470 and 563-566).
+//
+// All but about n * p of the passes end with their first skip, past the whole list; as
+// log(u) / log(1 - p) >= n whenever u <= 1 - n * p, those need no logarithm (the margin in
+// the test covers the rounding of both sides).  A lane tests its infector's passes; the few
+// that go on are queued by the warp and enumerated 32 at a time, so that the long path
+// (logarithms, members, their records, claims) runs in full warps rather than for one or
+// two lanes of almost every warp.
+struct PlaceQueue {
+    static constexpr int kCap = 64;
+    double p[kCap];
+    int i[kCap], link[kCap];
+    unsigned meta[kCap];   // place type, between groups << 3, care-home infector << 4, age group << 5, group << 16
+};
+
+__device__ __forceinline__ bool place_pass_goes_on(const StepScalars& st, int i, int pt, int n, double p, bool between)
+{
+    if (p <= 0 || n <= 0) return false;
+    if (p >= 1.0) return true;
+    Stream s(st.seed, between ? CS_RNG_PLACE_BETWEEN : CS_RNG_PLACE_GROUP, (uint32_t)st.ts, (uint32_t)i, (uint32_t)pt);
+    return !(s.next() < 1.0 - (double)n * p - 1e-9);
+}
+
+// One queued pass.
+__device__ __forceinline__ long long place_candidates(const DevPop& d, const cs_params& P, const StepScalars& st, int i,
+                                                      int link, unsigned meta, double p)
+{
+    const int pt = meta & 7u, gi = (int)(meta >> 16), iag = (int)(meta >> 5 & 0x7ffu);
+    const bool between = meta >> 3 & 1u, ich = meta >> 4 & 1u;
     const DevPlaces& pl = d.pl[pt];
-    int base = pl.member_ofs[link], n;
-    int gi = group_of(d, pt, i);
+    const PlaceRec rec = load_place(d, pt, link);
+    int base = rec.member_ofs, n = rec.n;
     if (!between) {
-        int g = pl.group_ofs[link] + gi;
-        base += pl.group_start[g];
-        n = pl.group_size[g];
-    } else
-        n = pl.member_ofs[link + 1] - pl.member_ofs[link];
-    if (p <= 0 || n <= 0) return;
-    int mc_place = pl.mcell[link];
-    Stream s(seed, between ? CS_RNG_PLACE_BETWEEN : CS_RNG_PLACE_GROUP, (uint32_t)st.ts, (uint32_t)i, (uint32_t)pt);
+        const int2 g = __ldg(pl.group + rec.group_ofs + gi);
+        base += g.x;
+        n = g.y;
+    }
+    Stream s(st.seed, between ? CS_RNG_PLACE_BETWEEN : CS_RNG_PLACE_GROUP, (uint32_t)st.ts, (uint32_t)i, (uint32_t)pt);
     double logq = (p < 1.0) ? log1p(-p) : 0.0;
     double pos = -1.0;
-    int iag = age_group(hi);
-    bool ich = is_ch(hi);
     long long ncand = 0;
     for (;;) {
         if (p >= 1.0) pos = pos + 1.0;
@@ -1456,159 +1610,148 @@ __device__ void place_candidates(const DevPop& d, const cs_params& P, const Step
             if ((pt == P.CareHomePlaceType) && ((!ich) || (!is_ch(hm)))) sc *= P.CareHomeWorkerGroupScaling;
             sc *= calc_person_susc(hm, iag, P) * p / p;
             if (st.blanket) {
-                if (dist2_hh_pt(d, P, hm.hh, pl.x[link], pl.y[link]) > P.MoveRestrRadius2) sc *= P.MoveRestrEffect;
-            } else if (moverest_differs(d, hm.mcell, mc_place))
+                if (dist2_hh_pt(d, *d.P, hm.hh, pl.x[link], pl.y[link]) > P.MoveRestrRadius2) sc *= P.MoveRestrEffect;
+            } else if (moverest_differs(d, hm.mcell, rec.mcell))
                 sc *= P.MoveRestrEffect;
             if ((sc == 1) || (s.next() < sc)) claim_infection(d, P, st, m, i, between ? 2 + pt + CS_MAX_PLACE_TYPES : 2 + pt);
         }
     }
+    return ncand;
+}
+
+__device__ __forceinline__ void k_places_body(const DevPop& d)
+{
+    __shared__ StagedParams sp;
+    struct Queues { PlaceQueue q[kThreads / 32]; };
+    const int nact = d.counts[kCntAct];
+    const Groups work(nact);
+    if (work.idle_block()) return;
+    const cs_params& P = stage_params(sp, d.P);
+    if (!P.DoPlaces) return;
+    const StepScalars st = *d.step;
+    const int lane = threadIdx.x & 31;
+    PlaceQueue& Q = sp.spare<Queues>()->q[threadIdx.x >> 5];
+    int nq = 0;
+    long long ncand = 0;
+    auto drain = [&](int keep) {   // enumerate queued passes while more than `keep` wait
+        while (nq > keep) {
+            __syncwarp();
+            const int take = min(nq, 32);
+            nq -= take;   // the last ones in
+            if (lane < take) ncand += place_candidates(d, P, st, Q.i[nq + lane], Q.link[nq + lane], Q.meta[nq + lane], Q.p[nq + lane]);
+            __syncwarp();
+        }
+    };
+    auto push = [&](bool on, int i, int link, unsigned meta, double p) {
+        const unsigned m = __ballot_sync(0xffffffffu, on);
+        if (on) {
+            const int at = nq + __popc(m & ((1u << lane) - 1u));
+            Q.p[at] = p;
+            Q.i[at] = i;
+            Q.link[at] = link;
+            Q.meta[at] = meta;
+        }
+        nq += __popc(m);
+        drain(31);
+    };
+    for (long long g = work.first(); work.more(g); g = work.next(g)) {
+        const int idx = work.item(g);
+        int i = 0;
+        PersonHot hi;
+        PersonLinks pli;
+        bool out = idx >= 0;
+        if (out) {
+            i = d.act[idx].x;
+            hi = d.hot[i];
+            pli = load_links(d, i);
+            out = !host_absent(hi, st.ts);
+        }
+        for (int pt = 0;;) {   // the n-th place of every lane's infector, whatever its type
+            int link = -1, gi = 0;
+            if (out) {
+#pragma unroll
+                for (int q = 0; q < CS_MAX_PLACE_TYPES; q++)
+                    if (link < 0 && q >= pt && q < d.NPT && pli.link[q] >= 0) { link = pli.link[q]; gi = pli.group[q]; pt = q; }
+            }
+            if (!__any_sync(0xffffffffu, link >= 0)) break;
+            double p1 = 0.0, p2 = 0.0;
+            bool on1 = false, on2 = false;
+            unsigned meta = 0;
+            if (link >= 0) {
+                const PlaceRec rec = load_place(d, pt, link);
+                const bool within = pt != P.HotelPlaceType;
+                const int ng = within ? __ldg(d.pl[pt].group + rec.group_ofs + gi).y : 0;
+                double PI = st.fp * st.seas * calc_place_inf(d, hi, P, pt, st.ts);
+                if (st.blanket) {
+                    if (dist2_hh_pt(d, *d.P, hi.hh, d.pl[pt].x[link], d.pl[pt].y[link]) > P.MoveRestrRadius2)
+                        PI *= P.MoveRestrEffect;
+                } else if (moverest_differs(d, hi.mcell, rec.mcell))
+                    PI *= P.MoveRestrEffect;
+                p1 = PI;
+                if (p1 > 1) p1 = 1;
+                on1 = within && place_pass_goes_on(st, i, pt, ng, p1, false);
+                p2 = PI * (P.PlaceTypePropBetweenGroupLinks[pt] * P.PlaceTypeGroupSizeParam1[pt] / ((double)rec.n));
+                if (p2 > 1) p2 = 1;
+                on2 = place_pass_goes_on(st, i, pt, rec.n, p2, true);
+                meta = (unsigned)pt | (is_ch(hi) ? 16u : 0u) | (unsigned)age_group(hi) << 5 | (unsigned)gi << 16;
+            }
+            push(on1, i, link, meta, p1);
+            push(on2, i, link, meta | 8u, p2);
+            pt++;
+        }
+    }
+    drain(0);
+    __syncwarp();
     cnt_add_warp(CSB_CTR(work_place_candidates), ncand);
 }
+__global__ void __launch_bounds__(kThreads, 3) k_places(DevPop d) { k_places_body(d); }
+__global__ void __launch_bounds__(kThreads, 3) k_places_multi(const DevPop* __restrict__ pops) { k_places_body(pops[blockIdx.y]); }
 
-// Household pass and spatial Poisson count of one infector (src/Sweep.cpp:331-377,
-// 656-698); one thread per infector.
-__device__ __forceinline__ void k_infector_hh_spatial_body(const DevPop& d)
-{
-    const cs_params& P = *d.P;
-    const StepScalars st = *d.step;
-    const uint64_t seed = st.seed;
-    int nact = d.counts[kCntAct];
-    const bool anyc = closures_possible(d, st.ts);
-    long long hh_members = 0;
-    // block-uniform loop: every thread takes part in the list reservations
-    for (int base = blockIdx.x * blockDim.x; base < nact; base += gridDim.x * blockDim.x) {
-        const int idx = base + threadIdx.x;
-        int links[CS_MAX_PLACE_TYPES];
-        int nwork = 0, k = 0;
-        uint8_t closed_i = 0;
-        bool absent_i = true;
-        if (idx < nact) {
-            const int2 ac = d.act[idx];
-            const int i = ac.x, ci = ac.y;
-            PersonHot hi = d.hot[i];
-            int h = hi.hh;
-            int iag = age_group(hi);
-            const HouseholdRec hr = load_household(d, h);
-            uint16_t nh = hr.nh;
-            if (st.hh_beta > 0 && nh > 1) {
-                int f0 = hr.first, f1 = f0 + nh;
-                double HI = st.hh_beta * calc_house_inf(hi, hr.nhr, P, st.ts);
-                bool absent = false;
-                for (int m = f0; anyc && (m < f1) && (!absent); m++) {
-                    // a member counts only when absent: its places are read only then
-                    if (!host_absent(d.hot[m], st.ts)) continue;
-                    for (int pt = 0; (pt < d.NPT) && (!absent); pt++) {
-                        int lk = link_of(d, pt, m);
-                        if (lk >= 0) absent = place_closed(d, pt, lk, st.ts);
-                    }
-                }
-                if (absent) HI *= P.Efficacies[CS_NPI_PLACE_CLOSURE][CS_SETTING_HOUSE];
-                Stream s(seed, CS_RNG_HOUSEHOLD, (uint32_t)st.ts, (uint32_t)i, 0);
-                for (int m = f0; m < f1; m++) {
-                    hh_members++;
-                    PersonHot hm = d.hot[m];
-                    if (hm.inf == CS_INF_SUSCEPTIBLE) {
-                        double foi = HI * calc_house_susc(d, hm, iag, P);
-                        if (s.next() < foi) claim_infection(d, P, st, m, i, 1);
-                    }
-                }
-            }
-            // the infector's place passes: one work entry per place it attends today
-            absent_i = host_absent(hi, st.ts);
-            const PersonLinks pli = load_links(d, i);
-            for (int pt = 0; pt < d.NPT; pt++) {
-                links[pt] = P.DoPlaces ? pli.link[pt] : -1;
-                if (links[pt] >= 0 && !absent_i) nwork++;
-            }
-            if (st.sp_beta > 0) {
-                double si = calc_spatial_inf(hi, P, st.ts);
-                bool closed = false;   // counts only for an absent infector
-                for (int pt = 0; anyc && absent_i && (pt < d.NPT) && (!closed); pt++)
-                    if (links[pt] >= 0) closed = place_closed(d, pt, links[pt], st.ts);
-                if (closed && absent_i) { si *= P.Efficacies[CS_NPI_PLACE_CLOSURE][CS_SETTING_SPATIAL]; closed_i = 1; }
-                double lambda = si * st.sp_beta * d.tot_prob[ci];
-                Stream s(seed, CS_RNG_SPATIAL_COUNT, (uint32_t)st.ts, (uint32_t)i, 0);
-                k = sample_poisson(s, lambda, CSB_CTR(err_spatial_tries));
-            }
-        }
-        // place-work entries [ow, ow + nwork) and contact-map entries [oc, oc + k)
-        const int2 o = block_reserve2(d.counts + kCntPlaceWork, nwork, d.counts + kCntContacts, k);
-        if (idx < nact) {
-            int ow = o.x;
-            for (int pt = 0; pt < d.NPT; pt++)
-                if (links[pt] >= 0 && !absent_i) d.place_work[ow++] = make_int2((idx << 3) | pt, links[pt]);
-            d.cnt_ofs[idx] = o.y;
-            for (int jj = 0; jj < k && o.y + jj < d.cmap_cap; jj++) d.cmap[o.y + jj] = idx;
-            d.act_closed[idx] = closed_i;
-        }
-    }
-    cnt_add_warp(CSB_CTR(work_hh_members), hh_members);
-}
-__global__ void __launch_bounds__(kThreads) k_infector_hh_spatial(DevPop d) { k_infector_hh_spatial_body(d); }
-__global__ void __launch_bounds__(kThreads) k_infector_hh_spatial_multi(const DevPop* __restrict__ pops) { k_infector_hh_spatial_body(pops[blockIdx.y]); }
-
-// Place passes (src/Sweep.cpp:379-647): one thread per (infector, place) work
-// entry, i.e. per place type the infector attends and is not absent from.
-__device__ __forceinline__ void k_infector_places_body(const DevPop& d)
-{
-    const cs_params& P = *d.P;
-    const StepScalars st = *d.step;
-    const uint64_t seed = st.seed;
-    int n = d.counts[kCntPlaceWork];
-    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
-        int2 e = d.place_work[t];
-        int idx = e.x >> 3, pt = e.x & 7, link = e.y;
-        int i = d.act[idx].x;
-        PersonHot hi = d.hot[i];
-        double PI = st.fp * st.seas * calc_place_inf(hi, P, pt, st.ts);
-        if (st.blanket) {
-            if (dist2_hh_pt(d, P, hi.hh, d.pl[pt].x[link], d.pl[pt].y[link]) > P.MoveRestrRadius2)
-                PI *= P.MoveRestrEffect;
-        } else if (moverest_differs(d, hi.mcell, d.pl[pt].mcell[link]))
-            PI *= P.MoveRestrEffect;
-        if (pt != P.HotelPlaceType) {
-            double p1 = PI;
-            if (p1 > 1) p1 = 1;
-            place_candidates(d, P, st, i, hi, pt, link, p1, false, seed);
-        }
-        int np = d.pl[pt].member_ofs[link + 1] - d.pl[pt].member_ofs[link];
-        double p2 = PI * (P.PlaceTypePropBetweenGroupLinks[pt] * P.PlaceTypeGroupSizeParam1[pt] / ((double)np));
-        if (p2 > 1) p2 = 1;
-        place_candidates(d, P, st, i, hi, pt, link, p2, true, seed);
-    }
-}
-__global__ void __launch_bounds__(kThreads) k_infector_places(DevPop d) { k_infector_places_body(d); }
-__global__ void __launch_bounds__(kThreads) k_infector_places_multi(const DevPop* __restrict__ pops) { k_infector_places_body(pops[blockIdx.y]); }
-
-// Spatial contacts (src/Sweep.cpp:742-856): pick a target block from the infector's
-// block row, a slot uniformly among the block's S0 slots, accept with K(d)/bound,
-// redraw on rejection or a dead target.  Draw t of a contact reads its uniforms
-// from Philox blocks 2t and 2t+1 of the contact's stream, so the draws are
-// independent of one another: LANES lanes (4, 8 or 16, a tuning choice that does
-// not change results) evaluate draws t0..t0+LANES-1 together and the lowest
-// accepted one wins, exactly as a sequential loop would.
+// Spatial pass (src/Sweep.cpp:656-856).  An infector has a contact in one step in twenty or
+// so.  A warp tests its infectors 32 at a time, u < 1 - lambda ending most of them, queues
+// the others and draws their numbers of contacts in full warps; and it works through those
+// in groups of LANES lanes (2, 4, 8 or 16, a tuning choice that does not change results), a
+// group taking the next contact as soon as it is done with one and the warp testing more
+// infectors before its groups run out.  A contact: pick a target block from the infector's block
+// row, a slot uniformly among the block's S0 slots, accept with K(d)/bound, redraw on
+// rejection or a dead target.  Draw t of a contact reads its uniforms from Philox blocks 2t
+// and 2t+1 of the contact's stream, so the draws are independent of one another: a group
+// evaluates LANES consecutive draws together and the lowest accepted one wins, exactly as
+// a sequential loop would.  Bound: a draw's chain of seven dependent gathers.
 constexpr uint32_t kSpatialBlocksPerDraw = 2;
 
 // One rejection draw; true when accepted (target alive, u < K(d)/bound).
-__device__ __forceinline__ bool spatial_draw(const DevPop& d, const cs_params& P, Stream& s, int b,
+__device__ __forceinline__ bool spatial_draw(const DevPop& d, const cs_params& Pg, Stream& s, int b,
                                              const double* row, const int16_t* guide_row, double total,
-                                             int hh_inf, int& m_out, int& slot_out, int& p_out,
+                                             float2 xy_inf, int& m_out, int& slot_out, int& p_out,
                                              PersonHot& hp_out, double& d2_out, int* oor)
 {
-    // smallest B with target < row[B]: guide-table start, then walk
+    // smallest B with target < row[B]: it lies between the cut points of target's guide entry
+    // and the next (the steps after the search cover their rounding)
     double u1 = s.next();
     double target = u1 * total;
-    int B = guide_row[min((int)(u1 * (double)d.NB), d.NB - 1)];
+    const int q1 = min((int)(u1 * (double)d.NB), d.NB - 1);
+    int B = guide_row[q1];
+    for (int hi = q1 + 1 < d.NB ? guide_row[q1 + 1] : d.NB - 1; B < hi;) {
+        const int mid = (B + hi) >> 1;
+        if (target < row[mid]) hi = mid; else B = mid + 1;
+    }
     while (B > 0 && row[B - 1] > target) B--;
     while (B < d.NB - 1 && !(target < row[B])) B++;
     const BlockInfo bi = d.block_info[B];
+    const double bound = bound_of(d, b, B);
     long long bS0 = bi.S0;
     if (bS0 <= 0) return false;
     double u2 = s.next();
     double r = floor(u2 * (double)bS0);
     // smallest cell k in block B with r < cum[k], the same way
     int kb = bi.kb, ke = bi.ke - 1;
-    int k0 = kb + d.cell_guide[kb + min((int)(u2 * (double)(ke - kb + 1)), ke - kb)];
+    const int q2 = min((int)(u2 * (double)(ke - kb + 1)), ke - kb);
+    int k0 = kb + d.cell_guide[kb + q2];
+    for (int hi = q2 < ke - kb ? kb + d.cell_guide[kb + q2 + 1] : ke; k0 < hi;) {
+        const int mid = (k0 + hi) >> 1;
+        if (r < (double)d.block_cell_info[mid].cum) hi = mid; else k0 = mid + 1;
+    }
     while (k0 > kb && r < (double)d.block_cell_info[k0 - 1].cum) k0--;
     while (k0 < ke && !(r < (double)d.block_cell_info[k0].cum)) k0++;
     const BlockCell bc = d.block_cell_info[k0];
@@ -1616,96 +1759,224 @@ __device__ __forceinline__ bool spatial_draw(const DevPop& d, const cs_params& P
     int slot = (int)(r - (double)(bc.cum - bc.s0));
     int p = d.slots[bc.start + slot];
     PersonHot hp = d.hot[p];
-    double d2 = dist2_hh(d, P, hh_inf, hp.hh);
-    double accept = knum_f32(d, P, d2, oor) / bound_of(d, b, B);
+    double d2 = dist2_xy(Pg, xy_inf, person_xy(d, p));
+    double accept = knum_f32(d, Pg, d2, oor) / bound;
     if ((s.next() >= accept) || !is_alive(hp.inf)) return false;
     m_out = m; slot_out = slot; p_out = p; hp_out = hp; d2_out = d2;
     return true;
 }
 
+// An accepted contact of infector ii (cell cc, bit 31: its places are closed) with person p.
+__device__ __forceinline__ void spatial_accept(const DevPop& d, const cs_params& P, const cs_params& Pg, const StepScalars& st,
+                                               Stream& s, bool anyc, int ii, int cc, int m, int slot, int p,
+                                               const PersonHot& hp, double d2w)
+{
+    const PersonHot hinf = d.hot[ii];
+    if (((cc & 0x7fffffff) == m) && (hp.hh == hinf.hh)) return;
+    const int iag = age_group(hinf);
+    double ss = calc_spatial_susc(d, hp, P, st.ts);
+    if (is_ch(hp) || is_ch(hinf)) ss *= P.CareHomeResidentSpatialScaling;
+    if (slot >= d.S[m]) return;
+    ss *= calc_person_susc(hp, iag, P);
+    ss *= P.WAIFW_Matrix_SpatialOnly[age_group(hp)][iag];
+    if (st.blanket) {   // the draw's distance is dist2_raw's with UTM coordinates
+        const double d2b = P.DoUTM_coords ? d2w : dist2_hh_raw(d, Pg, hinf.hh, hp.hh);
+        if (d2b > P.MoveRestrRadius2) ss *= P.MoveRestrEffect;
+    } else if (moverest_differs(d, hp.mcell, hinf.mcell))
+        ss *= P.MoveRestrEffect;
+    if (cc >= 0 && anyc && host_absent(hp, st.ts)) {
+        bool f = false;
+        for (int pt = 0; (pt < d.NPT) && (!f); pt++) {
+            int lk = link_of(d, pt, p);
+            if (lk >= 0) f = place_closed(d, pt, lk, st.ts);
+        }
+        if (f) ss *= P.Efficacies[CS_NPI_PLACE_CLOSURE][CS_SETTING_SPATIAL];
+    }
+    if ((ss == 1) || (s.next() < ss))
+        if (hp.inf == CS_INF_SUSCEPTIBLE) claim_infection(d, P, st, p, ii, 2 + 2 * CS_MAX_PLACE_TYPES);
+}
+
+// A warp's infectors with contacts still to be placed.
+struct ContactQueue {
+    static constexpr int kCap = 64;   // 32 more are drawn for while at most 32 wait
+    int i[kCap], cell[kCap], k[kCap];
+    float2 xy[kCap];
+};
+// Its infectors that may have contacts, to be drawn for (cell with bit 31: its places are closed).
+struct MaybeQueue {
+    double lambda[64];
+    int i[64], cell[64];
+};
+
 template <int kSpatialLanes>
 __device__ __forceinline__ void k_spatial_body(const DevPop& d)
 {
-    const cs_params& P = *d.P;
+    __shared__ StagedParams sp;
+    __shared__ ContactQueue s_queue[kThreads / 32];
+    struct Maybes { MaybeQueue q[kThreads / 32]; };
+    const cs_params& Pg = *d.P;
+    const int nact = d.counts[kCntAct];
+    if (blockIdx.x == 0 && threadIdx.x == 0 && nact) cnt_add(CSB_CTR(work_infectors), nact);
     const StepScalars st = *d.step;
-    const uint64_t seed = st.seed;
-    int nact = d.counts[kCntAct];
-    int nres = d.counts[kCntContacts];
-    int ncont = min(nres, d.cmap_cap);   // contacts beyond the map are counted as overflow
-    auto tile = cg::tiled_partition<kSpatialLanes>(cg::this_thread_block());
-    const int lane = (int)tile.thread_rank();
-    const int group = (blockIdx.x * blockDim.x + threadIdx.x) / kSpatialLanes;
-    const int ngroups = (gridDim.x * blockDim.x) / kSpatialLanes;
-    long long draws = 0, oor_count = 0, give_ups = 0;
-    for (int cidx = group; cidx < ncont; cidx += ngroups) {
-        int idx = d.cmap[cidx];            // the infector owning contact cidx
-        int j = cidx - d.cnt_ofs[idx];
-        const int2 ac = d.act[idx];
-        const int i = ac.x, ci = ac.y;
-        bool closed_i = d.act_closed[idx] != 0;
-        PersonHot hinf = d.hot[i];
-        int b = d.cell_block[ci];
-        const double* row = d.block_row_cum + (size_t)b * d.NB;
-        const int16_t* guide_row = d.block_guide + (size_t)b * d.NB;
-        double total = row[d.NB - 1];
-        if (!(total > 0)) { if (lane == 0) give_ups++; continue; }
-        int m = 0, slot = 0, p = 0, won = -1;
+    const Groups work(nact);
+    if (work.idle_block() || !(st.sp_beta > 0)) return;
+    const cs_params& P = stage_params(sp, d.P);
+    const bool anyc = closures_possible(d, st.ts);
+    const int lane = threadIdx.x & 31, sub = lane & ~(kSpatialLanes - 1), sl = lane & (kSpatialLanes - 1);
+    constexpr unsigned kSubMask = (1u << kSpatialLanes) - 1u;
+    unsigned leaders = 0;
+    for (int q = 0; q < 32; q += kSpatialLanes) leaders |= 1u << q;
+    long long draws = 0, contacts = 0, oor_count = 0, give_ups = 0;
+    ContactQueue& Q = s_queue[threadIdx.x >> 5];
+    MaybeQueue& M = sp.spare<Maybes>()->q[threadIdx.x >> 5];
+    int maybe = 0;   // infectors to be drawn for
+    int head = 0, tail = 0, waiting = 0, used = 0;   // queue ends, contacts waiting in it, contacts of the head taken
+    // this lane's group's contact: infector, cell (bit 31: its places are closed), number, next draw
+    int ii = 0, cc = 0, j = 0, t0 = 0, b = 0;
+    bool busy = false;
+    float2 xyi = make_float2(0.f, 0.f);
+    double total = 0.0;
+    long long g = work.first();
+    for (;;) {
+        // ---- infectors' numbers of contacts, until every group has one waiting
+        while ((work.more(g) || maybe) && waiting < 32 / kSpatialLanes && tail - head <= 32) {
+            if (work.more(g) && maybe < 32) {
+                const int idx = work.item(g);
+                g = work.next(g);
+                int i = 0, ci = 0;
+                double lambda = 0.0;
+                bool on = false;
+                if (idx >= 0) {
+                    const int2 ac = d.act[idx];
+                    i = ac.x;
+                    ci = ac.y;
+                    const PersonHot hi = d.hot[i];
+                    const double tp = d.tot_prob[ci];
+                    double si = calc_spatial_inf(d, hi, P, st.ts);
+                    bool closed_i = false;
+                    if (anyc && P.DoPlaces && host_absent(hi, st.ts)) {   // closures count only for an absent infector
+                        const PersonLinks pli = load_links(d, i);
+                        for (int pt = 0; (pt < d.NPT) && (!closed_i); pt++)
+                            if (pli.link[pt] >= 0) closed_i = place_closed(d, pt, pli.link[pt], st.ts);
+                    }
+                    if (closed_i) si *= P.Efficacies[CS_NPI_PLACE_CLOSURE][CS_SETTING_SPATIAL];
+                    lambda = si * st.sp_beta * tp;
+                    if (closed_i) ci |= (int)0x80000000;
+                    Stream s(st.seed, CS_RNG_SPATIAL_COUNT, (uint32_t)st.ts, (uint32_t)i, 0);
+                    on = lambda > 0 && (lambda >= 10.0 || !(s.next() < 1.0 - lambda - 1e-12));   // as sample_poisson tests
+                }
+                const unsigned m = __ballot_sync(0xffffffffu, on);
+                if (on) {
+                    const int at = maybe + __popc(m & ((1u << lane) - 1u));
+                    M.lambda[at] = lambda;
+                    M.i[at] = i;
+                    M.cell[at] = ci;
+                }
+                maybe += __popc(m);
+                __syncwarp();
+            }
+            if (maybe >= 32 || (!work.more(g) && maybe > 0)) {
+                const int take = min(maybe, 32);
+                maybe -= take;   // the last ones in
+                int i = 0, ci = 0, k = 0;
+                float2 xy = make_float2(0.f, 0.f);
+                if (lane < take) {
+                    i = M.i[maybe + lane];
+                    ci = M.cell[maybe + lane];
+                    xy = person_xy(d, i);
+                    Stream s(st.seed, CS_RNG_SPATIAL_COUNT, (uint32_t)st.ts, (uint32_t)i, 0);
+                    k = sample_poisson(s, M.lambda[maybe + lane], CSB_CTR(err_spatial_tries));
+                    contacts += k;
+                }
+                const unsigned m = __ballot_sync(0xffffffffu, k > 0);
+                if (k > 0) {
+                    const int at = (tail + __popc(m & ((1u << lane) - 1u))) & (ContactQueue::kCap - 1);
+                    Q.i[at] = i;
+                    Q.cell[at] = ci;
+                    Q.k[at] = k;
+                    Q.xy[at] = xy;
+                }
+                tail += __popc(m);
+                waiting += __reduce_add_sync(0xffffffffu, k);
+                __syncwarp();
+            }
+        }
+        // ---- idle groups take the next contacts, in order
+        const unsigned idle = __ballot_sync(0xffffffffu, !busy) & leaders;
+        const int nidle = min(__popc(idle), waiting), mine = busy ? -1 : __popc(idle & ((1u << sub) - 1u));
+        if (nidle == 0 && idle == leaders) break;   // nothing waiting, nothing in flight (and no infectors left)
+        for (int r = 0; r < nidle; r++) {
+            const int at = head & (ContactQueue::kCap - 1);
+            if (mine == r) {
+                ii = Q.i[at];
+                cc = Q.cell[at];
+                xyi = Q.xy[at];
+                j = used;
+            }
+            if (++used == Q.k[at]) { head++; used = 0; }
+        }
+        waiting -= nidle;
+        if (mine >= 0 && mine < nidle) {
+            t0 = 0;
+            b = d.cell_block[cc & 0x7fffffff];
+            total = d.block_row_cum[(size_t)b * d.NB + d.NB - 1];
+            busy = total > 0;
+            if (!busy && sl == 0) give_ups++;
+        }
+        __syncwarp();
+        // ---- one round of draws
+        int m = 0, slot = 0, p = 0, oor = 0;
         double d2w = 0.0;
         PersonHot hp;
-        Stream s(seed, CS_RNG_SPATIAL_CONTACT, (uint32_t)st.ts, (uint32_t)i, (uint32_t)j);
-        for (int t0 = 0; t0 < kMaxSpatialTries; t0 += kSpatialLanes) {
-            int t = t0 + lane, oor = 0;
-            s = Stream(seed, CS_RNG_SPATIAL_CONTACT, (uint32_t)st.ts, (uint32_t)i, (uint32_t)j);
-            s.block = kSpatialBlocksPerDraw * (uint32_t)t;
-            bool acc = (t < kMaxSpatialTries) && spatial_draw(d, P, s, b, row, guide_row, total, hinf.hh,
-                                                              m, slot, p, hp, d2w, &oor);
-            unsigned mask = tile.ballot(acc);
-            int w = mask ? __ffs(mask) - 1 : kSpatialLanes;
-            if (lane < w) oor_count += oor;   // draws up to the winner count, as in a sequential loop
-            if (lane == w) oor_count += oor;
-            if (mask) { won = t0 + w; break; }
+        bool acc = false;
+        Stream s(st.seed, CS_RNG_SPATIAL_CONTACT, (uint32_t)st.ts, (uint32_t)ii, (uint32_t)j);
+        if (busy) {
+            s.block = kSpatialBlocksPerDraw * (uint32_t)(t0 + sl);
+            acc = spatial_draw(d, Pg, s, b, d.block_row_cum + (size_t)b * d.NB, d.block_guide + (size_t)b * d.NB, total, xyi,
+                               m, slot, p, hp, d2w, &oor);
         }
-        if (lane == 0) draws += (won >= 0) ? won + 1 : kMaxSpatialTries;
-        if (won < 0) { if (lane == 0) give_ups++; continue; }
-        if (lane != won % kSpatialLanes) continue;
-        if ((ci != m) || (hp.hh != hinf.hh)) {
-            int iag = age_group(hinf);
-            double ss = calc_spatial_susc(d, hp, P, st.ts);
-            if (is_ch(hp) || is_ch(hinf)) ss *= P.CareHomeResidentSpatialScaling;
-            if (slot < d.S[m]) {
-                ss *= calc_person_susc(hp, iag, P);
-                ss *= P.WAIFW_Matrix_SpatialOnly[age_group(hp)][iag];
-                if (st.blanket) {   // the draw's distance is dist2_raw's with UTM coordinates
-                    const double d2b = P.DoUTM_coords ? d2w : dist2_hh_raw(d, P, hinf.hh, hp.hh);
-                    if (d2b > P.MoveRestrRadius2) ss *= P.MoveRestrEffect;
-                } else if (moverest_differs(d, hp.mcell, hinf.mcell))
-                    ss *= P.MoveRestrEffect;
-                if ((!closed_i) && closures_possible(d, st.ts) && host_absent(hp, st.ts)) {
-                    bool f = false;
-                    for (int pt = 0; (pt < d.NPT) && (!f); pt++) {
-                        int lk = link_of(d, pt, p);
-                        if (lk >= 0) f = place_closed(d, pt, lk, st.ts);
-                    }
-                    if (f) ss *= P.Efficacies[CS_NPI_PLACE_CLOSURE][CS_SETTING_SPATIAL];
+        const unsigned won = (__ballot_sync(0xffffffffu, acc) >> sub) & kSubMask;
+        if (busy) {
+            const int w = won ? __ffs(won) - 1 : kSpatialLanes;
+            if (sl <= w) oor_count += oor;   // draws up to the winner count, as in a sequential loop
+            if (won) {
+                busy = false;
+                if (sl == 0) draws += t0 + w + 1;
+                if (sl == w) spatial_accept(d, P, Pg, st, s, anyc, ii, cc, m, slot, p, hp, d2w);
+            } else {
+                t0 += kSpatialLanes;
+                if (t0 >= kMaxSpatialTries) {
+                    if (sl == 0) { draws += kMaxSpatialTries; give_ups++; }
+                    busy = false;
                 }
-                if ((ss == 1) || (s.next() < ss))
-                    if (hp.inf == CS_INF_SUSCEPTIBLE) claim_infection(d, P, st, p, i, 2 + 2 * CS_MAX_PLACE_TYPES);
             }
         }
     }
+    __syncwarp();
     cnt_add_warp(CSB_CTR(work_spatial_draws), draws);
     cnt_add_warp(CSB_CTR(err_kernel_range), oor_count);
     cnt_add_warp(CSB_CTR(err_spatial_tries), give_ups);
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-        cnt_add(CSB_CTR(work_infectors), nact);
-        cnt_add(CSB_CTR(work_spatial_contacts), ncont);
-        if (nres > ncont) cnt_add(CSB_CTR(err_queue_overflow), nres - ncont);
+    {
+        long long sum = contacts;
+        for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+        if (lane == 0 && sum) {
+            cnt_add(CSB_CTR(work_spatial_contacts), sum);
+            atomicAdd(d.counts + kCntContacts, (int32_t)sum);
+        }
     }
 }
 template <int kSpatialLanes>
 __global__ void __launch_bounds__(kThreads, 3) k_spatial(DevPop d) { k_spatial_body<kSpatialLanes>(d); }
 template <int kSpatialLanes>
 __global__ void __launch_bounds__(kThreads, 3) k_spatial_multi(const DevPop* __restrict__ pops) { k_spatial_body<kSpatialLanes>(pops[blockIdx.y]); }
+
+// More spatial contacts in a step than two per person are an overflow of the step (an
+// infectiousness far outside the model's range); reported with the bounded loops' give-ups.
+__device__ __forceinline__ void check_contacts(const DevPop& d)
+{
+    const int n = d.counts[kCntContacts], cap = (int)min(2ll * d.N, 0x7fffffffll);
+    if (n > cap) cnt_add(CSB_CTR(err_queue_overflow), n - cap);
+}
 
 // Tallies of DoInfect that every infection adds to, summed per thread and added once per
 // warp: one atomic per thread on a single address would serialise the launch.
@@ -1786,6 +2057,7 @@ __device__ __forceinline__ void k_apply_infections_body(const DevPop& d)
     const int ts = d.step->ts;
     const uint64_t seed = d.step->seed;
     const int nq = d.counts[kCntQueue];
+    if (blockIdx.x == 0 && threadIdx.x == 0) check_contacts(d);
     if (blockIdx.x * blockDim.x >= nq) return;   // a block without work stages nothing
     const bool staged = nq >= kStageMinItems;
     stage_begin(d.C, staged);
@@ -2256,36 +2528,6 @@ __device__ __forceinline__ void k_apply_false_cases_body(const DevPop& d)
 __global__ void k_apply_false_cases(DevPop d) { k_apply_false_cases_body(d); }
 __global__ void k_apply_false_cases_multi(const DevPop* __restrict__ pops) { k_apply_false_cases_body(pops[blockIdx.y]); }
 
-// How a launch of warps takes a list of n items: `per` items a warp at a time, group g of
-// them by warp g / blocks of block g % blocks.  With few items a launch lasts as long as one
-// item's chain of dependent loads and double-precision draws, and lanes that take different
-// branches of it add theirs up, so while there are fewer items than schedulers (148 SMs
-// of four; shared by a batch's members) each gets a warp of its own, on as many SMs as there
-// are groups.  With many, whole warps in whole blocks: every warp and block adds its
-// tallies to the same few counters at its end.
-struct Groups {
-    int n, per, blocks;
-    __device__ __forceinline__ explicit Groups(int items) : n(items)
-    {
-        const int slots = 592 / (int)gridDim.y, wpb = blockDim.x >> 5;
-        per = max(1, min(32, n / max(1, slots)));
-        const int groups = (n + per - 1) / per;
-        blocks = max(1, min((int)gridDim.x, max(min(groups, 148), (groups + wpb - 1) / wpb)));
-    }
-    __device__ __forceinline__ bool idle_block() const { return (int)blockIdx.x >= blocks || (long long)blockIdx.x * per >= n; }
-    // f(item) for every item of the calling thread; all lanes of a warp make the same calls
-    template <typename F>
-    __device__ __forceinline__ void each(F f) const
-    {
-        const int lane = threadIdx.x & 31;
-        if ((int)blockIdx.x >= blocks) return;
-        for (long long g = blockIdx.x + (long long)blocks * (threadIdx.x >> 5); g * per < n; g += (long long)blocks * (blockDim.x >> 5)) {
-            const long long e = g * per + lane;
-            if (lane < per && e < n) f((int)e);
-        }
-    }
-};
-
 // The step's state changes, one kernel per kind, run side by side: DoInfect for every
 // claimed person (kInfections), DoIncub for the latent people whose time is now (kOnsets),
 // DoCase / severity / recovery / death for the infectious ones (kProgress).  They touch
@@ -2309,6 +2551,7 @@ __device__ __forceinline__ void k_changes_body(const DevPop& d)
     const DevIv iv = *d.iv;
     const int n = d.counts[kKind == kInfections ? kCntQueue : kKind == kOnsets ? kCntEvents : kCntEventsInf];
     if (kKind == kOnsets && blockIdx.x == 0 && threadIdx.x == 0) *d.ev_init = 0;   // the scan before this formed next_ev
+    if (kKind == kInfections && blockIdx.x == 0 && threadIdx.x == 0) check_contacts(d);
     const Groups work(n);
     if (work.idle_block()) return;   // a block without work stages nothing
     const bool staged = n >= kStageMinItems;
@@ -2718,6 +2961,10 @@ __global__ void k_place_events(DevPop d, const cs_place_event* __restrict__ ev, 
 __global__ void k_mcell_status(DevPop d, const int32_t* __restrict__ m, const uint8_t* __restrict__ sd,
                                const uint8_t* __restrict__ mr, int n)
 {
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        if (sd) d.status_any[kAnySocdist] = 1;
+        if (mr) d.status_any[kAnyMoverest] = 1;
+    }
     for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
         if (sd) d.socdist[m[k]] = sd[k];
         if (mr) d.moverest[m[k]] = mr[k];
@@ -2876,6 +3123,7 @@ __device__ __forceinline__ void k_socdist_fill_body(const DevPop& d, const DayCt
     if (!ctl->socd_write) return;
     const bool per_unit = ctl->pol.per_adunit != 0;
     const uint8_t on = ctl->pol.social_distancing ? CS_TREAT_TREATED : CS_TREAT_UNTREATED;
+    if (blockIdx.x == 0 && threadIdx.x == 0 && ctl->pol.social_distancing) d.status_any[kAnySocdist] = 1;
     for (int m = blockIdx.x * blockDim.x + threadIdx.x; m < d.NM; m += gridDim.x * blockDim.x) {
         if (!per_unit) {
             d.socdist[m] = ctl->socd_value;
@@ -2982,6 +3230,8 @@ static int alloc_dynamic(cs_gpu_ctx* c)
     AL(d.socdist, NM); AL(d.moverest, NM);
     CK(cudaMemsetAsync(d.socdist, 0, NM, c->stream));
     CK(cudaMemsetAsync(d.moverest, 0, NM, c->stream));
+    AL(d.status_any, 2);
+    CK(cudaMemsetAsync(d.status_any, 0, 2 * sizeof(int32_t), c->stream));
     AL(d.block_cell_info, NC); AL(d.block_info, (size_t)d.NB); AL(d.block_row_cum, (size_t)d.NB * d.NB);
     if (!d.bounds_static) AL(d.block_bound_tab, (size_t)d.NB * d.NB);   // else shared, filled once
     AL(d.block_guide, (size_t)d.NB * d.NB); AL(d.cell_guide, NC);
@@ -2993,12 +3243,10 @@ static int alloc_dynamic(cs_gpu_ctx* c)
         AL(c->rowS, (size_t)params->nch);
     }
     AL(d.claim, N); AL(d.queue, N); AL(d.counts, kCntN); AL(d.touched, NC); AL(d.cell_flag, NC + 4);
-    AL(d.act, N); AL(d.events, N); AL(d.cnt, NC); AL(d.cnt_s, NC); AL(d.cnt_ofs, N);
-    AL(d.cmap, 2 * N); d.cmap_cap = (int32_t)(2 * N);
-    AL(d.act_closed, N); AL(d.hh_flag, NH + 4); AL(d.hh_list, NH);
+    AL(d.act, N); AL(d.events, N); AL(d.cnt, NC); AL(d.cnt_s, NC);
+    AL(d.hh_flag, NH + 4); AL(d.hh_list, NH);
     AL(d.carer_win, NH); AL(d.carer_list, NH);
     CK(cudaMemsetAsync(d.carer_win, 0, sizeof(uint32_t) * NH, c->stream));
-    AL(d.place_work, N * (size_t)(NPT > 0 ? NPT : 1));
     AL(d.close_window, 2);
     CK(cudaMemcpyAsync(d.close_window, kNoClosures, sizeof(kNoClosures), cudaMemcpyHostToDevice, c->stream));
     CK(cudaMemsetAsync(d.claim, 0xff, sizeof(unsigned long long) * N, c->stream));
@@ -3043,9 +3291,8 @@ int cs_gpu_create(const cs_population* pop, const cs_params* params, int device,
     CK(cudaSetDevice(device));
     CK(cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking));
     CK(c->br.create());
-    int nsm = 148;
-    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, device);
-    c->grid = nsm * 8;
+    cudaDeviceGetAttribute(&c->nsm, cudaDevAttrMultiProcessorCount, device);
+    c->grid = c->nsm * 8;
     c->hp = *params;
     c->stat = std::make_shared<StaticStore>();
     c->stat->device = device;
@@ -3098,6 +3345,17 @@ int cs_gpu_create(const cs_population* pop, const cs_params* params, int device,
         CK(cudaStreamSynchronize(c->stream));
     }
     {
+        std::vector<float2> xy(N);
+        for (size_t p = 0; p < N; p++) {
+            const int32_t h = pop->person_hh[p];
+            xy[p] = make_float2(pop->hh_x[h], pop->hh_y[h]);
+        }
+        float2* t;
+        UP(t, xy.data(), N);
+        d.pxy = t;
+        CK(cudaStreamSynchronize(c->stream));
+    }
+    {
         std::vector<HouseholdRec> hh(NH);
         for (size_t h = 0; h < NH; h++)
             hh[h] = HouseholdRec{pop->hh_x[h], pop->hh_y[h], pop->hh_first[h], pop->hh_nh[h], pop->hh_nhr[h]};
@@ -3135,6 +3393,17 @@ int cs_gpu_create(const cs_population* pop, const cs_params* params, int device,
         { int32_t* t; UP(t, pop->place_group_ofs[pt], np + 1); pl.group_ofs = t; }
         { int32_t* t; UP(t, pop->group_start[pt], ng); pl.group_start = t; }
         { int32_t* t; UP(t, pop->group_size[pt], ng); pl.group_size = t; }
+        {
+            std::vector<PlaceRec> rec(np);
+            std::vector<int2> grp(ng);
+            for (size_t l = 0; l < np; l++)
+                rec[l] = PlaceRec{pop->place_member_ofs[pt][l], pop->place_member_ofs[pt][l + 1] - pop->place_member_ofs[pt][l],
+                                  pop->place_group_ofs[pt][l], pop->place_mcell[pt][l]};
+            for (size_t g = 0; g < ng; g++) grp[g] = make_int2(pop->group_start[pt][g], pop->group_size[pt][g]);
+            { PlaceRec* t; UP(t, rec.data(), np); pl.rec = t; }
+            { int2* t; UP(t, grp.data(), ng); pl.group = t; }
+            CK(cudaStreamSynchronize(c->stream));   // before rec and grp go out of scope
+        }
         { float* t; UP(t, pop->place_x[pt], np); pl.x = t; }
         { float* t; UP(t, pop->place_y[pt], np); pl.y = t; }
     }
@@ -3203,6 +3472,7 @@ int cs_gpu_create_replica(const cs_gpu_ctx* base, cs_gpu_ctx** out)
     CK(cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking));
     CK(c->br.create());
     c->grid = base->grid;
+    c->nsm = base->nsm;
     c->hp = base->hp;
     c->stat = base->stat;
     c->d = base->d;           // static pointers and sizes; dynamic ones are replaced below
@@ -3532,6 +3802,7 @@ static int reset_run_level(cs_gpu_ctx* c, uint64_t seed)
     CK(cudaMemcpyAsync(d.close_window, kNoClosures, sizeof(kNoClosures), cudaMemcpyHostToDevice, c->stream));
     CK(cudaMemsetAsync(d.socdist, 0, d.NM, c->stream));
     CK(cudaMemsetAsync(d.moverest, 0, d.NM, c->stream));
+    CK(cudaMemsetAsync(d.status_any, 0, 2 * sizeof(int32_t), c->stream));
     LAUNCH(k_iv_reset, 1, kThreads, c->dIv, d.NA);
     return CS_OK;
 }
@@ -3558,6 +3829,13 @@ int cs_gpu_begin_run(cs_gpu_ctx* c, uint64_t seed, const int32_t* seed_people, i
     c->run_started = true;
     return cs_gpu_seed_infections(c, 0.0, seed_people, n_seed);
 }
+
+// Blocks of a step kernel that deals its list out itself (Groups): the context's grid, but no
+// more than the SMs hold at once.  Blocks past the first wave find the list dealt out or, at
+// high load, repeat the staging of the parameters for little of it; every wave of blocks
+// costs a launch about 1.5 us.
+constexpr int kWave3 = 3, kWave4 = 4, kWave6 = 6;   // resident blocks per SM of the kernels below
+static int wave_grid(const cs_gpu_ctx* c, int per_sm) { return std::min(c->grid, c->nsm * per_sm); }
 
 // Every tile of kThreads cells shared by enough blocks to fill the grid.
 static int scan_grid(int NC, int grid)
@@ -3593,22 +3871,20 @@ static int begin_step(cs_gpu_ctx* c, double t, bool empty_lists)
 }
 }
 
-// The infectors' passes over the list the scan built.  The place pass and the spatial pass
-// both read the infector pass's lists and only claim infections (atomicMin on the claim
-// key) and add to counters, so they run side by side.
+// The infectors' passes over the list the scan built.
 static int infector_passes(cs_gpu_ctx* c)
 {
     DevPop& d = c->d;
-    LAUNCH(k_infector_hh_spatial, c->grid, kThreads, d);
-    FORK(1);
-    LAUNCH_ON(0, k_infector_places, c->grid, kThreads, d);
+    FORK(2);
+    LAUNCH_ON(0, k_household, wave_grid(c, kWave6), kThreads, d);
+    LAUNCH_ON(1, k_places, wave_grid(c, kWave3), kThreads, d);
     switch (c->spatial_lanes) {
-    case 2: LAUNCH(k_spatial<2>, c->grid, kThreads, d); break;
-    case 4: LAUNCH(k_spatial<4>, c->grid, kThreads, d); break;
-    case 16: LAUNCH(k_spatial<16>, c->grid, kThreads, d); break;
-    default: LAUNCH(k_spatial<8>, c->grid, kThreads, d); break;
+    case 2: LAUNCH(k_spatial<2>, wave_grid(c, kWave3), kThreads, d); break;
+    case 4: LAUNCH(k_spatial<4>, wave_grid(c, kWave3), kThreads, d); break;
+    case 16: LAUNCH(k_spatial<16>, wave_grid(c, kWave3), kThreads, d); break;
+    default: LAUNCH(k_spatial<8>, wave_grid(c, kWave3), kThreads, d); break;
     }
-    JOIN(1);
+    JOIN(2);
     return CS_OK;
 }
 
@@ -3625,11 +3901,11 @@ static int incub_alone(cs_gpu_ctx* c, double t)
     int r = begin_step<false, true>(c, t, false);
     if (r) return r;
     FORK(1);
-    LAUNCH_ON(0, k_progress, c->grid, kThreads, d);
-    LAUNCH(k_onsets, c->grid, kThreads, d);
+    LAUNCH_ON(0, k_progress, wave_grid(c, kWave3), kThreads, d);
+    LAUNCH(k_onsets, wave_grid(c, kWave3), kThreads, d);
     JOIN(1);
     FORK(1);
-    LAUNCH_ON(0, k_households, c->grid, kThreads, d);
+    LAUNCH_ON(0, k_households, wave_grid(c, kWave4), kThreads, d);
     LAUNCH(k_moves<false>, c->grid, kThreads, d);
     JOIN(1);
     CK(cudaMemsetAsync(d.counts, 0, sizeof(int32_t) * kCntN, c->stream));   // all list counters
@@ -3671,12 +3947,12 @@ static int step_eager(cs_gpu_ctx* c, double t, int run)
     if (!r) r = infector_passes(c);
     if (r) return r;
     FORK(2);
-    LAUNCH_ON(0, k_progress, c->grid, kThreads, d);
-    LAUNCH_ON(1, k_infections, c->grid, kThreads, d);
-    LAUNCH(k_onsets, c->grid, kThreads, d);
+    LAUNCH_ON(0, k_progress, wave_grid(c, kWave3), kThreads, d);
+    LAUNCH_ON(1, k_infections, wave_grid(c, kWave3), kThreads, d);
+    LAUNCH(k_onsets, wave_grid(c, kWave3), kThreads, d);
     JOIN(2);
     FORK(1);
-    LAUNCH_ON(0, k_households, c->grid, kThreads, d);
+    LAUNCH_ON(0, k_households, wave_grid(c, kWave4), kThreads, d);
     LAUNCH(k_moves<true>, c->grid, kThreads, d);
     JOIN(1);
     return CS_OK;
@@ -4108,47 +4384,50 @@ static int batch_enqueue(cs_gpu_batch* b, const DevPop* pops)
 {
     const int R = (int)b->members.size();
     const int grid = b->members[0]->grid;
-    const dim3 g(grid, R);
     int maxc = 0;
     for (const cs_gpu_ctx* m : b->members) maxc = std::max(maxc, m->d.NC);
-    const dim3 gs(scan_grid(maxc, grid), R);
+    // one wave of blocks per kernel over all members, and half as much again for members
+    // with more than their share
+    const int nsm = b->members[0]->nsm;
+    auto wave = [&](int per_sm) { return dim3(std::min(grid, std::max(8, (3 * nsm * per_sm / 2 + R - 1) / R)), R); };
+    const dim3 gs(scan_grid(maxc, wave(kWave4).x), R);
     const bool fused = batch_fused(b);
     BCK(b->br.begin(b->stream, 1));
     BLAUNCH_ON(0, k_set_step_multi, R, 1, pops, fused ? 1 : 0);
     if (fused) BLAUNCH((k_scan_multi<true, true>), gs, kThreads, pops);
     else BLAUNCH((k_scan_multi<true, false>), gs, kThreads, pops);
     BCK(b->br.end(b->stream, 1));
-    BLAUNCH(k_infector_hh_spatial_multi, g, kThreads, pops);
-    BCK(b->br.begin(b->stream, 1));
-    BLAUNCH_ON(0, k_infector_places_multi, g, kThreads, pops);
+    BCK(b->br.begin(b->stream, 2));
+    BLAUNCH_ON(0, k_household_multi, wave(kWave6), kThreads, pops);
+    BLAUNCH_ON(1, k_places_multi, wave(kWave3), kThreads, pops);
     switch (b->lanes) {
-    case 2: BLAUNCH(k_spatial_multi<2>, g, kThreads, pops); break;
-    case 4: BLAUNCH(k_spatial_multi<4>, g, kThreads, pops); break;
-    case 16: BLAUNCH(k_spatial_multi<16>, g, kThreads, pops); break;
-    default: BLAUNCH(k_spatial_multi<8>, g, kThreads, pops); break;
+    case 2: BLAUNCH(k_spatial_multi<2>, wave(kWave3), kThreads, pops); break;
+    case 4: BLAUNCH(k_spatial_multi<4>, wave(kWave3), kThreads, pops); break;
+    case 16: BLAUNCH(k_spatial_multi<16>, wave(kWave3), kThreads, pops); break;
+    default: BLAUNCH(k_spatial_multi<8>, wave(kWave3), kThreads, pops); break;
     }
-    BCK(b->br.end(b->stream, 1));
+    BCK(b->br.end(b->stream, 2));
     if (fused) {
         BCK(b->br.begin(b->stream, 2));
-        BLAUNCH_ON(0, k_progress_multi, g, kThreads, pops);
-        BLAUNCH_ON(1, k_infections_multi, g, kThreads, pops);
-        BLAUNCH(k_onsets_multi, g, kThreads, pops);
+        BLAUNCH_ON(0, k_progress_multi, wave(kWave3), kThreads, pops);
+        BLAUNCH_ON(1, k_infections_multi, wave(kWave3), kThreads, pops);
+        BLAUNCH(k_onsets_multi, wave(kWave3), kThreads, pops);
         BCK(b->br.end(b->stream, 2));
         BCK(b->br.begin(b->stream, 1));
-        BLAUNCH_ON(0, k_households_multi, g, kThreads, pops);
-        BLAUNCH(k_moves_multi<true>, g, kThreads, pops);
+        BLAUNCH_ON(0, k_households_multi, wave(kWave4), kThreads, pops);
+        BLAUNCH(k_moves_multi<true>, wave(kWave4), kThreads, pops);
         BCK(b->br.end(b->stream, 1));
         return CS_OK;
     }
-    BLAUNCH(k_apply_infections_multi, g, kThreads, pops);
-    BLAUNCH(k_partition_S_multi, g, kThreads, pops);
-    BLAUNCH(k_apply_false_cases_multi, g, kThreads, pops);
+    BLAUNCH(k_apply_infections_multi, wave(kWave4), kThreads, pops);
+    BLAUNCH(k_partition_S_multi, wave(kWave4), kThreads, pops);
+    BLAUNCH(k_apply_false_cases_multi, wave(kWave4), kThreads, pops);
     BLAUNCH(k_zero_counts_multi, R, 32, pops, (int)(kCntN - 1));   // the household list is the incub sweep's
     BLAUNCH((k_scan_multi<false, true>), gs, kThreads, pops);
-    BLAUNCH(k_onsets_multi, g, kThreads, pops);
-    BLAUNCH(k_progress_multi, g, kThreads, pops);
-    BLAUNCH(k_moves_multi<false>, g, kThreads, pops);
-    BLAUNCH(k_households_multi, g, kThreads, pops);
+    BLAUNCH(k_onsets_multi, wave(kWave3), kThreads, pops);
+    BLAUNCH(k_progress_multi, wave(kWave3), kThreads, pops);
+    BLAUNCH(k_moves_multi<false>, wave(kWave4), kThreads, pops);
+    BLAUNCH(k_households_multi, wave(kWave4), kThreads, pops);
     BLAUNCH(k_zero_counts_multi, R, 32, pops, (int)kCntN);
     return CS_OK;
 }
@@ -4446,6 +4725,8 @@ int cs_gpu_set_interventions(cs_gpu_ctx* c, const cs_interventions* iv)
     CK(cudaMemcpyAsync(c->iv_ci, ci.data(), sizeof(double) * na, cudaMemcpyHostToDevice, c->stream));
     CK(cudaMemcpyAsync(c->iv_hq, hq.data(), sizeof(double) * na, cudaMemcpyHostToDevice, c->stream));
     CK(cudaMemcpyAsync(c->dIv, &div, sizeof(div), cudaMemcpyHostToDevice, c->stream));
+    if (iv->mcell_socdist) CK(cudaMemsetAsync(c->d.status_any + kAnySocdist, 0xff, sizeof(int32_t), c->stream));
+    if (iv->mcell_moverest) CK(cudaMemsetAsync(c->d.status_any + kAnyMoverest, 0xff, sizeof(int32_t), c->stream));
     if (iv->mcell_socdist) CK(cudaMemcpyAsync(c->d.socdist, iv->mcell_socdist, c->d.NM, cudaMemcpyHostToDevice, c->stream));
     if (iv->mcell_moverest) CK(cudaMemcpyAsync(c->d.moverest, iv->mcell_moverest, c->d.NM, cudaMemcpyHostToDevice, c->stream));
     CK(cudaStreamSynchronize(c->stream));
