@@ -134,6 +134,10 @@ __device__ inline double sample_gamma(Stream& s, double beta, double alpha, unsi
         v = 1.0 + z * c;
         v = v * v * v;
         if (++it > kMaxLoop) { atomicAdd(err, 1ull); break; }
+        // their squeeze: u < 1 - 0.0331 z^4 implies acceptance, without the two logarithms
+        // (the margin covers the rounding of the test it stands for)
+        const double z2 = z * z;
+        if (z > (-1.0 / c) && u < 1.0 - 0.0331 * z2 * z2 - 1e-10) break;
     } while ((z <= (-1.0 / c)) || (log(u) >= (0.5 * z * z + d - d * v + d * log(v))));
     double g = (beta != 1.0) ? (d * v) / beta : d * v;
     if (alpha < 1.0) g = g * pow(s.next(), 1.0 / alpha);

@@ -116,6 +116,7 @@ struct DevPop {
     PersonHot* hot;
     const PersonLinks* links;  // [N]
     const HouseholdRec* hhr;   // [NH]
+    const int32_t* pcell;      // [N] the person's cell
     const float2* pxy;         // [N] the person's household's location, for the spatial draws (no detour by the record)
     const int32_t* mcell_cell;
     const int32_t* mcell_adunit;

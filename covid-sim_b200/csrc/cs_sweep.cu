@@ -92,6 +92,16 @@ __device__ __forceinline__ void cnt_add_warp(unsigned long long* p, long long v)
     if (g.thread_rank() == 0 && sum != 0) atomicAdd(p, (unsigned long long)sum);
 }
 
+// The same where all 32 lanes of the warp call it together: a few shuffles, none for a warp
+// whose lanes have nothing (a group of whichever lanes are there reduces 64-bit values in a
+// software loop: seven of them took 3 us at the end of a launch).
+__device__ __forceinline__ void cnt_add_all(unsigned long long* p, long long v)
+{
+    if (!__any_sync(0xffffffffu, v != 0)) return;
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    if ((threadIdx.x & 31) == 0 && v != 0) atomicAdd(p, (unsigned long long)v);
+}
+
 // Warp-aggregated append to a device list.
 __device__ __forceinline__ int32_t append(int32_t* count)
 {
@@ -1547,7 +1557,7 @@ __device__ __forceinline__ void k_household_body(const DevPop& d)
         }
     });
     __syncwarp();
-    cnt_add_warp(CSB_CTR(work_hh_members), hh_members);
+    cnt_add_all(CSB_CTR(work_hh_members), hh_members);
 }
 __global__ void __launch_bounds__(kThreads) k_household(DevPop d) { k_household_body(d); }
 __global__ void __launch_bounds__(kThreads) k_household_multi(const DevPop* __restrict__ pops) { k_household_body(pops[blockIdx.y]); }
@@ -1702,7 +1712,7 @@ __device__ __forceinline__ void k_places_body(const DevPop& d)
     }
     drain(0);
     __syncwarp();
-    cnt_add_warp(CSB_CTR(work_place_candidates), ncand);
+    cnt_add_all(CSB_CTR(work_place_candidates), ncand);
 }
 __global__ void __launch_bounds__(kThreads, 3) k_places(DevPop d) { k_places_body(d); }
 __global__ void __launch_bounds__(kThreads, 3) k_places_multi(const DevPop* __restrict__ pops) { k_places_body(pops[blockIdx.y]); }
@@ -1953,10 +1963,10 @@ __device__ __forceinline__ void k_spatial_body(const DevPop& d)
         }
     }
     __syncwarp();
-    cnt_add_warp(CSB_CTR(work_spatial_draws), draws);
-    cnt_add_warp(CSB_CTR(err_kernel_range), oor_count);
-    cnt_add_warp(CSB_CTR(err_spatial_tries), give_ups);
-    {
+    cnt_add_all(CSB_CTR(work_spatial_draws), draws);
+    cnt_add_all(CSB_CTR(err_kernel_range), oor_count);
+    cnt_add_all(CSB_CTR(err_spatial_tries), give_ups);
+    if (__any_sync(0xffffffffu, contacts != 0)) {
         long long sum = contacts;
         for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
         if (lane == 0 && sum) {
@@ -1985,13 +1995,15 @@ struct InfectTally {
 };
 __device__ __forceinline__ void infect_tally_add(const DevPop& d, const InfectTally& q)
 {
-    cnt_add_warp(CSB_CTR(cumI), q.n);
-    cnt_add_warp(CSB_CTR(cumI_keyworker[1]), q.kw);
-    cnt_add_warp(CSB_CTR(cumI_keyworker[0]), q.n - q.kw);
-    cnt_add_warp(CSB_CTR(cumTG), q.tg);
-    cnt_add_warp(CSB_CTR(cumSI), q.si);
-    cnt_add_warp(CSB_CTR(nTG), q.n_tg);
-    cnt_add_warp(CSB_CTR(sumRad2_q), q.rad_q);
+    __syncwarp();
+    if (!__any_sync(0xffffffffu, q.n != 0)) return;
+    cnt_add_all(CSB_CTR(cumI), q.n);
+    cnt_add_all(CSB_CTR(cumI_keyworker[1]), q.kw);
+    cnt_add_all(CSB_CTR(cumI_keyworker[0]), q.n - q.kw);
+    cnt_add_all(CSB_CTR(cumTG), q.tg);
+    cnt_add_all(CSB_CTR(cumSI), q.si);
+    cnt_add_all(CSB_CTR(nTG), q.n_tg);
+    cnt_add_all(CSB_CTR(sumRad2_q), q.rad_q);
     long long m = q.rad_max;
     for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
     if ((threadIdx.x & 31) == 0 && m > 0) atomicMax((long long*)CSB_CTR(maxRad2_bits), m);
@@ -2014,7 +2026,7 @@ __device__ __forceinline__ int do_infect(const DevPop& d, const cs_params& P, in
     d.infection_time[p] = (uint16_t)ts;
     d.infector[p] = infector;
     d.infect_type[p] = it;
-    const int cell = d.mcell_cell[h.mcell];
+    const int cell = d.pcell[p];
     atomicSub(d.S + cell, 1);
     atomicAdd(d.L + cell, 1);
     d.mark[d.cell_start[cell] + d.listpos[p]] = 1;
@@ -2071,7 +2083,6 @@ __device__ __forceinline__ void k_apply_infections_body(const DevPop& d)
         d.hot[p] = h;
         d.next_ev[p] = h.latent_time;
     }
-    __syncwarp();
     infect_tally_add(d, tally);
     if (blockIdx.x == 0 && threadIdx.x == 0) cnt_add(CSB_STAGED(work_new_infections), nq);
     stage_flush(d.C, staged);
@@ -2284,7 +2295,6 @@ __device__ void do_incub(const DevPop& d, const cs_params& P, int p, PersonHot& 
         else
             d.recovery_time[p] = tm.rec = (uint16_t)(h.latent_time + icdf_choose(P.infectious_icdf, P.InfectiousPeriod, s.next(), spd));
     } else {
-        int CaseTime = h.latent_time + ((int)(P.LatentToSymptDelay / P.ModelTimeStep));
         double x = s.next();
         int fin;
         if (x < P.Prop_ILI_ByAge[age]) fin = CS_SEV_ILI;
@@ -2292,45 +2302,47 @@ __device__ void do_incub(const DevPop& d, const cs_params& P, int p, PersonHot& 
         else if (x < P.Prop_ILI_ByAge[age] + P.Prop_SARI_ByAge[age] + P.Prop_Critical_ByAge[age]) fin = CS_SEV_CRITICAL;
         else fin = CS_SEV_MILD;
         bool to_die = false;
-        if (fin == CS_SEV_CRITICAL) { if (s.next() < (P.CFR_Critical_ByAge[age] * P.CFR_Critical_Scale_Current)) to_die = true; }
-        else if (fin == CS_SEV_SARI) { if (s.next() < (P.CFR_SARI_ByAge[age] * P.CFR_SARI_Scale_Current)) to_die = true; }
-        else if (fin == CS_SEV_ILI) { if (s.next() < (P.CFR_ILI_ByAge[age] * P.CFR_ILI_Scale_Current)) to_die = true; }
+        if (fin != CS_SEV_MILD) {
+            const double die = fin == CS_SEV_CRITICAL ? P.CFR_Critical_ByAge[age] * P.CFR_Critical_Scale_Current
+                             : fin == CS_SEV_SARI     ? P.CFR_SARI_ByAge[age] * P.CFR_SARI_Scale_Current
+                                                      : P.CFR_ILI_ByAge[age] * P.CFR_ILI_Scale_Current;
+            to_die = s.next() < die;
+        }
         if (is_ch(h) && ((fin == CS_SEV_CRITICAL) || (fin == CS_SEV_SARI)) && (s.next() > P.CareHomeRelProbHosp)) {
             to_die = true;
             fin = CS_SEV_ILI;
         }
         h.sev = (uint8_t)((h.sev & 0x0f) | (fin << 4));
         if (to_die) h.dflags |= CS_DF_TO_DIE;
-        uint16_t rec;
-        if (fin == CS_SEV_MILD)
-            rec = (uint16_t)(CaseTime + icdf_choose(P.MildToRecovery_icdf, P.Mean_MildToRecovery[age], s.next(), spd));
-        else if (fin == CS_SEV_CRITICAL) {
-            uint16_t sari = (uint16_t)(CaseTime + icdf_choose(P.ILIToSARI_icdf, P.Mean_ILIToSARI[age], s.next(), spd));
-            uint16_t crit = (uint16_t)(sari + icdf_choose(P.SARIToCritical_icdf, P.Mean_SARIToCritical[age], s.next(), spd));
-            d.sari_time[p] = tm.sari = sari;
-            d.critical_time[p] = tm.crit = crit;
-            if (to_die) {
-                if (P.IncludeStepDownToDeath == 1) {
-                    uint16_t sd = (uint16_t)(crit + icdf_choose(P.CriticalToCritRecov_icdf, P.Mean_CriticalToCritRecov[age], s.next(), spd));
-                    d.stepdown_time[p] = tm.sd = sd;
-                    rec = (uint16_t)(sd + icdf_choose(P.StepdownToDeath_icdf, P.Mean_StepdownToDeath[age], s.next(), spd));
-                } else
-                    rec = (uint16_t)(crit + icdf_choose(P.CriticalToDeath_icdf, P.Mean_CriticalToDeath[age], s.next(), spd));
-            } else {
-                uint16_t sd = (uint16_t)(crit + icdf_choose(P.CriticalToCritRecov_icdf, P.Mean_CriticalToCritRecov[age], s.next(), spd));
-                d.stepdown_time[p] = tm.sd = sd;
-                rec = (uint16_t)(sd + icdf_choose(P.CritRecovToRecov_icdf, P.Mean_CritRecovToRecov[age], s.next(), spd));
-            }
-        } else if (fin == CS_SEV_SARI) {
-            uint16_t sari = (uint16_t)(CaseTime + icdf_choose(P.ILIToSARI_icdf, P.Mean_ILIToSARI[age], s.next(), spd));
-            d.sari_time[p] = tm.sari = sari;
-            if (to_die) rec = (uint16_t)(sari + icdf_choose(P.SARIToDeath_icdf, P.Mean_SARIToDeath[age], s.next(), spd));
-            else rec = (uint16_t)(sari + icdf_choose(P.SARIToRecovery_icdf, P.Mean_SARIToRecovery[age], s.next(), spd));
-        } else {
-            if (to_die) rec = (uint16_t)(CaseTime + icdf_choose(P.ILIToDeath_icdf, P.Mean_ILIToDeath[age], s.next(), spd));
-            else rec = (uint16_t)(CaseTime + icdf_choose(P.ILIToRecovery_icdf, P.Mean_ILIToRecovery[age], s.next(), spd));
+        // from case onset through SARI, critical care and stepdown as far as the final
+        // severity goes, one delay after the other: one call site for all, so that a warp's
+        // lanes draw together and the code stays in the instruction cache
+        int when = h.latent_time + ((int)(P.LatentToSymptDelay / P.ModelTimeStep));
+        for (int at = 0;; at++) {
+            const cs_icdf* tab;
+            const double* mean;
+            bool last = true;
+            if (at == 0) {
+                if (fin == CS_SEV_MILD) { tab = &P.MildToRecovery_icdf; mean = P.Mean_MildToRecovery; }
+                else if (fin != CS_SEV_ILI) { tab = &P.ILIToSARI_icdf; mean = P.Mean_ILIToSARI; last = false; }
+                else if (to_die) { tab = &P.ILIToDeath_icdf; mean = P.Mean_ILIToDeath; }
+                else { tab = &P.ILIToRecovery_icdf; mean = P.Mean_ILIToRecovery; }
+            } else if (at == 1) {
+                if (fin != CS_SEV_SARI) { tab = &P.SARIToCritical_icdf; mean = P.Mean_SARIToCritical; last = false; }
+                else if (to_die) { tab = &P.SARIToDeath_icdf; mean = P.Mean_SARIToDeath; }
+                else { tab = &P.SARIToRecovery_icdf; mean = P.Mean_SARIToRecovery; }
+            } else if (at == 2) {
+                if (to_die && P.IncludeStepDownToDeath != 1) { tab = &P.CriticalToDeath_icdf; mean = P.Mean_CriticalToDeath; }
+                else { tab = &P.CriticalToCritRecov_icdf; mean = P.Mean_CriticalToCritRecov; last = false; }
+            } else if (to_die) { tab = &P.StepdownToDeath_icdf; mean = P.Mean_StepdownToDeath; }
+            else { tab = &P.CritRecovToRecov_icdf; mean = P.Mean_CritRecovToRecov; }
+            when = (uint16_t)(when + icdf_choose(*tab, mean[age], s.next(), spd));
+            if (last) break;
+            if (at == 0) d.sari_time[p] = tm.sari = (uint16_t)when;
+            else if (at == 1) d.critical_time[p] = tm.crit = (uint16_t)when;
+            else d.stepdown_time[p] = tm.sd = (uint16_t)when;
         }
-        d.recovery_time[p] = tm.rec = rec;
+        d.recovery_time[p] = tm.rec = (uint16_t)when;
     }
     if (h.inf == CS_INF_INFECTIOUS_ALMOST_SYMPTOMATIC && ((P.ControlPropCasesId == 1) || (s.next() < P.ControlPropCasesId))) {
         h.dflags |= CS_DF_DETECTED;
@@ -2620,7 +2632,6 @@ __device__ __forceinline__ void k_changes_body(const DevPop& d)
         }
     });
     if (kKind == kInfections) {
-        __syncwarp();
         infect_tally_add(d, tally);
         if (blockIdx.x == 0 && threadIdx.x == 0) {
             cnt_add(CSB_STAGED(work_new_infections), n);
@@ -3342,6 +3353,14 @@ int cs_gpu_create(const cs_population* pop, const cs_params* params, int device,
         PersonLinks* t;
         UP(t, lk.data(), N);
         d.links = t;
+        CK(cudaStreamSynchronize(c->stream));
+    }
+    {
+        std::vector<int32_t> pc(N);
+        for (size_t p = 0; p < N; p++) pc[p] = pop->mcell_cell[pop->person_mcell[p]];
+        int32_t* t;
+        UP(t, pc.data(), N);
+        d.pcell = t;
         CK(cudaStreamSynchronize(c->stream));
     }
     {
