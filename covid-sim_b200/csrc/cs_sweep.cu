@@ -193,11 +193,12 @@ struct StaticStore {
 // of the captured graphs).
 struct Branches {
     static constexpr int kN = 2;
-    cudaStream_t s[kN] = {};
+    cudaStream_t s[kN] = {}, body = nullptr;   // body: conditional parts of a graph are captured on it
     cudaEvent_t fork = nullptr, join[kN] = {};
     cudaError_t create()
     {
         cudaError_t e = cudaEventCreateWithFlags(&fork, cudaEventDisableTiming);
+        if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&body, cudaStreamNonBlocking);
         for (int i = 0; i < kN && e == cudaSuccess; i++) {
             e = cudaStreamCreateWithFlags(&s[i], cudaStreamNonBlocking);
             if (e == cudaSuccess) e = cudaEventCreateWithFlags(&join[i], cudaEventDisableTiming);
@@ -211,6 +212,7 @@ struct Branches {
             if (join[i]) cudaEventDestroy(join[i]);
         }
         if (fork) cudaEventDestroy(fork);
+        if (body) cudaStreamDestroy(body);
     }
     cudaError_t begin(cudaStream_t main, int n)   // branches 0..n-1 start after main's work so far
     {
@@ -2768,6 +2770,9 @@ struct DayCtl {
     double a_on_until[CS_MAX_ADUNITS];
     int8_t a_switch[CS_MAX_ADUNITS];    // this day: -1 none, 1 on, 0 off
     uint16_t a_close_start[CS_MAX_ADUNITS], a_close_stop[CS_MAX_ADUNITS];
+    // k_day_check's sums of S, L, I, R, D and its finished blocks; zero between launches
+    unsigned long long totals[5];
+    int32_t blocks_done;
 };
 
 // ------------------------------------------------------------ place closure
@@ -2992,8 +2997,8 @@ __global__ void k_close_places_multi(const DevPop* __restrict__ pops, int pt, Da
 }
 
 // The test after a timestep whether the susceptible fraction fell by more than 0.2
-// since UpdateProbs last ran (src/CovidSim.cpp:1520-1526); S is fresh from k_cell_totals.
-__device__ __forceinline__ void k_probs_check_body(const DevPop& d, DayCtl* ctl, int day_end)
+// since UpdateProbs last ran (src/CovidSim.cpp:1520-1526); S is fresh.
+__device__ __forceinline__ void probs_check(const DevPop& d, DayCtl* ctl, int day_end)
 {
     if (!day_end && !ctl->pol.probs_every_step) {   // this realisation tests at day ends only
         ctl->update = 0;
@@ -3006,11 +3011,6 @@ __device__ __forceinline__ void k_probs_check_body(const DevPop& d, DayCtl* ctl,
         up = 1;
     }
     ctl->update = up;
-}
-__global__ void k_probs_check(DevPop d, DayCtl* ctl, int day_end) { k_probs_check_body(d, ctl, day_end); }
-__global__ void k_probs_check_multi(const DevPop* __restrict__ pops, DayCtl* const* ctls, int day_end)
-{
-    k_probs_check_body(pops[blockIdx.x], ctls[blockIdx.x], day_end);
 }
 
 // End of a day of the run loop: the day's counters into the series, and the global
@@ -3120,13 +3120,44 @@ __device__ void k_day_logic_body(const DevPop& d, DayCtl* ctl, const int32_t* cl
     }
     if (threadIdx.x == 0) ctl->day = day + 1;
 }
-__global__ void k_day_logic(DevPop d, DayCtl* ctl, const int32_t* clock, DevIv* iv) { k_day_logic_body(d, ctl, clock, iv); }
-// one block per member; the window struct is the member's own (written only here and
-// by cs_gpu_set_interventions)
-__global__ void k_day_logic_multi(const DevPop* __restrict__ pops, DayCtl* const* ctls)
+// What follows a timestep of the run loop before anything else may: the cells' totals into
+// the counters, the UpdateProbs test, and at a day's end the day's logic, as one launch:
+// every block adds its cells' sums, and the last one to finish goes on with the rest.  The
+// rare work decided here (UpdateProbs; the switch's flags and closures) is in a conditional
+// part of the day graph, which `part` switches on; without one (a graph with timing nodes,
+// eager launches) it is launched every time and returns at its gates.
+__device__ __forceinline__ void k_day_check_body(const DevPop& d, DayCtl* ctl, int day_end, cudaGraphConditionalHandle part)
 {
-    const DevPop& d = pops[blockIdx.x];
-    k_day_logic_body(d, ctls[blockIdx.x], d.step_clock, const_cast<DevIv*>(d.iv));
+    __shared__ int s_last;
+    long long v[5] = {0, 0, 0, 0, 0};
+    for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < d.NC; c += gridDim.x * blockDim.x) {
+        v[0] += d.S[c]; v[1] += d.L[c]; v[2] += d.I[c]; v[3] += d.R[c]; v[4] += d.D[c];
+    }
+#pragma unroll
+    for (int k = 0; k < 5; k++) {
+        for (int o = 16; o > 0; o >>= 1) v[k] += __shfl_down_sync(0xffffffffu, v[k], o);
+        if ((threadIdx.x & 31) == 0 && v[k]) cnt_add(ctl->totals + k, v[k]);
+    }
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) s_last = atomicAdd(&ctl->blocks_done, 1) == (int)gridDim.x - 1;
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();
+    if (threadIdx.x < 5) {
+        (&d.C->S)[threadIdx.x] = (int64_t)atomicExch(ctl->totals + threadIdx.x, 0ull);
+        if (threadIdx.x == 0) ctl->blocks_done = 0;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) probs_check(d, ctl, day_end);
+    if (day_end) k_day_logic_body(d, ctl, d.step_clock, const_cast<DevIv*>(d.iv));
+    __syncthreads();
+    if (threadIdx.x == 0 && part && (ctl->update || (day_end && (ctl->socd_write || ctl->close)))) cudaGraphSetConditional(part, 1);
+}
+__global__ void __launch_bounds__(kThreads) k_day_check(DevPop d, DayCtl* ctl, int day_end, cudaGraphConditionalHandle part) { k_day_check_body(d, ctl, day_end, part); }
+__global__ void __launch_bounds__(kThreads) k_day_check_multi(const DevPop* __restrict__ pops, DayCtl* const* ctls, int day_end, cudaGraphConditionalHandle part)
+{
+    k_day_check_body(pops[blockIdx.y], ctls[blockIdx.y], day_end, part);
 }
 
 __device__ __forceinline__ void k_socdist_fill_body(const DevPop& d, const DayCtl* ctl)
@@ -3170,13 +3201,6 @@ __device__ __forceinline__ void k_cell_totals_body(const DevPop& d)
     }
 }
 __global__ void k_cell_totals(DevPop d) { k_cell_totals_body(d); }
-__global__ void k_cell_totals_multi(const DevPop* __restrict__ pops) { k_cell_totals_body(pops[blockIdx.y]); }
-// S..D of each member's counter block to zero before k_cell_totals_multi
-__global__ void k_zero_totals_multi(const DevPop* __restrict__ pops)
-{
-    if (threadIdx.x < 5) (&pops[blockIdx.x].C->S)[threadIdx.x] = 0;
-}
-
 // ================================================================ host API
 extern "C" {
 
@@ -4082,11 +4106,61 @@ int cs_gpu_use_graphs(cs_gpu_ctx* c, int enable)
 }
 
 // ------------------------------------------------------- device run loop
-// S..D of the counter block from the cells, as cs_gpu_get_counters does.
-static int enqueue_totals(cs_gpu_ctx* c)
+// A part of the graph being captured on `main` that runs only when a kernel before it set
+// its handle: add the conditional node behind main's work so far and capture what follows
+// on `body` into it, up to cond_end.
+static cudaError_t cond_graph(cudaStream_t main, cudaGraph_t* g, const cudaGraphNode_t** deps, size_t* n)
 {
-    CK(cudaMemsetAsync(c->d.C, 0, 5 * sizeof(int64_t), c->stream));
-    LAUNCH(k_cell_totals, 64, kThreads, c->d);
+    cudaStreamCaptureStatus st;
+    unsigned long long id;
+    cudaError_t e = cudaStreamGetCaptureInfo_v2(main, &st, &id, g, deps, n);
+    return e != cudaSuccess ? e : st == cudaStreamCaptureStatusActive ? cudaSuccess : cudaErrorIllegalState;
+}
+static cudaError_t cond_handle(cudaStream_t main, cudaGraphConditionalHandle* h)
+{
+    cudaGraph_t g;
+    const cudaGraphNode_t* deps;
+    size_t n;
+    cudaError_t e = cond_graph(main, &g, &deps, &n);
+    return e != cudaSuccess ? e : cudaGraphConditionalHandleCreate(h, g, 0, cudaGraphCondAssignDefault);
+}
+static cudaError_t cond_begin(cudaStream_t main, cudaStream_t body, cudaGraphConditionalHandle h)
+{
+    cudaGraph_t g;
+    const cudaGraphNode_t* deps;
+    size_t n;
+    cudaError_t e = cond_graph(main, &g, &deps, &n);
+    if (e != cudaSuccess) return e;
+    cudaGraphNodeParams np = {};
+    np.type = cudaGraphNodeTypeConditional;
+    np.conditional.handle = h;
+    np.conditional.type = cudaGraphCondTypeIf;
+    np.conditional.size = 1;
+    cudaGraphNode_t node;
+    e = cudaGraphAddNode(&node, g, deps, n, &np);
+    if (e == cudaSuccess) e = cudaStreamUpdateCaptureDependencies(main, &node, 1, cudaStreamSetCaptureDependencies);
+    if (e == cudaSuccess)
+        e = cudaStreamBeginCaptureToGraph(body, np.conditional.phGraph_out[0], nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal);
+    return e;
+}
+static cudaError_t cond_end(cudaStream_t body)
+{
+    cudaGraph_t g;
+    return cudaStreamEndCapture(body, &g);
+}
+
+// A switch's social-distancing flags and closures, behind their gates.
+static int enqueue_change(cs_gpu_ctx* c)
+{
+    DevPop& d = c->d;
+    const int mgrid = std::max(1, std::min(c->grid, (d.NM + kThreads - 1) / kThreads));
+    LAUNCH(k_socdist_fill, mgrid, kThreads, d, (const DayCtl*)c->d_ctl);
+    for (int pt = 0; pt < d.NPT; pt++)
+        LAUNCH(k_close_places, c->grid, kThreads, d, pt, (const uint8_t*)nullptr, (uint16_t)0, (uint16_t)0, (const DayCtl*)c->d_ctl);
+    if (d.NPT > 0) {
+        LAUNCH(k_carer_pass, c->grid, kThreads, d);
+        LAUNCH(k_carer_reset, 1, 1, d);
+    }
     return CS_OK;
 }
 
@@ -4094,29 +4168,38 @@ static int enqueue_totals(cs_gpu_ctx* c)
 // (k_set_step takes t from it) and the UpdateProbs gate (&ctl->update), so the
 // same launches serve every day and can be captured once.  Order as the host loop:
 // the timesteps; after each (or the day's last) the counters and the UpdateProbs
-// test; at the day's end the series and the trigger, then the gated UpdateProbs,
-// and the switch's social-distancing flags and closures.
-static int enqueue_day(cs_gpu_ctx* c, int spd, bool every_step)
+// test; at the day's end the series and the trigger, then UpdateProbs, and the switch's
+// social-distancing flags and closures.  parts: these into a conditional part of the graph
+// being captured, else gated.  (On all but a few days the 18 launches returned at their
+// gates, about 2 us each; the part's node takes 5 to 10 us when it does not run.  Tested
+// after every timestep, 1.5 M people with admin units: 68.5 -> 63 ms.)
+static int enqueue_day(cs_gpu_ctx* c, int spd, bool every_step, bool parts)
 {
     DevPop& d = c->d;
+    const int cgrid = std::max(1, std::min(64, (d.NC + kThreads - 1) / kThreads));
     for (int s = 0; s < spd; s++) {
         int r = step_eager(c, 0.0, 0);
         if (r) return r;
-        if (!every_step && s < spd - 1) continue;
-        r = enqueue_totals(c);
-        if (r) return r;
-        LAUNCH(k_probs_check, 1, 1, d, c->d_ctl, s == spd - 1 ? 1 : 0);
-        if (s == spd - 1) LAUNCH(k_day_logic, 1, kThreads, d, c->d_ctl, (const int32_t*)c->d_clock, c->dIv);
+        const bool day_end = s == spd - 1;
+        if (!every_step && !day_end) continue;
+        cudaGraphConditionalHandle part = 0;
+        if (parts) CK(cond_handle(c->stream, &part));
+        LAUNCH(k_day_check, cgrid, kThreads, d, c->d_ctl, day_end ? 1 : 0, part);
+        const cudaStream_t main = c->stream;
+        const long long l0 = c->launches;
+        if (parts) {
+            CK(cond_begin(main, c->br.body, part));
+            c->stream = c->br.body;
+        }
         r = cs_gpu_update_probs(c, 0);
+        if (!r && day_end) r = enqueue_change(c);
+        c->launches = l0;   // neither form counts what does its work on few days
+        c->stream = main;
+        if (parts) {
+            cudaError_t e = cond_end(c->br.body);
+            if (!r && e != cudaSuccess) r = set_err(c, CS_E_CUDA, "conditional part of the day graph: %s", cudaGetErrorString(e));
+        }
         if (r) return r;
-    }
-    const int mgrid = std::max(1, std::min(c->grid, (d.NM + kThreads - 1) / kThreads));
-    LAUNCH(k_socdist_fill, mgrid, kThreads, d, (const DayCtl*)c->d_ctl);
-    for (int pt = 0; pt < d.NPT; pt++)
-        LAUNCH(k_close_places, c->grid, kThreads, d, pt, (const uint8_t*)nullptr, (uint16_t)0, (uint16_t)0, (const DayCtl*)c->d_ctl);
-    if (d.NPT > 0) {
-        LAUNCH(k_carer_pass, 64, kThreads, d);
-        LAUNCH(k_carer_reset, 1, 1, d);
     }
     return CS_OK;
 }
@@ -4128,7 +4211,7 @@ static int capture_day(cs_gpu_ctx* c, int spd, bool every_step)
     cudaGraph_t g = nullptr;
     CK(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
     long long l0 = c->launches;
-    r = enqueue_day(c, spd, every_step);
+    r = enqueue_day(c, spd, every_step, !c->capturing_prof);
     cudaError_t e = cudaStreamEndCapture(c->stream, &g);
     if (r || e != cudaSuccess) {
         if (g) cudaGraphDestroy(g);
@@ -4169,7 +4252,7 @@ static int run_days(cs_gpu_ctx* c, int days, int spd, bool every_step)
             c->launches += c->day_launches;
             if (c->day_graph_prof) prof_graph_collect(c);
         } else {
-            int r = enqueue_day(c, spd, every_step);
+            int r = enqueue_day(c, spd, every_step, false);
             if (r) return r;
         }
     }
@@ -4282,7 +4365,7 @@ struct cs_gpu_batch {
     Branches br;              // kernels of a batched timestep that run side by side
     bool fused = false;       // the form of the timestep the graphs were captured with
     // device run loop (cs_gpu_batch_run): members' DevPop with step clocks and
-    // UpdateProbs gates, their control blocks, one graph per day
+    // UpdateProbs gates, their control blocks, one graph per day (with conditional parts)
     DevPop* d_pops_day = nullptr;
     DayCtl** d_ctls = nullptr;
     cudaGraph_t day_graph = nullptr;
@@ -4543,14 +4626,14 @@ int cs_gpu_batch_sync(cs_gpu_batch* b)
 }
 
 // ------------------------------------------------------- batched run loop
-// The single-context day (enqueue_day) for every member at once: the batched
-// timesteps, then the members' totals, UpdateProbs tests and day logic as one
-// launch each (blockIdx selects the member), and each member's gated UpdateProbs
-// chain on one of kSide side streams, forked from and joined back into the
-// batch's stream, so that the chains' mostly empty launches overlap.
-static int batch_updates(cs_gpu_batch* b)
+// The single-context day (enqueue_day) for every member at once: the batched timesteps,
+// then the members' totals, UpdateProbs tests and day logic as one launch (blockIdx selects
+// the member), and, in a conditional part of the graph, each member's gated UpdateProbs
+// chain on one of kSide side streams, forked from and joined back into the part's stream,
+// so that the chains overlap.
+static int batch_updates(cs_gpu_batch* b, cudaStream_t main)
 {
-    BCK(cudaEventRecord(b->ev_fork, b->stream));
+    BCK(cudaEventRecord(b->ev_fork, main));
     for (int i = 0; i < cs_gpu_batch::kSide; i++) BCK(cudaStreamWaitEvent(b->side[i], b->ev_fork, 0));
     int r = CS_OK;
     for (size_t k = 0; k < b->members.size() && !r; k++) {
@@ -4558,7 +4641,6 @@ static int batch_updates(cs_gpu_batch* b)
         m->stream = b->side[k % cs_gpu_batch::kSide];
         const long long l0 = m->launches;
         r = cs_gpu_update_probs(m, 0);
-        b->member_day_launches[k] += m->launches - l0;
         m->launches = l0;
         m->stream = b->stream;
         if (r) batch_err(b, r, "member %zu UpdateProbs: %s", k, m->err);
@@ -4566,39 +4648,50 @@ static int batch_updates(cs_gpu_batch* b)
     // joined even after an error, so that the capture can end
     for (int i = 0; i < cs_gpu_batch::kSide; i++) {
         cudaEventRecord(b->ev_join[i], b->side[i]);
-        cudaStreamWaitEvent(b->stream, b->ev_join[i], 0);
+        cudaStreamWaitEvent(main, b->ev_join[i], 0);
     }
     return r;
 }
 
+// enqueue_day for the batch: the parts run on a day on which any member needs them, each
+// member's kernels behind its own gates.
 static int batch_enqueue_day(cs_gpu_batch* b, int spd, bool every_step)
 {
     const int R = (int)b->members.size();
     const DevPop* pops = b->d_pops_day;
-    int npt = 0;
-    for (cs_gpu_ctx* m : b->members) npt = std::max(npt, m->d.NPT);
+    int npt = 0, maxc = 0;
+    for (cs_gpu_ctx* m : b->members) {
+        npt = std::max(npt, m->d.NPT);
+        maxc = std::max(maxc, m->d.NC);
+    }
+    const int cgrid = std::max(1, std::min(64, (maxc + kThreads - 1) / kThreads));
     for (int s = 0; s < spd; s++) {
         int r = batch_enqueue(b, pops);
         if (r) return r;
         for (int k = 0; k < R; k++) b->member_day_launches[k] += batch_kernels(b);
-        if (!every_step && s < spd - 1) continue;
-        const int day_end = s == spd - 1 ? 1 : 0;
-        BLAUNCH(k_zero_totals_multi, R, 32, pops);
-        BLAUNCH(k_cell_totals_multi, dim3(64, R), kThreads, pops);
-        BLAUNCH(k_probs_check_multi, R, 1, pops, b->d_ctls, day_end);
-        if (day_end) BLAUNCH(k_day_logic_multi, R, kThreads, pops, b->d_ctls);
-        for (int k = 0; k < R; k++) b->member_day_launches[k] += 2 + day_end;
-        r = batch_updates(b);
+        const bool day_end = s == spd - 1;
+        if (!every_step && !day_end) continue;
+        cudaGraphConditionalHandle part;
+        BCK(cond_handle(b->stream, &part));
+        BLAUNCH(k_day_check_multi, dim3(cgrid, R), kThreads, pops, b->d_ctls, day_end ? 1 : 0, part);
+        for (int k = 0; k < R; k++) b->member_day_launches[k]++;
+        const cudaStream_t body = b->br.body;
+        BCK(cond_begin(b->stream, body, part));
+        r = batch_updates(b, body);
+        if (!r && day_end) {
+            const dim3 g(std::min(b->members[0]->grid, std::max(64, (6 * b->members[0]->nsm + R - 1) / R)), R);
+            k_socdist_fill_multi<<<g, kThreads, 0, body>>>(pops, b->d_ctls);
+            for (int pt = 0; pt < npt; pt++) k_close_places_multi<<<g, kThreads, 0, body>>>(pops, pt, b->d_ctls);
+            if (npt > 0) {
+                k_carer_pass_multi<<<g, kThreads, 0, body>>>(pops);
+                k_carer_reset_multi<<<R, 1, 0, body>>>(pops);
+            }
+        }
+        const cudaError_t el = cudaGetLastError(), e = cond_end(body);
         if (r) return r;
+        BCK(el);
+        BCK(e);
     }
-    const dim3 g(b->members[0]->grid, R);
-    BLAUNCH(k_socdist_fill_multi, g, kThreads, pops, b->d_ctls);
-    for (int pt = 0; pt < npt; pt++) BLAUNCH(k_close_places_multi, g, kThreads, pops, pt, b->d_ctls);
-    if (npt > 0) {
-        BLAUNCH(k_carer_pass_multi, dim3(64, R), kThreads, pops);
-        BLAUNCH(k_carer_reset_multi, R, 1, pops);
-    }
-    for (int k = 0; k < R; k++) b->member_day_launches[k] += 1 + b->members[k]->d.NPT + (npt > 0 ? 2 : 0);
     return CS_OK;
 }
 
@@ -4764,7 +4857,7 @@ int cs_gpu_close_places(cs_gpu_ctx* c, int pt, const int32_t* mcells, int n_mcel
         CK(cudaMemcpyAsync(sel, h.data(), c->d.NM, cudaMemcpyHostToDevice, c->stream));
     }
     LAUNCH(k_close_places, c->grid, kThreads, c->d, pt, sel, start, stop, (const DayCtl*)nullptr);
-    LAUNCH(k_carer_pass, 64, kThreads, c->d);
+    LAUNCH(k_carer_pass, c->grid, kThreads, c->d);
     LAUNCH(k_carer_reset, 1, 1, c->d);
     if (sel) {
         CK(cudaStreamSynchronize(c->stream));
@@ -4806,7 +4899,7 @@ int cs_gpu_place_events(cs_gpu_ctx* c, const cs_place_event* ev, int n)
         int i1 = i0;
         while (i1 < n && key(v[i1]) == key(v[i0])) i1++;
         if (v[i0].kind == CS_PLACE_EV_HOLIDAY && closes) {   // the closures' carers before the holidays
-            LAUNCH(k_carer_pass, 64, kThreads, c->d);
+            LAUNCH(k_carer_pass, c->grid, kThreads, c->d);
             LAUNCH(k_carer_reset, 1, 1, c->d);
             closes = false;
         }
@@ -4815,7 +4908,7 @@ int cs_gpu_place_events(cs_gpu_ctx* c, const cs_place_event* ev, int n)
         i0 = i1;
     }
     if (closes) {
-        LAUNCH(k_carer_pass, 64, kThreads, c->d);
+        LAUNCH(k_carer_pass, c->grid, kThreads, c->d);
         LAUNCH(k_carer_reset, 1, 1, c->d);
     }
     CK(cudaStreamSynchronize(c->stream));
