@@ -53,7 +53,8 @@ __device__ __forceinline__ void mma_bf16(float c[4], const uint32_t a[4], const 
 // and writes its partial product to C + z * cstride (no bias, ReLU or BF16 output).
 __global__ void __launch_bounds__(128) k_gemm_nt(const bf16* __restrict__ A, int lda, const bf16* __restrict__ B, int ldb,
                                                  float* __restrict__ C, int ldc, bf16* __restrict__ Cb, int ldcb,
-                                                 const float* __restrict__ bias, int relu, int K, int kchunk, size_t cstride)
+                                                 const float* __restrict__ bias, int relu, int K, int kchunk, size_t cstride,
+                                                 const bf16* __restrict__ mask)
 {
     if (gridDim.z > 1) {
         const int z = blockIdx.z;
@@ -117,6 +118,10 @@ __global__ void __launch_bounds__(128) k_gemm_nt(const bf16* __restrict__ A, int
                 float v0 = acc[mi][ni][2 * h], v1 = acc[mi][ni][2 * h + 1];
                 if (bias) { v0 += bias[c]; v1 += bias[c + 1]; }
                 if (relu) { v0 = fmaxf(v0, 0.f); v1 = fmaxf(v1, 0.f); }
+                if (mask) {
+                    if (!(__bfloat162float(mask[(size_t)r * ldc + c]) > 0.f)) v0 = 0.f;
+                    if (!(__bfloat162float(mask[(size_t)r * ldc + c + 1]) > 0.f)) v1 = 0.f;
+                }
                 if (C) { C[(size_t)r * ldc + c] = v0; C[(size_t)r * ldc + c + 1] = v1; }
                 if (Cb) *reinterpret_cast<__nv_bfloat162*>(Cb + (size_t)r * ldcb + c) = __floats2bfloat162_rn(v0, v1);
             }
@@ -234,6 +239,8 @@ __device__ __forceinline__ void stage_conv_rows(unsigned char* dst, const bf16* 
 
 }  // namespace tc
 
+// mask (leading dimension ldc, may be null): outputs where it is not positive are zero, the
+// backward ReLU of the activation it holds.
 // C[M,N] = A[M,K] B[N,K]^T (+ bias) (ReLU) on tcgen05; N a multiple of BN, K of 64;
 // split K as k_gemm_nt (gridDim.z slices of kchunk, partial products at C + z * cstride).
 // With H set, A is the column matrix of a convolution of H (hT time points, hCin
@@ -242,7 +249,8 @@ template <int BN>
 __global__ void __launch_bounds__(128) k_gemm_tc(const bf16* __restrict__ A, int lda, const bf16* __restrict__ B, int ldb,
                                                  float* __restrict__ C, int ldc, bf16* __restrict__ Cb, int ldcb,
                                                  const float* __restrict__ bias, int relu, int M, int K, int kchunk,
-                                                 size_t cstride, int* err, const bf16* __restrict__ H, int hT, int hCin)
+                                                 size_t cstride, int* err, const bf16* __restrict__ H, int hT, int hCin,
+                                                 const bf16* __restrict__ mask)
 {
     using namespace tc;
     extern __shared__ unsigned char smem_raw[];
@@ -317,6 +325,11 @@ __global__ void __launch_bounds__(128) k_gemm_tc(const bf16* __restrict__ A, int
                     if (nk == 0) v0 = v1 = 0.f;
                     if (bias) { v0 += bias[col + j]; v1 += bias[col + j + 1]; }
                     if (relu) { v0 = fmaxf(v0, 0.f); v1 = fmaxf(v1, 0.f); }
+                    if (mask) {
+                        const __nv_bfloat162 h = *reinterpret_cast<const __nv_bfloat162*>(mask + (size_t)row * ldc + col + j);
+                        if (!(__low2float(h) > 0.f)) v0 = 0.f;
+                        if (!(__high2float(h) > 0.f)) v1 = 0.f;
+                    }
                     if (C) *reinterpret_cast<float2*>(C + (size_t)row * ldc + col + j) = make_float2(v0, v1);
                     if (Cb) *reinterpret_cast<__nv_bfloat162*>(Cb + (size_t)row * ldcb + col + j) = __floats2bfloat162_rn(v0, v1);
                 }
@@ -333,7 +346,8 @@ __global__ void __launch_bounds__(128) k_gemm_tc(const bf16* __restrict__ A, int
 // C[r, c] = sum over the slices z, in ascending order, of part[z][r, c] ([M, N] each),
 // then the product's epilogue (bias, ReLU, FP32 and/or BF16 stores).
 __global__ void k_splitk_reduce(const float* __restrict__ part, int nsplit, int M, int N, float* __restrict__ C, int ldc,
-                                bf16* __restrict__ Cb, int ldcb, const float* __restrict__ bias, int relu)
+                                bf16* __restrict__ Cb, int ldcb, const float* __restrict__ bias, int relu,
+                                const bf16* __restrict__ mask)
 {
     const size_t MN = (size_t)M * N;
     for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < MN; e += (size_t)gridDim.x * blockDim.x) {
@@ -342,6 +356,7 @@ __global__ void k_splitk_reduce(const float* __restrict__ part, int nsplit, int 
         const size_t r = e / N, c = e % N;
         if (bias) acc += bias[c];
         if (relu) acc = fmaxf(acc, 0.f);
+        if (mask && !(__bfloat162float(mask[r * ldc + c]) > 0.f)) acc = 0.f;
         if (C) C[r * ldc + c] = acc;
         if (Cb) Cb[r * ldcb + c] = __float2bfloat16_rn(acc);
     }
@@ -426,17 +441,6 @@ __global__ void k_col2im_up_relu(const float* __restrict__ dcols, int ldd, int B
     }
 }
 
-// dz = dh * (h > 0), FP32 and BF16 copies (dense [rows, ld]).
-__global__ void k_relu_back(const float* __restrict__ dh, const bf16* __restrict__ h, size_t n, float* __restrict__ dz,
-                            bf16* __restrict__ dzb)
-{
-    for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < n; e += (size_t)gridDim.x * blockDim.x) {
-        float v = __bfloat162float(h[e]) > 0.f ? dh[e] : 0.f;
-        dz[e] = v;
-        dzb[e] = __float2bfloat16(v);
-    }
-}
-
 // Column sums of dz [rows, ld] in a fixed order: part[chunk, col] over row chunks
 // of 256, then the chunks in ascending order.
 // Column sums of dz [rows, ld] in a fixed order.  Block (x, y) covers 32 columns
@@ -476,10 +480,10 @@ __global__ void k_colsum_final(const float* __restrict__ part, int nchunks, int 
     if (threadIdx.y == 0 && col < ld) out[col] = v;
 }
 
-// Loss terms and the output gradient: y is [B*368, 64] (channels < 4 used), target
+// Loss terms and the output gradient (FP32 and BF16): y is [B*368, 64] (channels < 4 used), target
 // [n, 365, 4]; rows of samples >= n and time points >= 365 get zero gradient.
 __global__ void k_mse(const float* __restrict__ y, const float* __restrict__ target, int n, int Bp, float scale,
-                      float* __restrict__ dy, float* __restrict__ sq)
+                      float* __restrict__ dy, bf16* __restrict__ dyb, float* __restrict__ sq)
 {
     const int T = 2 * 2 * 2 * kT0;   // 368
     const size_t total = (size_t)Bp * T * kCh;
@@ -494,6 +498,7 @@ __global__ void k_mse(const float* __restrict__ y, const float* __restrict__ tar
             sq[((size_t)b * kTOut + t) * kNOut + c] = d * d;
         }
         dy[e] = g;
+        dyb[e] = __float2bfloat16(g);
     }
 }
 
@@ -529,8 +534,10 @@ __global__ void k_sum_final(const double* __restrict__ part, int n, double* __re
 }
 
 __global__ void k_adam(float* __restrict__ w, float* __restrict__ m, float* __restrict__ v, const float* __restrict__ g,
-                       bf16* __restrict__ wb, size_t n, float lr, float b1, float b2, float eps, float c1, float c2, float wd)
+                       bf16* __restrict__ wb, size_t n, float lr, float b1, float b2, float eps, float c1, float c2, float wd,
+                       const int* __restrict__ err)
 {
+    if (*err) return;   // a product of this step gave up: the weights stay
     for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < n; e += (size_t)gridDim.x * blockDim.x) {
         float gi = g[e];
         float mi = b1 * m[e] + (1.f - b1) * gi;
@@ -583,6 +590,19 @@ struct Layer {
     size_t wofs, bofs;  // offsets in the padded parameter arrays
 };
 
+// A chain of kernels with scratch of its own.  A training step is four such chains: the
+// forward pass and the gradients of the activations (0); the weight gradients, alternate
+// layers (1 and 2); the bias gradients, transposed weights and loss (3).
+constexpr int kLanes = 4;
+struct Lane {
+    cudaStream_t st = nullptr;
+    cudaEvent_t done = nullptr;
+    float* kpart = nullptr;                 // split-K partial products
+    size_t kpart_n = 0;
+    bf16 *dzT = nullptr, *colsT = nullptr;  // transposed operands of a weight gradient
+    float* part = nullptr;                  // column sums
+};
+
 struct cs_sur {
     int device = 0;
     int bmax = 0;       // batch capacity (multiple of 64)
@@ -596,16 +616,28 @@ struct cs_sur {
     // activations and scratch sized for bmax
     std::vector<bf16*> act;                 // act[0] = input, act[l+1] = output of layer l (BF16)
     float* yout = nullptr;                  // last layer output FP32 [bmax*368, 64]
-    bf16 *cols[3] = {nullptr, nullptr, nullptr};
-    bf16 *colsT = nullptr, *dzT = nullptr, *wT = nullptr, *hT = nullptr;
-    float *dz = nullptr, *dh = nullptr, *dcols = nullptr, *part = nullptr;
-    float* kpart = nullptr;                 // split-K partial products
-    size_t kpart_n = 0;
+    bf16* cols[3] = {nullptr, nullptr, nullptr};   // column matrices of the mma.sync path
+    std::vector<float*> dz;                 // gradient at layer l's output before its ReLU (FP32, BF16); one per
+    std::vector<bf16*> dzb;                 // layer, as a layer's weight gradient runs beside the layers below it
+    std::vector<bf16*> wT;                  // transposed BF16 weights per layer
+    float* dcols = nullptr;
+    Lane lane[kLanes];                      // [0] the main chain, the others beside it
+    cudaEvent_t fork = nullptr;
+    std::vector<cudaEvent_t> dz_ready;      // per layer: its dz is written
     double *lpart = nullptr, *lsum = nullptr;   // loss reduction
     int* d_err = nullptr;                   // set by a tensor-core GEMM whose wait gave up
     int gemm_impl = 0;                      // 0: tcgen05, 1: mma.sync
-    bf16* dzb = nullptr;
     float *xdev = nullptr, *tdev = nullptr, *sq = nullptr, *ydev = nullptr;
+    // one training step (or loss and gradient) of n rows as a graph
+    struct StepGraph {
+        int n = 0;
+        bool update = false;
+        cudaGraph_t graph = nullptr;
+        cudaGraphExec_t exec = nullptr;
+        cudaGraphNode_t adam = nullptr;
+        cudaKernelNodeParams adam_params{};
+    };
+    std::vector<StepGraph> graphs;          // the most recent batch sizes
     std::vector<void*> allocs;
 };
 
@@ -638,6 +670,15 @@ static int salloc(cs_sur* s, T** p, size_t n)
     return CS_OK;
 }
 
+static void drop_graphs(cs_sur* s)
+{
+    for (auto& g : s->graphs) {
+        if (g.exec) cudaGraphExecDestroy(g.exec);
+        if (g.graph) cudaGraphDestroy(g.graph);
+    }
+    s->graphs.clear();
+}
+
 static void build_layers(cs_sur* s)
 {
     s->L.clear();
@@ -664,30 +705,31 @@ static void build_layers(cs_sur* s)
 constexpr int kLossBlocks = 296;
 
 // One product (or, with nsplit > 1, its K slices of kchunk) on the selected path.
-static int gemm_launch(cs_sur* s, const bf16* A, int lda, const bf16* B, int ldb, float* C, int ldc, bf16* Cb, int ldcb,
-                       const float* bias, int relu, int M, int N, int K, int nsplit, int kchunk, size_t cstride)
+static int gemm_launch(cs_sur* s, const Lane& w, const bf16* A, int lda, const bf16* B, int ldb, float* C, int ldc, bf16* Cb,
+                       int ldcb, const float* bias, int relu, int M, int N, int K, int nsplit, int kchunk, size_t cstride,
+                       const bf16* mask)
 {
     if (s->gemm_impl == 0 && K % 64 == 0 && kchunk % 64 == 0) {
         dim3 grid(N / 64, (M + tc::BM - 1) / tc::BM, nsplit);
-        k_gemm_tc<64><<<grid, 128, tc::smem_bytes(64), s->stream>>>(A, lda, B, ldb, C, ldc, Cb, ldcb, bias, relu, M, K,
-                                                                    kchunk, cstride, s->d_err, nullptr, 0, 0);
+        k_gemm_tc<64><<<grid, 128, tc::smem_bytes(64), w.st>>>(A, lda, B, ldb, C, ldc, Cb, ldcb, bias, relu, M, K,
+                                                               kchunk, cstride, s->d_err, nullptr, 0, 0, mask);
     } else {
         dim3 grid(N / 64, M / 64, nsplit);
-        sur::k_gemm_nt<<<grid, 128, 0, s->stream>>>(A, lda, B, ldb, C, ldc, Cb, ldcb, bias, relu, K, kchunk, cstride);
+        sur::k_gemm_nt<<<grid, 128, 0, w.st>>>(A, lda, B, ldb, C, ldc, Cb, ldcb, bias, relu, K, kchunk, cstride, mask);
     }
     SCK(cudaGetLastError());
     return CS_OK;
 }
 
-// C = A B^T (+ bias) (ReLU).  A product with few output tiles and a long K (the
+// C = A B^T (+ bias) (ReLU) (mask).  A product with few output tiles and a long K (the
 // convolutions' weight gradients, K = batch x time points; the linear layers at
 // batch sizes of a few hundred) is split along K so that about two blocks per SM
 // run; the slices' partial products are then summed in a fixed order and the
 // epilogue applied.
 constexpr int kMaxSplit = 64;
 
-static int gemm(cs_sur* s, const bf16* A, int lda, const bf16* B, int ldb, float* C, int ldc, bf16* Cb, int ldcb,
-                const float* bias, int relu, int M, int N, int K)
+static int gemm(cs_sur* s, const Lane& w, const bf16* A, int lda, const bf16* B, int ldb, float* C, int ldc, bf16* Cb,
+                int ldcb, const float* bias, int relu, int M, int N, int K, const bf16* mask = nullptr)
 {
     if (M % 64 || N % 64 || K % 32) return sur_err(s, CS_E_ARG, "gemm shape %d x %d x %d not padded", M, N, K);
     const int tiles = (s->gemm_impl == 0 ? (M + tc::BM - 1) / tc::BM : M / 64) * (N / 64);
@@ -695,24 +737,24 @@ static int gemm(cs_sur* s, const bf16* A, int lda, const bf16* B, int ldb, float
     if (nsplit > 1 && K % 64 == 0) {
         const int kchunk = ((K + nsplit - 1) / nsplit + 63) / 64 * 64;
         nsplit = (K + kchunk - 1) / kchunk;
-        if (nsplit > 1 && (size_t)nsplit * M * N <= s->kpart_n) {
-            int r = gemm_launch(s, A, lda, B, ldb, s->kpart, N, nullptr, 0, nullptr, 0, M, N, K, nsplit, kchunk,
-                                (size_t)M * N);
+        if (nsplit > 1 && (size_t)nsplit * M * N <= w.kpart_n) {
+            int r = gemm_launch(s, w, A, lda, B, ldb, w.kpart, N, nullptr, 0, nullptr, 0, M, N, K, nsplit, kchunk,
+                                (size_t)M * N, nullptr);
             if (r) return r;
             const int rg = (int)std::min<size_t>(1184, ((size_t)M * N + 255) / 256);
-            sur::k_splitk_reduce<<<rg, 256, 0, s->stream>>>(s->kpart, nsplit, M, N, C, ldc, Cb, ldcb, bias, relu);
+            sur::k_splitk_reduce<<<rg, 256, 0, w.st>>>(w.kpart, nsplit, M, N, C, ldc, Cb, ldcb, bias, relu, mask);
             SCK(cudaGetLastError());
             return CS_OK;
         }
     }
-    return gemm_launch(s, A, lda, B, ldb, C, ldc, Cb, ldcb, bias, relu, M, N, K, 1, K, 0);
+    return gemm_launch(s, w, A, lda, B, ldb, C, ldc, Cb, ldcb, bias, relu, M, N, K, 1, K, 0, mask);
 }
 
 
-static int transpose(cs_sur* s, const bf16* in, int ldi, bf16* out, int ldo, int R, int Cc)
+static int transpose(cs_sur* s, const Lane& w, const bf16* in, int ldi, bf16* out, int ldo, int R, int Cc)
 {
     dim3 grid(Cc / 32, R / 32), block(32, 8);
-    sur::k_transpose<<<grid, block, 0, s->stream>>>(in, ldi, out, ldo, R, Cc);
+    sur::k_transpose<<<grid, block, 0, w.st>>>(in, ldi, out, ldo, R, Cc);
     SCK(cudaGetLastError());
     return CS_OK;
 }
@@ -767,17 +809,38 @@ int cs_sur_create(int max_batch, int device, cs_sur** out)
     }
     for (auto& l : s->L) maxw = std::max(maxw, (size_t)l.outP * l.inP);
     SA(s->yout, (size_t)B * 8 * kT0 * kCh);
-    SA(s->colsT, maxcol);
     SA(s->dcols, maxcol);
-    size_t maxz = std::max(maxc, (size_t)B * 8 * kT0 * kCh);
-    SA(s->dz, maxz); SA(s->dzb, maxz); SA(s->dzT, maxz); SA(s->dh, maxz); SA(s->hT, maxz);
-    SA(s->wT, maxw);
-    SA(s->part, (size_t)((B * 8 * kT0 + 255) / 256 + 1) * 3000);
-    {
-        size_t mn = 0;
-        for (int i = 0; i < 3; i++) mn = std::max(mn, (size_t)s->L[6 + i].outP * s->L[6 + i].inP);
-        s->kpart_n = std::max(mn * kMaxSplit, (size_t)4 << 20);
-        SA(s->kpart, s->kpart_n);
+    const size_t maxz = std::max(maxc, (size_t)B * 8 * kT0 * kCh);
+    s->dz.assign(s->L.size(), nullptr);
+    s->dzb.assign(s->L.size(), nullptr);
+    s->wT.assign(s->L.size(), nullptr);
+    s->dz_ready.assign(s->L.size(), nullptr);
+    for (size_t li = 0; li < s->L.size(); li++) {
+        const Layer& l = s->L[li];
+        const size_t n = l.conv ? (size_t)B * l.T * kCh : (size_t)B * l.outP;
+        SA(s->dz[li], n); SA(s->dzb[li], n);
+        SA(s->wT[li], (size_t)l.outP * l.inP);
+        SCK(cudaEventCreateWithFlags(&s->dz_ready[li], cudaEventDisableTiming));
+    }
+    SCK(cudaEventCreateWithFlags(&s->fork, cudaEventDisableTiming));
+    size_t mn = 0;
+    for (int i = 0; i < 3; i++) mn = std::max(mn, (size_t)s->L[6 + i].outP * s->L[6 + i].inP);
+    for (int k = 0; k < kLanes; k++) {
+        Lane& w = s->lane[k];
+        if (k == 0) w.st = s->stream;
+        else {
+            SCK(cudaStreamCreateWithFlags(&w.st, cudaStreamNonBlocking));
+            SCK(cudaEventCreateWithFlags(&w.done, cudaEventDisableTiming));
+        }
+        if (k < 3) {
+            w.kpart_n = std::max(mn * kMaxSplit, (size_t)4 << 20);
+            SA(w.kpart, w.kpart_n);
+        }
+        if (k == 1 || k == 2) {
+            SA(w.dzT, maxz);
+            SA(w.colsT, std::max(maxcol, maxz));
+        }
+        if (k == 3) SA(w.part, (size_t)((B * 8 * kT0 + 255) / 256 + 1) * 3000);
     }
     SA(s->lpart, (size_t)kLossBlocks); SA(s->lsum, (size_t)1); SA(s->d_err, (size_t)1);
     SCK(cudaMemsetAsync(s->d_err, 0, sizeof(int), s->stream));
@@ -793,7 +856,15 @@ void cs_sur_destroy(cs_sur* s)
 {
     if (!s) return;
     if (s->stream) cudaStreamSynchronize(s->stream);
+    drop_graphs(s);
     for (void* p : s->allocs) cudaFree(p);
+    for (Lane& w : s->lane) {
+        if (w.st && w.st != s->stream) cudaStreamDestroy(w.st);
+        if (w.done) cudaEventDestroy(w.done);
+    }
+    for (cudaEvent_t e : s->dz_ready)
+        if (e) cudaEventDestroy(e);
+    if (s->fork) cudaEventDestroy(s->fork);
     if (s->stream) cudaStreamDestroy(s->stream);
     delete s;
 }
@@ -841,9 +912,10 @@ int cs_sur_get_params(cs_sur* s, float* flat)
 static int forward(cs_sur* s, int Bp)
 {
     int r;
+    const Lane& w = s->lane[0];
     for (int li = 0; li < 6; li++) {
         const Layer& l = s->L[li];
-        if ((r = gemm(s, s->act[li], l.inP, s->wb + l.wofs, l.inP, nullptr, 0, s->act[li + 1], l.outP,
+        if ((r = gemm(s, w, s->act[li], l.inP, s->wb + l.wofs, l.inP, nullptr, 0, s->act[li + 1], l.outP,
                       s->w + l.bofs, 1, Bp, l.outP, l.inP))) return r;
     }
     int T = kT0;
@@ -855,14 +927,14 @@ static int forward(cs_sur* s, int Bp)
         const int M = Bp * 2 * T;
         if (s->gemm_impl == 0) {   // the column matrix is generated while staging
             dim3 grid(l.outP / 64, (M + tc::BM - 1) / tc::BM, 1);
-            k_gemm_tc<64><<<grid, 128, tc::smem_bytes(64), s->stream>>>(nullptr, 0, s->wb + l.wofs, l.inP, C, kCh, Cb, kCh,
-                                                                        s->w + l.bofs, l.relu ? 1 : 0, M, l.inP, l.inP, 0,
-                                                                        s->d_err, s->act[6 + ci], T, l.cin);
+            k_gemm_tc<64><<<grid, 128, tc::smem_bytes(64), w.st>>>(nullptr, 0, s->wb + l.wofs, l.inP, C, kCh, Cb, kCh,
+                                                                   s->w + l.bofs, l.relu ? 1 : 0, M, l.inP, l.inP, 0,
+                                                                   s->d_err, s->act[6 + ci], T, l.cin, nullptr);
             SCK(cudaGetLastError());
         } else {
-            sur::k_im2col_up<<<1184, 256, 0, s->stream>>>(s->act[6 + ci], Bp, T, l.cin, s->cols[ci], l.inP);
+            sur::k_im2col_up<<<1184, 256, 0, w.st>>>(s->act[6 + ci], Bp, T, l.cin, s->cols[ci], l.inP);
             SCK(cudaGetLastError());
-            if ((r = gemm(s, s->cols[ci], l.inP, s->wb + l.wofs, l.inP, C, kCh, Cb, kCh, s->w + l.bofs, l.relu ? 1 : 0,
+            if ((r = gemm(s, w, s->cols[ci], l.inP, s->wb + l.wofs, l.inP, C, kCh, Cb, kCh, s->w + l.bofs, l.relu ? 1 : 0,
                           M, l.outP, l.inP))) return r;
         }
         T *= 2;
@@ -870,60 +942,84 @@ static int forward(cs_sur* s, int Bp)
     return CS_OK;
 }
 
-static int colsum(cs_sur* s, const float* dz, int rows, int ld, float* out)
+static int colsum(cs_sur* s, const Lane& w, const float* dz, int rows, int ld, float* out)
 {
     const int nch = (rows + kColChunk - 1) / kColChunk;
     const dim3 blk(32, 8);
-    sur::k_colsum_part<<<dim3((ld + 31) / 32, nch), blk, 0, s->stream>>>(dz, rows, ld, s->part);
-    sur::k_colsum_final<<<(ld + 31) / 32, blk, 0, s->stream>>>(s->part, nch, ld, out);
+    sur::k_colsum_part<<<dim3((ld + 31) / 32, nch), blk, 0, w.st>>>(dz, rows, ld, w.part);
+    sur::k_colsum_final<<<(ld + 31) / 32, blk, 0, w.st>>>(w.part, nch, ld, out);
     SCK(cudaGetLastError());
     return CS_OK;
 }
 
-// Backward pass from dy (in s->dh as [Bp*368, 64] FP32) to gradients in s->g.
+// The side chains of a step start here: transposed weights for the backward products.
+static int begin_lanes(cs_sur* s)
+{
+    int r;
+    SCK(cudaEventRecord(s->fork, s->stream));
+    for (int k = 1; k < kLanes; k++) SCK(cudaStreamWaitEvent(s->lane[k].st, s->fork, 0));
+    for (size_t li = 1; li < s->L.size(); li++) {
+        const Layer& l = s->L[li];
+        if ((r = transpose(s, s->lane[3], s->wb + l.wofs, l.inP, s->wT[li], l.outP, l.outP, l.inP))) return r;
+    }
+    SCK(cudaEventRecord(s->lane[3].done, s->lane[3].st));
+    return CS_OK;
+}
+
+// Weight and bias gradients of layer li from its dz (rows x outP), beside the main chain.
+static int weight_grad(cs_sur* s, int li, int rows, int Tin)
+{
+    int r;
+    const Layer& l = s->L[li];
+    const int ld = l.conv ? kCh : l.outP;
+    SCK(cudaEventRecord(s->dz_ready[li], s->stream));
+    const Lane& w = s->lane[1 + (li & 1)];
+    SCK(cudaStreamWaitEvent(w.st, s->dz_ready[li], 0));
+    SCK(cudaStreamWaitEvent(s->lane[3].st, s->dz_ready[li], 0));
+    // dW = dz^T in: A = dz^T [outP, rows], B = in^T [inP, rows]
+    if ((r = transpose(s, w, s->dzb[li], ld, w.dzT, rows, rows, l.outP))) return r;
+    if (l.conv) {   // the transposed column matrix of the convolution's input, from the input itself
+        dim3 grid(l.inP / 32, rows / 32), blk(32, 8);
+        sur::k_im2colT_up<<<grid, blk, 0, w.st>>>(s->act[li], Tin, l.cin, w.colsT, rows);
+        SCK(cudaGetLastError());
+    } else if ((r = transpose(s, w, s->act[li], l.inP, w.colsT, rows, rows, l.inP)))
+        return r;
+    if ((r = gemm(s, w, w.dzT, rows, w.colsT, rows, s->g + l.wofs, l.inP, nullptr, 0, nullptr, 0, l.outP, l.inP, rows))) return r;
+    return colsum(s, s->lane[3], s->dz[li], rows, ld, s->g + l.bofs);
+}
+
+// Backward pass from dy (in the last layer's dz, FP32 and BF16) to gradients in s->g; the
+// side chains are joined.
 static int backward(cs_sur* s, int Bp)
 {
     int r;
+    const Lane& w = s->lane[0];
+    SCK(cudaStreamWaitEvent(w.st, s->lane[3].done, 0));   // the transposed weights
     // ---- convolutions, last to first
-    // dz of the last conv is dy (no ReLU)
-    {
-        size_t n = (size_t)Bp * 8 * kT0 * kCh;
-        sur::k_to_bf16<<<1184, 256, 0, s->stream>>>(s->dh, s->dzb, n);
-        SCK(cudaMemcpyAsync(s->dz, s->dh, sizeof(float) * n, cudaMemcpyDeviceToDevice, s->stream));
-    }
     int T = 8 * kT0;
-    for (int ci = 2; ci >= 0; ci--) {
-        const Layer& l = s->L[6 + ci];
+    for (int li = 8; li >= 6; li--) {
+        const Layer& l = s->L[li];
         const int M = Bp * T;
-        // dW = dz^T cols: A = dz^T [outP, M], B = cols^T [inP, M]
-        if ((r = transpose(s, s->dzb, kCh, s->dzT, M, M, l.outP))) return r;
-        {   // the transposed column matrix of this convolution's input, from the input itself
-            dim3 grid(l.inP / 32, M / 32), blk(32, 8);
-            sur::k_im2colT_up<<<grid, blk, 0, s->stream>>>(s->act[6 + ci], T / 2, l.cin, s->colsT, M);
-            SCK(cudaGetLastError());
-        }
-        if ((r = gemm(s, s->dzT, M, s->colsT, M, s->g + l.wofs, l.inP, nullptr, 0, nullptr, 0, l.outP, l.inP, M))) return r;
-        if ((r = colsum(s, s->dz, M, kCh, s->g + l.bofs))) return r;
+        if ((r = weight_grad(s, li, M, T / 2))) return r;
         // dcols = dz W: A = dz [M, outP], B = W^T [inP, outP]
-        if ((r = transpose(s, s->wb + l.wofs, l.inP, s->wT, l.outP, l.outP, l.inP))) return r;
-        if ((r = gemm(s, s->dzb, kCh, s->wT, l.outP, s->dcols, l.inP, nullptr, 0, nullptr, 0, M, l.inP, l.outP))) return r;
+        if ((r = gemm(s, w, s->dzb[li], kCh, s->wT[li], l.outP, s->dcols, l.inP, nullptr, 0, nullptr, 0, M, l.inP, l.outP))) return r;
         // dz of the layer below: col2im with the ReLU mask of this conv's input
         T /= 2;
-        sur::k_col2im_up_relu<<<1184, 256, 0, s->stream>>>(s->dcols, l.inP, Bp, T, l.cin, s->act[6 + ci], s->dz, s->dzb);
+        sur::k_col2im_up_relu<<<1184, 256, 0, w.st>>>(s->dcols, l.inP, Bp, T, l.cin, s->act[li], s->dz[li - 1], s->dzb[li - 1]);
         SCK(cudaGetLastError());
     }
-    // ---- linear layers, last to first; s->dz/dzb hold dz of layer li's output
+    // ---- linear layers, last to first: the product's epilogue applies the ReLU mask of the
+    // layer's input and leaves the dz of the layer below
     for (int li = 5; li >= 0; li--) {
         const Layer& l = s->L[li];
-        if ((r = transpose(s, s->dzb, l.outP, s->dzT, Bp, Bp, l.outP))) return r;
-        if ((r = transpose(s, s->act[li], l.inP, s->hT, Bp, Bp, l.inP))) return r;
-        if ((r = gemm(s, s->dzT, Bp, s->hT, Bp, s->g + l.wofs, l.inP, nullptr, 0, nullptr, 0, l.outP, l.inP, Bp))) return r;
-        if ((r = colsum(s, s->dz, Bp, l.outP, s->g + l.bofs))) return r;
+        if ((r = weight_grad(s, li, Bp, 0))) return r;
         if (li == 0) break;
-        if ((r = transpose(s, s->wb + l.wofs, l.inP, s->wT, l.outP, l.outP, l.inP))) return r;
-        if ((r = gemm(s, s->dzb, l.outP, s->wT, l.outP, s->dh, l.inP, nullptr, 0, nullptr, 0, Bp, l.inP, l.outP))) return r;
-        sur::k_relu_back<<<1184, 256, 0, s->stream>>>(s->dh, s->act[li], (size_t)Bp * l.inP, s->dz, s->dzb);
-        SCK(cudaGetLastError());
+        if ((r = gemm(s, w, s->dzb[li], l.outP, s->wT[li], l.outP, s->dz[li - 1], l.inP, s->dzb[li - 1], l.inP, nullptr, 0, Bp,
+                      l.inP, l.outP, s->act[li]))) return r;
+    }
+    for (int k = 1; k < kLanes; k++) {
+        SCK(cudaEventRecord(s->lane[k].done, s->lane[k].st));
+        SCK(cudaStreamWaitEvent(s->stream, s->lane[k].done, 0));
     }
     return CS_OK;
 }
@@ -952,24 +1048,109 @@ static int load_batch(cs_sur* s, const float* x, const float* target, int n, int
     return CS_OK;
 }
 
-static int loss_grad(cs_sur* s, const float* x, const float* target, int n, float* loss)
+// The kernels of one step on n rows whose inputs and targets are in xdev and tdev: loss
+// terms summed into lsum, gradients in g and, with `update`, the weights' update.
+static int enqueue_step(cs_sur* s, int n, bool update)
 {
-    int Bp, r;
-    if ((r = load_batch(s, x, target, n, &Bp))) return r;
+    int r;
+    const int Bp = up64(n);
+    if ((r = begin_lanes(s))) return r;
+    sur::k_load_x<<<(Bp * 64 + 255) / 256, 256, 0, s->stream>>>(s->xdev, n, Bp, s->act[0]);
+    SCK(cudaGetLastError());
     if ((r = forward(s, Bp))) return r;
-    const float scale = 1.f / ((float)n * kTOut * kNOut);
-    sur::k_mse<<<1184, 256, 0, s->stream>>>(s->yout, s->tdev, n, Bp, scale, s->dh, s->sq);
+    const size_t nsq = (size_t)n * kTOut * kNOut;
+    sur::k_mse<<<1184, 256, 0, s->stream>>>(s->yout, s->tdev, n, Bp, 1.f / ((float)n * kTOut * kNOut), s->dz[8], s->dzb[8], s->sq);
+    SCK(cudaGetLastError());
+    SCK(cudaEventRecord(s->fork, s->stream));
+    SCK(cudaStreamWaitEvent(s->lane[3].st, s->fork, 0));
+    sur::k_sum_part<<<kLossBlocks, 256, 0, s->lane[3].st>>>(s->sq, nsq, s->lpart);
+    sur::k_sum_final<<<1, 256, 0, s->lane[3].st>>>(s->lpart, kLossBlocks, s->lsum);
     SCK(cudaGetLastError());
     if ((r = backward(s, Bp))) return r;
-    if (loss) {
-        const size_t nsq = (size_t)n * kTOut * kNOut;
-        sur::k_sum_part<<<kLossBlocks, 256, 0, s->stream>>>(s->sq, nsq, s->lpart);
-        sur::k_sum_final<<<1, 256, 0, s->stream>>>(s->lpart, kLossBlocks, s->lsum);
+    if (update) {
+        sur::k_adam<<<1184, 256, 0, s->stream>>>(s->w, s->m, s->v, s->g, s->wb, s->np, 0.f, 0.f, 0.f, 0.f, 1.f, 1.f, 0.f, s->d_err);
         SCK(cudaGetLastError());
+    }
+    return CS_OK;
+}
+
+// The step's graph for n rows, captured on first use.  A step is about 90 launches, most of
+// a few microseconds, in four chains; replayed as one graph the chains overlap and the
+// launches leave no gaps (0.93 ms a step of 64 rows when launched one after the other, half
+// of it gaps and transposes that nothing had to wait for).
+constexpr size_t kMaxGraphs = 8;   // batch sizes kept (a training run uses one or two)
+static int step_graph(cs_sur* s, int n, bool update, cs_sur::StepGraph** out)
+{
+    for (auto& g : s->graphs)
+        if (g.n == n && g.update == update) { *out = &g; return CS_OK; }
+    if (s->graphs.size() >= kMaxGraphs) {
+        SCK(cudaStreamSynchronize(s->stream));
+        drop_graphs(s);
+    }
+    cs_sur::StepGraph g;
+    g.n = n;
+    g.update = update;
+    SCK(cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal));
+    int r = enqueue_step(s, n, update);
+    cudaError_t e = cudaStreamEndCapture(s->stream, &g.graph);
+    if (r || e != cudaSuccess) {
+        if (g.graph) cudaGraphDestroy(g.graph);
+        (void)cudaGetLastError();
+        return r ? r : sur_err(s, CS_E_CUDA, "step graph capture: %s", cudaGetErrorString(e));
+    }
+    if (update) {
+        size_t nn = 0;
+        SCK(cudaGraphGetNodes(g.graph, nullptr, &nn));
+        std::vector<cudaGraphNode_t> nodes(nn);
+        SCK(cudaGraphGetNodes(g.graph, nodes.data(), &nn));
+        for (cudaGraphNode_t nd : nodes) {
+            cudaGraphNodeType ty;
+            SCK(cudaGraphNodeGetType(nd, &ty));
+            if (ty != cudaGraphNodeTypeKernel) continue;
+            cudaKernelNodeParams kp;
+            SCK(cudaGraphKernelNodeGetParams(nd, &kp));
+            if (kp.func == (void*)sur::k_adam) { g.adam = nd; g.adam_params = kp; }
+        }
+    }
+    e = cudaGraphInstantiate(&g.exec, g.graph, 0);
+    if (e != cudaSuccess) {
+        cudaGraphDestroy(g.graph);
+        return sur_err(s, CS_E_CUDA, "step graph instantiate: %s", cudaGetErrorString(e));
+    }
+    s->graphs.push_back(g);
+    *out = &s->graphs.back();
+    return CS_OK;
+}
+
+// One step on the host's batch: inputs and targets to the device, the step's graph, and the
+// loss back when asked for (which waits for the step).
+static int run_step(cs_sur* s, const float* x, const float* target, int n, float* loss, bool update, float lr, float wd)
+{
+    if (n <= 0 || n > s->bmax) return sur_err(s, CS_E_RANGE, "batch of %d outside 1..%d", n, s->bmax);
+    cs_sur::StepGraph* g;
+    int r = step_graph(s, n, update, &g);
+    if (r) return r;
+    SCK(cudaMemcpyAsync(s->xdev, x, sizeof(float) * n * kIn, cudaMemcpyHostToDevice, s->stream));
+    SCK(cudaMemcpyAsync(s->tdev, target, sizeof(float) * n * kTOut * kNOut, cudaMemcpyHostToDevice, s->stream));
+    if (update) {
+        s->t++;
+        float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
+        float c1 = 1.f - powf(b1, (float)s->t), c2 = 1.f - powf(b2, (float)s->t);
+        void* args[] = {&s->w, &s->m, &s->v, &s->g, &s->wb, &s->np, &lr, &b1, &b2, &eps, &c1, &c2, &wd, &s->d_err};
+        cudaKernelNodeParams kp = g->adam_params;
+        kp.kernelParams = args;
+        kp.extra = nullptr;
+        SCK(cudaGraphExecKernelNodeSetParams(g->exec, g->adam, &kp));
+    }
+    SCK(cudaGraphLaunch(g->exec, s->stream));
+    if (loss) {
         double acc = 0.0;
         SCK(cudaMemcpyAsync(&acc, s->lsum, sizeof(double), cudaMemcpyDeviceToHost, s->stream));
-        if ((r = sync_check(s))) return r;
-        *loss = (float)(acc / (double)nsq);
+        if ((r = sync_check(s))) {
+            if (update) s->t--;
+            return r;
+        }
+        *loss = (float)(acc / (double)((size_t)n * kTOut * kNOut));
     }
     return CS_OK;
 }
@@ -994,7 +1175,7 @@ int cs_sur_forward(cs_sur* s, const float* x, int n, float* y)
 int cs_sur_loss_grad(cs_sur* s, const float* x, const float* target, int n, float* loss, float* grad)
 {
     if (!s || !x || !target) return CS_E_ARG;
-    int r = loss_grad(s, x, target, n, loss);
+    int r = run_step(s, x, target, n, loss, false, 0.f, 0.f);
     if (r) return r;
     if (grad) {
         std::vector<float> h(s->np);
@@ -1013,15 +1194,11 @@ int cs_sur_loss_grad(cs_sur* s, const float* x, const float* target, int n, floa
 int cs_sur_train_step(cs_sur* s, const float* x, const float* target, int n, float lr, float weight_decay, float* loss)
 {
     if (!s || !x || !target) return CS_E_ARG;
-    int r = loss_grad(s, x, target, n, loss);
+    int r = run_step(s, x, target, n, loss, true, lr, weight_decay);
     if (r) return r;
-    s->t++;
-    const float b1 = 0.9f, b2 = 0.999f;
-    const float c1 = 1.f - powf(b1, (float)s->t), c2 = 1.f - powf(b2, (float)s->t);
-    sur::k_adam<<<1184, 256, 0, s->stream>>>(s->w, s->m, s->v, s->g, s->wb, s->np, lr, b1, b2, 1e-8f, c1, c2, weight_decay);
-    SCK(cudaGetLastError());
-    if (!loss) return sync_check(s);
-    return CS_OK;
+    if (loss) return CS_OK;
+    if ((r = sync_check(s))) s->t--;
+    return r;
 }
 
 int cs_sur_set_gemm(cs_sur* s, int impl)
@@ -1029,6 +1206,7 @@ int cs_sur_set_gemm(cs_sur* s, int impl)
     if (!s) return CS_E_ARG;
     if (impl != 0 && impl != 1) return sur_err(s, CS_E_ARG, "GEMM path must be 0 (tcgen05) or 1 (mma.sync)");
     SCK(cudaStreamSynchronize(s->stream));
+    drop_graphs(s);
     s->gemm_impl = impl;
     return CS_OK;
 }
