@@ -129,13 +129,12 @@ __global__ void __launch_bounds__(128) k_gemm_nt(const bf16* __restrict__ A, int
 
 // ------------------------------------------------------- tcgen05 GEMM
 // The same product on the 5th-generation tensor cores.  A block computes a 128 x BN
-// tile: its 128 threads stage 64-wide K slices of A and B in shared memory in the
-// K-major 128-byte-swizzled layout (two stages, so the loads of slice k+1 overlap
-// the products of slice k), one thread issues the tcgen05.mma instructions
-// (M = 128, N = BN, K = 16 each, BF16 in, FP32 accumulator in tensor memory) and
-// commits them to the stage's mbarrier, and after the last slice every warp reads
-// its 32 accumulator rows from tensor memory for the epilogue (bias, ReLU, FP32
-// and/or BF16 stores).  Rows of A past M are staged as zeros and not stored.
+// tile: its 128 threads copy 64-wide K slices of A and B into shared memory in the
+// K-major 128-byte-swizzled layout (cp.async, kStages - 1 slices ahead of the products),
+// one thread issues the tcgen05.mma instructions (M = 128, N = BN, K = 16 each, BF16 in,
+// FP32 accumulator in tensor memory) and commits them to the stage's mbarrier, and after
+// the last slice every warp reads its 32 accumulator rows from tensor memory for the
+// epilogue (bias, ReLU, mask, FP32 and/or BF16 stores, 16 bytes each).  Rows of A past M are staged as zeros and not stored.
 // Every wait is bounded: on a give-up the block records it in *err, waits (bounded)
 // for its issued products, frees its tensor memory and returns.
 namespace tc {
@@ -143,7 +142,7 @@ namespace tc {
 constexpr int BM = 128, BK = 64;          // BK bf16 = 128 bytes, one swizzle row
 constexpr unsigned kSpin = 1u << 22;      // try_wait rounds before a wait gives up
 
-__host__ __device__ constexpr size_t smem_bytes(int BN) { return 1024 + 2 * (size_t)(BM + BN) * BK * 2; }
+__host__ __device__ constexpr size_t smem_bytes(int BN, int stages) { return 1024 + stages * (size_t)(BM + BN) * BK * 2; }
 
 __device__ __forceinline__ uint32_t saddr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
@@ -202,40 +201,62 @@ __device__ __forceinline__ void ld32(uint32_t taddr, uint32_t (&r)[32])
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
 
-// rows x 64 BF16 of a row-major matrix (row stride ld elements, rows from r0, k from
-// k0) into a 128-byte-swizzled stage: 16-byte chunk j of row r lands at
-// r * 128 + ((j ^ (r & 7)) * 16).  Rows at or past nrows are zero.
-__device__ __forceinline__ void stage_rows(unsigned char* dst, const bf16* __restrict__ src, int ld, int r0, int nrows,
-                                           int k0, int rows)
+// 16 bytes into shared memory, or zeros.
+__device__ __forceinline__ void copy16(uint32_t dst, const bf16* src, bool valid)
 {
-    for (int i = threadIdx.x; i < rows * 8; i += blockDim.x) {
-        const int r = i >> 3, j = i & 7;
-        uint4 v = make_uint4(0, 0, 0, 0);
-        if (r0 + r < nrows) v = *reinterpret_cast<const uint4*>(src + (size_t)(r0 + r) * ld + k0 + j * 8);
-        *reinterpret_cast<uint4*>(dst + r * 128 + ((j ^ (r & 7)) << 4)) = v;
-    }
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" :: "r"(dst), "l"(src), "r"(valid ? 16 : 0) : "memory");
 }
+
+// A thread's 16-byte chunks of a rows x 64 slice (128-byte-swizzled: chunk j of row r lands
+// at r * 128 + ((j ^ (r & 7)) * 16)): chunk j = threadIdx & 7 of every 16th row, the same j
+// for all, so what depends on the row is formed once per tile and what depends on k once per
+// slice.
+template <int kRows>
+struct RowSource {   // rows of a row-major matrix; rows at or past nrows are zero
+    static constexpr int kN = kRows / 16;
+    const bf16 *base, *p;   // base: an address to name where nothing is read
+    int ld, left;
+    __device__ __forceinline__ RowSource(const bf16* src, int ld_, int r0, int nrows)
+        : base(src), p(src + (size_t)(r0 + (int)(threadIdx.x >> 3)) * ld_ + (threadIdx.x & 7) * 8), ld(ld_), left(nrows - r0 - (int)(threadIdx.x >> 3)) {}
+    __device__ __forceinline__ void stage(uint32_t dst, int k0) const
+    {
+        const int r = threadIdx.x >> 3, j = threadIdx.x & 7;
+        dst += r * 128 + ((j ^ (r & 7)) << 4);   // r + 16 q has the same low bits
+#pragma unroll
+        for (int q = 0; q < kN; q++) copy16(dst + q * 2048, 16 * q < left ? p + (size_t)(16 * q) * ld + k0 : base, 16 * q < left);
+    }
+};
 
 // The A operand of a convolution read straight from its input H [Bn*T, kCh] (no
 // column matrix): row m = b*2T + t, column k = tap*Cin + c holds
 // H[b*T + (t+tap-2)/2, c] when 0 <= t+tap-2 < 2T, else zero (as k_im2col_up).  Cin is
 // a multiple of 8, so a 16-byte chunk never straddles two taps.
-__device__ __forceinline__ void stage_conv_rows(unsigned char* dst, const bf16* __restrict__ H, int T, int Cin, int r0,
-                                                int nrows, int k0)
-{
-    for (int i = threadIdx.x; i < BM * 8; i += blockDim.x) {
-        const int r = i >> 3, j = i & 7;
-        uint4 v = make_uint4(0, 0, 0, 0);
-        const int m = r0 + r, k = k0 + j * 8;
-        const int tap = k / Cin;
-        if (m < nrows && tap < kTap) {
-            const int b = m / (2 * T), t = m - b * 2 * T, u = t + tap - kTap / 2;
-            if (u >= 0 && u < 2 * T)
-                v = *reinterpret_cast<const uint4*>(H + ((size_t)b * T + (u >> 1)) * kCh + (k - tap * Cin));
+struct ConvSource {
+    static constexpr int kN = BM / 16;
+    const bf16* H;
+    int T, Cin, nrows, m0;
+    int b[kN], t[kN];
+    __device__ __forceinline__ ConvSource(const bf16* H_, int T_, int Cin_, int r0, int nrows_)
+        : H(H_), T(T_), Cin(Cin_), nrows(nrows_), m0(r0 + (int)(threadIdx.x >> 3))
+    {
+#pragma unroll
+        for (int q = 0; q < kN; q++) {
+            b[q] = (m0 + 16 * q) / (2 * T);
+            t[q] = m0 + 16 * q - b[q] * 2 * T;
         }
-        *reinterpret_cast<uint4*>(dst + r * 128 + ((j ^ (r & 7)) << 4)) = v;
     }
-}
+    __device__ __forceinline__ void stage(uint32_t dst, int k0) const
+    {
+        const int r = threadIdx.x >> 3, j = threadIdx.x & 7, k = k0 + j * 8, tap = k / Cin, c = k - tap * Cin;
+        dst += r * 128 + ((j ^ (r & 7)) << 4);
+#pragma unroll
+        for (int q = 0; q < kN; q++) {
+            const int u = t[q] + tap - kTap / 2;
+            const bool on = m0 + 16 * q < nrows && tap < kTap && u >= 0 && u < 2 * T;
+            copy16(dst + q * 2048, on ? H + ((size_t)b[q] * T + (u >> 1)) * kCh + c : H, on);
+        }
+    }
+};
 
 }  // namespace tc
 
@@ -245,7 +266,7 @@ __device__ __forceinline__ void stage_conv_rows(unsigned char* dst, const bf16* 
 // split K as k_gemm_nt (gridDim.z slices of kchunk, partial products at C + z * cstride).
 // With H set, A is the column matrix of a convolution of H (hT time points, hCin
 // channels), generated while staging (not split).
-template <int BN>
+template <int BN, int kStages>
 __global__ void __launch_bounds__(128) k_gemm_tc(const bf16* __restrict__ A, int lda, const bf16* __restrict__ B, int ldb,
                                                  float* __restrict__ C, int ldc, bf16* __restrict__ Cb, int ldcb,
                                                  const float* __restrict__ bias, int relu, int M, int K, int kchunk,
@@ -254,12 +275,11 @@ __global__ void __launch_bounds__(128) k_gemm_tc(const bf16* __restrict__ A, int
 {
     using namespace tc;
     extern __shared__ unsigned char smem_raw[];
-    __shared__ uint64_t bar[2];
+    __shared__ uint64_t bar[kStages];
     __shared__ uint32_t tmem_base;
     __shared__ int s_ok;
-    unsigned char* base = smem_raw + ((1024 - (saddr(smem_raw) & 1023)) & 1023);
-    unsigned char* As = base;                          // [2][BM * 128 B]
-    unsigned char* Bs = base + 2 * BM * BK * 2;        // [2][BN * 128 B]
+    const uint32_t As = (saddr(smem_raw) + 1023) & ~1023u;   // [kStages][BM * 128 B]
+    const uint32_t Bs = As + kStages * BM * BK * 2;          // [kStages][BN * 128 B]
     if (gridDim.z > 1) {
         const int z = blockIdx.z;
         A += (size_t)z * kchunk;
@@ -269,13 +289,27 @@ __global__ void __launch_bounds__(128) k_gemm_tc(const bf16* __restrict__ A, int
     }
     const int bm = blockIdx.y * BM, bn = blockIdx.x * BN;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int nk = K / BK;
+    const RowSource<BM> arows(H ? B : A, H ? 0 : lda, H ? 0 : bm, H ? 0 : M);
+    const ConvSource aconv(H, H ? hT : 1, H ? hCin : 64, bm, H ? M : 0);
+    const RowSource<BN> brows(B, ldb, bn, 1 << 30);
+    auto load = [&](int kc) {   // slice kc on its way (an empty group past the last, so that groups count slices)
+        if (kc < nk) {
+            const uint32_t st = kc % kStages;
+            if (H) aconv.stage(As + st * BM * 128, kc * BK);
+            else arows.stage(As + st * BM * 128, kc * BK);
+            brows.stage(Bs + st * BN * 128, kc * BK);
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    for (int kc = 0; kc < kStages - 1; kc++) load(kc);
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" :: "r"(saddr(&tmem_base)), "r"(BN));
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
     }
     if (threadIdx.x == 0) {
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" :: "r"(saddr(&bar[0])));
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" :: "r"(saddr(&bar[1])));
+#pragma unroll
+        for (int i = 0; i < kStages; i++) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" :: "r"(saddr(&bar[i])));
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         s_ok = 1;
     }
@@ -283,32 +317,30 @@ __global__ void __launch_bounds__(128) k_gemm_tc(const bf16* __restrict__ A, int
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tm = tmem_base;
-    const int nk = K / BK;
     int issued = 0;                    // slices whose products were committed
+    bool ok = true;                    // this thread's waits came through
     for (int kc = 0; kc < nk; kc++) {
-        const int st = kc & 1;
-        if (kc >= 2) {                 // the products that read this stage are done
-            if (threadIdx.x == 0 && !mbar_wait(&bar[st], ((kc - 2) >> 1) & 1)) s_ok = 0;
-            __syncthreads();
-            if (!s_ok) break;
-        }
-        if (H) stage_conv_rows(As + st * BM * 128, H, hT, hCin, bm, M, kc * BK);
-        else stage_rows(As + st * BM * 128, A, lda, bm, M, kc * BK, BM);
-        stage_rows(Bs + st * BN * 128, B, ldb, bn, 1 << 30, kc * BK, BN);
+        const int st = kc % kStages;
+        asm volatile("cp.async.wait_group %0;" :: "n"(kStages - 2) : "memory");   // slice kc is in
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        __syncthreads();
+        if (!__syncthreads_and(ok)) break;
         if (threadIdx.x == 0) {
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            const uint32_t a0 = saddr(As + st * BM * 128), b0 = saddr(Bs + st * BN * 128);
+            const uint32_t a0 = As + st * BM * 128, b0 = Bs + st * BN * 128;
 #pragma unroll
             for (int k = 0; k < BK / 16; k++)
                 tc::mma(tm, sdesc(a0 + 32 * k), sdesc(b0 + 32 * k), idesc(BM, BN), (kc | k) != 0);
             commit(&bar[st]);
         }
         issued = kc + 1;
+        // the next slice to fetch goes where slice kc - 1 was, once its products are done
+        if (kc >= 1 && kc + kStages - 1 < nk) ok = mbar_wait(&bar[(kc - 1) % kStages], ((kc - 1) / kStages) & 1);
+        if (ok) load(kc + kStages - 1);
+        else asm volatile("cp.async.commit_group;" ::: "memory");
     }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
     // the last committed slice's barrier completes after all earlier products
-    if (threadIdx.x == 0 && issued > 0 && !mbar_wait(&bar[(issued - 1) & 1], ((issued - 1) >> 1) & 1)) s_ok = 0;
+    if (threadIdx.x == 0 && issued > 0 && !mbar_wait(&bar[(issued - 1) % kStages], ((issued - 1) / kStages) & 1)) s_ok = 0;
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     if (s_ok && issued == nk) {
@@ -319,19 +351,43 @@ __global__ void __launch_bounds__(128) k_gemm_tc(const bf16* __restrict__ A, int
             ld32(tm + ((uint32_t)(warp * 32) << 16) + (uint32_t)c0, r);
             if (row < M) {
                 const int col = bn + c0;
+                float v[32];
 #pragma unroll
-                for (int j = 0; j < 32; j += 2) {
-                    float v0 = __uint_as_float(r[j]), v1 = __uint_as_float(r[j + 1]);
-                    if (nk == 0) v0 = v1 = 0.f;
-                    if (bias) { v0 += bias[col + j]; v1 += bias[col + j + 1]; }
-                    if (relu) { v0 = fmaxf(v0, 0.f); v1 = fmaxf(v1, 0.f); }
-                    if (mask) {
-                        const __nv_bfloat162 h = *reinterpret_cast<const __nv_bfloat162*>(mask + (size_t)row * ldc + col + j);
-                        if (!(__low2float(h) > 0.f)) v0 = 0.f;
-                        if (!(__high2float(h) > 0.f)) v1 = 0.f;
+                for (int j = 0; j < 32; j++) v[j] = nk == 0 ? 0.f : __uint_as_float(r[j]);
+                if (bias) {
+#pragma unroll
+                    for (int j = 0; j < 32; j++) v[j] += bias[col + j];
+                }
+                if (relu) {
+#pragma unroll
+                    for (int j = 0; j < 32; j++) v[j] = fmaxf(v[j], 0.f);
+                }
+                if (mask) {
+#pragma unroll
+                    for (int j = 0; j < 32; j += 8) {
+                        const uint4 h4 = *reinterpret_cast<const uint4*>(mask + (size_t)row * ldc + col + j);
+                        const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&h4);
+#pragma unroll
+                        for (int q = 0; q < 4; q++) {
+                            if (!(__low2float(h[q]) > 0.f)) v[j + 2 * q] = 0.f;
+                            if (!(__high2float(h[q]) > 0.f)) v[j + 2 * q + 1] = 0.f;
+                        }
                     }
-                    if (C) *reinterpret_cast<float2*>(C + (size_t)row * ldc + col + j) = make_float2(v0, v1);
-                    if (Cb) *reinterpret_cast<__nv_bfloat162*>(Cb + (size_t)row * ldcb + col + j) = __floats2bfloat162_rn(v0, v1);
+                }
+                if (C) {
+#pragma unroll
+                    for (int j = 0; j < 32; j += 4)
+                        *reinterpret_cast<float4*>(C + (size_t)row * ldc + col + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
+                }
+                if (Cb) {
+#pragma unroll
+                    for (int j = 0; j < 32; j += 8) {
+                        uint4 o4;
+                        __nv_bfloat162* o = reinterpret_cast<__nv_bfloat162*>(&o4);
+#pragma unroll
+                        for (int q = 0; q < 4; q++) o[q] = __floats2bfloat162_rn(v[j + 2 * q], v[j + 2 * q + 1]);
+                        *reinterpret_cast<uint4*>(Cb + (size_t)row * ldcb + col + j) = o4;
+                    }
                 }
             }
         }
@@ -341,6 +397,17 @@ __global__ void __launch_bounds__(128) k_gemm_tc(const bf16* __restrict__ A, int
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" :: "r"(tm), "r"(BN));
+}
+
+// Stages: four put a short product's whole K in flight at once (the linear layers: 64 to 512
+// wide, split); with more blocks than two an SM, two leave room for four blocks an SM, which
+// hide one another's loads.
+static int tc_stages(const dim3& grid) { return (size_t)grid.x * grid.y * grid.z <= 296 ? 4 : 2; }
+template <typename... Args>
+static void tc_launch(const dim3& grid, cudaStream_t st, Args... args)
+{
+    if (tc_stages(grid) == 4) k_gemm_tc<64, 4><<<grid, 128, tc::smem_bytes(64, 4), st>>>(args...);
+    else k_gemm_tc<64, 2><<<grid, 128, tc::smem_bytes(64, 2), st>>>(args...);
 }
 
 // C[r, c] = sum over the slices z, in ascending order, of part[z][r, c] ([M, N] each),
@@ -711,8 +778,8 @@ static int gemm_launch(cs_sur* s, const Lane& w, const bf16* A, int lda, const b
 {
     if (s->gemm_impl == 0 && K % 64 == 0 && kchunk % 64 == 0) {
         dim3 grid(N / 64, (M + tc::BM - 1) / tc::BM, nsplit);
-        k_gemm_tc<64><<<grid, 128, tc::smem_bytes(64), w.st>>>(A, lda, B, ldb, C, ldc, Cb, ldcb, bias, relu, M, K,
-                                                               kchunk, cstride, s->d_err, nullptr, 0, 0, mask);
+        tc_launch(grid, w.st, A, lda, B, ldb, C, ldc, Cb, ldcb, bias, relu, M, K, kchunk, cstride, s->d_err,
+                  (const bf16*)nullptr, 0, 0, mask);
     } else {
         dim3 grid(N / 64, M / 64, nsplit);
         sur::k_gemm_nt<<<grid, 128, 0, w.st>>>(A, lda, B, ldb, C, ldc, Cb, ldcb, bias, relu, K, kchunk, cstride, mask);
@@ -844,7 +911,8 @@ int cs_sur_create(int max_batch, int device, cs_sur** out)
     }
     SA(s->lpart, (size_t)kLossBlocks); SA(s->lsum, (size_t)1); SA(s->d_err, (size_t)1);
     SCK(cudaMemsetAsync(s->d_err, 0, sizeof(int), s->stream));
-    SCK(cudaFuncSetAttribute(k_gemm_tc<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tc::smem_bytes(64)));
+    SCK(cudaFuncSetAttribute(k_gemm_tc<64, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tc::smem_bytes(64, 4)));
+    SCK(cudaFuncSetAttribute(k_gemm_tc<64, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tc::smem_bytes(64, 2)));
     SA(s->xdev, (size_t)B * kIn); SA(s->tdev, (size_t)B * kTOut * kNOut); SA(s->sq, (size_t)B * kTOut * kNOut);
     SA(s->ydev, (size_t)B * kTOut * kNOut);
 #undef SA
@@ -927,9 +995,9 @@ static int forward(cs_sur* s, int Bp)
         const int M = Bp * 2 * T;
         if (s->gemm_impl == 0) {   // the column matrix is generated while staging
             dim3 grid(l.outP / 64, (M + tc::BM - 1) / tc::BM, 1);
-            k_gemm_tc<64><<<grid, 128, tc::smem_bytes(64), w.st>>>(nullptr, 0, s->wb + l.wofs, l.inP, C, kCh, Cb, kCh,
-                                                                   s->w + l.bofs, l.relu ? 1 : 0, M, l.inP, l.inP, 0,
-                                                                   s->d_err, s->act[6 + ci], T, l.cin, nullptr);
+            tc_launch(grid, w.st, (const bf16*)nullptr, 0, (const bf16*)(s->wb + l.wofs), l.inP, C, kCh, Cb, kCh,
+                      (const float*)(s->w + l.bofs), l.relu ? 1 : 0, M, l.inP, l.inP, (size_t)0, s->d_err,
+                      (const bf16*)s->act[6 + ci], T, l.cin, (const bf16*)nullptr);
             SCK(cudaGetLastError());
         } else {
             sur::k_im2col_up<<<1184, 256, 0, w.st>>>(s->act[6 + ci], Bp, T, l.cin, s->cols[ci], l.inP);
