@@ -23,6 +23,7 @@
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
+#include <thread>
 #include <vector>
 
 #include "covidsim_b200.h"
@@ -271,9 +272,11 @@ __global__ void __launch_bounds__(128) k_gemm_tc(const bf16* __restrict__ A, int
                                                  float* __restrict__ C, int ldc, bf16* __restrict__ Cb, int ldcb,
                                                  const float* __restrict__ bias, int relu, int M, int K, int kchunk,
                                                  size_t cstride, int* err, const bf16* __restrict__ H, int hT, int hCin,
-                                                 const bf16* __restrict__ mask)
+                                                 const bf16* __restrict__ mask, float* __restrict__ Y, int yn)
 {
     using namespace tc;
+    constexpr int kCols = BN < 32 ? 32 : BN;   // tensor memory comes in 32 columns at least
+    constexpr int kW = BN < 32 ? BN : 32;      // columns of a 32-column read that hold outputs
     extern __shared__ unsigned char smem_raw[];
     __shared__ uint64_t bar[kStages];
     __shared__ uint32_t tmem_base;
@@ -304,7 +307,7 @@ __global__ void __launch_bounds__(128) k_gemm_tc(const bf16* __restrict__ A, int
     };
     for (int kc = 0; kc < kStages - 1; kc++) load(kc);
     if (warp == 0) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" :: "r"(saddr(&tmem_base)), "r"(BN));
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" :: "r"(saddr(&tmem_base)), "r"(kCols));
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
     }
     if (threadIdx.x == 0) {
@@ -351,20 +354,20 @@ __global__ void __launch_bounds__(128) k_gemm_tc(const bf16* __restrict__ A, int
             ld32(tm + ((uint32_t)(warp * 32) << 16) + (uint32_t)c0, r);
             if (row < M) {
                 const int col = bn + c0;
-                float v[32];
+                float v[kW];
 #pragma unroll
-                for (int j = 0; j < 32; j++) v[j] = nk == 0 ? 0.f : __uint_as_float(r[j]);
+                for (int j = 0; j < kW; j++) v[j] = nk == 0 ? 0.f : __uint_as_float(r[j]);
                 if (bias) {
 #pragma unroll
-                    for (int j = 0; j < 32; j++) v[j] += bias[col + j];
+                    for (int j = 0; j < kW; j++) v[j] += bias[col + j];
                 }
                 if (relu) {
 #pragma unroll
-                    for (int j = 0; j < 32; j++) v[j] = fmaxf(v[j], 0.f);
+                    for (int j = 0; j < kW; j++) v[j] = fmaxf(v[j], 0.f);
                 }
                 if (mask) {
 #pragma unroll
-                    for (int j = 0; j < 32; j += 8) {
+                    for (int j = 0; j < kW; j += 8) {
                         const uint4 h4 = *reinterpret_cast<const uint4*>(mask + (size_t)row * ldc + col + j);
                         const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&h4);
 #pragma unroll
@@ -374,14 +377,18 @@ __global__ void __launch_bounds__(128) k_gemm_tc(const bf16* __restrict__ A, int
                         }
                     }
                 }
+                if (Y && bn + c0 == 0) {   // the network's outputs: [yn, 365, 4] from [yn * 368, ...]
+                    const int yb = row / (8 * kT0), yt = row - yb * (8 * kT0);
+                    if (yb < yn && yt < kTOut) *reinterpret_cast<float4*>(Y + ((size_t)yb * kTOut + yt) * kNOut) = make_float4(v[0], v[1], v[2], v[3]);
+                }
                 if (C) {
 #pragma unroll
-                    for (int j = 0; j < 32; j += 4)
+                    for (int j = 0; j < kW; j += 4)
                         *reinterpret_cast<float4*>(C + (size_t)row * ldc + col + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
                 }
                 if (Cb) {
 #pragma unroll
-                    for (int j = 0; j < 32; j += 8) {
+                    for (int j = 0; j < kW; j += 8) {
                         uint4 o4;
                         __nv_bfloat162* o = reinterpret_cast<__nv_bfloat162*>(&o4);
 #pragma unroll
@@ -396,18 +403,26 @@ __global__ void __launch_bounds__(128) k_gemm_tc(const bf16* __restrict__ A, int
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
-    if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" :: "r"(tm), "r"(BN));
+    if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" :: "r"(tm), "r"(kCols));
 }
 
 // Stages: four put a short product's whole K in flight at once (the linear layers: 64 to 512
 // wide, split); with more blocks than two an SM, two leave room for four blocks an SM, which
-// hide one another's loads.
+// hide one another's loads.  BN: the output columns that are there (64, or 32 and 16 for the
+// last two convolutions' 32 and 4 channels, whose padding to 64 was product work for nothing).
 static int tc_stages(const dim3& grid) { return (size_t)grid.x * grid.y * grid.z <= 296 ? 4 : 2; }
-template <typename... Args>
+template <int BN, typename... Args>
 static void tc_launch(const dim3& grid, cudaStream_t st, Args... args)
 {
-    if (tc_stages(grid) == 4) k_gemm_tc<64, 4><<<grid, 128, tc::smem_bytes(64, 4), st>>>(args...);
-    else k_gemm_tc<64, 2><<<grid, 128, tc::smem_bytes(64, 2), st>>>(args...);
+    if (tc_stages(grid) == 4) k_gemm_tc<BN, 4><<<grid, 128, tc::smem_bytes(BN, 4), st>>>(args...);
+    else k_gemm_tc<BN, 2><<<grid, 128, tc::smem_bytes(BN, 2), st>>>(args...);
+}
+template <int BN>
+static cudaError_t tc_enable()
+{
+    cudaError_t e = cudaFuncSetAttribute(k_gemm_tc<BN, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tc::smem_bytes(BN, 4));
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_gemm_tc<BN, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tc::smem_bytes(BN, 2));
+    return e;
 }
 
 // C[r, c] = sum over the slices z, in ascending order, of part[z][r, c] ([M, N] each),
@@ -694,7 +709,16 @@ struct cs_sur {
     double *lpart = nullptr, *lsum = nullptr;   // loss reduction
     int* d_err = nullptr;                   // set by a tensor-core GEMM whose wait gave up
     int gemm_impl = 0;                      // 0: tcgen05, 1: mma.sync
-    float *xdev = nullptr, *tdev = nullptr, *sq = nullptr, *ydev = nullptr;
+    float *xdev = nullptr, *tdev = nullptr, *sq = nullptr;
+    struct Predict {                        // the prediction path's workspace (predict_space)
+        int rows = 0;
+        float* dev = nullptr;               // one allocation; the rest points into it
+        std::vector<bf16*> act;
+        float *xdev[2] = {}, *ydev[2] = {}, *kpart = nullptr;
+        size_t kpart_n = 0;
+        cudaStream_t copy = nullptr;
+        cudaEvent_t ready[2] = {};
+    } pred;
     // one training step (or loss and gradient) of n rows as a graph
     struct StepGraph {
         int n = 0;
@@ -735,6 +759,13 @@ static int salloc(cs_sur* s, T** p, size_t n)
     SCK(cudaMemsetAsync(q, 0, sizeof(T) * (n ? n : 1), s->stream));
     *p = (T*)q;
     return CS_OK;
+}
+
+static void free_predict(cs_sur* s)
+{
+    cudaFree(s->pred.dev);
+    s->pred.dev = nullptr;
+    s->pred.rows = 0;
 }
 
 static void drop_graphs(cs_sur* s)
@@ -778,8 +809,8 @@ static int gemm_launch(cs_sur* s, const Lane& w, const bf16* A, int lda, const b
 {
     if (s->gemm_impl == 0 && K % 64 == 0 && kchunk % 64 == 0) {
         dim3 grid(N / 64, (M + tc::BM - 1) / tc::BM, nsplit);
-        tc_launch(grid, w.st, A, lda, B, ldb, C, ldc, Cb, ldcb, bias, relu, M, K, kchunk, cstride, s->d_err,
-                  (const bf16*)nullptr, 0, 0, mask);
+        tc_launch<64>(grid, w.st, A, lda, B, ldb, C, ldc, Cb, ldcb, bias, relu, M, K, kchunk, cstride, s->d_err,
+                      (const bf16*)nullptr, 0, 0, mask, (float*)nullptr, 0);
     } else {
         dim3 grid(N / 64, M / 64, nsplit);
         sur::k_gemm_nt<<<grid, 128, 0, w.st>>>(A, lda, B, ldb, C, ldc, Cb, ldcb, bias, relu, K, kchunk, cstride, mask);
@@ -792,14 +823,16 @@ static int gemm_launch(cs_sur* s, const Lane& w, const bf16* A, int lda, const b
 // convolutions' weight gradients, K = batch x time points; the linear layers at
 // batch sizes of a few hundred) is split along K so that about two blocks per SM
 // run; the slices' partial products are then summed in a fixed order and the
-// epilogue applied.
+// epilogue applied.  Msplit: the rows the split is chosen for, when several batches go
+// through as one (their sums must be those of the batch alone).
 constexpr int kMaxSplit = 64;
 
 static int gemm(cs_sur* s, const Lane& w, const bf16* A, int lda, const bf16* B, int ldb, float* C, int ldc, bf16* Cb,
-                int ldcb, const float* bias, int relu, int M, int N, int K, const bf16* mask = nullptr)
+                int ldcb, const float* bias, int relu, int M, int N, int K, const bf16* mask = nullptr, int Msplit = 0)
 {
     if (M % 64 || N % 64 || K % 32) return sur_err(s, CS_E_ARG, "gemm shape %d x %d x %d not padded", M, N, K);
-    const int tiles = (s->gemm_impl == 0 ? (M + tc::BM - 1) / tc::BM : M / 64) * (N / 64);
+    const int Mt = Msplit ? Msplit : M;
+    const int tiles = (s->gemm_impl == 0 ? (Mt + tc::BM - 1) / tc::BM : Mt / 64) * (N / 64);
     int nsplit = tiles < 74 ? std::min(kMaxSplit, std::max(1, std::min(K / 128, 296 / tiles))) : 1;
     if (nsplit > 1 && K % 64 == 0) {
         const int kchunk = ((K + nsplit - 1) / nsplit + 63) / 64 * 64;
@@ -911,10 +944,10 @@ int cs_sur_create(int max_batch, int device, cs_sur** out)
     }
     SA(s->lpart, (size_t)kLossBlocks); SA(s->lsum, (size_t)1); SA(s->d_err, (size_t)1);
     SCK(cudaMemsetAsync(s->d_err, 0, sizeof(int), s->stream));
-    SCK(cudaFuncSetAttribute(k_gemm_tc<64, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tc::smem_bytes(64, 4)));
-    SCK(cudaFuncSetAttribute(k_gemm_tc<64, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tc::smem_bytes(64, 2)));
+    SCK(tc_enable<64>());
+    SCK(tc_enable<32>());
+    SCK(tc_enable<16>());
     SA(s->xdev, (size_t)B * kIn); SA(s->tdev, (size_t)B * kTOut * kNOut); SA(s->sq, (size_t)B * kTOut * kNOut);
-    SA(s->ydev, (size_t)B * kTOut * kNOut);
 #undef SA
     SCK(cudaStreamSynchronize(s->stream));
     return CS_OK;
@@ -925,6 +958,10 @@ void cs_sur_destroy(cs_sur* s)
     if (!s) return;
     if (s->stream) cudaStreamSynchronize(s->stream);
     drop_graphs(s);
+    if (s->pred.copy) { cudaStreamSynchronize(s->pred.copy); cudaStreamDestroy(s->pred.copy); }
+    for (cudaEvent_t e : s->pred.ready)
+        if (e) cudaEventDestroy(e);
+    free_predict(s);
     for (void* p : s->allocs) cudaFree(p);
     for (Lane& w : s->lane) {
         if (w.st && w.st != s->stream) cudaStreamDestroy(w.st);
@@ -945,9 +982,9 @@ int cs_sur_set_params(cs_sur* s, const float* flat)
     std::vector<float> h(s->np, 0.f);
     size_t k = 0;
     for (auto& l : s->L) {
-        for (int o = 0; o < l.out; o++)
-            for (int i = 0; i < l.in; i++) h[l.wofs + (size_t)o * l.inP + i] = flat[k++];
-        for (int o = 0; o < l.out; o++) h[l.bofs + o] = flat[k++];
+        for (int o = 0; o < l.out; o++, k += l.in) memcpy(&h[l.wofs + (size_t)o * l.inP], flat + k, sizeof(float) * l.in);
+        memcpy(&h[l.bofs], flat + k, sizeof(float) * l.out);
+        k += l.out;
     }
     SCK(cudaMemcpyAsync(s->w, h.data(), sizeof(float) * s->np, cudaMemcpyHostToDevice, s->stream));
     SCK(cudaMemsetAsync(s->m, 0, sizeof(float) * s->np, s->stream));
@@ -967,43 +1004,54 @@ int cs_sur_get_params(cs_sur* s, float* flat)
     SCK(cudaStreamSynchronize(s->stream));
     size_t k = 0;
     for (auto& l : s->L) {
-        for (int o = 0; o < l.out; o++)
-            for (int i = 0; i < l.in; i++) flat[k++] = h[l.wofs + (size_t)o * l.inP + i];
-        for (int o = 0; o < l.out; o++) flat[k++] = h[l.bofs + o];
+        for (int o = 0; o < l.out; o++, k += l.in) memcpy(flat + k, &h[l.wofs + (size_t)o * l.inP], sizeof(float) * l.in);
+        memcpy(flat + k, &h[l.bofs], sizeof(float) * l.out);
+        k += l.out;
     }
     return CS_OK;
 }
 
 }  // extern "C"
 
-// Forward pass of Bp rows (x already in act[0]); leaves y in s->yout.
-static int forward(cs_sur* s, int Bp)
+// Forward pass of Bp rows (x already in act[0]) through the activation buffers `act`; the
+// outputs go to y64 ([Bp*368, 64], channels 0..3) or, for `n` rows, to y ([n, 365, 4]).
+// Msplit: the batch size whose summation order the products take (0: Bp).
+static int forward(cs_sur* s, const Lane& w, bf16* const* act, int Bp, float* y64, float* y, int n, int Msplit)
 {
     int r;
-    const Lane& w = s->lane[0];
     for (int li = 0; li < 6; li++) {
         const Layer& l = s->L[li];
-        if ((r = gemm(s, w, s->act[li], l.inP, s->wb + l.wofs, l.inP, nullptr, 0, s->act[li + 1], l.outP,
-                      s->w + l.bofs, 1, Bp, l.outP, l.inP))) return r;
+        if ((r = gemm(s, w, act[li], l.inP, s->wb + l.wofs, l.inP, nullptr, 0, act[li + 1], l.outP,
+                      s->w + l.bofs, 1, Bp, l.outP, l.inP, nullptr, Msplit))) return r;
     }
     int T = kT0;
     for (int ci = 0; ci < 3; ci++) {
         const Layer& l = s->L[6 + ci];
         const bool last = ci == 2;
-        float* C = last ? s->yout : nullptr;
-        bf16* Cb = last ? nullptr : s->act[7 + ci];
+        float* C = last ? y64 : nullptr;
+        bf16* Cb = last ? nullptr : act[7 + ci];
         const int M = Bp * 2 * T;
         if (s->gemm_impl == 0) {   // the column matrix is generated while staging
-            dim3 grid(l.outP / 64, (M + tc::BM - 1) / tc::BM, 1);
-            tc_launch(grid, w.st, (const bf16*)nullptr, 0, (const bf16*)(s->wb + l.wofs), l.inP, C, kCh, Cb, kCh,
-                      (const float*)(s->w + l.bofs), l.relu ? 1 : 0, M, l.inP, l.inP, (size_t)0, s->d_err,
-                      (const bf16*)s->act[6 + ci], T, l.cin, (const bf16*)nullptr);
+            dim3 grid(1, (M + tc::BM - 1) / tc::BM, 1);
+            const bf16 *none = nullptr, *wl = s->wb + l.wofs, *in = act[6 + ci];
+            const float* bias = s->w + l.bofs;
+            auto args = [&](auto launch) {
+                launch(grid, w.st, none, 0, wl, l.inP, C, kCh, Cb, kCh, bias, l.relu ? 1 : 0, M, l.inP, l.inP, (size_t)0,
+                       s->d_err, in, T, l.cin, none, last ? y : nullptr, n);
+            };
+            if (ci == 0) args([](auto... a) { tc_launch<64>(a...); });
+            else if (ci == 1) args([](auto... a) { tc_launch<32>(a...); });
+            else args([](auto... a) { tc_launch<16>(a...); });
             SCK(cudaGetLastError());
         } else {
-            sur::k_im2col_up<<<1184, 256, 0, w.st>>>(s->act[6 + ci], Bp, T, l.cin, s->cols[ci], l.inP);
+            sur::k_im2col_up<<<1184, 256, 0, w.st>>>(act[6 + ci], Bp, T, l.cin, s->cols[ci], l.inP);
             SCK(cudaGetLastError());
             if ((r = gemm(s, w, s->cols[ci], l.inP, s->wb + l.wofs, l.inP, C, kCh, Cb, kCh, s->w + l.bofs, l.relu ? 1 : 0,
                           M, l.outP, l.inP))) return r;
+            if (last && y) {
+                sur::k_store_y<<<512, 256, 0, w.st>>>(y64, n, y);
+                SCK(cudaGetLastError());
+            }
         }
         T *= 2;
     }
@@ -1105,17 +1153,6 @@ static int sync_check(cs_sur* s)
     return CS_OK;
 }
 
-static int load_batch(cs_sur* s, const float* x, const float* target, int n, int* Bp)
-{
-    if (n <= 0 || n > s->bmax) return sur_err(s, CS_E_RANGE, "batch of %d outside 1..%d", n, s->bmax);
-    *Bp = up64(n);
-    SCK(cudaMemcpyAsync(s->xdev, x, sizeof(float) * n * kIn, cudaMemcpyHostToDevice, s->stream));
-    sur::k_load_x<<<(*Bp * 64 + 255) / 256, 256, 0, s->stream>>>(s->xdev, n, *Bp, s->act[0]);
-    SCK(cudaGetLastError());
-    if (target) SCK(cudaMemcpyAsync(s->tdev, target, sizeof(float) * n * kTOut * kNOut, cudaMemcpyHostToDevice, s->stream));
-    return CS_OK;
-}
-
 // The kernels of one step on n rows whose inputs and targets are in xdev and tdev: loss
 // terms summed into lsum, gradients in g and, with `update`, the weights' update.
 static int enqueue_step(cs_sur* s, int n, bool update)
@@ -1125,7 +1162,7 @@ static int enqueue_step(cs_sur* s, int n, bool update)
     if ((r = begin_lanes(s))) return r;
     sur::k_load_x<<<(Bp * 64 + 255) / 256, 256, 0, s->stream>>>(s->xdev, n, Bp, s->act[0]);
     SCK(cudaGetLastError());
-    if ((r = forward(s, Bp))) return r;
+    if ((r = forward(s, s->lane[0], s->act.data(), Bp, s->yout, nullptr, 0, 0))) return r;
     const size_t nsq = (size_t)n * kTOut * kNOut;
     sur::k_mse<<<1184, 256, 0, s->stream>>>(s->yout, s->tdev, n, Bp, 1.f / ((float)n * kTOut * kNOut), s->dz[8], s->dzb[8], s->sq);
     SCK(cudaGetLastError());
@@ -1223,21 +1260,149 @@ static int run_step(cs_sur* s, const float* x, const float* target, int n, float
     return CS_OK;
 }
 
+// ---------------------------------------------------------------- prediction
+// Workspace of the prediction path: activations for `rows` rows, and two slots of inputs and
+// outputs, so that one group of rows is computed while the one before goes to the caller.
+// Made for as many rows as the calls so far asked for, up to the largest group.
+static cudaError_t make_predict(cs_sur* s, int rows)
+{
+    cs_sur::Predict& P = s->pred;
+    const size_t nx = (size_t)rows * 64, ny = (size_t)rows * kTOut * kNOut;   // rows are 16-byte multiples throughout
+    std::vector<size_t> at;   // activations, in floats from the start
+    size_t n = 2 * (nx + ny);
+    if (rows > s->bmax) {
+        for (size_t li = 0; li < s->L.size(); li++) {
+            at.push_back(n);
+            n += (act_elems(s, (int)li, rows) + 1) / 2;
+        }
+        size_t wide = 0;   // slices x columns of the widest split: a linear layer has K / 128 slices at most
+        for (int li = 0; li < 6; li++) wide = std::max(wide, (size_t)(s->L[li].inP / 128) * s->L[li].outP);
+        P.kpart_n = wide * rows;
+        P.kpart = nullptr;
+        n += P.kpart_n;
+    }
+    cudaError_t e = cudaMalloc(&P.dev, sizeof(float) * n);
+    if (e == cudaSuccess) e = cudaMemsetAsync(P.dev, 0, sizeof(float) * n, s->stream);
+    if (e == cudaSuccess && !P.copy) e = cudaStreamCreateWithFlags(&P.copy, cudaStreamNonBlocking);
+    for (int k = 0; k < 2; k++) {
+        if (e == cudaSuccess && !P.ready[k]) e = cudaEventCreateWithFlags(&P.ready[k], cudaEventDisableTiming);
+    }
+    if (e != cudaSuccess) return e;
+    for (int k = 0; k < 2; k++) {
+        P.xdev[k] = P.dev + k * nx;
+        P.ydev[k] = P.dev + 2 * nx + k * ny;
+    }
+    P.act.clear();
+    for (size_t a : at) P.act.push_back((bf16*)(P.dev + a));
+    if (!at.empty()) P.kpart = P.dev + (n - P.kpart_n);
+    P.rows = rows;
+    return cudaSuccess;
+}
+
+static int predict_space(cs_sur* s, int n)
+{
+    // as many whole batches as about 2048 rows hold: enough blocks for every product
+    const int batches = std::min(std::max(1, 2048 / s->bmax), n / s->bmax);
+    const int rows = s->bmax * std::max(1, batches);
+    if (rows <= s->pred.rows) return CS_OK;
+    if (s->pred.rows) SCK(cudaStreamSynchronize(s->stream));
+    free_predict(s);
+    if (make_predict(s, rows) == cudaSuccess) return CS_OK;
+    cudaGetLastError();   // no memory for a group: one batch at a time
+    free_predict(s);
+    SCK(make_predict(s, s->bmax));
+    return CS_OK;
+}
+
+// Has the pages of the caller's output mapped by a few threads while the first groups are
+// computed: left to the copies, one page fault after the other takes 20 of the 27 ms that
+// 117 MB need to reach memory the caller has just allocated (eight threads: 2.8 ms).  One
+// byte a page is written back as it is, before the first copy into the output.
+struct PageMapper {
+    std::thread th[8];
+    PageMapper(float* y, size_t n)
+    {
+        constexpr size_t kPage = 4096, kLeast = (size_t)4 << 20;
+        const size_t bytes = sizeof(float) * n;
+        if (bytes < kLeast) return;
+        const size_t nt = std::min<size_t>(8, std::max(1u, std::thread::hardware_concurrency()));
+        const size_t per = (bytes / nt + kPage) / kPage * kPage;
+        volatile char* p = (volatile char*)y;
+        try {
+            for (size_t t = 0; t < nt; t++)
+                th[t] = std::thread([=] {
+                    for (size_t i = t * per; i < std::min(bytes, (t + 1) * per); i += kPage) p[i] = p[i];
+                });
+        } catch (...) {   // no more threads to be had: the copies map what is left
+        }
+    }
+    void done()
+    {
+        for (std::thread& t : th)
+            if (t.joinable()) t.join();
+    }
+    ~PageMapper() { done(); }
+};
+
+// Predictions for n rows in groups of whole batches (several as one pass, each product
+// summed as for one batch, so a row's outputs do not depend on the grouping), the rows past
+// the last whole batch as a batch of their own.  Bound by the outputs' way into the caller's
+// memory: 20,000 rows are 117 MB, 7 ms of copying into mapped pages, beside 2.2 ms of kernels.
+static int predict(cs_sur* s, const float* x, int n, float* y)
+{
+    int r = predict_space(s, n);
+    if (r) return r;
+    cs_sur::Predict& P = s->pred;
+    const size_t ny = (size_t)kTOut * kNOut;
+    const bool wide = P.rows > s->bmax && s->gemm_impl == 0;
+    PageMapper map(y, (size_t)n * ny);
+    struct { int at, rows; } made[2] = {{0, 0}, {0, 0}};
+    auto take = [&](int k) -> int {   // slot k's outputs to the caller
+        if (made[k].rows == 0) return CS_OK;
+        map.done();
+        SCK(cudaStreamWaitEvent(P.copy, P.ready[k], 0));
+        SCK(cudaMemcpyAsync(y + (size_t)made[k].at * ny, P.ydev[k], sizeof(float) * made[k].rows * ny, cudaMemcpyDeviceToHost,
+                            P.copy));
+        SCK(cudaStreamSynchronize(P.copy));
+        made[k].rows = 0;
+        return CS_OK;
+    };
+    int k = 0;
+    for (int at = 0; at < n; k ^= 1) {
+        const int left = n - at;
+        const int nb = left < s->bmax ? left : wide ? std::min(P.rows, left / s->bmax * s->bmax) : s->bmax;
+        const bool group = nb > s->bmax;
+        const int Bp = up64(nb);
+        SCK(cudaMemcpyAsync(P.xdev[k], x + (size_t)at * kIn, sizeof(float) * nb * kIn, cudaMemcpyHostToDevice, s->stream));
+        bf16* const* act = group ? P.act.data() : s->act.data();
+        sur::k_load_x<<<(Bp * 64 + 255) / 256, 256, 0, s->stream>>>(P.xdev[k], nb, Bp, act[0]);
+        SCK(cudaGetLastError());
+        Lane w = s->lane[0];
+        if (group) {
+            w.kpart = P.kpart;
+            w.kpart_n = P.kpart_n;
+        }
+        if ((r = forward(s, w, act, Bp, s->gemm_impl == 0 ? nullptr : s->yout, P.ydev[k], nb, group ? s->bmax : 0))) return r;
+        SCK(cudaEventRecord(P.ready[k], s->stream));
+        made[k].at = at;
+        made[k].rows = nb;
+        at += nb;
+        if ((r = take(k ^ 1))) return r;
+    }
+    return take(k ^ 1);
+}
+
 extern "C" {
 
 int cs_sur_forward(cs_sur* s, const float* x, int n, float* y)
 {
     if (!s || !x || !y) return CS_E_ARG;
-    for (int b0 = 0; b0 < n; b0 += s->bmax) {
-        int nb = std::min(s->bmax, n - b0), Bp, r;
-        if ((r = load_batch(s, x + (size_t)b0 * kIn, nullptr, nb, &Bp))) return r;
-        if ((r = forward(s, Bp))) return r;
-        sur::k_store_y<<<512, 256, 0, s->stream>>>(s->yout, nb, s->ydev);
-        SCK(cudaGetLastError());
-        SCK(cudaMemcpyAsync(y + (size_t)b0 * kTOut * kNOut, s->ydev, sizeof(float) * nb * kTOut * kNOut,
-                            cudaMemcpyDeviceToHost, s->stream));
-    }
-    return sync_check(s);
+    if (n <= 0) return sync_check(s);
+    const int r = predict(s, x, n, y);
+    if (r == CS_OK) return sync_check(s);
+    cudaStreamSynchronize(s->stream);   // nothing of the call is left in flight
+    if (s->pred.copy) cudaStreamSynchronize(s->pred.copy);
+    return r;
 }
 
 int cs_sur_loss_grad(cs_sur* s, const float* x, const float* target, int n, float* loss, float* grad)
@@ -1251,9 +1416,9 @@ int cs_sur_loss_grad(cs_sur* s, const float* x, const float* target, int n, floa
         if ((r = sync_check(s))) return r;
         size_t k = 0;
         for (auto& l : s->L) {
-            for (int o = 0; o < l.out; o++)
-                for (int i = 0; i < l.in; i++) grad[k++] = h[l.wofs + (size_t)o * l.inP + i];
-            for (int o = 0; o < l.out; o++) grad[k++] = h[l.bofs + o];
+            for (int o = 0; o < l.out; o++, k += l.in) memcpy(grad + k, &h[l.wofs + (size_t)o * l.inP], sizeof(float) * l.in);
+            memcpy(grad + k, &h[l.bofs], sizeof(float) * l.out);
+            k += l.out;
         }
     }
     return CS_OK;

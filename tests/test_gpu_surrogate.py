@@ -1,0 +1,75 @@
+"""The surrogate network's paths that depend on how many rows a call has: predictions in
+groups of batches, in two slots, against the same rows batch by batch (tolerance: none, a
+group's products are summed as a batch's) and against the CPU reference (the tolerance of a
+forward pass in bfloat16 operands, 1e-2 as for one batch); gradients at ragged sizes, with
+products of few and of many blocks; and training steps whose recorded forms are made, kept
+and dropped again as sizes come and go (tolerance: none)."""
+import numpy as np
+import pytest
+
+import surrogate_ref as ref
+
+pytestmark = pytest.mark.gpu
+
+
+def _case(n, seed):
+    rng = np.random.default_rng(seed)
+    flat = (ref.init_params(seed) + rng.normal(0.0, 0.02, ref.init_params(seed).shape)).astype(np.float32)
+    return flat, rng.random((n, ref.N_IN)).astype(np.float32), rng.normal(0.0, 1.0, (n, ref.T_OUT, ref.N_OUT)).astype(np.float32)
+
+
+def _rel(a, b):
+    return float(np.linalg.norm(a - b) / max(np.linalg.norm(b), 1e-30))
+
+
+@pytest.mark.parametrize("max_batch,n", [(64, 1), (64, 65), (64, 2048), (64, 4200), (200, 2047), (200, 5121), (2100, 2200)])
+def test_predictions_in_groups_are_those_of_single_batches(max_batch, n):
+    from covidsim_b200 import surrogate
+    flat, x, _ = _case(n, 21)
+    net = surrogate.Surrogate(max_batch=max_batch, params=flat)
+    step = (max_batch + 63) // 64 * 64                 # the capacity that the batch is rounded up to
+    single = np.concatenate([net.predict(x[i:i + step]) for i in range(0, n, step)])
+    for _ in range(2):                                 # the second call finds the workspace in place
+        assert np.array_equal(net.predict(x), single)
+    pick = np.unique(np.linspace(0, n - 1, 40).astype(int))
+    assert _rel(single[pick], ref.forward(flat, x[pick], round_bf16=True)) < 1e-2
+    net.set_gemm("mma.sync")                           # one batch at a time; only summation order differs
+    assert _rel(net.predict(x), single) < 2e-3
+    net.close()
+
+
+@pytest.mark.parametrize("n", [1, 63, 129, 300])
+def test_gradients_at_ragged_sizes(n):
+    from covidsim_b200 import surrogate
+    flat, x, target = _case(n, 23)
+    out = {}
+    for impl in ("tcgen05", "mma.sync"):
+        net = surrogate.Surrogate(max_batch=320, params=flat)
+        net.set_gemm(impl)
+        out[impl] = net.loss_grad(x, target)
+        again = net.loss_grad(x, target)
+        assert again[0] == out[impl][0] and np.array_equal(again[1], out[impl][1])
+        net.close()
+    assert abs(out["tcgen05"][0] - out["mma.sync"][0]) <= 1e-4 * abs(out["mma.sync"][0])
+    k = 0
+    for name, (o, i) in ref.layer_shapes():
+        for part, m in (("W", o * i), ("b", o)):
+            e = _rel(out["tcgen05"][1][k:k + m], out["mma.sync"][1][k:k + m])
+            assert e < 1e-2, (name, part, e)
+            k += m
+
+
+def test_training_steps_do_not_depend_on_what_is_recorded():
+    from covidsim_b200 import surrogate
+    flat, x, target = _case(200, 25)
+    sizes = [200, 1, 64, 65, 100, 127, 128, 129, 190, 7, 200, 1, 64, 100]   # ten sizes, then some again
+    a, b = (surrogate.Surrogate(max_batch=256, params=flat) for _ in range(2))
+    for k, n in enumerate(sizes):
+        la = a.train_step(x[:n], target[:n], 1e-3)
+        if k % 2:
+            b.loss_grad(x[:n + 3], target[:n + 3]) if n + 3 <= 200 else b.predict(x)
+        lb = b.train_step(x[:n], target[:n], 1e-3)
+        assert la == lb, (k, n)
+        assert np.array_equal(a.get_params(), b.get_params()), (k, n)
+    a.close()
+    b.close()
