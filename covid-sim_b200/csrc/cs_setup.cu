@@ -7,8 +7,8 @@
 // every sum is an integer sum or has a fixed order, and the only atomics are
 // integer counts, so the result is a function of the spec alone.
 //
-// Work is one thread per microcell, person, household or place; the passes that
-// need an order (people per cell, households per microcell, places' member lists)
+// Work is one thread per microcell, person, household or place (a warp per person who
+// is still without a place, and per place for its groups); the passes that need an order (people per cell, households per microcell, places' member lists)
 // take it from exclusive scans and one stable radix sort, written below.
 #include <algorithm>
 #include <cmath>
@@ -17,6 +17,7 @@
 #include <cstdarg>
 #include <cstring>
 #include <string>
+#include <thread>
 #include <vector>
 
 #include <cuda_runtime.h>
@@ -543,127 +544,339 @@ __global__ void k_bucket_count(int npl, Buckets B, const float* __restrict__ px,
     atomicAdd(bcnt + b, 1);
 }
 
+// A place as the proposals read it: one 16-byte record, bucket by bucket, so that a bucket's
+// (and a column of buckets') candidates are one run of memory.
+struct __align__(16) PlaceSeen {
+    float x, y;
+    int32_t pl, room;
+};
+
 __global__ void k_bucket_fill(int npl, const int32_t* __restrict__ pb, int32_t* __restrict__ cursor,
-                              int32_t* __restrict__ items)
+                              const float* __restrict__ px, const float* __restrict__ py, const int32_t* __restrict__ rem,
+                              PlaceSeen* __restrict__ seen, int32_t* __restrict__ seen_at)
 {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < npl) items[atomicAdd(cursor + pb[i], 1)] = i;   // order within a bucket is immaterial
+    if (i >= npl) return;
+    const int e = atomicAdd(cursor + pb[i], 1);   // order within a bucket is immaterial
+    seen[e] = PlaceSeen{px[i], py[i], i, rem[i]};
+    seen_at[i] = e;
 }
 
-struct Cand { double d2; int32_t pl; };
+// The nn nearest candidates of one attendee, rank by lane: lane k holds the k-th of all that
+// were put in, (d2, place) ascending; lanes past the number put in hold +inf.
+struct Nearest {
+    double d2;
+    int32_t pl;
 
-// (d2, place) ascending: the candidates' order does not depend on the visit order.
-__device__ __forceinline__ bool cand_less(double d2, int pl, const Cand& c)
-{
-    return d2 < c.d2 || (d2 == c.d2 && pl < c.pl);
-}
+    __device__ __forceinline__ bool before(double od2, int opl) const   // is (od2, opl) before this lane's entry
+    {
+        return od2 < d2 || (od2 == d2 && opl < pl);
+    }
+    // The warp's 32 candidates (+inf where a lane has none) as the first entries: a bitonic sort.
+    __device__ __forceinline__ void start(double cd2, int cpl, int lane)
+    {
+        d2 = cd2;
+        pl = cpl;
+#pragma unroll
+        for (int k = 2; k <= 32; k <<= 1)
+#pragma unroll
+            for (int j = k >> 1; j > 0; j >>= 1) {
+                const double od2 = __shfl_xor_sync(0xffffffffu, d2, j);
+                const int opl = __shfl_xor_sync(0xffffffffu, pl, j);
+                // the pair's lower lane keeps the smaller entry, in a descending run the larger
+                if (before(od2, opl) == (((lane & j) == 0) == ((lane & k) == 0))) {
+                    d2 = od2;
+                    pl = opl;
+                }
+            }
+    }
+    // Candidates of the lanes with `in`, one after the other; entries past rank 31 drop out.
+    __device__ __forceinline__ void add(double cd2, int cpl, bool in, int nn, int lane)
+    {
+        const double wd2 = __shfl_sync(0xffffffffu, d2, nn - 1);
+        const int wpl = __shfl_sync(0xffffffffu, pl, nn - 1);
+        in = in && (cd2 < wd2 || (cd2 == wd2 && cpl < wpl));
+        for (unsigned m = __ballot_sync(0xffffffffu, in); m; m &= m - 1) {
+            const int j = __ffs(m) - 1;
+            const double xd2 = __shfl_sync(0xffffffffu, cd2, j);
+            const int xpl = __shfl_sync(0xffffffffu, cpl, j);
+            const bool moves = before(xd2, xpl);
+            const unsigned mm = __ballot_sync(0xffffffffu, moves);
+            const double ud2 = __shfl_up_sync(0xffffffffu, d2, 1);
+            const int upl = __shfl_up_sync(0xffffffffu, pl, 1);
+            if (moves) {
+                const bool here = lane == __ffs(mm) - 1;
+                d2 = here ? xd2 : ud2;
+                pl = here ? xpl : upl;
+            }
+        }
+    }
+};
 
-// One round of proposals: attendee a (person p) without a place gathers the nn
-// nearest places with room (rings of buckets until nn are in hand, then one ring
-// more) and proposes to one with probability proportional to K(d) * room (K alone
-// in the capacity-free round).
-__global__ void __launch_bounds__(128) k_propose(uint64_t seed, int t, int round, int free_round, int n_att, int nn,
-                                                 Buckets B, const cs_params* __restrict__ Pp,
-                                                 const double* __restrict__ lk, const double* __restrict__ hr,
-                                                 const int32_t* __restrict__ list, const int32_t* __restrict__ person_hh,
-                                                 const float* __restrict__ hh_x, const float* __restrict__ hh_y,
-                                                 const float* __restrict__ px, const float* __restrict__ py,
-                                                 const int32_t* __restrict__ bstart, const int32_t* __restrict__ items,
-                                                 const int32_t* __restrict__ rem, const int32_t* __restrict__ link,
-                                                 int32_t* __restrict__ prop)
+// The rings of buckets around a household, as runs of place records: rings 0 and 1 together
+// (ring 1 is always needed) are the 3 columns of their square, the middle one first; a
+// further ring r is its two outer columns and the two ends of the others.  A column's
+// buckets, and so their records, lie one after the other.
+struct Rings {
+    int bx, by, rmax, r = 1, found = 0, found0 = 0, extra = -1;
+
+    __device__ __forceinline__ Rings(const Buckets& B, int b0) : bx(b0 / B.nby), by(b0 % B.nby), rmax(max(B.nbx, B.nby)) {}
+    __device__ __forceinline__ int runs() const { return r == 1 ? 3 : 4 * r; }
+    __device__ __forceinline__ void run(const Buckets& B, const int32_t* __restrict__ bstart, int k, int* start, int* end) const
+    {
+        int x, y0 = by - r, y1 = by + r;
+        if (r == 1) x = k == 0 ? bx : bx + 2 * k - 3;
+        else if (k < 2) x = k ? bx + r : bx - r;
+        else {
+            x = bx - r + 1 + ((k - 2) >> 1);
+            if (k & 1) y0 = y1; else y1 = y0;
+        }
+        y0 = max(y0, 0);
+        y1 = min(y1, B.nby - 1);
+        *start = *end = 0;
+        if (x >= 0 && x < B.nbx && y0 <= y1) {
+            *start = bstart[x * B.nby + y0];
+            *end = bstart[x * B.nby + y1 + 1];
+        }
+    }
+    // The ring is through: rings go on until nn places with room were found, then one more.
+    __device__ __forceinline__ bool more(int nn)
+    {
+        if (r == 1 && found0 >= nn) extra = 1;
+        if (extra > 0) extra--;
+        else if (found >= nn) extra = 1;
+        r++;
+        return r < rmax && extra != 0;
+    }
+};
+
+// One round of proposals: an attendee (person p) without a place gathers the nn nearest
+// places with room (rings of buckets until nn are in hand, then one ring more) and
+// proposes to one with probability proportional to K(d) * room (K alone in the
+// capacity-free round).  Two forms of it:
+//
+// The first round, a thread per attendee: neighbours look through the same runs in step, so
+// a record is one broadcast load, and few candidates are among the nearest so far.
+// Bound by the instructions per candidate.  1,000,000 people, 480,000 workers choosing among
+// 24 places: 1420 us with places, rooms and locations gathered one by one, 830 now; a warp
+// per attendee took 1830.
+__global__ void __launch_bounds__(128) k_propose_first(uint64_t seed, int t, int free_round, int n_att, int nn, Buckets B,
+                                                       const cs_params* __restrict__ Pp,
+                                                       const double* __restrict__ lk, const double* __restrict__ hr,
+                                                       const int32_t* __restrict__ list, const int32_t* __restrict__ person_hh,
+                                                       const float* __restrict__ hh_x, const float* __restrict__ hh_y,
+                                                       const int32_t* __restrict__ bstart, const PlaceSeen* __restrict__ seen,
+                                                       const int32_t* __restrict__ rem,
+                                                       int32_t* __restrict__ prop, int32_t* __restrict__ nprop)
 {
     int a = blockIdx.x * blockDim.x + threadIdx.x;
     if (a >= n_att) return;
     prop[a] = -1;
-    if (link[a] >= 0) return;
     const cs_params& P = *Pp;
     const int p = list[a];
     const int h = person_hh[p];
     const float hx = hh_x[h], hy = hh_y[h];
     const int b0 = bucket_of(B, hx, hy);
-    const int bx = b0 / B.nby, by = b0 % B.nby;
-    Cand top[CS_SETUP_MAX_NEAREST];
-    int ntop = 0, found = 0, extra = -1;
-    const int rmax = max(B.nbx, B.nby);
-    for (int r = 0; r < rmax && extra != 0; r++) {
-        // the ring's buckets: the square's perimeter at Chebyshev distance r
-        const int side = (r == 0) ? 1 : 8 * r;
-        for (int q = 0; q < side; q++) {
-            int x, y;
-            if (r == 0) { x = bx; y = by; }
-            else if (q < 2 * r + 1) { x = bx - r + q; y = by - r; }                    // bottom row
-            else if (q < 4 * r + 2) { x = bx - r + (q - 2 * r - 1); y = by + r; }      // top row
-            else if (q < 6 * r + 1) { x = bx - r; y = by - r + 1 + (q - 4 * r - 2); }  // left column
-            else { x = bx + r; y = by - r + 1 + (q - 6 * r - 1); }                      // right column
-            if (x < 0 || y < 0 || x >= B.nbx || y >= B.nby) continue;
-            const int bk = x * B.nby + y;
-            for (int e = bstart[bk]; e < bstart[bk + 1]; e++) {
-                const int pl = items[e];
-                if (!free_round && rem[pl] <= 0) continue;
-                found++;
-                const double d2 = dist2_pts(P, hx, hy, px[pl], py[pl]);
-                if (ntop == nn && !cand_less(d2, pl, top[nn - 1])) continue;
-                int k = (ntop < nn) ? ntop++ : nn - 1;
-                while (k > 0 && cand_less(d2, pl, top[k - 1])) { top[k] = top[k - 1]; k--; }
-                top[k].d2 = d2;
-                top[k].pl = pl;
+    const int e0 = bstart[b0], e1 = bstart[b0 + 1];   // ring 0
+    Rings R(B, b0);
+    double td2[CS_SETUP_MAX_NEAREST];
+    int tpl[CS_SETUP_MAX_NEAREST];
+    double wd2 = __longlong_as_double(0x7ff0000000000000LL);   // the last of a full list
+    int ntop = 0, wpl = 0x7fffffff;
+    do {
+        for (int k = 0; k < R.runs(); k++) {
+            int e, end;
+            R.run(B, bstart, k, &e, &end);
+            for (; e < end; e++) {
+                const int4 q = *reinterpret_cast<const int4*>(seen + e);
+                if (!free_round && q.w <= 0) continue;
+                R.found++;
+                if (e >= e0 && e < e1) R.found0++;
+                const double d2 = dist2_pts(P, hx, hy, __int_as_float(q.x), __int_as_float(q.y));
+                if (d2 > wd2 || (d2 == wd2 && q.z > wpl)) continue;
+                int j = ntop < nn ? ntop++ : nn - 1;
+                for (; j > 0 && (d2 < td2[j - 1] || (d2 == td2[j - 1] && q.z < tpl[j - 1])); j--) {
+                    td2[j] = td2[j - 1];
+                    tpl[j] = tpl[j - 1];
+                }
+                td2[j] = d2;
+                tpl[j] = q.z;
+                if (ntop == nn) {
+                    wd2 = td2[nn - 1];
+                    wpl = tpl[nn - 1];
+                }
             }
         }
-        if (extra > 0) extra--;
-        else if (extra < 0 && found >= nn) extra = 1;
-    }
+    } while (R.more(nn));
     if (ntop == 0) return;
-    double w[CS_SETUP_MAX_NEAREST];
     double tot = 0.0;
     for (int k = 0; k < ntop; k++) {
-        w[k] = knum_tab(lk, hr, P, top[k].d2) * (free_round ? 1.0 : (double)rem[top[k].pl]);
-        tot = tot + w[k];
+        td2[k] = knum_tab(lk, hr, P, td2[k]) * (free_round ? 1.0 : (double)rem[tpl[k]]);   // its weight from here on
+        tot = tot + td2[k];
     }
     int k = 0;
     if (tot > 0) {
-        Stream s(seed, CS_RNG_SETUP_CHOOSE, (uint32_t)round, (uint32_t)p, (uint32_t)t);
+        Stream s(seed, CS_RNG_SETUP_CHOOSE, 0u, (uint32_t)p, (uint32_t)t);
         double u = s.next() * tot;
-        while (k + 1 < ntop && u >= w[k]) { u -= w[k]; k++; }
+        while (k + 1 < ntop && u >= td2[k]) { u -= td2[k]; k++; }
     } else if (!free_round) {
         return;   // every place in reach is beyond the kernel: wait for the last round
     }
-    prop[a] = top[k].pl;
+    prop[a] = tpl[k];
+    atomicAdd(nprop + tpl[k], 1);
 }
 
-__global__ void k_count_props(int n_att, const int32_t* __restrict__ prop, int32_t* __restrict__ nprop)
+// The later rounds, a warp per attendee that is still without a place (`open`, as many as
+// n_open says), dealt one by one: these live where places are short, side by side in the
+// list, and search wide.  The lanes take a run's candidates 32 at a time and hold the
+// nearest in order of rank.  Bound by the gathers' and shuffles' latency.  1,000,000 people,
+// 24 such launches: a thread per attendee of the whole list took 4.5 ms (its last searches
+// alone in their warps), a warp per 32 attendees of the list 4.0, this 1.5.
+__global__ void __launch_bounds__(128) k_propose(uint64_t seed, int t, int round, int free_round, int nn, Buckets B,
+                                                 const cs_params* __restrict__ Pp,
+                                                 const double* __restrict__ lk, const double* __restrict__ hr,
+                                                 const int32_t* __restrict__ list, const int32_t* __restrict__ person_hh,
+                                                 const float* __restrict__ hh_x, const float* __restrict__ hh_y,
+                                                 const int32_t* __restrict__ bstart, const PlaceSeen* __restrict__ seen,
+                                                 const int32_t* __restrict__ rem, const int32_t* __restrict__ open,
+                                                 const int32_t* __restrict__ n_open, int32_t* __restrict__ next,
+                                                 int32_t* __restrict__ prop, int32_t* __restrict__ nprop)
 {
-    int a = blockIdx.x * blockDim.x + threadIdx.x;
-    if (a < n_att && prop[a] >= 0) atomicAdd(nprop + prop[a], 1);
-}
-
-__global__ void k_accept(uint64_t seed, int t, int round, int free_round, int n_att, const int32_t* __restrict__ list,
-                         const int32_t* __restrict__ prop, const int32_t* __restrict__ nprop,
-                         const int32_t* __restrict__ rem, int32_t* __restrict__ link, int32_t* __restrict__ taken,
-                         int32_t* __restrict__ forced)
-{
-    int a = blockIdx.x * blockDim.x + threadIdx.x;
-    if (a >= n_att) return;
-    const int pl = prop[a];
-    if (pl < 0) return;
-    bool ok = true;
-    if (!free_round) {
-        const int n = nprop[pl], r = rem[pl];
-        if (n > r) {
-            Stream s(seed, CS_RNG_SETUP_ACCEPT, (uint32_t)round, (uint32_t)list[a], (uint32_t)t);
-            ok = s.next() * (double)n < (double)r;
+    constexpr unsigned kAll = 0xffffffffu;
+    const int lane = threadIdx.x & 31, n = *n_open;
+    const cs_params& P = *Pp;
+    for (;;) {
+        int i = 0;
+        if (lane == 0) i = atomicAdd(next, 1);
+        i = __shfl_sync(kAll, i, 0);
+        if (i >= n) return;
+        const int p = list[open[i]];
+        const int h = person_hh[p];
+        const float hx = hh_x[h], hy = hh_y[h];
+        const int b0 = bucket_of(B, hx, hy);
+        const int e0 = bstart[b0], e1 = bstart[b0 + 1];   // ring 0
+        Rings R(B, b0);
+        Nearest top;
+        bool empty = true;
+        do {
+            const int nruns = R.runs();
+            for (int s0 = 0; s0 < nruns; s0 += 32) {
+                int start = 0, end = 0;
+                if (s0 + lane < nruns) R.run(B, bstart, s0 + lane, &start, &end);
+                int inc = end - start;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const int y = __shfl_up_sync(kAll, inc, o);
+                    if (lane >= o) inc += y;
+                }
+                const int total = __shfl_sync(kAll, inc, 31), ofs = end - inc;
+                auto at = [&](int c) {   // the record of candidate c
+                    int sg = 0;          // its run
+#pragma unroll
+                    for (int o = 16; o > 0; o >>= 1)
+                        if (__shfl_sync(kAll, inc, sg + o - 1) <= c) sg += o;
+                    return c + __shfl_sync(kAll, ofs, sg);
+                };
+                auto load = [&](int c, int e) {
+                    return c < total ? *reinterpret_cast<const int4*>(seen + e) : make_int4(0, 0, 0, 0);
+                };
+                int e = at(lane);
+                int4 q = load(lane, e);
+                for (int c0 = 0; c0 < total; c0 += 32) {
+                    const int en = at(c0 + 32 + lane);
+                    const int4 qn = load(c0 + 32 + lane, en);   // on its way while this one is looked at
+                    int pl = 0x7fffffff;
+                    double d2 = __longlong_as_double(0x7ff0000000000000LL);   // +inf
+                    const bool ok = c0 + lane < total && (free_round || q.w > 0);
+                    if (ok) {
+                        pl = q.z;
+                        d2 = dist2_pts(P, hx, hy, __int_as_float(q.x), __int_as_float(q.y));
+                    }
+                    const unsigned got = __ballot_sync(kAll, ok);
+                    R.found += __popc(got);
+                    if (R.r == 1) R.found0 += __popc(__ballot_sync(kAll, ok && e >= e0 && e < e1));
+                    if (got) {
+                        if (empty) top.start(d2, pl, lane);
+                        else top.add(d2, pl, ok, nn, lane);
+                        empty = false;
+                    }
+                    q = qn;
+                    e = en;
+                }
+            }
+        } while (R.more(nn));
+        int pick = -1;
+        const int ntop = min(R.found, nn);
+        if (ntop > 0) {
+            const double w = lane < ntop ? knum_tab(lk, hr, P, top.d2) * (free_round ? 1.0 : (double)rem[top.pl]) : 0.0;
+            double tot = 0.0;
+            for (int k = 0; k < ntop; k++) tot = tot + __shfl_sync(kAll, w, k);
+            int k = 0;
+            if (tot > 0) {
+                Stream s(seed, CS_RNG_SETUP_CHOOSE, (uint32_t)round, (uint32_t)p, (uint32_t)t);
+                double u = s.next() * tot;
+                for (; k + 1 < ntop; k++) {
+                    const double wk = __shfl_sync(kAll, w, k);
+                    if (!(u >= wk)) break;
+                    u -= wk;
+                }
+            } else if (!free_round) {
+                k = -1;   // every place in reach is beyond the kernel: wait for the last round
+            }
+            if (k >= 0) pick = __shfl_sync(kAll, top.pl, k);
+        }
+        if (lane == 0) {
+            prop[i] = pick;
+            if (pick >= 0) atomicAdd(nprop + pick, 1);
         }
     }
-    if (!ok) return;
-    link[a] = pl;
-    atomicAdd(taken + pl, 1);
-    if (free_round) atomicAdd(forced, 1);
 }
 
-__global__ void k_take(int npl, int32_t* __restrict__ rem, int32_t* __restrict__ taken, int32_t* __restrict__ nprop)
+// The places' answers to the proposals of the attendees in `open` (null: all n_att); those
+// left without a place are the next round's.
+__global__ void k_accept(uint64_t seed, int t, int round, int free_round, int n_att, const int32_t* __restrict__ open,
+                         const int32_t* __restrict__ n_open, const int32_t* __restrict__ list,
+                         const int32_t* __restrict__ prop, const int32_t* __restrict__ nprop,
+                         const int32_t* __restrict__ rem, int32_t* __restrict__ link, int32_t* __restrict__ taken,
+                         int32_t* __restrict__ left, int32_t* __restrict__ n_left)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const bool in = i < (open ? *n_open : n_att);
+    int a = 0;
+    bool ok = false;
+    if (in) {
+        a = open ? open[i] : i;
+        const int pl = prop[i];
+        ok = pl >= 0;
+        if (ok && !free_round) {
+            const int n = nprop[pl], r = rem[pl];
+            if (n > r) {
+                Stream s(seed, CS_RNG_SETUP_ACCEPT, (uint32_t)round, (uint32_t)list[a], (uint32_t)t);
+                ok = s.next() * (double)n < (double)r;
+            }
+        }
+        if (ok) {
+            link[a] = pl;
+            atomicAdd(taken + pl, 1);
+        }
+    }
+    const unsigned m = __ballot_sync(0xffffffffu, in && !ok);
+    if (!m) return;
+    const int lane = threadIdx.x & 31;
+    int base = 0;
+    if (lane == 0) base = atomicAdd(n_left, __popc(m));
+    base = __shfl_sync(0xffffffffu, base, 0);
+    if (in && !ok) left[base + __popc(m & ((1u << lane) - 1u))] = a;
+}
+
+__global__ void k_take(int npl, int32_t* __restrict__ rem, int32_t* __restrict__ taken, int32_t* __restrict__ nprop,
+                       PlaceSeen* __restrict__ seen, const int32_t* __restrict__ seen_at)
 {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= npl) return;
-    rem[i] = max(rem[i] - taken[i], 0);
+    const int room = max(rem[i] - taken[i], 0);
+    rem[i] = room;
+    seen[seen_at[i]].room = room;
     taken[i] = 0;
     nprop[i] = 0;
 }
@@ -694,21 +907,24 @@ __global__ void k_group_counts(int npl, int g1, const int32_t* __restrict__ mcou
     if (i < npl) ng[i] = max(1, (int)floor((double)mcount[i] / (double)g1 + 0.5));
 }
 
-// Group k of a place of n members covers members [k n / ng, (k+1) n / ng).
+// Group k of a place of n members covers members [k n / ng, (k+1) n / ng).  A warp per
+// place, its lanes side by side over groups and members: the writes to the members are
+// scattered, and a thread per place waited for its own (1,000,000 people 968 us, 184 now).
 __global__ void k_groups(int npl, const int32_t* __restrict__ mcount, const int32_t* __restrict__ mofs,
                          const int32_t* __restrict__ ng, const int32_t* __restrict__ gofs,
                          const int32_t* __restrict__ members, int32_t* __restrict__ gstart,
                          int32_t* __restrict__ gsize, uint16_t* __restrict__ person_group)
 {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const long long i = ((long long)blockIdx.x * blockDim.x + threadIdx.x) / 32;
     if (i >= npl) return;
-    const long long n = mcount[i], g = ng[i];
-    for (long long k = 0; k < g; k++) {
+    const long long n = mcount[i], g = ng[i], lane = threadIdx.x & 31;
+    for (long long k = lane; k < g; k += 32) {
         const long long s = (k * n) / g, e = ((k + 1) * n) / g;
         gstart[gofs[i] + k] = (int32_t)s;
         gsize[gofs[i] + k] = (int32_t)(e - s);
-        for (long long q = s; q < e; q++) person_group[members[mofs[i] + q]] = (uint16_t)k;
     }
+    // member q's group: the largest k with floor(k n / g) <= q, that is k n < (q + 1) g
+    for (long long q = lane; q < n; q += 32) person_group[members[mofs[i] + q]] = (uint16_t)(((q + 1) * g - 1) / n);
 }
 
 __global__ void k_fill_i32(int32_t* p, long long n, int32_t v)
@@ -734,6 +950,8 @@ struct cs_setup {
     cudaStream_t stream = nullptr;
     std::string err;
     std::vector<void*> allocs;
+    char* slab = nullptr;                      // what is left of the newest slab (dalloc)
+    size_t slab_left = 0, slab_total = 0;
     int32_t N = 0, NH = 0, NC = 0, NM = 0, n_adunits = 1, npt = 0;
     double device_ms = 0;
     int32_t *person_hh = nullptr, *person_mcell = nullptr, *person_place = nullptr, *hh_first = nullptr,
@@ -770,13 +988,30 @@ int fail(cs_setup* s, int code, const char* fmt, ...)
         if (e_ != cudaSuccess) return fail(s, CS_E_CUDA, "%s: %s", #kern, cudaGetErrorString(e_)); \
     } while (0)
 
+// Device memory comes in slabs, each as large as all before it (32 MB at least), and is
+// given back with the set-up: its some 200 arrays, allocated and freed one by one, took
+// some 20 of the 44 ms that a set-up of 1,000,000 people lasted.
 template <typename T>
 int dalloc(cs_setup* s, T** p, long long n)
 {
-    void* q = nullptr;
-    SK(cudaMalloc(&q, (size_t)std::max(n, 1LL) * sizeof(T)));
-    s->allocs.push_back(q);
-    *p = (T*)q;
+    const size_t bytes = ((size_t)std::max(n, 1LL) * sizeof(T) + 255) / 256 * 256;
+    if (bytes > s->slab_left) {
+        size_t take = std::max(bytes, std::max(s->slab_total, (size_t)32 << 20));
+        void* q = nullptr;
+        cudaError_t e = cudaMalloc(&q, take);
+        if (e != cudaSuccess && take > bytes) {   // no room for a slab: the array alone
+            cudaGetLastError();
+            e = cudaMalloc(&q, take = bytes);
+        }
+        if (e != cudaSuccess) return fail(s, CS_E_CUDA, "cudaMalloc(%zu bytes): %s", bytes, cudaGetErrorString(e));
+        s->allocs.push_back(q);
+        s->slab = (char*)q;
+        s->slab_left = take;
+        s->slab_total += take;
+    }
+    *p = (T*)s->slab;
+    s->slab += bytes;
+    s->slab_left -= bytes;
     return CS_OK;
 }
 
@@ -852,6 +1087,48 @@ int radix_sort(cs_setup* s, uint64_t* keys, int32_t* vals, long long n, int bits
     return CS_OK;
 }
 
+// Copies of host arrays to the device by a thread of their own, so that the copy through the
+// driver's staging buffers (5.5 ms for two tables of 2,000,000 entries) does not hold up the
+// launches.  done() waits for them; so does leaving the set-up on an error.
+struct TableCopies {
+    struct Item { void* dst; const void* src; size_t bytes; };
+    Item items[2 * CS_MAX_PLACE_TYPES];
+    int n = 0, device;
+    cudaError_t err = cudaSuccess;
+    std::thread th;
+
+    explicit TableCopies(int dev) : device(dev) {}
+    ~TableCopies() { done(); }
+    void add(void* dst, const void* src, size_t bytes) { items[n++] = {dst, src, bytes}; }
+    void copy()
+    {
+        cudaStream_t st = nullptr;
+        err = cudaSetDevice(device);
+        if (err == cudaSuccess) err = cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking);
+        for (int k = 0; k < n && err == cudaSuccess; k++)
+            err = cudaMemcpyAsync(items[k].dst, items[k].src, items[k].bytes, cudaMemcpyHostToDevice, st);
+        if (st) {
+            const cudaError_t e = cudaStreamSynchronize(st);
+            if (err == cudaSuccess) err = e;
+            cudaStreamDestroy(st);
+        }
+    }
+    void start()
+    {
+        if (n == 0) return;
+        try {
+            th = std::thread([this] { copy(); });
+        } catch (...) {
+            copy();   // no thread to be had
+        }
+    }
+    cudaError_t done()
+    {
+        if (th.joinable()) th.join();
+        return err;
+    }
+};
+
 int check_spec(cs_setup* s, const cs_setup_spec& S, const cs_params& P)
 {
     if (S.n_people <= 0 || S.ncw <= 0 || S.nch <= 0 || S.nmcl <= 0)
@@ -908,6 +1185,29 @@ int run_setup(cs_setup* s, const cs_setup_spec& S, const cs_params& P)
     cs_params* Pd;
     SALLOC(Pd, 1);
     SK(cudaMemcpyAsync(Pd, &P, sizeof(cs_params), cudaMemcpyHostToDevice, s->stream));
+    // The place types' kernel tables are host arrays: each distinct one is copied to the
+    // device once, beside everything up to the first proposals.
+    const int npt = S.num_place_types;
+    const size_t ktab = (size_t)P.kernel_size + 1;
+    const double* klk[CS_MAX_PLACE_TYPES] = {};
+    const double* khr[CS_MAX_PLACE_TYPES] = {};
+    TableCopies tables(s->device);
+    for (int t = 0; t < npt; t++) {
+        for (int u = 0; u < t && !klk[t]; u++)
+            if (S.pt[u].kernel_lookup == S.pt[t].kernel_lookup && S.pt[u].kernel_hi_res == S.pt[t].kernel_hi_res) {
+                klk[t] = klk[u];
+                khr[t] = khr[u];
+            }
+        if (klk[t]) continue;
+        double *a, *b;
+        SALLOC(a, ktab);
+        SALLOC(b, ktab);
+        tables.add(a, S.pt[t].kernel_lookup, sizeof(double) * ktab);
+        tables.add(b, S.pt[t].kernel_hi_res, sizeof(double) * ktab);
+        klk[t] = a;
+        khr[t] = b;
+    }
+    tables.start();
     unsigned long long* err;
     SALLOC(err, 1);
     SK(cudaMemsetAsync(err, 0, sizeof(unsigned long long), s->stream));
@@ -998,27 +1298,7 @@ int run_setup(cs_setup* s, const cs_setup_spec& S, const cs_params& P)
     SALLOC(s->person_age, N);
     SLAUNCH(k_ages, nblk(N), kT, seed, N, ar, s->person_age);
 
-    // 6. places.  The spec's kernel tables are host arrays: each distinct one is
-    // copied to the device once.
-    const int npt = S.num_place_types;
-    const size_t ktab = (size_t)P.kernel_size + 1;
-    const double* klk[CS_MAX_PLACE_TYPES] = {};
-    const double* khr[CS_MAX_PLACE_TYPES] = {};
-    for (int t = 0; t < npt; t++) {
-        for (int u = 0; u < t && !klk[t]; u++)
-            if (S.pt[u].kernel_lookup == S.pt[t].kernel_lookup && S.pt[u].kernel_hi_res == S.pt[t].kernel_hi_res) {
-                klk[t] = klk[u];
-                khr[t] = khr[u];
-            }
-        if (klk[t]) continue;
-        double *a, *b;
-        SALLOC(a, ktab);
-        SALLOC(b, ktab);
-        SK(cudaMemcpyAsync(a, S.pt[t].kernel_lookup, sizeof(double) * ktab, cudaMemcpyHostToDevice, s->stream));
-        SK(cudaMemcpyAsync(b, S.pt[t].kernel_hi_res, sizeof(double) * ktab, cudaMemcpyHostToDevice, s->stream));
-        klk[t] = a;
-        khr[t] = b;
-    }
+    // 6. places
     SALLOC(s->person_place, (long long)std::max(npt, 1) * N);
     SALLOC(s->person_group, (long long)std::max(npt, 1) * N);
     SLAUNCH(k_fill_i32, nblk((long long)npt * N), kT, s->person_place, (long long)npt * N, -1);
@@ -1080,38 +1360,55 @@ int run_setup(cs_setup* s, const cs_setup_spec& S, const cs_params& P)
         B.nbx = (ncw + B.bs - 1) / B.bs;
         B.nby = (nch + B.bs - 1) / B.bs;
         const int NBK = B.nbx * B.nby;
-        int32_t *pb, *bcnt, *bstart, *cursor, *items;
+        int32_t *pb, *bcnt, *bstart, *cursor, *seen_at;
+        PlaceSeen* seen;
         SALLOC(pb, npl);
         SALLOC(bcnt, NBK + 1);
         SALLOC(bstart, NBK + 1);
         SALLOC(cursor, NBK + 1);
-        SALLOC(items, npl);
+        SALLOC(seen, npl);
+        SALLOC(seen_at, npl);
         SK(cudaMemsetAsync(bcnt, 0, sizeof(int32_t) * (NBK + 1), s->stream));
         SLAUNCH(k_bucket_count, nblk(npl), kT, npl, B, O.x, O.y, pb, bcnt);
         SSCAN(bcnt, NBK + 1, bstart, false, (int32_t*)nullptr);
         SK(cudaMemcpyAsync(cursor, bstart, sizeof(int32_t) * (NBK + 1), cudaMemcpyDeviceToDevice, s->stream));
-        SLAUNCH(k_bucket_fill, nblk(npl), kT, npl, pb, cursor, items);
-        // rounds of proposals
-        int32_t *link, *prop, *nprop, *taken, *forced;
+        SLAUNCH(k_bucket_fill, nblk(npl), kT, npl, pb, cursor, O.x, O.y, rem, seen, seen_at);
+        // rounds of proposals; after round k, n_left[k] attendees without a place
+        int32_t *link, *prop, *nprop, *taken, *open[2], *n_left, *next;
         SALLOC(link, n_att);
         SALLOC(prop, n_att);
         SALLOC(nprop, npl);
         SALLOC(taken, npl);
-        SALLOC(forced, 1);
+        SALLOC(open[0], n_att);
+        SALLOC(open[1], n_att);
+        SALLOC(n_left, 2 * (S.rounds + 1));
+        next = n_left + S.rounds + 1;
         SLAUNCH(k_fill_i32, nblk(n_att), kT, link, (long long)n_att, -1);
         SK(cudaMemsetAsync(nprop, 0, sizeof(int32_t) * npl, s->stream));
         SK(cudaMemsetAsync(taken, 0, sizeof(int32_t) * npl, s->stream));
-        SK(cudaMemsetAsync(forced, 0, sizeof(int32_t), s->stream));
+        SK(cudaMemsetAsync(n_left, 0, sizeof(int32_t) * 2 * (S.rounds + 1), s->stream));
+        SK(tables.done());
+        // six blocks of four warps an SM hold at k_propose's registers
+        const unsigned dealers = std::min(148u * 6, nblk(n_att, 4));
         for (int rd = 0; rd <= S.rounds; rd++) {
             const int free_round = rd == S.rounds;
-            SLAUNCH(k_propose, nblk(n_att, 128), 128, seed, t, rd, free_round, n_att, T.nearest, B, Pd, klk[t],
-                    khr[t], list, s->person_hh, s->hh_x, s->hh_y, O.x, O.y, bstart, items, rem, link, prop);
-            SLAUNCH(k_count_props, nblk(n_att), kT, n_att, prop, nprop);
-            SLAUNCH(k_accept, nblk(n_att), kT, seed, t, rd, free_round, n_att, list, prop, nprop, rem, link, taken,
-                    forced);
-            SLAUNCH(k_take, nblk(npl), kT, npl, rem, taken, nprop);
+            const int32_t* from = rd > 0 ? open[(rd - 1) & 1] : nullptr;
+            const int32_t* n_from = rd > 0 ? n_left + rd - 1 : nullptr;
+            if (rd == 0)
+                SLAUNCH(k_propose_first, nblk(n_att, 128), 128, seed, t, free_round, n_att, T.nearest, B, Pd, klk[t], khr[t],
+                        list, s->person_hh, s->hh_x, s->hh_y, bstart, seen, rem, prop, nprop);
+            else
+                SLAUNCH(k_propose, dealers, 128, seed, t, rd, free_round, T.nearest, B, Pd, klk[t], khr[t], list, s->person_hh,
+                        s->hh_x, s->hh_y, bstart, seen, rem, from, n_from, next + rd, prop, nprop);
+            SLAUNCH(k_accept, nblk(n_att), kT, seed, t, rd, free_round, n_att, from, n_from, list, prop, nprop, rem, link,
+                    taken, open[rd & 1], n_left + rd);
+            SLAUNCH(k_take, nblk(npl), kT, npl, rem, taken, nprop, seen, seen_at);
         }
-        SREAD(forced, &O.forced);
+        int32_t last[2] = {n_att, 0};   // without a place before and after the last round
+        if (S.rounds > 0) SK(cudaMemcpyAsync(last, n_left + S.rounds - 1, sizeof last, cudaMemcpyDeviceToHost, s->stream));
+        else SK(cudaMemcpyAsync(last + 1, n_left, sizeof(int32_t), cudaMemcpyDeviceToHost, s->stream));
+        SK(cudaStreamSynchronize(s->stream));
+        O.forced = last[0] - last[1];
         // members: by (place, random key)
         uint64_t* keys;
         int32_t *vals, *mcount, *ng;
@@ -1143,7 +1440,7 @@ int run_setup(cs_setup* s, const cs_setup_spec& S, const cs_params& P)
         SREAD(tot32 + 3, &O.n_groups);
         SALLOC(O.gstart, O.n_groups);
         SALLOC(O.gsize, O.n_groups);
-        SLAUNCH(k_groups, nblk(npl), kT, npl, mcount, O.member_ofs, ng, O.group_ofs, O.members, O.gstart, O.gsize,
+        SLAUNCH(k_groups, nblk(32LL * npl), kT, npl, mcount, O.member_ofs, ng, O.group_ofs, O.members, O.gstart, O.gsize,
                 s->person_group + (long long)t * N);
     }
     SK(cudaEventRecord(e1, s->stream));
