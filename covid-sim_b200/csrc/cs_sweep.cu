@@ -266,7 +266,7 @@ struct cs_gpu_ctx {
     bool lists_stale = false;   // the last timestep left its touched-cell and household lists for the next scan to empty
     int grid = 148 * 8;
     int nsm = 148;
-    int spatial_lanes = 8;   // lanes per spatial contact (2, 4, 8 or 16)
+    int spatial_lanes = 0;   // lanes per spatial contact (2, 4, 8 or 16; 0: by the load)
     // one timestep captured as a CUDA graph and replayed
     bool use_graph = true;
     cudaGraph_t graph = nullptr;
@@ -1741,13 +1741,13 @@ __global__ void __launch_bounds__(kThreads, 3) k_places_multi(const DevPop* __re
 // Spatial pass (src/Sweep.cpp:656-856).  An infector has a contact in one step in twenty or
 // so.  A warp tests its infectors 32 at a time, u < 1 - lambda ending most of them, queues
 // the others and draws their numbers of contacts in full warps; and it works through those
-// in groups of LANES lanes (2, 4, 8 or 16, a tuning choice that does not change results), a
-// group taking the next contact as soon as it is done with one and the warp testing more
-// infectors before its groups run out.  A contact: pick a target block from the infector's block
+// in groups of kLanes lanes (2, 4, 8 or 16, a tuning choice that does not change results;
+// k_spatial_any), a group taking the next contact as soon as it is done with one and the
+// warp testing more infectors before its groups run out.  A contact: pick a target block from the infector's block
 // row, a slot uniformly among the block's S0 slots, accept with K(d)/bound, redraw on
 // rejection or a dead target.  Draw t of a contact reads its uniforms from Philox blocks 2t
 // and 2t+1 of the contact's stream, so the draws are independent of one another: a group
-// evaluates LANES consecutive draws together and the lowest accepted one wins, exactly as
+// evaluates kLanes consecutive draws together and the lowest accepted one wins, exactly as
 // a sequential loop would.  Bound: a draw's chain of seven dependent gathers.
 constexpr uint32_t kSpatialBlocksPerDraw = 2;
 
@@ -1839,26 +1839,27 @@ struct MaybeQueue {
     int i[64], cell[64];
 };
 
-template <int kSpatialLanes>
-__device__ __forceinline__ void k_spatial_body(const DevPop& d)
+struct SpatialShared {
+    StagedParams sp;
+    ContactQueue queue[kThreads / 32];
+};
+
+template <int kLanes>
+__device__ __forceinline__ void k_spatial_body(const DevPop& d, SpatialShared& sh, int nact)
 {
-    __shared__ StagedParams sp;
-    __shared__ ContactQueue s_queue[kThreads / 32];
+    StagedParams& sp = sh.sp;
     struct Maybes { MaybeQueue q[kThreads / 32]; };
     const cs_params& Pg = *d.P;
-    const int nact = d.counts[kCntAct];
     if (blockIdx.x == 0 && threadIdx.x == 0 && nact) cnt_add(CSB_CTR(work_infectors), nact);
     const StepScalars st = *d.step;
     const Groups work(nact);
     if (work.idle_block() || !(st.sp_beta > 0)) return;
     const cs_params& P = stage_params(sp, d.P);
     const bool anyc = closures_possible(d, st.ts);
-    const int lane = threadIdx.x & 31, sub = lane & ~(kSpatialLanes - 1), sl = lane & (kSpatialLanes - 1);
-    constexpr unsigned kSubMask = (1u << kSpatialLanes) - 1u;
-    unsigned leaders = 0;
-    for (int q = 0; q < 32; q += kSpatialLanes) leaders |= 1u << q;
+    const int lane = threadIdx.x & 31, sub = lane & ~(kLanes - 1), sl = lane & (kLanes - 1);
+    constexpr unsigned kSubMask = (1u << kLanes) - 1u, kLeaders = 0xffffffffu / kSubMask;   // the lowest lane of each group
     long long draws = 0, contacts = 0, oor_count = 0, give_ups = 0;
-    ContactQueue& Q = s_queue[threadIdx.x >> 5];
+    ContactQueue& Q = sh.queue[threadIdx.x >> 5];
     MaybeQueue& M = sp.spare<Maybes>()->q[threadIdx.x >> 5];
     int maybe = 0;   // infectors to be drawn for
     int head = 0, tail = 0, waiting = 0, used = 0;   // queue ends, contacts waiting in it, contacts of the head taken
@@ -1870,7 +1871,7 @@ __device__ __forceinline__ void k_spatial_body(const DevPop& d)
     long long g = work.first();
     for (;;) {
         // ---- infectors' numbers of contacts, until every group has one waiting
-        while ((work.more(g) || maybe) && waiting < 32 / kSpatialLanes && tail - head <= 32) {
+        while ((work.more(g) || maybe) && waiting < 32 / kLanes && tail - head <= 32) {
             if (work.more(g) && maybe < 32) {
                 const int idx = work.item(g);
                 g = work.next(g);
@@ -1933,9 +1934,9 @@ __device__ __forceinline__ void k_spatial_body(const DevPop& d)
             }
         }
         // ---- idle groups take the next contacts, in order
-        const unsigned idle = __ballot_sync(0xffffffffu, !busy) & leaders;
+        const unsigned idle = __ballot_sync(0xffffffffu, !busy) & kLeaders;
         const int nidle = min(__popc(idle), waiting), mine = busy ? -1 : __popc(idle & ((1u << sub) - 1u));
-        if (nidle == 0 && idle == leaders) break;   // nothing waiting, nothing in flight (and no infectors left)
+        if (nidle == 0 && idle == kLeaders) break;   // nothing waiting, nothing in flight (and no infectors left)
         for (int r = 0; r < nidle; r++) {
             const int at = head & (ContactQueue::kCap - 1);
             if (mine == r) {
@@ -1968,14 +1969,14 @@ __device__ __forceinline__ void k_spatial_body(const DevPop& d)
         }
         const unsigned won = (__ballot_sync(0xffffffffu, acc) >> sub) & kSubMask;
         if (busy) {
-            const int w = won ? __ffs(won) - 1 : kSpatialLanes;
+            const int w = won ? __ffs(won) - 1 : kLanes;
             if (sl <= w) oor_count += oor;   // draws up to the winner count, as in a sequential loop
             if (won) {
                 busy = false;
                 if (sl == 0) draws += t0 + w + 1;
                 if (sl == w) spatial_accept(d, P, Pg, st, s, anyc, ii, cc, m, slot, p, hp, d2w);
             } else {
-                t0 += kSpatialLanes;
+                t0 += kLanes;
                 if (t0 >= kMaxSpatialTries) {
                     if (sl == 0) { draws += kMaxSpatialTries; give_ups++; }
                     busy = false;
@@ -1996,10 +1997,25 @@ __device__ __forceinline__ void k_spatial_body(const DevPop& d)
         }
     }
 }
-template <int kSpatialLanes>
-__global__ void __launch_bounds__(kThreads, 3) k_spatial(DevPop d) { k_spatial_body<kSpatialLanes>(d); }
-template <int kSpatialLanes>
-__global__ void __launch_bounds__(kThreads, 3) k_spatial_multi(const DevPop* __restrict__ pops) { k_spatial_body<kSpatialLanes>(pops[blockIdx.y]); }
+// Lanes per contact, unless a number was set.  Eight keep a contact's chain short while
+// there are groups to spare; with more contacts (one in twenty infectors) than the grid has
+// groups of eight, groups of four place more of them at a time.  Measured with 8 and 4:
+// 1,000,000 people alone 39.6 and 40.7 ms, two such side by side 44.3 and 45.5, four 73.5
+// both, eight 108.7 and 108.0, sixteen 188.5 and 182.5; 500,000 infectors of 10,000,000
+// 10.59 and 10.15.
+template <int kLanes>   // 0: by the load
+__device__ __forceinline__ void k_spatial_any(const DevPop& d)
+{
+    __shared__ SpatialShared sh;
+    const int nact = d.counts[kCntAct];
+    if constexpr (kLanes != 0) k_spatial_body<kLanes>(d, sh, nact);
+    else if (nact > 20 * (int)(gridDim.x * (kThreads / 8))) k_spatial_body<4>(d, sh, nact);
+    else k_spatial_body<8>(d, sh, nact);
+}
+template <int kLanes>
+__global__ void __launch_bounds__(kThreads, 3) k_spatial(DevPop d) { k_spatial_any<kLanes>(d); }
+template <int kLanes>
+__global__ void __launch_bounds__(kThreads, 3) k_spatial_multi(const DevPop* __restrict__ pops) { k_spatial_any<kLanes>(pops[blockIdx.y]); }
 
 // More spatial contacts in a step than two per person are an overflow of the step (an
 // infectiousness far outside the model's range); reported with the bounded loops' give-ups.
@@ -3942,8 +3958,9 @@ static int infector_passes(cs_gpu_ctx* c)
     switch (c->spatial_lanes) {
     case 2: LAUNCH(k_spatial<2>, wave_grid(c, kWave3), kThreads, d); break;
     case 4: LAUNCH(k_spatial<4>, wave_grid(c, kWave3), kThreads, d); break;
+    case 8: LAUNCH(k_spatial<8>, wave_grid(c, kWave3), kThreads, d); break;
     case 16: LAUNCH(k_spatial<16>, wave_grid(c, kWave3), kThreads, d); break;
-    default: LAUNCH(k_spatial<8>, wave_grid(c, kWave3), kThreads, d); break;
+    default: LAUNCH(k_spatial<0>, wave_grid(c, kWave3), kThreads, d); break;
     }
     JOIN(2);
     return CS_OK;
@@ -4379,7 +4396,7 @@ struct cs_gpu_batch {
     std::vector<long long> member_launches;
     double* d_t = nullptr;   // the timestep's t, read by every member's k_set_step
     DevPop* d_pops = nullptr; // members' DevPop (t taken from d_t)
-    int lanes = 8;            // spatial lanes of the batched launches
+    int lanes = 0;            // lanes per spatial contact of the batched launches (0: by the load)
     Branches br;              // kernels of a batched timestep that run side by side
     bool fused = false;       // the form of the timestep the graphs were captured with
     // device run loop (cs_gpu_batch_run): members' DevPop with step clocks and
@@ -4523,8 +4540,9 @@ static int batch_enqueue(cs_gpu_batch* b, const DevPop* pops)
     switch (b->lanes) {
     case 2: BLAUNCH(k_spatial_multi<2>, wave(kWave3), kThreads, pops); break;
     case 4: BLAUNCH(k_spatial_multi<4>, wave(kWave3), kThreads, pops); break;
+    case 8: BLAUNCH(k_spatial_multi<8>, wave(kWave3), kThreads, pops); break;
     case 16: BLAUNCH(k_spatial_multi<16>, wave(kWave3), kThreads, pops); break;
-    default: BLAUNCH(k_spatial_multi<8>, wave(kWave3), kThreads, pops); break;
+    default: BLAUNCH(k_spatial_multi<0>, wave(kWave3), kThreads, pops); break;
     }
     BCK(b->br.end(b->stream, 2));
     if (fused) {
