@@ -707,7 +707,7 @@ struct cs_sur {
     cudaEvent_t fork = nullptr;
     std::vector<cudaEvent_t> dz_ready;      // per layer: its dz is written
     double *lpart = nullptr, *lsum = nullptr;   // loss reduction
-    int* d_err = nullptr;                   // set by a tensor-core GEMM whose wait gave up
+    int* d_err = nullptr;                   // set by a tensor-core GEMM whose wait gave up; right behind lsum
     int gemm_impl = 0;                      // 0: tcgen05, 1: mma.sync
     float *xdev = nullptr, *tdev = nullptr, *sq = nullptr;
     struct Predict {                        // the prediction path's workspace (predict_space)
@@ -942,8 +942,8 @@ int cs_sur_create(int max_batch, int device, cs_sur** out)
         }
         if (k == 3) SA(w.part, (size_t)((B * 8 * kT0 + 255) / 256 + 1) * 3000);
     }
-    SA(s->lpart, (size_t)kLossBlocks); SA(s->lsum, (size_t)1); SA(s->d_err, (size_t)1);
-    SCK(cudaMemsetAsync(s->d_err, 0, sizeof(int), s->stream));
+    SA(s->lpart, (size_t)kLossBlocks); SA(s->lsum, (size_t)2);
+    s->d_err = reinterpret_cast<int*>(s->lsum + 1);
     SCK(tc_enable<64>());
     SCK(tc_enable<32>());
     SCK(tc_enable<16>());
@@ -1071,9 +1071,15 @@ static int colsum(cs_sur* s, const Lane& w, const float* dz, int rows, int ld, f
 // The side chains of a step start here: transposed weights for the backward products.
 static int begin_lanes(cs_sur* s)
 {
-    int r;
     SCK(cudaEventRecord(s->fork, s->stream));
     for (int k = 1; k < kLanes; k++) SCK(cudaStreamWaitEvent(s->lane[k].st, s->fork, 0));
+    return CS_OK;
+}
+
+// The transposed weights, beside the forward pass.
+static int transpose_weights(cs_sur* s)
+{
+    int r;
     for (size_t li = 1; li < s->L.size(); li++) {
         const Layer& l = s->L[li];
         if ((r = transpose(s, s->lane[3], s->wb + l.wofs, l.inP, s->wT[li], l.outP, l.outP, l.inP))) return r;
@@ -1140,13 +1146,15 @@ static int backward(cs_sur* s, int Bp)
     return CS_OK;
 }
 
-// Wait for the stream; an error if a tensor-core GEMM's bounded wait gave up.
-static int sync_check(cs_sur* s)
+// Wait for the stream; the loss sum of the last step, and an error if a tensor-core GEMM's bounded
+// wait gave up (one copy of both).
+static int sync_check(cs_sur* s, double* lsum = nullptr)
 {
-    int e = 0;
-    SCK(cudaMemcpyAsync(&e, s->d_err, sizeof(int), cudaMemcpyDeviceToHost, s->stream));
+    struct { double lsum; int err, pad; } st = {};   // as they lie on the device
+    SCK(cudaMemcpyAsync(&st, s->lsum, sizeof st, cudaMemcpyDeviceToHost, s->stream));
     SCK(cudaStreamSynchronize(s->stream));
-    if (e) {
+    if (lsum) *lsum = st.lsum;
+    if (st.err) {
         SCK(cudaMemsetAsync(s->d_err, 0, sizeof(int), s->stream));
         return sur_err(s, CS_E_CUDA, "a tensor-core GEMM gave up waiting for its products");
     }
@@ -1163,6 +1171,7 @@ static int enqueue_step(cs_sur* s, int n, bool update)
     sur::k_load_x<<<(Bp * 64 + 255) / 256, 256, 0, s->stream>>>(s->xdev, n, Bp, s->act[0]);
     SCK(cudaGetLastError());
     if ((r = forward(s, s->lane[0], s->act.data(), Bp, s->yout, nullptr, 0, 0))) return r;
+    if ((r = transpose_weights(s))) return r;
     const size_t nsq = (size_t)n * kTOut * kNOut;
     sur::k_mse<<<1184, 256, 0, s->stream>>>(s->yout, s->tdev, n, Bp, 1.f / ((float)n * kTOut * kNOut), s->dz[8], s->dzb[8], s->sq);
     SCK(cudaGetLastError());
@@ -1250,8 +1259,7 @@ static int run_step(cs_sur* s, const float* x, const float* target, int n, float
     SCK(cudaGraphLaunch(g->exec, s->stream));
     if (loss) {
         double acc = 0.0;
-        SCK(cudaMemcpyAsync(&acc, s->lsum, sizeof(double), cudaMemcpyDeviceToHost, s->stream));
-        if ((r = sync_check(s))) {
+        if ((r = sync_check(s, &acc))) {
             if (update) s->t--;
             return r;
         }
