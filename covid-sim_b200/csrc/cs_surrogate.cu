@@ -475,49 +475,50 @@ __global__ void k_im2col_up(const bf16* __restrict__ H, int Bn, int T, int Cin, 
 }
 
 // The transposed column matrix, colsT[k, m] = cols[m, k] of k_im2col_up, for m < M
-// (= Bn*2T) and k < ldk (columns past kTap*Cin zero), through a 32 x 32 shared tile
-// so that both the reads of H and the writes are coalesced.
-__global__ void k_im2colT_up(const bf16* __restrict__ H, int T, int Cin, bf16* __restrict__ colsT, int M)
+// (= Bn*2T, a multiple of 64) and k < ldk (columns past kTap*Cin zero), through a shared tile
+// of 32 k by 64 m: a thread reads 8 channels of one tap and writes 8 time points of one
+// column, 16 bytes each.  Bound: the matrix' writes (36 MB for 256 rows' last convolution);
+// 2 bytes an access took 66 us for that (with the products beside it), now 22.
+__global__ void __launch_bounds__(256) k_im2colT_up(const bf16* __restrict__ H, int T, int Cin, bf16* __restrict__ colsT, int M)
 {
-    __shared__ bf16 tile[32][34];
-    const int m0 = blockIdx.y * 32, k0 = blockIdx.x * 32;
-    for (int q = threadIdx.y; q < 32; q += blockDim.y) {
-        const int m = m0 + q, k = k0 + threadIdx.x;
-        bf16 v = __float2bfloat16(0.f);
-        const int tap = k / Cin;
+    __shared__ __align__(16) bf16 tile[32][72];   // rows of 144 B: 16-byte reads, neighbouring columns in other banks
+    const int m0 = blockIdx.y * 64, k0 = blockIdx.x * 32;
+    {
+        const int i = threadIdx.x & 63, m = m0 + i, k = k0 + 8 * (threadIdx.x >> 6), tap = k / Cin;
+        union { uint4 q; bf16 h[8]; } u;
+        u.q = make_uint4(0, 0, 0, 0);
         if (tap < kTap) {
-            const int b = m / (2 * T), t = m - b * 2 * T, u = t + tap - kTap / 2;
-            if (u >= 0 && u < 2 * T) v = H[((size_t)b * T + (u >> 1)) * kCh + (k - tap * Cin)];
+            const int b = m / (2 * T), t = m - b * 2 * T, v = t + tap - kTap / 2;
+            if (v >= 0 && v < 2 * T) u.q = *reinterpret_cast<const uint4*>(H + ((size_t)b * T + (v >> 1)) * kCh + (k - tap * Cin));
         }
-        tile[q][threadIdx.x] = v;
+#pragma unroll
+        for (int j = 0; j < 8; j++) tile[k - k0 + j][i] = u.h[j];
     }
     __syncthreads();
-    for (int q = threadIdx.y; q < 32; q += blockDim.y)
-        colsT[(size_t)(k0 + q) * M + m0 + threadIdx.x] = tile[threadIdx.x][q];
+    const int r = threadIdx.x >> 3, c = 8 * (threadIdx.x & 7);
+    *reinterpret_cast<uint4*>(colsT + (size_t)(k0 + r) * M + m0 + c) = *reinterpret_cast<const uint4*>(&tile[r][c]);
 }
 
 // Adjoint of k_im2col_up, fused with the ReLU mask of H: for channel c < Cin,
 // dz[b*T+s, c] = (H > 0) * sum over u in {2s, 2s+1}, k of dcols[b*2T + u-k+2, k*Cin + c];
-// FP32 and BF16 copies; channels >= Cin are zero.
+// FP32 and BF16 copies; channels >= Cin are zero from the start and stay so.
 __global__ void k_col2im_up_relu(const float* __restrict__ dcols, int ldd, int Bn, int T, int Cin,
                                  const bf16* __restrict__ H, float* __restrict__ dz, bf16* __restrict__ dzb)
 {
-    const size_t n = (size_t)Bn * T * kCh;
-    for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < n; e += (size_t)gridDim.x * blockDim.x) {
-        int c = (int)(e % kCh);
-        size_t bs = e / kCh;
+    const size_t n = (size_t)Bn * T * Cin;
+    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
+        const int c = (int)(i % Cin);
+        const size_t bs = i / Cin, e = bs * kCh + c;
         int b = (int)(bs / T), s = (int)(bs % T);
         float acc = 0.f;
-        if (c < Cin) {
-            for (int du = 0; du < 2; du++) {
-                int u = 2 * s + du;
-                for (int k = 0; k < kTap; k++) {
-                    int t = u - k + kTap / 2;
-                    if (t >= 0 && t < 2 * T) acc += dcols[((size_t)b * 2 * T + t) * ldd + k * Cin + c];
-                }
+        for (int du = 0; du < 2; du++) {
+            int u = 2 * s + du;
+            for (int k = 0; k < kTap; k++) {
+                int t = u - k + kTap / 2;
+                if (t >= 0 && t < 2 * T) acc += dcols[((size_t)b * 2 * T + t) * ldd + k * Cin + c];
             }
-            if (!(__bfloat162float(H[e]) > 0.f)) acc = 0.f;
         }
+        if (!(__bfloat162float(H[e]) > 0.f)) acc = 0.f;
         dz[e] = acc;
         dzb[e] = __float2bfloat16(acc);
     }
@@ -542,12 +543,25 @@ __device__ __forceinline__ float lanes_tree(float v, float (*sh)[33])
 }
 __global__ void k_colsum_part(const float* __restrict__ dz, int rows, int ld, float* __restrict__ part)
 {
+    // Bound: the latency of the loads; 16 rows of a thread are on their way at once (and added
+    // one by one, in order).  256 rows' three convolutions, with the products beside them:
+    // 52 + 38 + 33 us four at a time, at most 39 + 20 + 20 now.
+    constexpr int kAhead = 16;
     __shared__ float sh[8][33];
     const int col = blockIdx.x * 32 + threadIdx.x;
     const int r0 = blockIdx.y * kColChunk, r1 = min(rows, r0 + kColChunk);
     float v = 0.f;
-    if (col < ld)
-        for (int r = r0 + threadIdx.y; r < r1; r += 8) v += dz[(size_t)r * ld + col];
+    if (col < ld) {
+        int r = r0 + threadIdx.y;
+        for (; r + 8 * (kAhead - 1) < r1; r += 8 * kAhead) {
+            float x[kAhead];
+#pragma unroll
+            for (int q = 0; q < kAhead; q++) x[q] = dz[(size_t)(r + 8 * q) * ld + col];
+#pragma unroll
+            for (int q = 0; q < kAhead; q++) v += x[q];
+        }
+        for (; r < r1; r += 8) v += dz[(size_t)r * ld + col];
+    }
     v = lanes_tree(v, sh);
     if (threadIdx.y == 0 && col < ld) part[(size_t)blockIdx.y * ld + col] = v;
 }
@@ -563,24 +577,38 @@ __global__ void k_colsum_final(const float* __restrict__ part, int nchunks, int 
 }
 
 // Loss terms and the output gradient (FP32 and BF16): y is [B*368, 64] (channels < 4 used), target
-// [n, 365, 4]; rows of samples >= n and time points >= 365 get zero gradient.
+// [n, 365, 4]; rows of samples >= n and time points >= 365 get zero gradient.  A thread per
+// row, its four channels in one access; the gradients' other channels are zero from the
+// start and stay so.  (All 64 written: 21 us for 256 rows, now 7.)
 __global__ void k_mse(const float* __restrict__ y, const float* __restrict__ target, int n, int Bp, float scale,
                       float* __restrict__ dy, bf16* __restrict__ dyb, float* __restrict__ sq)
 {
+    static_assert(kNOut == 4, "a row's outputs are one 16-byte access");
     const int T = 2 * 2 * 2 * kT0;   // 368
-    const size_t total = (size_t)Bp * T * kCh;
-    for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < total; e += (size_t)gridDim.x * blockDim.x) {
-        int c = (int)(e % kCh);
-        size_t bt = e / kCh;
-        int b = (int)(bt / T), t = (int)(bt % T);
-        float g = 0.f;
-        if (c < kNOut && t < kTOut && b < n) {
-            float d = y[e] - target[((size_t)b * kTOut + t) * kNOut + c];
-            g = 2.f * d * scale;
-            sq[((size_t)b * kTOut + t) * kNOut + c] = d * d;
+    const size_t total = (size_t)Bp * T;
+    for (size_t bt = blockIdx.x * (size_t)blockDim.x + threadIdx.x; bt < total; bt += (size_t)gridDim.x * blockDim.x) {
+        const int b = (int)(bt / T), t = (int)(bt % T);
+        union F4 { float4 q; float f[4]; };
+        F4 g;
+        g.q = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (t < kTOut && b < n) {
+            const size_t at = ((size_t)b * kTOut + t) * kNOut;
+            F4 yv, tv, s2;
+            yv.q = *reinterpret_cast<const float4*>(y + bt * kCh);
+            tv.q = *reinterpret_cast<const float4*>(target + at);
+#pragma unroll
+            for (int c = 0; c < kNOut; c++) {
+                const float d = yv.f[c] - tv.f[c];
+                g.f[c] = 2.f * d * scale;
+                s2.f[c] = d * d;
+            }
+            *reinterpret_cast<float4*>(sq + at) = s2.q;
         }
-        dy[e] = g;
-        dyb[e] = __float2bfloat16(g);
+        *reinterpret_cast<float4*>(dy + bt * kCh) = g.q;
+        union { uint2 q; bf16 h[4]; } gb;
+#pragma unroll
+        for (int c = 0; c < kNOut; c++) gb.h[c] = __float2bfloat16(g.f[c]);
+        *reinterpret_cast<uint2*>(dyb + bt * kCh) = gb.q;
     }
 }
 
@@ -1058,12 +1086,13 @@ static int forward(cs_sur* s, const Lane& w, bf16* const* act, int Bp, float* y6
     return CS_OK;
 }
 
-static int colsum(cs_sur* s, const Lane& w, const float* dz, int rows, int ld, float* out)
+// Sums of the first `cols` columns (the others are padding: zero, as are their sums from the start).
+static int colsum(cs_sur* s, const Lane& w, const float* dz, int rows, int ld, int cols, float* out)
 {
     const int nch = (rows + kColChunk - 1) / kColChunk;
     const dim3 blk(32, 8);
-    sur::k_colsum_part<<<dim3((ld + 31) / 32, nch), blk, 0, w.st>>>(dz, rows, ld, w.part);
-    sur::k_colsum_final<<<(ld + 31) / 32, blk, 0, w.st>>>(w.part, nch, ld, out);
+    sur::k_colsum_part<<<dim3((cols + 31) / 32, nch), blk, 0, w.st>>>(dz, rows, ld, w.part);
+    sur::k_colsum_final<<<(cols + 31) / 32, blk, 0, w.st>>>(w.part, nch, ld, out);
     SCK(cudaGetLastError());
     return CS_OK;
 }
@@ -1101,13 +1130,12 @@ static int weight_grad(cs_sur* s, int li, int rows, int Tin)
     // dW = dz^T in: A = dz^T [outP, rows], B = in^T [inP, rows]
     if ((r = transpose(s, w, s->dzb[li], ld, w.dzT, rows, rows, l.outP))) return r;
     if (l.conv) {   // the transposed column matrix of the convolution's input, from the input itself
-        dim3 grid(l.inP / 32, rows / 32), blk(32, 8);
-        sur::k_im2colT_up<<<grid, blk, 0, w.st>>>(s->act[li], Tin, l.cin, w.colsT, rows);
+        sur::k_im2colT_up<<<dim3(l.inP / 32, rows / 64), 256, 0, w.st>>>(s->act[li], Tin, l.cin, w.colsT, rows);
         SCK(cudaGetLastError());
     } else if ((r = transpose(s, w, s->act[li], l.inP, w.colsT, rows, rows, l.inP)))
         return r;
     if ((r = gemm(s, w, w.dzT, rows, w.colsT, rows, s->g + l.wofs, l.inP, nullptr, 0, nullptr, 0, l.outP, l.inP, rows))) return r;
-    return colsum(s, s->lane[3], s->dz[li], rows, ld, s->g + l.bofs);
+    return colsum(s, s->lane[3], s->dz[li], rows, ld, l.out, s->g + l.bofs);
 }
 
 // Backward pass from dy (in the last layer's dz, FP32 and BF16) to gradients in s->g; the
