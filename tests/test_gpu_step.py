@@ -73,3 +73,30 @@ def test_step_matches_single_sweeps_and_oracle(n_people, cells, latent, infectio
         assert cs[0][k] == cs[2][k], k
     for s in (whole, single, orac):
         s.close()
+
+
+@pytest.mark.parametrize("n_people,cells,n_seed", [(2001, 4, 40), (40000, 30, 16000)])
+def test_lanes_per_contact_by_the_load(n_people, cells, n_seed):
+    """A grid of eight blocks has 256 groups of eight lanes, so that more than 5,120 infectors
+    take groups of four: the states are those of every number that can be set."""
+    pop, P, lk, hr = _world(n_people, cells, 0.3, None)
+    sims = {lanes: sim.Simulation(pop, P, lk, hr) for lanes in (0, 2, 4, 8, 16)}
+    seeds = sims[0].choose_seeds(9, n_seed)
+    for lanes, s in sims.items():
+        s.backend.set_grid(8 if lanes == 0 else 592)
+        if lanes:
+            s.backend.set_spatial_lanes(lanes)
+        s.backend.begin_run(9, seeds)
+    most, before = 0, 0
+    for k in range(16):
+        for s in sims.values():
+            s.backend.step(k * P.ModelTimeStep, 0)
+        now = int(sims[0].backend.counters().work_infectors)
+        most, before = max(most, now - before), now
+    assert (most > 5120) == (n_people == 40000)
+    want = snapshot(sims[8].backend, pop)
+    for lanes, s in sims.items():
+        _same(snapshot(s.backend, pop), want, "%d lanes" % lanes)
+        assert abi.counters_to_dict(s.backend.counters()) == abi.counters_to_dict(sims[8].backend.counters())
+    for s in sims.values():
+        s.close()
