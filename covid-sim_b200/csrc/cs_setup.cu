@@ -8,8 +8,9 @@
 // integer counts, so the result is a function of the spec alone.
 //
 // Work is one thread per microcell, person, household or place (a warp per person who
-// is still without a place, and per place for its groups); the passes that need an order (people per cell, households per microcell, places' member lists)
-// take it from exclusive scans and one stable radix sort, written below.
+// is still without a place, and per place for its groups); the passes that need an
+// order (people per cell, households per microcell, places' member lists) take it from
+// exclusive scans and one stable radix sort, written below.
 #include <algorithm>
 #include <cmath>
 #include <cstdint>
@@ -951,7 +952,7 @@ struct cs_setup {
     std::string err;
     std::vector<void*> allocs;
     char* slab = nullptr;                      // what is left of the newest slab (dalloc)
-    size_t slab_left = 0, slab_total = 0;
+    size_t slab_left = 0, slab_total = 0, slab_first = 0;
     int32_t N = 0, NH = 0, NC = 0, NM = 0, n_adunits = 1, npt = 0;
     double device_ms = 0;
     int32_t *person_hh = nullptr, *person_mcell = nullptr, *person_place = nullptr, *hh_first = nullptr,
@@ -988,15 +989,17 @@ int fail(cs_setup* s, int code, const char* fmt, ...)
         if (e_ != cudaSuccess) return fail(s, CS_E_CUDA, "%s: %s", #kern, cudaGetErrorString(e_)); \
     } while (0)
 
-// Device memory comes in slabs, each as large as all before it (32 MB at least), and is
-// given back with the set-up: its some 200 arrays, allocated and freed one by one, took
-// some 20 of the 44 ms that a set-up of 1,000,000 people lasted.
+// Device memory comes in slabs and is given back with the set-up: its some 200 arrays,
+// allocated and freed one by one, took some 20 of the 44 ms that a set-up of 1,000,000
+// people lasted.  The first slab is about what the set-up needs (run_setup), a further one
+// half of all before it (32 MB at least).  With five slabs, of 32 MB and doubling, and one
+// thread for the tables the same set-up took 19.6 ms, now 16.3.
 template <typename T>
 int dalloc(cs_setup* s, T** p, long long n)
 {
     const size_t bytes = ((size_t)std::max(n, 1LL) * sizeof(T) + 255) / 256 * 256;
     if (bytes > s->slab_left) {
-        size_t take = std::max(bytes, std::max(s->slab_total, (size_t)32 << 20));
+        size_t take = std::max(bytes, std::max(s->slab_total ? s->slab_total / 2 : s->slab_first, (size_t)32 << 20));
         void* q = nullptr;
         cudaError_t e = cudaMalloc(&q, take);
         if (e != cudaSuccess && take > bytes) {   // no room for a slab: the array alone
@@ -1087,45 +1090,49 @@ int radix_sort(cs_setup* s, uint64_t* keys, int32_t* vals, long long n, int bits
     return CS_OK;
 }
 
-// Copies of host arrays to the device by a thread of their own, so that the copy through the
-// driver's staging buffers (5.5 ms for two tables of 2,000,000 entries) does not hold up the
-// launches.  done() waits for them; so does leaving the set-up on an error.
+// Copies of host arrays to the device by threads of their own, one each, so that the copies
+// through the driver's staging buffers (5.5 ms one after the other for four tables of
+// 2,000,000 entries) do not hold up the launches.  done() waits for them; so does leaving
+// the set-up on an error.
 struct TableCopies {
-    struct Item { void* dst; const void* src; size_t bytes; };
+    struct Item { void* dst; const void* src; size_t bytes; cudaError_t err; std::thread th; };
     Item items[2 * CS_MAX_PLACE_TYPES];
     int n = 0, device;
-    cudaError_t err = cudaSuccess;
-    std::thread th;
 
     explicit TableCopies(int dev) : device(dev) {}
     ~TableCopies() { done(); }
-    void add(void* dst, const void* src, size_t bytes) { items[n++] = {dst, src, bytes}; }
-    void copy()
+    static void copy(Item& it, int device)
     {
         cudaStream_t st = nullptr;
-        err = cudaSetDevice(device);
-        if (err == cudaSuccess) err = cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking);
-        for (int k = 0; k < n && err == cudaSuccess; k++)
-            err = cudaMemcpyAsync(items[k].dst, items[k].src, items[k].bytes, cudaMemcpyHostToDevice, st);
+        it.err = cudaSetDevice(device);
+        if (it.err == cudaSuccess) it.err = cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking);
+        if (it.err == cudaSuccess) it.err = cudaMemcpyAsync(it.dst, it.src, it.bytes, cudaMemcpyHostToDevice, st);
         if (st) {
             const cudaError_t e = cudaStreamSynchronize(st);
-            if (err == cudaSuccess) err = e;
+            if (it.err == cudaSuccess) it.err = e;
             cudaStreamDestroy(st);
         }
     }
-    void start()
+    void start(void* dst, const void* src, size_t bytes)
     {
-        if (n == 0) return;
+        Item& it = items[n++];
+        it.dst = dst;
+        it.src = src;
+        it.bytes = bytes;
         try {
-            th = std::thread([this] { copy(); });
+            it.th = std::thread(copy, std::ref(it), device);
         } catch (...) {
-            copy();   // no thread to be had
+            copy(it, device);   // no thread to be had
         }
     }
     cudaError_t done()
     {
-        if (th.joinable()) th.join();
-        return err;
+        cudaError_t e = cudaSuccess;
+        for (int k = 0; k < n; k++) {
+            if (items[k].th.joinable()) items[k].th.join();
+            if (e == cudaSuccess) e = items[k].err;
+        }
+        return e;
     }
 };
 
@@ -1182,6 +1189,9 @@ int run_setup(cs_setup* s, const cs_setup_spec& S, const cs_params& P)
     s->npt = S.num_place_types;
     s->n_adunits = S.adunit_grid > 0 ? S.adunit_grid * S.adunit_grid : 1;
 
+    // microcells' weights, prefix sums and counts; people's arrays, attendees' lists and
+    // sorts; two kernel tables twice; and room for what is per cell, household and place
+    s->slab_first = (size_t)(S.n_blobs > 0 ? 28 : 20) * M + (size_t)100 * N + 4 * sizeof(double) * (size_t)P.kernel_size + ((size_t)16 << 20);
     cs_params* Pd;
     SALLOC(Pd, 1);
     SK(cudaMemcpyAsync(Pd, &P, sizeof(cs_params), cudaMemcpyHostToDevice, s->stream));
@@ -1202,12 +1212,11 @@ int run_setup(cs_setup* s, const cs_setup_spec& S, const cs_params& P)
         double *a, *b;
         SALLOC(a, ktab);
         SALLOC(b, ktab);
-        tables.add(a, S.pt[t].kernel_lookup, sizeof(double) * ktab);
-        tables.add(b, S.pt[t].kernel_hi_res, sizeof(double) * ktab);
+        tables.start(a, S.pt[t].kernel_lookup, sizeof(double) * ktab);
+        tables.start(b, S.pt[t].kernel_hi_res, sizeof(double) * ktab);
         klk[t] = a;
         khr[t] = b;
     }
-    tables.start();
     unsigned long long* err;
     SALLOC(err, 1);
     SK(cudaMemsetAsync(err, 0, sizeof(unsigned long long), s->stream));
