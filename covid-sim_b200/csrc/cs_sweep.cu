@@ -32,6 +32,7 @@
 #include <cooperative_groups/reduce.h>
 
 #include <algorithm>
+#include <climits>
 #include <cmath>
 #include <cstdarg>
 #include <cstdio>
@@ -807,20 +808,30 @@ static TotPairGeom tot_pair_geom(int ncw, int nch, bool partial)
     g.nchunks = (nch + kTotProbRowChunk - 1) / kTotProbRowChunk;
     g.chunks_per_block = partial ? 1 : g.nchunks;
     g.need = (ncw + kTotProbCols - 1) / kTotProbCols;
-    // Row pairs per block: the count that leaves the fewest lanes idle in a multiple of
-    // 128 threads.  Four warps are the unit because a block's warps go round the SM's four
-    // schedulers: at 600 columns two pairs (150 threads, five warps) gave one scheduler
-    // two warps of every block and the others one, and ran at 53 % of the FP32 pipe.
+    // Row pairs per block: the count with the fewest threads on the busiest SM.  A block's
+    // threads are a multiple of 128: a block's warps go round the SM's four schedulers, and at
+    // 600 columns two pairs (150 threads, five warps) gave one scheduler two warps of every
+    // block and the others one, and ran at 53 % of the FP32 pipe.  Measured over 13 grids from
+    // 20 x 20 to 600 x 600, the time is about columns x (0.2 us + 0.37 us per 128 threads on an
+    // SM).  Fewest idle lanes alone, the same choice from about 300 x 300 cells on, left small
+    // grids a few large blocks: 160 x 200 cells 267 us in 42 blocks, now 103; 100 x 80 cells
+    // 166 in 6, now 57; 20 x 20 cells 45 in one, now 19.
     g.npair = 1;
     g.threads = 256;
-    double best = 0.0;
+    int best = INT_MAX;
+    double best_blocks = 0.0;
     for (int k = 1; k * g.need <= kTotPairThreads && 2 * (k - 1) < nch; k++) {
         const int t = (k * g.need + 127) / 128 * 128;
-        const double used = (double)(k * g.need) / (double)t;
         TotPairGeom h = g;
         h.npair = k;
-        if (used > best + 0.02 && (k == 1 || h.smem() <= kMaxBlockSmem)) {
-            best = used;
+        if (k > 1 && h.smem() > kMaxBlockSmem) break;
+        // blocks with a whole chunk of rows (a last, shorter chunk counts as its part)
+        const double blocks = (nch + 2 * k - 1) / (2 * k) * (partial ? (double)nch / kTotProbRowChunk : 1.0);
+        const int load = std::max(1, (int)ceil(blocks / 148 - 0.05)) * t;
+        // alike: few large blocks where there are more than SMs, else many small ones
+        if (load < best || (load == best && best_blocks > 148)) {
+            best = load;
+            best_blocks = blocks;
             g.npair = k;
             g.threads = t;
         }
