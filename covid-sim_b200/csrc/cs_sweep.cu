@@ -3731,13 +3731,15 @@ static int tot_prob_smem(cs_gpu_ctx* c, bool denominators, size_t smem)
 
 // Numerators on the packed pipe, unless a grid is so wide that its interleaved kernel
 // rows do not fit shared memory twice (about 4,400 columns); k_tot_prob_rows needs a quarter.
-static bool tot_prob_packed(const cs_params& P) { return tot_pair_geom(P.ncw, P.nch, true).smem() <= kMaxBlockSmem; }
+static bool tot_prob_packed(const cs_params& P, bool partial) { return tot_pair_geom(P.ncw, P.nch, partial).smem() <= kMaxBlockSmem; }
 
-static int tot_prob_prepare(cs_gpu_ctx* c)
+// partial: the form that is launched, as the row pairs a block has (and with them its shared
+// memory) differ between the two.
+static int tot_prob_prepare(cs_gpu_ctx* c, bool partial)
 {
     const cs_params& P = c->hp;
-    if (!tot_prob_packed(P)) return tot_prob_smem(c, false, tot_prob_geom(P.ncw, P.nch, true).smem(false));
-    const size_t smem = tot_pair_geom(P.ncw, P.nch, true).smem();
+    if (!tot_prob_packed(P, partial)) return tot_prob_smem(c, false, tot_prob_geom(P.ncw, P.nch, partial).smem(false));
+    const size_t smem = tot_pair_geom(P.ncw, P.nch, partial).smem();
     if (smem <= 48 * 1024 || smem <= c->tp_pair_smem) return CS_OK;
     CK(cudaFuncSetAttribute(k_tot_prob_pairs, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     c->tp_pair_smem = smem;
@@ -3749,10 +3751,10 @@ static int tot_prob_prepare(cs_gpu_ctx* c)
 static int tot_prob_numerators(cs_gpu_ctx* c, const float* S0g, const uint8_t* rowS, float* out, bool partial)
 {
     const cs_params& P = c->hp;
-    int r = tot_prob_prepare(c);
+    int r = tot_prob_prepare(c, partial);
     if (r) return r;
     if (c->prof) prof_begin(c, partial ? "k_tot_prob_rows" : "k_tot_prob_rows_static");
-    if (tot_prob_packed(P)) {
+    if (tot_prob_packed(P, partial)) {
         const TotPairGeom gm = tot_pair_geom(P.ncw, P.nch, partial);
         const dim3 grid(gm.xblocks, (P.nch + 2 * gm.npair - 1) / (2 * gm.npair), gm.nchunks / gm.chunks_per_block);
         k_tot_prob_pairs<<<grid, gm.threads, gm.smem(), c->stream>>>(c->d, S0g, rowS, out, gm, c->Gtab);
@@ -4252,7 +4254,7 @@ static int enqueue_day(cs_gpu_ctx* c, int spd, bool every_step, bool parts)
 
 static int capture_day(cs_gpu_ctx* c, int spd, bool every_step)
 {
-    int r = tot_prob_prepare(c);
+    int r = tot_prob_prepare(c, true);
     if (r) return r;
     cudaGraph_t g = nullptr;
     CK(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
@@ -4753,7 +4755,7 @@ static int batch_capture_day(cs_gpu_batch* b, int spd, bool every_step)
         }
     }
     for (cs_gpu_ctx* m : b->members)
-        if (int r = tot_prob_prepare(m)) return batch_err(b, r, "%s", m->err);
+        if (int r = tot_prob_prepare(m, true)) return batch_err(b, r, "%s", m->err);
     b->member_day_launches.assign(n, 0);
     // the members' own launches (their UpdateProbs chains) read the clock and gate too
     for (cs_gpu_ctx* m : b->members) {

@@ -1,0 +1,49 @@
+"""UpdateProbs over the shapes of grid that choose its launch: the fixed-scratch form
+against the allocating one where it takes more row pairs a block (and so more shared memory)
+than that does.  All sums have one order, so every value must be equal (tolerance: none)."""
+import numpy as np
+import pytest
+
+from covidsim_b200 import population, params as prm, sim
+from tests.helpers import snapshot, STATE_FIELDS
+
+pytestmark = pytest.mark.gpu
+
+
+def _world(ncw, nch, n_people=3000):
+    grid = population.make_grid(nmcl=1)
+    cell = min(1.0 / 120, 2.0 / max(ncw, nch))
+    grid.update(ncw=ncw, nch=nch, cell_width=cell, cell_height=cell)
+    pop = population.generate(n_people, grid, sigma=1.5, seed=3 + ncw)
+    P, lk, hr = prm.build_params(grid, kernel_size=200000)
+    P.LocalBeta = 0.9
+    return pop, P, lk, hr
+
+
+def _started(world, steps=12):
+    """A Simulation `steps` timesteps into an epidemic."""
+    s = sim.Simulation(*world)
+    s.backend.begin_run(3, s.choose_seeds(3, 200))
+    for k in range(steps):
+        s.backend.step(k * world[1].ModelTimeStep)
+    return s
+
+
+def _same(a, b, where):
+    for k in STATE_FIELDS:
+        assert np.array_equal(a[k], b[k]), "%s: %s differs at %d entries" % (where, k, int(np.sum(a[k] != b[k])))
+
+
+@pytest.mark.parametrize("ncw,nch", [(769, 311), (456, 648), (792, 632)])
+def test_static_form_where_it_needs_more_shared_memory(ncw, nch):
+    """One, two and one row pairs a block in the allocating form, two, three and three in the
+    fixed-scratch one.  A small grid is brought up to date first, so that what an earlier call
+    of this process enabled is not what the static call lives on."""
+    small = _started(_world(200, 160), 0)
+    small.backend.update_probs(0)
+    ref, var = (_started(_world(ncw, nch)) for _ in range(2))
+    var.backend.update_probs_static(0)
+    ref.backend.update_probs(0)
+    _same(snapshot(var.backend, var.pop), snapshot(ref.backend, ref.pop), "%d x %d" % (ncw, nch))
+    for s in (small, ref, var):
+        s.close()
