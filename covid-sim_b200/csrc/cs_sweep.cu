@@ -282,8 +282,6 @@ struct cs_gpu_ctx {
     int series_cap = 0;
     int day_every_step = -1;    // the probs_every_step the day graph was captured with
     long long geometry_gen = 0; // bumped when set_params replaces the kernel-row table
-    size_t tp_pair_smem = 0;    // dynamic shared memory enabled for k_tot_prob_pairs
-    size_t tp_smem[2] = {0, 0}; // dynamic shared memory enabled for k_tot_prob_rows<false>, <true>
     // staging of cs_gpu_place_events / cs_gpu_set_mcell_status
     cs_place_event* d_ev = nullptr;
     int ev_cap = 0;
@@ -439,6 +437,7 @@ extern "C" {
 static int tot_prob_pass(cs_gpu_ctx* c, bool denominators);
 static int build_kernel_rows(cs_gpu_ctx* c);
 static int build_block_bounds(cs_gpu_ctx* c);
+static int enable_shared_memory(cs_gpu_ctx* c);
 }
 
 // ================================================================ run start
@@ -3539,6 +3538,8 @@ int cs_gpu_create(const cs_population* pop, const cs_params* params, int device,
     // ---- dynamic state of this realisation
     r = alloc_dynamic(c);
     if (r) return r;
+    r = enable_shared_memory(c);
+    if (r) return r;
     r = build_block_bounds(c);
     if (r) return r;
     r = build_kernel_rows(c);
@@ -3658,8 +3659,6 @@ int cs_gpu_set_params(cs_gpu_ctx* c, const cs_params* params)
 static int build_block_bounds(cs_gpu_ctx* c)
 {
     DevPop& d = c->d;
-    if (2 * (size_t)d.NB > (48u << 10))   // k_block_guides' marks
-        CK(cudaFuncSetAttribute(k_block_guides, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 * 32767));
     if (!d.bounds_static) return CS_OK;
     unsigned long long* oor = nullptr;
     CK(cudaMalloc(&oor, sizeof(unsigned long long)));
@@ -3717,32 +3716,20 @@ __global__ void k_zero_gated(float* p, size_t n, unsigned char* q, size_t m, con
     for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < m; e += (size_t)gridDim.x * blockDim.x) q[e] = 0;
 }
 
-// The dynamic shared memory the row kernel needs, raised above the default before
-// its first launch (and so never inside a graph capture that follows one).
-static int tot_prob_smem(cs_gpu_ctx* c, bool denominators, size_t smem)
-{
-    size_t& have = c->tp_smem[denominators ? 1 : 0];
-    if (smem <= 48 * 1024 || smem <= have) return CS_OK;
-    if (denominators) CK(cudaFuncSetAttribute(k_tot_prob_rows<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    else CK(cudaFuncSetAttribute(k_tot_prob_rows<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    have = smem;
-    return CS_OK;
-}
-
 // Numerators on the packed pipe, unless a grid is so wide that its interleaved kernel
 // rows do not fit shared memory twice (about 4,400 columns); k_tot_prob_rows needs a quarter.
 static bool tot_prob_packed(const cs_params& P, bool partial) { return tot_pair_geom(P.ncw, P.nch, partial).smem() <= kMaxBlockSmem; }
 
-// partial: the form that is launched, as the row pairs a block has (and with them its shared
-// memory) differ between the two.
-static int tot_prob_prepare(cs_gpu_ctx* c, bool partial)
+// Dynamic shared memory above the default for the kernels that may need it, in time for
+// their first launch (and never inside a capture).  The limit belongs to the kernel on its
+// device, not to a context, and each call sets it anew, downwards too: so it is always set
+// to the same value, the most a block can have.
+static int enable_shared_memory(cs_gpu_ctx* c)
 {
-    const cs_params& P = c->hp;
-    if (!tot_prob_packed(P, partial)) return tot_prob_smem(c, false, tot_prob_geom(P.ncw, P.nch, partial).smem(false));
-    const size_t smem = tot_pair_geom(P.ncw, P.nch, partial).smem();
-    if (smem <= 48 * 1024 || smem <= c->tp_pair_smem) return CS_OK;
-    CK(cudaFuncSetAttribute(k_tot_prob_pairs, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    c->tp_pair_smem = smem;
+    CK(cudaFuncSetAttribute(k_tot_prob_pairs, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxBlockSmem));
+    CK(cudaFuncSetAttribute(k_tot_prob_rows<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxBlockSmem));
+    CK(cudaFuncSetAttribute(k_tot_prob_rows<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxBlockSmem));
+    CK(cudaFuncSetAttribute(k_block_guides, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 * 32767));   // its marks
     return CS_OK;
 }
 
@@ -3751,8 +3738,6 @@ static int tot_prob_prepare(cs_gpu_ctx* c, bool partial)
 static int tot_prob_numerators(cs_gpu_ctx* c, const float* S0g, const uint8_t* rowS, float* out, bool partial)
 {
     const cs_params& P = c->hp;
-    int r = tot_prob_prepare(c, partial);
-    if (r) return r;
     if (c->prof) prof_begin(c, partial ? "k_tot_prob_rows" : "k_tot_prob_rows_static");
     if (tot_prob_packed(P, partial)) {
         const TotPairGeom gm = tot_pair_geom(P.ncw, P.nch, partial);
@@ -3798,7 +3783,6 @@ static int tot_prob_pass(cs_gpu_ctx* c, bool denominators)
         int tpb;
         tot_prob_launch_shape(P.ncw, P.nch, gm, &grid, &tpb);
         const size_t smem = gm.smem(true);
-        if ((r = tot_prob_smem(c, true, smem))) return r;
         if (c->prof) prof_begin(c, "k_tot_prob_rows");
         k_tot_prob_rows<true><<<grid, tpb, smem, c->stream>>>(d, c->S0g, c->Ng, c->rowS, c->rowN, c->Apart, c->Bpart, gm, c->Gtab);
         if (c->prof) prof_end(c);
@@ -4254,12 +4238,10 @@ static int enqueue_day(cs_gpu_ctx* c, int spd, bool every_step, bool parts)
 
 static int capture_day(cs_gpu_ctx* c, int spd, bool every_step)
 {
-    int r = tot_prob_prepare(c, true);
-    if (r) return r;
     cudaGraph_t g = nullptr;
     CK(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
     long long l0 = c->launches;
-    r = enqueue_day(c, spd, every_step, !c->capturing_prof);
+    int r = enqueue_day(c, spd, every_step, !c->capturing_prof);
     cudaError_t e = cudaStreamEndCapture(c->stream, &g);
     if (r || e != cudaSuccess) {
         if (g) cudaGraphDestroy(g);
@@ -4754,8 +4736,6 @@ static int batch_capture_day(cs_gpu_batch* b, int spd, bool every_step)
             BCK(cudaEventCreateWithFlags(&b->ev_join[i], cudaEventDisableTiming));
         }
     }
-    for (cs_gpu_ctx* m : b->members)
-        if (int r = tot_prob_prepare(m, true)) return batch_err(b, r, "%s", m->err);
     b->member_day_launches.assign(n, 0);
     // the members' own launches (their UpdateProbs chains) read the clock and gate too
     for (cs_gpu_ctx* m : b->members) {

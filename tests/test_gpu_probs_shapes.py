@@ -1,6 +1,7 @@
 """UpdateProbs over the shapes of grid that choose its launch: the fixed-scratch form
 against the allocating one where it takes more row pairs a block (and so more shared memory)
-than that does.  All sums have one order, so every value must be equal (tolerance: none)."""
+than that does, and contexts of different grids in one process, in turn.  All sums
+have one order, so every value must be equal (tolerance: none)."""
 import numpy as np
 import pytest
 
@@ -46,4 +47,28 @@ def test_static_form_where_it_needs_more_shared_memory(ncw, nch):
     ref.backend.update_probs(0)
     _same(snapshot(var.backend, var.pop), snapshot(ref.backend, ref.pop), "%d x %d" % (ncw, nch))
     for s in (small, ref, var):
+        s.close()
+
+
+@pytest.mark.parametrize("large,small", [((600, 600), (240, 240)), ((340, 260), (240, 240)), ((6000, 4), (5000, 4))])
+def test_contexts_of_other_grids_take_turns(large, small):
+    """More than 48 KB of shared memory a block each, the larger grid before, between and
+    after calls of the smaller one: by direct calls, in a day graph captured after them, and
+    from a replica made after them (above about 4,400 columns the unpacked kernel)."""
+    a, b = _started(_world(*large)), _started(_world(*small))
+    a.backend.update_probs(0)
+    first = snapshot(a.backend, a.pop)
+    for _ in range(2):
+        b.backend.update_probs(0)
+        a.backend.update_probs(0)
+        _same(snapshot(a.backend, a.pop), first, "in turn")
+    want, _ = a.run(5, 3, n_seed=100, probs_every_step=True, blocks=True)
+    b.run(5, 3, n_seed=100, probs_every_step=True)
+    a.backend.set_params(a.params)          # drops the day graph
+    again, _ = a.run(5, 3, n_seed=100, probs_every_step=True, blocks=True)
+    r = a.replica()
+    other, _ = r.run(5, 3, n_seed=100, probs_every_step=True, blocks=True)
+    for k in want:
+        assert np.array_equal(want[k], again[k]) and np.array_equal(want[k], other[k]), k
+    for s in (a, b, r):
         s.close()
