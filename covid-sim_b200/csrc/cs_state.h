@@ -214,9 +214,11 @@ struct DevPop {
 // the incub sweep's household pass.  The step's transition events are two lists in
 // `events`: latent people from the front (kCntEvents), infectious people from the
 // back (kCntEventsInf), so that a warp of the transition kernel mostly takes one
-// branch.
+// branch.  kCntDone is no list's: 1 when the touched-cell and household lists are those of
+// a whole timestep that has worked them off, for the next one to empty (a household list
+// without it still waits for its pass).
 enum { kCntQueue = 0, kCntTouched = 1, kCntAct = 2, kCntContacts = 3, kCntEvents = 4,
-       kCntCarer = 5, kCntFalse = 6, kCntEventsInf = 7, kCntHH = 8, kCntN = 9 };
+       kCntCarer = 5, kCntFalse = 6, kCntEventsInf = 7, kCntDone = 8, kCntHH = 9, kCntN = 10 };
 enum { kAnySocdist = 0, kAnyMoverest = 1 };
 
 }  // namespace csb

@@ -1212,7 +1212,8 @@ __device__ __forceinline__ double step_time(const DevPop& d, const cs_params& P,
 __device__ __forceinline__ int step_number(const cs_params& P, double t) { return (int)(uint16_t)(P.TimeStepsPerDay * t); }
 
 // The step's scalars from the parameters, on the device (src/Sweep.cpp:292-301);
-// empty_lists: also the lists that the timestep before left for this one to empty.
+// empty_lists: also the lists that a timestep before left for this one to empty (not the
+// households that an infection sweep alone left to the next transitions).
 __device__ __forceinline__ void k_set_step_body(const DevPop& d, double t, unsigned long long seed, int empty_lists)
 {
     const cs_params& P = *d.P;
@@ -1228,7 +1229,7 @@ __device__ __forceinline__ void k_set_step_body(const DevPop& d, double t, unsig
     st.hh_beta = P.DoHouseholds ? st.seas * st.fp * P.HouseholdTrans : 0.0;
     st.seed = seed;
     *d.step = st;
-    if (empty_lists) d.counts[kCntTouched] = d.counts[kCntHH] = 0;
+    if (empty_lists && d.counts[kCntDone]) d.counts[kCntTouched] = d.counts[kCntHH] = 0;
 }
 __global__ void k_set_step(DevPop d, double t, unsigned long long seed, int empty_lists) { k_set_step_body(d, t, seed, empty_lists); }
 __global__ void k_set_step_multi(const DevPop* __restrict__ pops, int empty_lists) { k_set_step_body(pops[blockIdx.x], 0.0, 0ull, empty_lists); }
@@ -2761,7 +2762,8 @@ __device__ __forceinline__ void k_moves_body(const DevPop& d)
     const int n = partition_touched<kS, true>(d);
     if (kS) {
         if ((threadIdx.x & 31) == 0 && n) cnt_add(CSB_CTR(work_cells_touched), n);
-        if (blockIdx.x == 0 && threadIdx.x < kCntN && threadIdx.x != kCntTouched && threadIdx.x != kCntHH) d.counts[threadIdx.x] = 0;
+        if (blockIdx.x == 0 && threadIdx.x < kCntN && threadIdx.x != kCntTouched && threadIdx.x != kCntHH)
+            d.counts[threadIdx.x] = threadIdx.x == kCntDone ? 1 : 0;
     }
     if (d.step_clock && blockIdx.x == 0 && threadIdx.x == 0) *d.step_clock += 1;
 }

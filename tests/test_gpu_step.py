@@ -100,3 +100,44 @@ def test_lanes_per_contact_by_the_load(n_people, cells, n_seed):
         assert abi.counters_to_dict(s.backend.counters()) == abi.counters_to_dict(sims[8].backend.counters())
     for s in sims.values():
         s.close()
+
+
+@pytest.mark.parametrize("device_loop", [False, True])
+def test_households_left_by_an_infect_sweep_alone(device_loop):
+    """The false cases of an infection sweep leave flagged households to the next transitions,
+    also when those are a whole timestep's or the device run loop's, with false positives off."""
+    pop, P, lk, hr = _world(6000, 4, None, None)
+    whole, single = sim.Simulation(pop, P, lk, hr), sim.Simulation(pop, P, lk, hr)
+    orac = sim.Simulation(pop, P, lk, hr, backend=oracle_py.OracleBackend)
+    sims, dt = (whole, single, orac), P.ModelTimeStep
+    on, off = abi.cs_params.from_buffer_copy(P), abi.cs_params.from_buffer_copy(P)
+    on.FalsePositiveRate = 0.5
+    iv = abi.cs_interventions()
+    iv.CaseIsolationPolicyDuration = iv.HQuarantinePolicyDuration = 1000.0
+    seeds = whole.choose_seeds(5, 100)   # few enough that the day's end recomputes no probabilities
+    for s in sims:
+        s.backend.begin_run(5, seeds)
+        s.backend.set_interventions(iv)
+        for k in range(12):
+            s.backend.step(k * dt, 0)
+        s.backend.set_params(on)
+        s.backend.infect_sweep(12 * dt, 0)
+        s.backend.set_params(off)
+    before = snapshot(orac.backend, pop)
+    steps = int(P.TimeStepsPerDay) if device_loop else 3
+    for s in sims:
+        if s is whole and device_loop:
+            s.backend.run_device(1, sim.run_policy(None, pop.num_place_types))
+            continue
+        for k in range(0 if device_loop else 13, steps if device_loop else 16):
+            if s is whole:
+                s.backend.step(k * dt, 0)
+            else:
+                s.backend.infect_sweep(k * dt, 0)
+                s.backend.incub_recovery_sweep(k * dt)
+    want = snapshot(orac.backend, pop)
+    assert not np.array_equal(before["quar_start_time"], want["quar_start_time"])
+    _same(snapshot(single.backend, pop), want, "sweeps")
+    _same(snapshot(whole.backend, pop), want, "whole timesteps")
+    for s in sims:
+        s.close()
