@@ -32,6 +32,7 @@
 #include <cooperative_groups/reduce.h>
 
 #include <algorithm>
+#include <array>
 #include <climits>
 #include <cmath>
 #include <cstdarg>
@@ -291,6 +292,7 @@ struct cs_gpu_ctx {
     cudaGraph_t day_graph = nullptr;
     cudaGraphExec_t day_exec = nullptr;
     long long day_launches = 0;
+    long long part_launches[2] = {0, 0};   // of a conditional part within a day and at a day's end
     // optional per-launch timing with events on the context's stream
     bool prof = false;
     struct Rec { const char* name; cudaEvent_t a, b; };
@@ -2820,6 +2822,10 @@ struct DayCtl {
     // k_day_check's sums of S, L, I, R, D and its finished blocks; zero between launches
     unsigned long long totals[5];
     int32_t blocks_done;
+    int32_t need;               // the rare work (UpdateProbs, the switch's flags and closures) has something to do
+    // times a conditional part of the graph ran, within a day and at days' ends, and the step
+    // of the last one (a batch's first member counts for all)
+    int32_t part_step, parts[2];
 };
 
 // ------------------------------------------------------------ place closure
@@ -3171,9 +3177,9 @@ __device__ void k_day_logic_body(const DevPop& d, DayCtl* ctl, const int32_t* cl
 // the counters, the UpdateProbs test, and at a day's end the day's logic, as one launch:
 // every block adds its cells' sums, and the last one to finish goes on with the rest.  The
 // rare work decided here (UpdateProbs; the switch's flags and closures) is in a conditional
-// part of the day graph, which `part` switches on; without one (a graph with timing nodes,
-// eager launches) it is launched every time and returns at its gates.
-__device__ __forceinline__ void k_day_check_body(const DevPop& d, DayCtl* ctl, int day_end, cudaGraphConditionalHandle part)
+// part of the day graph, which `part` switches on; a graph with timing nodes launches it every
+// time and it returns at its gates; without a graph the host asks (`need`).
+__device__ __forceinline__ void k_day_check_body(const DevPop& d, DayCtl* ctl, DayCtl* first, int day_end, cudaGraphConditionalHandle part)
 {
     __shared__ int s_last;
     long long v[5] = {0, 0, 0, 0, 0};
@@ -3199,12 +3205,19 @@ __device__ __forceinline__ void k_day_check_body(const DevPop& d, DayCtl* ctl, i
     if (threadIdx.x == 0) probs_check(d, ctl, day_end);
     if (day_end) k_day_logic_body(d, ctl, d.step_clock, const_cast<DevIv*>(d.iv));
     __syncthreads();
-    if (threadIdx.x == 0 && part && (ctl->update || (day_end && (ctl->socd_write || ctl->close)))) cudaGraphSetConditional(part, 1);
+    if (threadIdx.x == 0) {
+        ctl->need = ctl->update || (day_end && (ctl->socd_write || ctl->close));
+        if (part && ctl->need) {
+            cudaGraphSetConditional(part, 1);
+            const int step = *d.step_clock;   // the same for every member of a batch
+            if (atomicExch(&first->part_step, step) != step) atomicAdd(first->parts + day_end, 1);
+        }
+    }
 }
-__global__ void __launch_bounds__(kThreads) k_day_check(DevPop d, DayCtl* ctl, int day_end, cudaGraphConditionalHandle part) { k_day_check_body(d, ctl, day_end, part); }
+__global__ void __launch_bounds__(kThreads) k_day_check(DevPop d, DayCtl* ctl, int day_end, cudaGraphConditionalHandle part) { k_day_check_body(d, ctl, ctl, day_end, part); }
 __global__ void __launch_bounds__(kThreads) k_day_check_multi(const DevPop* __restrict__ pops, DayCtl* const* ctls, int day_end, cudaGraphConditionalHandle part)
 {
-    k_day_check_body(pops[blockIdx.y], ctls[blockIdx.y], day_end, part);
+    k_day_check_body(pops[blockIdx.y], ctls[blockIdx.y], ctls[0], day_end, part);
 }
 
 __device__ __forceinline__ void k_socdist_fill_body(const DevPop& d, const DayCtl* ctl)
@@ -4203,11 +4216,15 @@ static int enqueue_change(cs_gpu_ctx* c)
 // same launches serve every day and can be captured once.  Order as the host loop:
 // the timesteps; after each (or the day's last) the counters and the UpdateProbs
 // test; at the day's end the series and the trigger, then UpdateProbs, and the switch's
-// social-distancing flags and closures.  parts: these into a conditional part of the graph
-// being captured, else gated.  (On all but a few days the 18 launches returned at their
-// gates, about 2 us each; the part's node takes 5 to 10 us when it does not run.  Tested
-// after every timestep, 1.5 M people with admin units: 68.5 -> 63 ms.)
-static int enqueue_day(cs_gpu_ctx* c, int spd, bool every_step, bool parts)
+// social-distancing flags and closures, which are wanted on few days (on the others their 18
+// launches returned at their gates, about 2 us each; the part's node takes 5 to 10 us when it
+// does not run.  Tested after every timestep, 1.5 M people with admin units: 68.5 -> 63 ms.)
+enum class Rare {
+    kPart,    // into a conditional part of the graph being captured
+    kGated,   // launched, behind their gates (a graph with timing nodes)
+    kAsked,   // launched when the host has read that they are wanted (no graph)
+};
+static int enqueue_day(cs_gpu_ctx* c, int spd, bool every_step, Rare rare)
 {
     DevPop& d = c->d;
     const int cgrid = std::max(1, std::min(64, (d.NC + kThreads - 1) / kThreads));
@@ -4217,19 +4234,26 @@ static int enqueue_day(cs_gpu_ctx* c, int spd, bool every_step, bool parts)
         const bool day_end = s == spd - 1;
         if (!every_step && !day_end) continue;
         cudaGraphConditionalHandle part = 0;
-        if (parts) CK(cond_handle(c->stream, &part));
+        if (rare == Rare::kPart) CK(cond_handle(c->stream, &part));
         LAUNCH(k_day_check, cgrid, kThreads, d, c->d_ctl, day_end ? 1 : 0, part);
+        if (rare == Rare::kAsked) {
+            int32_t need = 0;
+            CK(cudaMemcpyAsync(&need, &c->d_ctl->need, sizeof(need), cudaMemcpyDeviceToHost, c->stream));
+            CK(cudaStreamSynchronize(c->stream));
+            if (!need) continue;
+        }
         const cudaStream_t main = c->stream;
         const long long l0 = c->launches;
-        if (parts) {
+        if (rare == Rare::kPart) {
             CK(cond_begin(main, c->br.body, part));
             c->stream = c->br.body;
         }
         r = cs_gpu_update_probs(c, 0);
         if (!r && day_end) r = enqueue_change(c);
-        c->launches = l0;   // neither form counts what does its work on few days
         c->stream = main;
-        if (parts) {
+        if (rare == Rare::kPart) {
+            c->part_launches[day_end] = c->launches - l0;   // counted when the part has run (cs_gpu_run)
+            c->launches = l0;
             cudaError_t e = cond_end(c->br.body);
             if (!r && e != cudaSuccess) r = set_err(c, CS_E_CUDA, "conditional part of the day graph: %s", cudaGetErrorString(e));
         }
@@ -4243,7 +4267,7 @@ static int capture_day(cs_gpu_ctx* c, int spd, bool every_step)
     cudaGraph_t g = nullptr;
     CK(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
     long long l0 = c->launches;
-    int r = enqueue_day(c, spd, every_step, !c->capturing_prof);
+    int r = enqueue_day(c, spd, every_step, c->capturing_prof ? Rare::kGated : Rare::kPart);
     cudaError_t e = cudaStreamEndCapture(c->stream, &g);
     if (r || e != cudaSuccess) {
         if (g) cudaGraphDestroy(g);
@@ -4284,7 +4308,7 @@ static int run_days(cs_gpu_ctx* c, int days, int spd, bool every_step)
             c->launches += c->day_launches;
             if (c->day_graph_prof) prof_graph_collect(c);
         } else {
-            int r = enqueue_day(c, spd, every_step, false);
+            int r = enqueue_day(c, spd, every_step, Rare::kAsked);
             if (r) return r;
         }
     }
@@ -4366,7 +4390,10 @@ int cs_gpu_run(cs_gpu_ctx* c, int days, const cs_run_policy* policy, cs_counters
     cs_counters last;
     r = day_series_out(c, days, daily, &last);
     if (r) return r;
+    int32_t parts[2] = {0, 0};   // conditional parts that ran (none in the other forms)
+    CK(cudaMemcpyAsync(parts, c->d_ctl->parts, sizeof(parts), cudaMemcpyDeviceToHost, c->stream));
     CK(cudaStreamSynchronize(c->stream));
+    for (int k = 0; k < 2; k++) c->launches += parts[k] * c->part_launches[k];
     return check_give_ups(c, last);
 }
 
@@ -4380,8 +4407,8 @@ __global__ void k_zero_counts_multi(const DevPop* __restrict__ pops, int n)
 // A batch steps many realisations (contexts, each with its own population or a
 // replica sharing one) with one CUDA graph per timestep.  Each of the step's
 // kernels is launched once for all members: blockIdx.y selects the member, whose
-// DevPop the kernel reads from a device array, so a timestep is the same 11
-// kernels and 2 counter resets whatever the number of members.  While the batch
+// DevPop the kernel reads from a device array, so a timestep is the same ten kernels
+// (with false positives fifteen, two of them counter resets) whatever the number of members.  While the batch
 // exists every member's work goes to the batch's stream, which keeps a member's
 // own calls (UpdateProbs, interventions, counters) ordered with the batched steps.
 struct cs_gpu_batch {
@@ -4390,7 +4417,8 @@ struct cs_gpu_batch {
     cudaStream_t stream = nullptr;
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
-    std::vector<long long> member_launches;
+    long long launched = 0;      // kernels of the batched launches, each for every member
+    long long step_launches = 0; // of one timestep's graph
     double* d_t = nullptr;   // the timestep's t, read by every member's k_set_step
     DevPop* d_pops = nullptr; // members' DevPop (t taken from d_t)
     int lanes = 0;            // lanes per spatial contact of the batched launches (0: by the load)
@@ -4405,7 +4433,9 @@ struct cs_gpu_batch {
     int day_every_step = -1;
     int day_spd = 0;
     std::vector<long long> day_geometry;       // members' geometry_gen when the day graph was captured
-    std::vector<long long> member_day_launches;
+    long long day_launches = 0;                // kernels of the day graph, each for every member
+    // a conditional part's kernels for each member, within a day and at a day's end
+    std::vector<std::array<long long, 2>> part_launches;
     static constexpr int kSide = 8;            // streams the members' UpdateProbs chains fan out to
     cudaStream_t side[kSide] = {};
     cudaEvent_t ev_fork = nullptr, ev_join[kSide] = {};
@@ -4459,7 +4489,6 @@ int cs_gpu_batch_create(cs_gpu_ctx* const* members, int n, cs_gpu_batch** out)
     BCK(cudaMalloc(&b->d_t, sizeof(double)));
     BCK(cudaMalloc(&b->d_pops, sizeof(DevPop) * n));
     b->members.assign(members, members + n);
-    b->member_launches.assign(n, 0);
     for (int k = 0; k < n; k++) {
         cs_gpu_ctx* m = b->members[k];
         BCK(cudaStreamSynchronize(m->stream));
@@ -4474,6 +4503,7 @@ const char* cs_gpu_batch_last_error(const cs_gpu_batch* b) { return b ? b->err :
 #define BLAUNCH(kernel, grid, block, ...)                                                          \
     do {                                                                                           \
         kernel<<<(grid), (block), 0, b->stream>>>(__VA_ARGS__);                                    \
+        b->launched++;                                                                             \
         cudaError_t e_ = cudaGetLastError();                                                       \
         if (e_ != cudaSuccess) return batch_err(b, CS_E_CUDA, "launch %s: %s", #kernel, cudaGetErrorString(e_)); \
     } while (0)
@@ -4481,6 +4511,7 @@ const char* cs_gpu_batch_last_error(const cs_gpu_batch* b) { return b ? b->err :
 #define BLAUNCH_ON(i, kernel, grid, block, ...)                                                    \
     do {                                                                                           \
         kernel<<<(grid), (block), 0, b->br.s[i]>>>(__VA_ARGS__);                                   \
+        b->launched++;                                                                             \
         cudaError_t e_ = cudaGetLastError();                                                       \
         if (e_ != cudaSuccess) return batch_err(b, CS_E_CUDA, "launch %s: %s", #kernel, cudaGetErrorString(e_)); \
     } while (0)
@@ -4492,8 +4523,6 @@ static bool batch_fused(const cs_gpu_batch* b)
         if (!fused_step(m)) return false;
     return true;
 }
-
-static long long batch_kernels(const cs_gpu_batch* b) { return batch_fused(b) ? 10 : 12; }
 
 // Members' list counters before a batched timestep or run, as cs_gpu_step and cs_gpu_run
 // treat a lone context's.
@@ -4590,6 +4619,7 @@ static int batch_capture(cs_gpu_batch* b, double t, int run)
     BCK(cudaMemcpyAsync(b->d_pops, hp.data(), sizeof(DevPop) * n, cudaMemcpyHostToDevice, b->stream));
     BCK(cudaStreamSynchronize(b->stream));
     BCK(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
+    const long long l0 = b->launched;
     int r = batch_enqueue(b, b->d_pops);
     cudaGraph_t g = nullptr;
     cudaError_t e = cudaStreamEndCapture(b->stream, &g);
@@ -4600,7 +4630,7 @@ static int batch_capture(cs_gpu_batch* b, double t, int run)
     }
     BCK(cudaGraphInstantiate(&b->exec, g, 0));
     b->graph = g;
-    for (int k = 0; k < n; k++) b->member_launches[k] = batch_kernels(b);   // kernels run for each member per step
+    b->step_launches = b->launched - l0;
     return CS_OK;
 }
 
@@ -4617,7 +4647,7 @@ int cs_gpu_batch_step(cs_gpu_batch* b, double t, int run)
     // every member's k_scan reads t (and its run's seed) from device memory
     BCK(cudaMemcpyAsync(b->d_t, &t, sizeof(double), cudaMemcpyHostToDevice, b->stream));
     BCK(cudaGraphLaunch(b->exec, b->stream));
-    for (size_t k = 0; k < b->members.size(); k++) b->members[k]->launches += b->member_launches[k];
+    for (cs_gpu_ctx* m : b->members) m->launches += b->step_launches;
     return CS_OK;
 }
 
@@ -4664,7 +4694,7 @@ int cs_gpu_batch_sync(cs_gpu_batch* b)
 // the member), and, in a conditional part of the graph, each member's gated UpdateProbs
 // chain on one of kSide side streams, forked from and joined back into the part's stream,
 // so that the chains overlap.
-static int batch_updates(cs_gpu_batch* b, cudaStream_t main)
+static int batch_updates(cs_gpu_batch* b, cudaStream_t main, int day_end)
 {
     BCK(cudaEventRecord(b->ev_fork, main));
     for (int i = 0; i < cs_gpu_batch::kSide; i++) BCK(cudaStreamWaitEvent(b->side[i], b->ev_fork, 0));
@@ -4674,6 +4704,7 @@ static int batch_updates(cs_gpu_batch* b, cudaStream_t main)
         m->stream = b->side[k % cs_gpu_batch::kSide];
         const long long l0 = m->launches;
         r = cs_gpu_update_probs(m, 0);
+        b->part_launches[k][day_end] = m->launches - l0;
         m->launches = l0;
         m->stream = b->stream;
         if (r) batch_err(b, r, "member %zu UpdateProbs: %s", k, m->err);
@@ -4701,16 +4732,14 @@ static int batch_enqueue_day(cs_gpu_batch* b, int spd, bool every_step)
     for (int s = 0; s < spd; s++) {
         int r = batch_enqueue(b, pops);
         if (r) return r;
-        for (int k = 0; k < R; k++) b->member_day_launches[k] += batch_kernels(b);
         const bool day_end = s == spd - 1;
         if (!every_step && !day_end) continue;
         cudaGraphConditionalHandle part;
         BCK(cond_handle(b->stream, &part));
         BLAUNCH(k_day_check_multi, dim3(cgrid, R), kThreads, pops, b->d_ctls, day_end ? 1 : 0, part);
-        for (int k = 0; k < R; k++) b->member_day_launches[k]++;
         const cudaStream_t body = b->br.body;
         BCK(cond_begin(b->stream, body, part));
-        r = batch_updates(b, body);
+        r = batch_updates(b, body, day_end ? 1 : 0);
         if (!r && day_end) {
             const dim3 g(std::min(b->members[0]->grid, std::max(64, (6 * b->members[0]->nsm + R - 1) / R)), R);
             k_socdist_fill_multi<<<g, kThreads, 0, body>>>(pops, b->d_ctls);
@@ -4719,6 +4748,7 @@ static int batch_enqueue_day(cs_gpu_batch* b, int spd, bool every_step)
                 k_carer_pass_multi<<<g, kThreads, 0, body>>>(pops);
                 k_carer_reset_multi<<<R, 1, 0, body>>>(pops);
             }
+            for (auto& n : b->part_launches) n[1] += 1 + npt + (npt > 0 ? 2 : 0);
         }
         const cudaError_t el = cudaGetLastError(), e = cond_end(body);
         if (r) return r;
@@ -4738,7 +4768,8 @@ static int batch_capture_day(cs_gpu_batch* b, int spd, bool every_step)
             BCK(cudaEventCreateWithFlags(&b->ev_join[i], cudaEventDisableTiming));
         }
     }
-    b->member_day_launches.assign(n, 0);
+    b->part_launches.assign(n, {0, 0});
+    const long long l0 = b->launched;
     // the members' own launches (their UpdateProbs chains) read the clock and gate too
     for (cs_gpu_ctx* m : b->members) {
         m->d.step_clock = m->d_clock;
@@ -4764,6 +4795,7 @@ static int batch_capture_day(cs_gpu_batch* b, int spd, bool every_step)
         return batch_err(b, CS_E_CUDA, "batch day graph instantiate: %s", cudaGetErrorString(ei));
     }
     b->day_graph = g;
+    b->day_launches = b->launched - l0;
     b->day_every_step = every_step ? 1 : 0;
     b->day_spd = spd;
     b->day_geometry.resize(n);
@@ -4820,12 +4852,15 @@ int cs_gpu_batch_run(cs_gpu_batch* b, int days, const cs_run_policy* policies, c
         if (int r = batch_capture_day(b, spd, every)) return r;
     }
     for (int d = 0; d < days; d++) BCK(cudaGraphLaunch(b->day_exec, b->stream));
-    for (int k = 0; k < n; k++) b->members[k]->launches += b->member_day_launches[k] * days;
     std::vector<cs_counters> last(n);
     for (int k = 0; k < n; k++)
         if (int r = day_series_out(b->members[k], days, daily ? daily + (size_t)k * days : nullptr, &last[k]))
             return batch_err(b, r, "member %d: %s", k, b->members[k]->err);
+    int32_t parts[2];   // conditional parts that ran
+    BCK(cudaMemcpyAsync(parts, b->members[0]->d_ctl->parts, sizeof(parts), cudaMemcpyDeviceToHost, b->stream));
     BCK(cudaStreamSynchronize(b->stream));
+    for (int k = 0; k < n; k++)
+        b->members[k]->launches += b->day_launches * days + parts[0] * b->part_launches[k][0] + parts[1] * b->part_launches[k][1];
     for (int k = 0; k < n; k++)
         if (int r = check_give_ups(b->members[k], last[k])) return batch_err(b, r, "member %d: %s", k, b->members[k]->err);
     return CS_OK;

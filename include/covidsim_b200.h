@@ -658,7 +658,8 @@ void cs_host_free(void* p);
 int cs_gpu_sync(cs_gpu_ctx* ctx);
 /* The CUDA stream the context launches on (a cudaStream_t), for host-side timing. */
 void* cs_gpu_stream(cs_gpu_ctx* ctx);
-/* Number of kernels launched on the context since creation. */
+/* Number of kernels launched on the context since creation (a batch's launches, which
+ * serve all members, count for each of them). */
 int64_t cs_gpu_launch_count(const cs_gpu_ctx* ctx);
 /*
  * Per-kernel device time: with enable = 1 every launch is bracketed by CUDA events
