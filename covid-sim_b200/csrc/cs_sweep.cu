@@ -402,14 +402,16 @@ static int set_err(cs_gpu_ctx* c, int code, const char* fmt, ...)
         if (e_ != cudaSuccess) return set_err(c, CS_E_CUDA, "%s: %s", #call, cudaGetErrorString(e_)); \
     } while (0)
 
-#define LAUNCH(kernel, grid, block, ...)                                                           \
+#define LAUNCH(kernel, grid, block, ...) LAUNCH_AS(#kernel, kernel, grid, block, __VA_ARGS__)
+// the name is what cs_gpu_profile_entry calls the kernel
+#define LAUNCH_AS(name, kernel, grid, block, ...)                                                  \
     do {                                                                                           \
-        if (c->prof) prof_begin(c, #kernel);                                                       \
+        if (c->prof) prof_begin(c, name);                                                          \
         kernel<<<(grid), (block), 0, c->stream>>>(__VA_ARGS__);                                    \
         if (c->prof) prof_end(c);                                                                  \
         c->launches++;                                                                             \
         cudaError_t e_ = cudaGetLastError();                                                       \
-        if (e_ != cudaSuccess) return set_err(c, CS_E_CUDA, "launch %s: %s", #kernel, cudaGetErrorString(e_)); \
+        if (e_ != cudaSuccess) return set_err(c, CS_E_CUDA, "launch %s: %s", name, cudaGetErrorString(e_)); \
     } while (0)
 
 template <typename T>
@@ -3954,7 +3956,7 @@ static int begin_step(cs_gpu_ctx* c, double t, bool empty_lists)
     DevPop& d = c->d;
     FORK(1);
     LAUNCH_ON(0, k_set_step, 1, 1, d, t, (unsigned long long)c->seed, empty_lists ? 1 : 0);
-    LAUNCH((k_scan<kActive, kEvents>), scan_grid(d.NC, c->grid), kThreads, d, t);
+    LAUNCH_AS("k_scan", (k_scan<kActive, kEvents>), scan_grid(d.NC, c->grid), kThreads, d, t);
     JOIN(1);
     return CS_OK;
 }

@@ -1,7 +1,10 @@
-"""The count of kernels launched (cs_gpu_launch_count) against the kernels that the profiler
-sees: direct calls, timesteps as graphs, the run loop as day graphs (with parts that run on
-few days), without graphs and with timing nodes, and a batch of one."""
+"""The count of kernels launched (cs_gpu_launch_count), and the names that per-launch timing
+gives them, against the kernels that the profiler sees: direct calls, timesteps as graphs, the
+run loop as day graphs (with parts that run on few days), without graphs and with timing
+nodes, and a batch of one."""
+import os
 import re
+import sys
 
 import pytest
 
@@ -48,6 +51,10 @@ def test_launch_count_of_a_run(form, every_step, fpr):
     run()   # graphs captured
     counted, seen = _counted(s, run)
     assert counted == seen > 40 * 4 * 9
+    names = set(s.backend.profile_entries()) if form == "timed" else set()
+    assert all(re.fullmatch(r"k_\w+(<\w+(, ?\w+)*>)?", n) for n in names), names
+    if names:
+        assert {"k_scan", "k_moves", "k_household", "k_day_check"} <= {n.split("<")[0] for n in names}
     s.close()
 
 
@@ -85,4 +92,18 @@ def test_launch_count_of_timesteps_sweeps_and_a_batch(fpr):
     counted, seen = _counted(s, run)
     assert counted == seen
     batch.close()
+    s.close()
+
+
+def test_timed_kernels_have_their_bytes_in_the_benchmark():
+    sys.path.insert(0, os.path.dirname(os.path.dirname(os.path.abspath(__file__))))
+    import bench
+    pop, P, lk, hr = tiny_world()
+    s = sim.Simulation(pop, P, lk, hr)
+    s.backend.profile(1)
+    s.run(5, 20, n_seed=200)
+    w = abi.counters_to_dict(s.backend.counters())
+    names = {n.split("<")[0] for n in s.backend.profile_entries()}
+    for k in ("k_scan", "k_household", "k_places", "k_spatial", "k_infections", "k_onsets", "k_progress", "k_moves"):
+        assert k in names and bench.kernel_bytes(k, w, pop.n_cells * 80) > 0, k
     s.close()
