@@ -755,8 +755,12 @@ struct cs_sur {
         cudaGraphExec_t exec = nullptr;
         cudaGraphNode_t adam = nullptr;
         cudaKernelNodeParams adam_params{};
+        long long used = 0;                 // the step that used it last
     };
-    std::vector<StepGraph> graphs;          // the most recent batch sizes
+    std::vector<StepGraph> graphs;          // kMaxGraphs batch sizes at most
+    struct Missed { int n; bool update; long long at; };
+    std::vector<Missed> missed;             // sizes that ran without a graph, and the last step that did
+    long long steps = 0;
     std::vector<void*> allocs;
 };
 
@@ -803,6 +807,7 @@ static void drop_graphs(cs_sur* s)
         if (g.graph) cudaGraphDestroy(g.graph);
     }
     s->graphs.clear();
+    s->missed.clear();
 }
 
 static void build_layers(cs_sur* s)
@@ -1189,9 +1194,14 @@ static int sync_check(cs_sur* s, double* lsum = nullptr)
     return CS_OK;
 }
 
+// What the weights' update takes from the step it belongs to.
+struct AdamStep {
+    float lr = 0.f, b1 = 0.9f, b2 = 0.999f, eps = 1e-8f, c1 = 1.f, c2 = 1.f, wd = 0.f;
+};
+
 // The kernels of one step on n rows whose inputs and targets are in xdev and tdev: loss
 // terms summed into lsum, gradients in g and, with `update`, the weights' update.
-static int enqueue_step(cs_sur* s, int n, bool update)
+static int enqueue_step(cs_sur* s, int n, bool update, const AdamStep& a)
 {
     int r;
     const int Bp = up64(n);
@@ -1210,30 +1220,56 @@ static int enqueue_step(cs_sur* s, int n, bool update)
     SCK(cudaGetLastError());
     if ((r = backward(s, Bp))) return r;
     if (update) {
-        sur::k_adam<<<1184, 256, 0, s->stream>>>(s->w, s->m, s->v, s->g, s->wb, s->np, 0.f, 0.f, 0.f, 0.f, 1.f, 1.f, 0.f, s->d_err);
+        sur::k_adam<<<1184, 256, 0, s->stream>>>(s->w, s->m, s->v, s->g, s->wb, s->np, a.lr, a.b1, a.b2, a.eps, a.c1,
+                                                  a.c2, a.wd, s->d_err);
         SCK(cudaGetLastError());
     }
     return CS_OK;
 }
 
-// The step's graph for n rows, captured on first use.  A step is about 90 launches, most of
-// a few microseconds, in four chains; replayed as one graph the chains overlap and the
-// launches leave no gaps (0.93 ms a step of 64 rows when launched one after the other, half
-// of it gaps and transposes that nothing had to wait for).
-constexpr size_t kMaxGraphs = 8;   // batch sizes kept (a training run uses one or two)
+// The step's graph for n rows, captured on first use, or null: the step then runs as its
+// launches.  A step is about 90 launches, most of a few microseconds, in four chains;
+// replayed as one graph the chains overlap and the launches leave no gaps (0.93 ms a step of
+// 64 rows when launched one after the other, half of it gaps and transposes that nothing had
+// to wait for).  Capturing one takes longer than the launches it saves once, so when all
+// places are taken a size gets that of the graph unused for longest only if it has itself
+// come twice since that was used.  (Twelve sizes in turn, each ninth capture dropping
+// the others: 14.7 ms for twelve steps, 11.4 in a single chain, now 4.7.)
+constexpr size_t kMaxGraphs = 8;    // batch sizes kept (a training run uses one or two)
+constexpr size_t kMaxMissed = 64;   // sizes without one that are remembered
 static int step_graph(cs_sur* s, int n, bool update, cs_sur::StepGraph** out)
 {
+    *out = nullptr;
+    const long long now = ++s->steps;
     for (auto& g : s->graphs)
-        if (g.n == n && g.update == update) { *out = &g; return CS_OK; }
+        if (g.n == n && g.update == update) {
+            g.used = now;
+            *out = &g;
+            return CS_OK;
+        }
     if (s->graphs.size() >= kMaxGraphs) {
+        auto oldest = std::min_element(s->graphs.begin(), s->graphs.end(),
+                                       [](const cs_sur::StepGraph& a, const cs_sur::StepGraph& b) { return a.used < b.used; });
+        auto m = std::find_if(s->missed.begin(), s->missed.end(),
+                              [&](const cs_sur::Missed& x) { return x.n == n && x.update == update; });
+        if (m == s->missed.end() || m->at < oldest->used) {
+            if (m != s->missed.end()) s->missed.erase(m);
+            else if (s->missed.size() >= kMaxMissed) s->missed.erase(s->missed.begin());
+            s->missed.push_back({n, update, now});
+            return CS_OK;
+        }
+        s->missed.erase(m);
         SCK(cudaStreamSynchronize(s->stream));
-        drop_graphs(s);
+        cudaGraphExecDestroy(oldest->exec);
+        cudaGraphDestroy(oldest->graph);
+        s->graphs.erase(oldest);
     }
     cs_sur::StepGraph g;
     g.n = n;
     g.update = update;
+    g.used = now;
     SCK(cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal));
-    int r = enqueue_step(s, n, update);
+    int r = enqueue_step(s, n, update, AdamStep());
     cudaError_t e = cudaStreamEndCapture(s->stream, &g.graph);
     if (r || e != cudaSuccess) {
         if (g.graph) cudaGraphDestroy(g.graph);
@@ -1274,17 +1310,26 @@ static int run_step(cs_sur* s, const float* x, const float* target, int n, float
     if (r) return r;
     SCK(cudaMemcpyAsync(s->xdev, x, sizeof(float) * n * kIn, cudaMemcpyHostToDevice, s->stream));
     SCK(cudaMemcpyAsync(s->tdev, target, sizeof(float) * n * kTOut * kNOut, cudaMemcpyHostToDevice, s->stream));
+    AdamStep a;
     if (update) {
         s->t++;
-        float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
-        float c1 = 1.f - powf(b1, (float)s->t), c2 = 1.f - powf(b2, (float)s->t);
-        void* args[] = {&s->w, &s->m, &s->v, &s->g, &s->wb, &s->np, &lr, &b1, &b2, &eps, &c1, &c2, &wd, &s->d_err};
-        cudaKernelNodeParams kp = g->adam_params;
-        kp.kernelParams = args;
-        kp.extra = nullptr;
-        SCK(cudaGraphExecKernelNodeSetParams(g->exec, g->adam, &kp));
+        a.lr = lr;
+        a.wd = wd;
+        a.c1 = 1.f - powf(a.b1, (float)s->t);
+        a.c2 = 1.f - powf(a.b2, (float)s->t);
     }
-    SCK(cudaGraphLaunch(g->exec, s->stream));
+    if (!g) {
+        if ((r = enqueue_step(s, n, update, a))) return r;
+    } else {
+        if (update) {
+            void* args[] = {&s->w, &s->m, &s->v, &s->g, &s->wb, &s->np, &a.lr, &a.b1, &a.b2, &a.eps, &a.c1, &a.c2, &a.wd, &s->d_err};
+            cudaKernelNodeParams kp = g->adam_params;
+            kp.kernelParams = args;
+            kp.extra = nullptr;
+            SCK(cudaGraphExecKernelNodeSetParams(g->exec, g->adam, &kp));
+        }
+        SCK(cudaGraphLaunch(g->exec, s->stream));
+    }
     if (loss) {
         double acc = 0.0;
         if ((r = sync_check(s, &acc))) {

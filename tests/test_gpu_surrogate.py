@@ -73,3 +73,40 @@ def test_training_steps_do_not_depend_on_what_is_recorded():
         assert np.array_equal(a.get_params(), b.get_params()), (k, n)
     a.close()
     b.close()
+
+
+def test_many_batch_sizes_in_turn_do_not_record_at_every_step():
+    """Twelve sizes in turn: once as many as are kept have been recorded, the others run
+    without, and all give the steps of a network that sees them for the first time."""
+    import torch
+    from torch.profiler import profile, ProfilerActivity
+    from covidsim_b200 import surrogate
+    flat, x, target = _case(200, 27)
+    net = surrogate.Surrogate(max_batch=256, params=flat)
+    sizes = [200 - 16 * k for k in range(12)]
+
+    def cycle():
+        return [net.train_step(x[:n], target[:n], 1e-3) for n in sizes]
+    cycle()
+    with profile(activities=[ProfilerActivity.CPU, ProfilerActivity.CUDA]) as p:
+        cycle()
+        cycle()
+    names = [e.name for e in p.events()]
+    if not names:
+        pytest.skip("the profiler records nothing here")
+    assert sum("GraphLaunch" in n for n in names) > 0
+    assert sum("GraphInstantiate" in n for n in names) == 0
+    fresh = surrogate.Surrogate(max_batch=256, params=net.get_params())
+    for n in sizes:
+        a, b = net.loss_grad(x[:n], target[:n]), fresh.loss_grad(x[:n], target[:n])
+        assert a[0] == b[0] and np.array_equal(a[1], b[1]), n
+    # sizes that are met from now on take the places of those that are not
+    for n in sizes[:2] * 200:
+        net.train_step(x[:n + 1], target[:n + 1], 1e-3)
+    with profile(activities=[ProfilerActivity.CPU, ProfilerActivity.CUDA]) as p:
+        for n in sizes[:2]:
+            net.train_step(x[:n + 1], target[:n + 1], 1e-3)
+    assert sum("GraphLaunch" in e.name for e in p.events()) == 2
+    net.close()
+    fresh.close()
+    torch.cuda.synchronize()
