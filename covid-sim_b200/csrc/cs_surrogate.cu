@@ -726,11 +726,12 @@ struct cs_sur {
     // activations and scratch sized for bmax
     std::vector<bf16*> act;                 // act[0] = input, act[l+1] = output of layer l (BF16)
     float* yout = nullptr;                  // last layer output FP32 [bmax*368, 64]
-    bf16* cols[3] = {nullptr, nullptr, nullptr};   // column matrices of the mma.sync path
     std::vector<float*> dz;                 // gradient at layer l's output before its ReLU (FP32, BF16); one per
     std::vector<bf16*> dzb;                 // layer, as a layer's weight gradient runs beside the layers below it
     std::vector<bf16*> wT;                  // transposed BF16 weights per layer
     float* dcols = nullptr;
+    bf16* cols = nullptr;                   // column matrix of the mma.sync path: one convolution's at a time, in the
+                                            // forward pass, which dcols (of the backward pass) leaves to it
     Lane lane[kLanes];                      // [0] the main chain, the others beside it
     cudaEvent_t fork = nullptr;
     std::vector<cudaEvent_t> dz_ready;      // per layer: its dz is written
@@ -928,7 +929,7 @@ int cs_sur_create(int max_batch, int device, cs_sur** out)
     SA(s->w, s->np); SA(s->m, s->np); SA(s->v, s->np); SA(s->g, s->np); SA(s->wb, s->np);
     const int B = s->bmax;
     s->act.assign(s->L.size() + 1, nullptr);
-    size_t maxc = 0, maxcol = 0, maxw = 0;
+    size_t maxc = 0, maxcol = 0;
     for (size_t li = 0; li <= s->L.size(); li++) {
         size_t n = act_elems(s, (int)li, B);
         SA(s->act[li], n);
@@ -936,13 +937,11 @@ int cs_sur_create(int max_batch, int device, cs_sur** out)
     }
     for (int i = 0; i < 3; i++) {
         const Layer& l = s->L[6 + i];
-        size_t n = (size_t)B * l.T * l.inP;
-        SA(s->cols[i], n);
-        maxcol = std::max(maxcol, n);
+        maxcol = std::max(maxcol, (size_t)B * l.T * l.inP);
     }
-    for (auto& l : s->L) maxw = std::max(maxw, (size_t)l.outP * l.inP);
     SA(s->yout, (size_t)B * 8 * kT0 * kCh);
     SA(s->dcols, maxcol);
+    s->cols = reinterpret_cast<bf16*>(s->dcols);
     const size_t maxz = std::max(maxc, (size_t)B * 8 * kT0 * kCh);
     s->dz.assign(s->L.size(), nullptr);
     s->dzb.assign(s->L.size(), nullptr);
@@ -1077,9 +1076,9 @@ static int forward(cs_sur* s, const Lane& w, bf16* const* act, int Bp, float* y6
             else args([](auto... a) { tc_launch<16>(a...); });
             SCK(cudaGetLastError());
         } else {
-            sur::k_im2col_up<<<1184, 256, 0, w.st>>>(act[6 + ci], Bp, T, l.cin, s->cols[ci], l.inP);
+            sur::k_im2col_up<<<1184, 256, 0, w.st>>>(act[6 + ci], Bp, T, l.cin, s->cols, l.inP);
             SCK(cudaGetLastError());
-            if ((r = gemm(s, w, s->cols[ci], l.inP, s->wb + l.wofs, l.inP, C, kCh, Cb, kCh, s->w + l.bofs, l.relu ? 1 : 0,
+            if ((r = gemm(s, w, s->cols, l.inP, s->wb + l.wofs, l.inP, C, kCh, Cb, kCh, s->w + l.bofs, l.relu ? 1 : 0,
                           M, l.outP, l.inP))) return r;
             if (last && y) {
                 sur::k_store_y<<<512, 256, 0, w.st>>>(y64, n, y);

@@ -110,3 +110,18 @@ def test_many_batch_sizes_in_turn_do_not_record_at_every_step():
     net.close()
     fresh.close()
     torch.cuda.synchronize()
+
+
+def test_memory_of_a_network_by_its_batch():
+    """Activations, their gradients, scratch and batch of one row: 1.30 MB at most, so that the
+    largest batch that fits the device does not shrink."""
+    import torch
+    from covidsim_b200 import surrogate
+    torch.cuda.synchronize()
+    used = {}
+    for rows in (1024, 4096):
+        free = torch.cuda.mem_get_info()[0]
+        net = surrogate.Surrogate(max_batch=rows)
+        used[rows] = free - torch.cuda.mem_get_info()[0]
+        net.close()
+    assert (used[4096] - used[1024]) / 3072 < 1.30e6
