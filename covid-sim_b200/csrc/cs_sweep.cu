@@ -4136,7 +4136,8 @@ int cs_gpu_grid(const cs_gpu_ctx* c) { return c ? c->grid : 0; }
 int cs_gpu_set_spatial_lanes(cs_gpu_ctx* c, int lanes)
 {
     if (!c) return CS_E_ARG;
-    if (lanes != 2 && lanes != 4 && lanes != 8 && lanes != 16) return set_err(c, CS_E_ARG, "spatial lanes must be 2, 4, 8 or 16");
+    if (lanes != 0 && lanes != 2 && lanes != 4 && lanes != 8 && lanes != 16)
+        return set_err(c, CS_E_ARG, "spatial lanes must be 2, 4, 8 or 16 (0: by the load)");
     CK(cudaStreamSynchronize(c->stream));
     c->spatial_lanes = lanes;
     drop_day_graph(c);
@@ -4674,7 +4675,8 @@ int cs_gpu_batch_set_grid(cs_gpu_batch* b, int blocks)
 int cs_gpu_batch_set_spatial_lanes(cs_gpu_batch* b, int lanes)
 {
     if (!b) return CS_E_ARG;
-    if (lanes != 2 && lanes != 4 && lanes != 8 && lanes != 16) return batch_err(b, CS_E_ARG, "spatial lanes must be 2, 4, 8 or 16");
+    if (lanes != 0 && lanes != 2 && lanes != 4 && lanes != 8 && lanes != 16)
+        return batch_err(b, CS_E_ARG, "spatial lanes must be 2, 4, 8 or 16 (0: by the load)");
     BCK(cudaStreamSynchronize(b->stream));
     b->lanes = lanes;
     batch_drop_graph(b);

@@ -141,3 +141,26 @@ def test_households_left_by_an_infect_sweep_alone(device_loop):
     _same(snapshot(whole.backend, pop), want, "whole timesteps")
     for s in sims:
         s.close()
+
+
+def test_the_choice_of_lanes_by_the_load_can_be_had_back():
+    pop, P, lk, hr = _world(2001, 4, 0.3, None)
+    a = sim.Simulation(pop, P, lk, hr)
+    b = a.replica()
+    batch = sim.Batch([b])
+    for be in (a.backend, batch):
+        be.set_spatial_lanes(4)
+        be.set_spatial_lanes(0)
+        for lanes in (-1, 1, 3, 32):
+            with pytest.raises(abi.CovidSimError):
+                be.set_spatial_lanes(lanes)
+    seeds = a.choose_seeds(9, 100)
+    for s in (a, b):
+        s.backend.begin_run(9, seeds)
+    for k in range(8):
+        a.backend.step(k * P.ModelTimeStep, 0)
+        batch.step(k * P.ModelTimeStep, 0)
+    _same(snapshot(a.backend, pop), snapshot(b.backend, pop), "alone and in a batch")
+    batch.close()
+    a.close()
+    b.close()
