@@ -1,11 +1,13 @@
 """UpdateProbs over the shapes of grid that choose its launch: the fixed-scratch form
 against the allocating one where it takes more row pairs a block (and so more shared memory)
-than that does, and contexts of different grids in one process, in turn.  All sums
-have one order, so every value must be equal (tolerance: none)."""
+than that does; contexts of different grids in one process, in turn; and several row pairs
+a block against the oracle.  All sums have one order, so every value must be equal
+(tolerance: none)."""
 import numpy as np
 import pytest
 
-from covidsim_b200 import population, params as prm, sim
+from covidsim_b200 import abi, population, params as prm, sim
+import oracle_py
 from tests.helpers import snapshot, STATE_FIELDS
 
 pytestmark = pytest.mark.gpu
@@ -71,4 +73,31 @@ def test_contexts_of_other_grids_take_turns(large, small):
     for k in want:
         assert np.array_equal(want[k], again[k]) and np.array_equal(want[k], other[k]), k
     for s in (a, b, r):
+        s.close()
+
+
+@pytest.mark.parametrize("ncw,nch,n_people", [(120, 121, 500), (97, 201, 500), (241, 243, 700), (340, 259, 700)])
+def test_several_row_pairs_a_block_match_the_oracle(ncw, nch, n_people):
+    """Two, five, seven and eight row pairs a block, rows that are no multiple of theirs (the
+    last block's pairs past the grid, the odd row among others), threads past the pairs, and
+    with the last two more than 48 KB of shared memory."""
+    world = _world(ncw, nch, n_people)
+    pop, P = world[:2]
+    sims = [sim.Simulation(*world), sim.Simulation(*world, backend=oracle_py.OracleBackend)]
+    seeds = sims[0].choose_seeds(3, n_people // 4)
+    for s in sims:
+        s.backend.begin_run(3, seeds)
+        for k in range(24):
+            s.backend.infect_sweep(k * P.ModelTimeStep, 0)
+            s.backend.incub_recovery_sweep(k * P.ModelTimeStep)
+        s.backend.update_probs(0)
+    a, b = (snapshot(s.backend, pop) for s in sims)
+    assert not np.all(b["cell_tot_prob"] == 1.0)
+    _same(a, b, "%d x %d" % (ncw, nch))
+    # the tables' counts are those of the oracle too: the sweep after them draws from both alike
+    for s in sims:
+        s.backend.infect_sweep(24 * P.ModelTimeStep, 0)
+    ca, cb = (abi.counters_to_dict(s.backend.counters()) for s in sims)
+    assert ca == cb
+    for s in sims:
         s.close()

@@ -164,3 +164,20 @@ def test_the_choice_of_lanes_by_the_load_can_be_had_back():
     batch.close()
     a.close()
     b.close()
+
+
+def test_counters_match_the_oracle_before_any_mid_run_seeding():
+    """Every counter, the radii of infection (summed by warps beside the transitions) too."""
+    for n_people, cells, latent, n_seed in ((6000, 4, 0.02, 300), (20000, 30, 0.3, 1000)):
+        pop, P, lk, hr = _world(n_people, cells, latent, None)
+        sims = [sim.Simulation(pop, P, lk, hr), sim.Simulation(pop, P, lk, hr, backend=oracle_py.OracleBackend)]
+        seeds = sims[0].choose_seeds(5, n_seed)
+        for s in sims:
+            s.backend.begin_run(5, seeds)
+            for k in range(29):
+                s.backend.step(k * P.ModelTimeStep, 0)
+        a, b = (abi.counters_to_dict(s.backend.counters()) for s in sims)
+        assert b["sumRad2_q"] > 0 and b["maxRad2_bits"] > 0
+        assert a == b
+        for s in sims:
+            s.close()
