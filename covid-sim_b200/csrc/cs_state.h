@@ -72,14 +72,11 @@ struct __align__(16) PlaceRec {
 
 struct DevPlaces {
     int32_t n;
-    const PlaceRec* rec;       // the next four arrays' entries of a place, together
-    const int2* group;         // (group_start, group_size)
+    const PlaceRec* rec;
+    const int2* group;         // (first member within the place, size) of each group
     const int32_t* mcell;
     const int32_t* member_ofs;
     const int32_t* members;
-    const int32_t* group_ofs;
-    const int32_t* group_start;
-    const int32_t* group_size;
     const float* x;            // location (blanket movement restrictions measure to it)
     const float* y;
     uint16_t* close_start;
@@ -118,7 +115,6 @@ struct DevPop {
     const HouseholdRec* hhr;   // [NH]
     const int32_t* pcell;      // [N] the person's cell
     const float2* pxy;         // [N] the person's household's location, for the spatial draws (no detour by the record)
-    const int32_t* mcell_cell;
     const int32_t* mcell_adunit;
     const int32_t* cell_grid;
     const int32_t* cell_start;

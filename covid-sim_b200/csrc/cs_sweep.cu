@@ -114,39 +114,6 @@ __device__ __forceinline__ int32_t append(int32_t* count)
     return base + (int32_t)g.thread_rank();
 }
 
-// Reserves na entries of list A and nb entries of list B for every thread of the
-// block, with one atomic per list per block.  Every thread of the block must call
-// it at the same point (block-uniform control flow); blockDim.x is a multiple of 32.
-__device__ __forceinline__ int2 block_reserve2(int32_t* count_a, int32_t na, int32_t* count_b, int32_t nb)
-{
-    __shared__ int2 warp_base[32];
-    __shared__ int2 block_base;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
-    int32_t ia = na, ib = nb;
-    for (int o = 1; o < 32; o <<= 1) {
-        int32_t ya = __shfl_up_sync(0xffffffffu, ia, o), yb = __shfl_up_sync(0xffffffffu, ib, o);
-        if (lane >= o) { ia += ya; ib += yb; }
-    }
-    if (lane == 31) warp_base[warp] = make_int2(ia, ib);
-    __syncthreads();
-    if (warp == 0) {
-        int2 v = lane < nwarps ? warp_base[lane] : make_int2(0, 0);
-        int32_t xa = v.x, xb = v.y;
-        for (int o = 1; o < 32; o <<= 1) {
-            int32_t ya = __shfl_up_sync(0xffffffffu, xa, o), yb = __shfl_up_sync(0xffffffffu, xb, o);
-            if (lane >= o) { xa += ya; xb += yb; }
-        }
-        int32_t ta = __shfl_sync(0xffffffffu, xa, 31), tb = __shfl_sync(0xffffffffu, xb, 31);
-        if (lane == 0)
-            block_base = make_int2(ta && count_a ? atomicAdd(count_a, ta) : 0, tb && count_b ? atomicAdd(count_b, tb) : 0);
-        if (lane < nwarps) warp_base[lane] = make_int2(xa - v.x, xb - v.y);
-    }
-    __syncthreads();
-    int2 r = make_int2(block_base.x + warp_base[warp].x + ia - na, block_base.y + warp_base[warp].y + ib - nb);
-    __syncthreads();   // the shared slots are reused by the next call
-    return r;
-}
-
 // Cell flags of a step: its lists change; someone infected this step also turned
 // infectious; someone who turned infectious this step also left the infectious block.
 enum : unsigned { kCellTouched = 1, kCellRelayS = 2, kCellRelayL = 4 };
@@ -3398,7 +3365,7 @@ int cs_gpu_create(const cs_population* pop, const cs_params* params, int device,
     d.NA = pop->n_adunits > 0 ? pop->n_adunits : 1;
     size_t N = d.N, NH = d.NH, NC = d.NC, NM = d.NM, NPT = d.NPT;
     if (d.NPT < 0 || d.NPT > CS_MAX_PLACE_TYPES) return set_err(c, CS_E_ARG, "num_place_types out of range");
-    if (N >= (1u << 28)) return set_err(c, CS_E_UNSUPPORTED, "at most 2^28 - 1 people (place work entries pack index << 3)");
+    if (N >= (1u << 28)) return set_err(c, CS_E_UNSUPPORTED, "at most 2^28 - 1 people (no larger population has been run)");
     if (N == 0 || NC == 0) return set_err(c, CS_E_ARG, "empty population");
 #define UP(field, src, n) do { if ((r = dupload(c, &field, src, n))) return r; } while (0)
 #define AL(field, n) do { if ((r = dalloc(c, &field, n))) return r; } while (0)
@@ -3469,7 +3436,6 @@ int cs_gpu_create(const cs_population* pop, const cs_params* params, int device,
         d.hhr = t;
         CK(cudaStreamSynchronize(c->stream));
     }
-    { int32_t* t; UP(t, pop->mcell_cell, NM); d.mcell_cell = t; }
     { int32_t* t; UP(t, pop->mcell_adunit, NM); d.mcell_adunit = t; }
     { int32_t* t; UP(t, pop->cell_grid, NC); d.cell_grid = t; }
     { int32_t* t; UP(t, pop->cell_start, NC + 1); d.cell_start = t; }
@@ -3495,9 +3461,6 @@ int cs_gpu_create(const cs_population* pop, const cs_params* params, int device,
         { int32_t* t; UP(t, pop->place_mcell[pt], np); pl.mcell = t; }
         { int32_t* t; UP(t, pop->place_member_ofs[pt], np + 1); pl.member_ofs = t; }
         { int32_t* t; UP(t, pop->place_members[pt], nm); pl.members = t; }
-        { int32_t* t; UP(t, pop->place_group_ofs[pt], np + 1); pl.group_ofs = t; }
-        { int32_t* t; UP(t, pop->group_start[pt], ng); pl.group_start = t; }
-        { int32_t* t; UP(t, pop->group_size[pt], ng); pl.group_size = t; }
         {
             std::vector<PlaceRec> rec(np);
             std::vector<int2> grp(ng);
