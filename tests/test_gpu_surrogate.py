@@ -125,3 +125,19 @@ def test_memory_of_a_network_by_its_batch():
         used[rows] = free - torch.cuda.mem_get_info()[0]
         net.close()
     assert (used[4096] - used[1024]) / 3072 < 1.30e6
+
+
+def test_a_network_takes_few_allocations():
+    """No more than the 36 arrays it had when its passes ran in one chain: each allocation is
+    host time of every creation."""
+    from torch.profiler import profile, ProfilerActivity
+    from covidsim_b200 import surrogate
+    flat = ref.init_params(3).astype(np.float32)
+    surrogate.Surrogate(max_batch=64, params=flat).close()
+    with profile(activities=[ProfilerActivity.CPU, ProfilerActivity.CUDA]) as p:
+        net = surrogate.Surrogate(max_batch=64, params=flat)
+    names = [e.name for e in p.events()]
+    net.close()
+    if not names:
+        pytest.skip("the profiler records nothing here")
+    assert 0 < sum(n == "cudaMalloc" for n in names) <= 36
