@@ -423,9 +423,22 @@ static_assert(kParamsHead >= offsetof(cs_params, infectiousness) + kProfileStage
 static_assert(kParamsMid <= offsetof(cs_params, PlaceTypeTrans) && kParamsMid % 16 == 0, "staged range");
 static_assert(kParamsEnd >= offsetof(cs_params, sinx) && kParamsEnd % 16 == 0, "staged range");
 
+// Entry k of the table of doubles at byte `table` of the parameter block, read in place: what
+// the block holds there when k lies outside the table but not outside the block (a sweep at a
+// time before its infectors' latent periods ended, a household larger than the table), else 0.
+static __device__ __noinline__ double param_at(const cs_params* Pg, size_t table, int k)
+{
+    const long long at = (long long)table + 8ll * k;
+    return at >= 0 && at + 8 <= (long long)sizeof(cs_params) ? *reinterpret_cast<const double*>(reinterpret_cast<const char*>(Pg) + at) : 0.0;
+}
 __device__ __forceinline__ double profile_at(const cs_params& P, const cs_params* Pg, int k)
 {
-    return k < kProfileStaged ? P.infectiousness[k] : Pg->infectiousness[k];
+    return (unsigned)k < (unsigned)kProfileStaged ? P.infectiousness[k] : param_at(Pg, offsetof(cs_params, infectiousness), k);
+}
+__device__ __forceinline__ double house_denom_at(const cs_params& P, const cs_params* Pg, int nhr)
+{
+    return (unsigned)(nhr - 1) < (unsigned)CS_MAX_HOUSEHOLD_SIZE ? P.HouseholdDenomLookup[nhr - 1]
+                                                                 : param_at(Pg, offsetof(cs_params, HouseholdDenomLookup), nhr - 1);
 }
 
 // --------------------------------------- CalcInfSusc (src/CalcInfSusc.cpp)
@@ -441,7 +454,7 @@ __device__ __forceinline__ double calc_house_inf(const DevPop& d, const PersonHo
     double infn = P.NoInfectiousnessSDinHH ? ((h.infness < 0) ? P.SymptInfectiousness : P.AsymptInfectiousness) : fabs(h.infness);
     return (iso ? P.Efficacies[CS_NPI_CASE_ISOLATION][CS_SETTING_HOUSE] : 1.0)
         * ((host_quarantined(h, P, ts) && !iso) ? P.Efficacies[CS_NPI_HOME_QUARANTINE][CS_SETTING_HOUSE] : 1.0)
-        * P.HouseholdDenomLookup[nhr - 1]
+        * house_denom_at(P, d.P, nhr)
         * (is_ch(h) ? P.CareHomeResidentHouseholdScaling : 1.0)
         * infn
         * profile_at(P, d.P, ts - h.latent_time - 1);

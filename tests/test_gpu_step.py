@@ -181,3 +181,32 @@ def test_counters_match_the_oracle_before_any_mid_run_seeding():
         assert a == b
         for s in sims:
             s.close()
+
+
+def test_parameters_beyond_their_tables():
+    """Households whose size for the kernel lies past its table read what the parameter block
+    holds there, as the oracle does; a sweep at a time long before its infectors turned
+    infectious reads nothing outside the block."""
+    pop, P, lk, hr = _world(2001, 4, None, None)
+    pop.hh_nhr = np.full_like(pop.hh_nhr, 300)          # entry 299: entry 289 of the profile behind it
+    q = abi.cs_params.from_buffer_copy(P)
+    q.infectiousness[289] = 0.7
+    q.LocalBeta = 0.5
+    sims = [sim.Simulation(pop, q, lk, hr), sim.Simulation(pop, q, lk, hr, backend=oracle_py.OracleBackend)]
+    seeds = sims[0].choose_seeds(5, 60)
+    for s in sims:
+        s.backend.begin_run(5, seeds)
+        for k in range(32):
+            s.backend.step(k * q.ModelTimeStep, 0)
+    a, b = (snapshot(s.backend, pop) for s in sims)
+    _same(a, b, "large households")
+    assert np.sum(b["infect_type"] % abi.CONST["CS_INFECT_TYPE_MASK"] == 1) > 20     # infections in households
+    g = sims[0].backend
+    for k in range(32, 240):
+        g.step(k * q.ModelTimeStep, 0)
+    g.infect_sweep(0.0, 0)
+    g.incub_recovery_sweep(0.0)
+    g.sync()
+    check_lists(snapshot(g, pop), pop)
+    for s in sims:
+        s.close()
