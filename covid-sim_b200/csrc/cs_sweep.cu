@@ -3718,8 +3718,11 @@ static int enable_shared_memory(cs_gpu_ctx* c)
 static int tot_prob_numerators(cs_gpu_ctx* c, const float* S0g, const uint8_t* rowS, float* out, bool partial)
 {
     const cs_params& P = c->hp;
-    if (c->prof) prof_begin(c, partial ? "k_tot_prob_rows" : "k_tot_prob_rows_static");
-    if (tot_prob_packed(P, partial)) {
+    const bool packed = tot_prob_packed(P, partial);
+    if (c->prof)
+        prof_begin(c, packed ? (partial ? "k_tot_prob_pairs" : "k_tot_prob_pairs_static")
+                             : (partial ? "k_tot_prob_rows" : "k_tot_prob_rows_static"));
+    if (packed) {
         const TotPairGeom gm = tot_pair_geom(P.ncw, P.nch, partial);
         const dim3 grid(gm.xblocks, (P.nch + 2 * gm.npair - 1) / (2 * gm.npair), gm.nchunks / gm.chunks_per_block);
         k_tot_prob_pairs<<<grid, gm.threads, gm.smem(), c->stream>>>(c->d, S0g, rowS, out, gm, c->Gtab);

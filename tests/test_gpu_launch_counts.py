@@ -107,3 +107,19 @@ def test_timed_kernels_have_their_bytes_in_the_benchmark():
     for k in ("k_scan", "k_household", "k_places", "k_spatial", "k_infections", "k_onsets", "k_progress", "k_moves"):
         assert k in names and bench.kernel_bytes(k, w, pop.n_cells * 80) > 0, k
     s.close()
+
+
+def test_timed_names_are_the_kernels_that_run():
+    pop, P, lk, hr = tiny_world(adunit_grid=2)
+    s = sim.Simulation(pop, P, lk, hr)
+    s.backend.profile(1)
+
+    def work():
+        s.run(505, 40, n_seed=20, policy=sim.InterventionPolicy(threshold=3, window=7, duration=12.0))
+        s.backend.update_probs(0)
+        s.backend.infect_sweep(40.0)
+        s.backend.incub_recovery_sweep(40.0)
+    ran = {re.search(r"k_\w+", n).group() for n in _kernels(work)}
+    timed = {n.split("<")[0] for n in s.backend.profile_entries()}
+    assert timed and timed <= ran, timed - ran
+    s.close()
