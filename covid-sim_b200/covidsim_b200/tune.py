@@ -19,7 +19,8 @@ LANES = (2, 4, 8, 16)
 
 def autotune(simulation, n_sm=148, grids_per_sm=GRIDS_PER_SM, lanes=LANES, steps=24, seed_frac=0.02, seed=4040):
     """Time `steps` timesteps of a realisation seeded with `seed_frac` of the
-    population under each (grid, lanes) setting; apply and return the fastest as
+    population under each (grid, lanes) setting (0 among `lanes`: by the load, the
+    library's default); apply and return the fastest as
     {"grid": blocks, "spatial_lanes": lanes, "ms": {setting: ms}}."""
     import torch
     be = simulation.backend

@@ -3887,11 +3887,14 @@ int cs_gpu_begin_run(cs_gpu_ctx* c, uint64_t seed, const int32_t* seed_people, i
     return cs_gpu_seed_infections(c, 0.0, seed_people, n_seed);
 }
 
-// Blocks of a step kernel that deals its list out itself (Groups): the context's grid, but no
-// more than the SMs hold at once.  Blocks past the first wave find the list dealt out or, at
-// high load, repeat the staging of the parameters for little of it; every wave of blocks
-// costs a launch about 1.5 us.
-constexpr int kWave3 = 3, kWave4 = 4, kWave6 = 6;   // resident blocks per SM of the kernels below
+// Blocks of a step kernel that deals its list out itself (Groups): the context's grid, but
+// about as many as the SMs hold at once.  Blocks past the first wave find the list dealt out
+// or, at high load, repeat the staging of the parameters for little of it; every wave of
+// blocks costs a launch about 1.5 us.  Blocks per SM: 3 of k_places, k_spatial and the
+// changes (80 registers a thread hold no more), 4 of k_households, 6 of k_household (46
+// registers: 5 of them resident).  k_scan and k_moves go by cells and take the context's grid
+// (8 an SM; 4 and 5 are resident); in a batch (batch_enqueue) their members share 6 an SM.
+constexpr int kWave3 = 3, kWave4 = 4, kWave6 = 6;
 static int wave_grid(const cs_gpu_ctx* c, int per_sm) { return std::min(c->grid, c->nsm * per_sm); }
 
 // Every tile of kThreads cells shared by enough blocks to fill the grid.
@@ -4518,8 +4521,8 @@ static int batch_enqueue(cs_gpu_batch* b, const DevPop* pops)
     const int grid = b->members[0]->grid;
     int maxc = 0;
     for (const cs_gpu_ctx* m : b->members) maxc = std::max(maxc, m->d.NC);
-    // one wave of blocks per kernel over all members, and half as much again for members
-    // with more than their share
+    // the blocks of wave_grid over all members, and half as much again for members with more
+    // than their share
     const int nsm = b->members[0]->nsm;
     auto wave = [&](int per_sm) { return dim3(std::min(grid, std::max(8, (3 * nsm * per_sm / 2 + R - 1) / R)), R); };
     const dim3 gs(scan_grid(maxc, wave(kWave4).x), R);
